@@ -3,6 +3,7 @@
 #include "redcuda_dot.cuh"
 #include "redcuda_kernels.cuh"
 #include "redcuda_moe_mma.cuh"
+#include "redcuda_stage.cuh"
 #include "../../include/redcuda.h"
 
 #include <math.h>
@@ -86,7 +87,12 @@ int require_device() {
 int DevMem::alloc(size_t n) {
     release();
     if (!n) n = 16;
-    RC_CUDA(cudaMalloc(&p, n));
+    if (cudaMalloc(&p, n) != cudaSuccess) {      // the buffers that idle host-call leases keep may be what is missing
+        cudaGetLastError();
+        p = nullptr;
+        stage_trim();
+        RC_CUDA(cudaMalloc(&p, n));
+    }
     bytes = n;
     return 1;
 }
@@ -667,22 +673,22 @@ int redcuda_quant_dequant_rows(uint32_t type, const uint8_t *rows, uint32_t nrow
     RC_REQUIRE(bytes, "dequant: %u columns is not a valid row length for type %u", ncols, type);
     const size_t n = (size_t)nrows * ncols;
     if (type == RC_F32) { memcpy(out, rows, n * 4u); return 1; }   // a copy, as in the reference (quant_cpu.c:159)
-    DevMem raw, planar, o;
-    if (!raw.alloc(bytes) || !planar.alloc(bytes) || !o.alloc(n * 4u)) return 0;
-    cudaStream_t s = 0;
+    Stage st;
+    if (!st.open(2u * Stage::pad(bytes) + Stage::pad(n * 4u))) return 0;
+    uint8_t *raw = st.take(bytes), *planar = st.take(bytes);
+    float *o = st.take<float>(n * 4u);
+    cudaStream_t s = st.stream();
+    if (!st.upload(raw, rows, bytes)) return 0;
     if (type == RC_F16) {
-        RC_CUDA(cudaMemcpyAsync(raw.p, rows, bytes, cudaMemcpyHostToDevice, s));
-        RC_LAUNCH((k_dequant_f16), (unsigned)((n + 255u) / 256u < 4096u ? (n + 255u) / 256u : 4096u), 256, 0, s, raw.as<unsigned short>(), n, o.as<float>());
+        RC_LAUNCH((k_dequant_f16), (unsigned)((n + 255u) / 256u < 4096u ? (n + 255u) / 256u : 4096u), 256, 0, s, (const unsigned short *)raw, n, o);
         RC_LAUNCHED();
     } else {
-        if (!upload_matrix(type, nrows, ncols, rows, false, planar.as<uint8_t>(), raw.as<uint8_t>(), s)) return 0;
+        if (!upload_matrix(type, nrows, ncols, raw, true, planar, nullptr, s)) return 0;
         const uint64_t nb = (uint64_t)nrows * (ncols / 256u), groups = nb * 32u;
-        RC_LAUNCH((k_dequant), (unsigned)((groups + 255u) / 256u < 4096u ? (groups + 255u) / 256u : 4096u), 256, 0, s, planar.as<uint8_t>(), type, nb, books_iq2(), books_iq3s(), o.as<float>());
+        RC_LAUNCH((k_dequant), (unsigned)((groups + 255u) / 256u < 4096u ? (groups + 255u) / 256u : 4096u), 256, 0, s, planar, type, nb, books_iq2(), books_iq3s(), o);
         RC_LAUNCHED();
     }
-    RC_CUDA(cudaMemcpyAsync(out, o.p, n * 4u, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaStreamSynchronize(s));
-    return 1;
+    return st.download(out, o, n * 4u) && st.finish();
 }
 
 int redcuda_quant_matvec(uint32_t type, const uint8_t *w, uint32_t nrows, uint32_t ncols, const float *x, uint32_t ntok, float *out) {
@@ -693,19 +699,18 @@ int redcuda_quant_matvec(uint32_t type, const uint8_t *w, uint32_t nrows, uint32
     RC_REQUIRE(rc_type_supported(type), "matvec: unsupported ggml type %u", type);
     const uint64_t bytes = rc_matrix_bytes(type, nrows, ncols);
     RC_REQUIRE(bytes, "matvec: %u columns is not a valid row length for type %u", ncols, type);
-    DevMem raw, planar, xd, od;
-    if (!raw.alloc(bytes) || !planar.alloc(bytes) || !xd.alloc((size_t)ntok * ncols * 4u) || !od.alloc((size_t)ntok * nrows * 4u)) return 0;
-    cudaStream_t s = 0;
-    if (!upload_matrix(type, nrows, ncols, w, false, planar.as<uint8_t>(), raw.as<uint8_t>(), s)) return 0;
-    RC_CUDA(cudaMemcpyAsync(xd.p, x, (size_t)ntok * ncols * 4u, cudaMemcpyHostToDevice, s));
+    const size_t xb = (size_t)ntok * ncols * 4u, ob = (size_t)ntok * nrows * 4u;
+    Stage st;
+    if (!st.open(2u * Stage::pad(bytes) + Stage::pad(xb) + Stage::pad(ob))) return 0;
+    uint8_t *raw = st.take(bytes), *planar = st.take(bytes);
+    float *xd = st.take<float>(xb), *od = st.take<float>(ob);
+    cudaStream_t s = st.stream();
+    if (!st.upload(xd, x, xb) || !st.upload(raw, w, bytes) || !upload_matrix(type, nrows, ncols, raw, true, planar, nullptr, s)) return 0;
     GemvArgs A{};
-    A.njobs = 1; A.ntok = ntok; A.x = xd.as<float>(); A.x_stride = ncols;
-    A.job[0].w0 = planar.as<uint8_t>(); A.job[0].w1 = nullptr; A.job[0].out = od.as<float>(); A.job[0].nb = (uint64_t)nrows * (ncols / 256u);
+    A.njobs = 1; A.ntok = ntok; A.x = xd; A.x_stride = ncols;
+    A.job[0].w0 = planar; A.job[0].w1 = nullptr; A.job[0].out = od; A.job[0].nb = (uint64_t)nrows * (ncols / 256u);
     A.job[0].type = type; A.job[0].nrows = nrows; A.job[0].ncols = ncols; A.job[0].out_stride = nrows; A.job[0].epi = GEMV_STORE;
-    if (!launch_gemv(A, s)) return 0;
-    RC_CUDA(cudaMemcpyAsync(out, od.p, (size_t)ntok * nrows * 4u, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaStreamSynchronize(s));
-    return 1;
+    return launch_gemv(A, s) && st.download(out, od, ob) && st.finish();
 }
 
 int redcuda_router_select_softmax_topk(const float *logits, uint32_t ntok, uint32_t n_expert, uint32_t top_k,
@@ -713,16 +718,13 @@ int redcuda_router_select_softmax_topk(const float *logits, uint32_t ntok, uint3
     if (!require_device()) return 0;
     RC_REQUIRE(logits && ids && weights && n_expert && top_k && top_k <= n_expert, "invalid router top-k selection arguments");
     if (!ntok) return 1;
-    DevMem l, i, w, p;
-    if (!l.alloc((size_t)ntok * n_expert * 4u) || !i.alloc((size_t)ntok * top_k * 4u) || !w.alloc((size_t)ntok * top_k * 4u)) return 0;
-    if (probs && !p.alloc((size_t)ntok * n_expert * 4u)) return 0;
-    cudaStream_t s = 0;
-    RC_CUDA(cudaMemcpyAsync(l.p, logits, (size_t)ntok * n_expert * 4u, cudaMemcpyHostToDevice, s));
-    if (!launch_route(l.as<float>(), ntok, n_expert, top_k, i.as<uint32_t>(), w.as<float>(), probs ? p.as<float>() : nullptr, s)) return 0;
-    RC_CUDA(cudaMemcpyAsync(ids, i.p, (size_t)ntok * top_k * 4u, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaMemcpyAsync(weights, w.p, (size_t)ntok * top_k * 4u, cudaMemcpyDeviceToHost, s));
-    if (probs) RC_CUDA(cudaMemcpyAsync(probs, p.p, (size_t)ntok * n_expert * 4u, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaStreamSynchronize(s));
+    const size_t lb = (size_t)ntok * n_expert * 4u, kb = (size_t)ntok * top_k * 4u;
+    Stage st;
+    if (!st.open(Stage::pad(lb) + 2u * Stage::pad(kb) + (probs ? Stage::pad(lb) : 0u))) return 0;
+    float *l = st.take<float>(lb), *w = st.take<float>(kb), *p = probs ? st.take<float>(lb) : nullptr;
+    uint32_t *i = st.take<uint32_t>(kb);
+    if (!st.upload(l, logits, lb) || !launch_route(l, ntok, n_expert, top_k, i, w, p, st.stream())) return 0;
+    if (!st.download(ids, i, kb) || !st.download(weights, w, kb) || (probs && !st.download(probs, p, lb)) || !st.finish()) return 0;
     return status_failed() ? 0 : 1;
 }
 

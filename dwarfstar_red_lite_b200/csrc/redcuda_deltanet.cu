@@ -9,6 +9,7 @@
 //   k_dn_tail   per value head RMSNorm(core) * w * SiLU(z)
 #include "redcuda_common.cuh"
 #include "redcuda_kernels.cuh"
+#include "redcuda_stage.cuh"
 #include "../../include/redcuda.h"
 
 #include <stdlib.h>
@@ -841,27 +842,17 @@ extern "C" int redcuda_deltanet_step(const redcuda_deltanet_params *p, uint32_t 
     const size_t b_ck = (size_t)D.channels * D.d_conv * 4u, b_r = (size_t)D.rank * 4u, b_nw = (size_t)D.S * 4u;
     const size_t b_qkv = (size_t)batch * D.channels * 4u, b_z = (size_t)batch * D.d_inner * 4u, b_ba = (size_t)batch * 2u * D.rank * 4u;
     const size_t b_cs = (size_t)batch * D.channels * ns * 4u, b_rs = (size_t)batch * D.rank * D.S * D.S * 4u;
-    DevMem ck, dt, sa, nw, dq, dz, dba, cs, rs, qk, v, beta, gate, core, o;
-    if (!ck.alloc(b_ck) || !dt.alloc(b_r) || !sa.alloc(b_r) || !nw.alloc(b_nw) || !dq.alloc(b_qkv) || !dz.alloc(b_z) || !dba.alloc(b_ba) ||
-        !cs.alloc(b_cs) || !rs.alloc(b_rs) || !qk.alloc(batch * nqk * 4u) || !v.alloc(b_z) || !beta.alloc(batch * b_r) || !gate.alloc(batch * b_r) ||
-        !core.alloc(b_z) || !o.alloc(b_z)) return 0;
-    cudaStream_t s = 0;
-    RC_CUDA(cudaMemcpyAsync(ck.p, p->conv_kernel, b_ck, cudaMemcpyHostToDevice, s));
-    RC_CUDA(cudaMemcpyAsync(dt.p, p->dt_bias, b_r, cudaMemcpyHostToDevice, s));
-    RC_CUDA(cudaMemcpyAsync(sa.p, p->ssm_a, b_r, cudaMemcpyHostToDevice, s));
-    RC_CUDA(cudaMemcpyAsync(nw.p, p->ssm_norm, b_nw, cudaMemcpyHostToDevice, s));
-    RC_CUDA(cudaMemcpyAsync(dq.p, qkv, b_qkv, cudaMemcpyHostToDevice, s));
-    RC_CUDA(cudaMemcpyAsync(dz.p, z, b_z, cudaMemcpyHostToDevice, s));
-    RC_CUDA(cudaMemcpyAsync(dba.p, ba, b_ba, cudaMemcpyHostToDevice, s));
-    RC_CUDA(cudaMemcpyAsync(cs.p, conv_state, b_cs, cudaMemcpyHostToDevice, s));
-    RC_CUDA(cudaMemcpyAsync(rs.p, rec_state, b_rs, cudaMemcpyHostToDevice, s));
-    if (!launch_deltanet(D, batch, ck.as<float>(), dt.as<float>(), sa.as<float>(), nw.as<float>(), dq.as<float>(), dz.as<float>(), dba.as<float>(),
-                         cs.as<float>(), rs.as<float>(), qk.as<float>(), v.as<float>(), beta.as<float>(), gate.as<float>(), core.as<float>(), o.as<float>(), s)) return 0;
-    RC_CUDA(cudaMemcpyAsync(conv_state, cs.p, b_cs, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaMemcpyAsync(rec_state, rs.p, b_rs, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaMemcpyAsync(out, o.p, b_z, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaStreamSynchronize(s));
-    return 1;
+    const size_t b_qk = batch * nqk * 4u;
+    Stage st;
+    if (!st.open(Stage::pad(b_ck) + 2u * Stage::pad(b_r) + Stage::pad(b_nw) + Stage::pad(b_qkv) + 4u * Stage::pad(b_z) + Stage::pad(b_ba) + Stage::pad(b_cs) + Stage::pad(b_rs) +
+                 Stage::pad(b_qk) + 2u * Stage::pad(batch * b_r))) return 0;
+    auto f32 = [&](size_t n) { return st.take<float>(n); };
+    float *ck = f32(b_ck), *dt = f32(b_r), *sa = f32(b_r), *nw = f32(b_nw), *dq = f32(b_qkv), *dz = f32(b_z), *dba = f32(b_ba), *cs = f32(b_cs), *rs = f32(b_rs),
+          *qk = f32(b_qk), *v = f32(b_z), *beta = f32(batch * b_r), *gate = f32(batch * b_r), *core = f32(b_z), *o = f32(b_z);
+    if (!st.upload(ck, p->conv_kernel, b_ck) || !st.upload(dt, p->dt_bias, b_r) || !st.upload(sa, p->ssm_a, b_r) || !st.upload(nw, p->ssm_norm, b_nw) || !st.upload(dq, qkv, b_qkv) ||
+        !st.upload(dz, z, b_z) || !st.upload(dba, ba, b_ba) || !st.upload(cs, conv_state, b_cs) || !st.upload(rs, rec_state, b_rs)) return 0;
+    if (!launch_deltanet(D, batch, ck, dt, sa, nw, dq, dz, dba, cs, rs, qk, v, beta, gate, core, o, st.stream())) return 0;
+    return st.download(conv_state, cs, b_cs) && st.download(rec_state, rs, b_rs) && st.download(out, o, b_z) && st.finish();
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -34,6 +34,7 @@
 #include "redcuda_dot.cuh"
 #include "redcuda_kernels.cuh"
 #include "redcuda_moe_mma.cuh"
+#include "redcuda_stage.cuh"
 #include "../../include/redcuda.h"
 
 #include <stdlib.h>
@@ -588,15 +589,15 @@ extern "C" int redcuda_nib_dequant_rows(const uint8_t *rows, uint32_t nrows, uin
     RC_REQUIRE(rows && out, "nib dequant: null argument");
     RC_REQUIRE(nib_shape_ok(nrows, ncols), "nib dequant: matrix %ux%u is not tileable (16 rows, 256/512/1024/2048 columns)", nrows, ncols);
     const uint64_t bytes = rc_matrix_bytes(RC_IQ2_XXS, nrows, ncols), nb = (uint64_t)nrows * (ncols / 256u);
-    DevMem raw, planar, nib, o;
-    if (!raw.alloc(bytes) || !planar.alloc(bytes) || !nib.alloc(nib_matrix_bytes(nrows, ncols)) || !o.alloc((size_t)nrows * ncols * 4u)) return 0;
-    cudaStream_t s = 0;
-    if (!upload_matrix(RC_IQ2_XXS, nrows, ncols, rows, false, planar.as<uint8_t>(), raw.as<uint8_t>(), s)) return 0;
-    if (!launch_nib_repack(planar.as<uint8_t>(), nrows, ncols, nib.as<uint8_t>(), s)) return 0;
+    const size_t ob = (size_t)nrows * ncols * 4u, nibb = nib_matrix_bytes(nrows, ncols);
+    Stage st;
+    if (!st.open(2u * Stage::pad(bytes) + Stage::pad(nibb) + Stage::pad(ob))) return 0;
+    uint8_t *raw = st.take(bytes), *planar = st.take(bytes), *nib = st.take(nibb);
+    float *o = st.take<float>(ob);
+    cudaStream_t s = st.stream();
+    if (!st.upload(raw, rows, bytes) || !upload_matrix(RC_IQ2_XXS, nrows, ncols, raw, true, planar, nullptr, s) || !launch_nib_repack(planar, nrows, ncols, nib, s)) return 0;
     const uint64_t total = nb * 32u;
-    RC_LAUNCH((k_nib_dequant), (unsigned)((total + 255u) / 256u < 4096u ? (total + 255u) / 256u : 4096u), 256, 0, s, nib.as<uint8_t>(), nb, nrows, ncols / 256u, o.as<float>());
+    RC_LAUNCH((k_nib_dequant), (unsigned)((total + 255u) / 256u < 4096u ? (total + 255u) / 256u : 4096u), 256, 0, s, nib, nb, nrows, ncols / 256u, o);
     RC_LAUNCHED();
-    RC_CUDA(cudaMemcpyAsync(out, o.p, (size_t)nrows * ncols * 4u, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaStreamSynchronize(s));
-    return 1;
+    return st.download(out, o, ob) && st.finish();
 }

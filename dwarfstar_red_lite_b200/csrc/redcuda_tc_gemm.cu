@@ -26,6 +26,7 @@
 #include "redcuda_formats.cuh"
 #include "redcuda_dot.cuh"
 #include "redcuda_kernels.cuh"
+#include "redcuda_stage.cuh"
 #include "redcuda_tc_gemm.cuh"
 
 #include <cuda_fp16.h>
@@ -516,24 +517,26 @@ extern "C" int redcuda_quant_matmul_tc(uint32_t type, const uint8_t *w, uint32_t
     RC_REQUIRE(ncols % 256u == 0, "matmul_tc: %u columns is not a multiple of 256", ncols);
     const uint64_t bytes = rc_matrix_bytes(type, nrows, ncols);
     const uint32_t tn = tc_token_tile(ntok, tc_row_tiles(nrows));
-    DevMem raw, planar, xd, od, xs, xinv, err, wd, winv;
-    if (!raw.alloc(bytes) || !planar.alloc(bytes) || !xd.alloc((size_t)ntok * ncols * 4u) || !od.alloc((size_t)ntok * nrows * 4u) ||
-        !xs.alloc(tc_xs_halves(ntok, ncols, tn) * 2u) || !xinv.alloc((size_t)((ntok + tn - 1u) / tn) * tn * 4u) || !err.alloc(4u) ||
-        !wd.alloc(tc_wd_bytes(tc_row_tiles(nrows), ncols)) || !winv.alloc((size_t)tc_row_tiles(nrows) * 4u)) return 0;
-    cudaStream_t s = 0;
-    if (!upload_matrix(type, nrows, ncols, w, false, planar.as<uint8_t>(), raw.as<uint8_t>(), s)) return 0;
-    RC_CUDA(cudaMemcpyAsync(xd.p, x, (size_t)ntok * ncols * 4u, cudaMemcpyHostToDevice, s));
-    RC_CUDA(cudaMemsetAsync(err.p, 0, 4u, s));
-    if (!launch_tc_prep_x(xd.as<float>(), nullptr, ncols, ntok, ncols, tn, xs.as<__half>(), xinv.as<float>(), s)) return 0;
+    const size_t xb = (size_t)ntok * ncols * 4u, ob = (size_t)ntok * nrows * 4u, xsb = tc_xs_halves(ntok, ncols, tn) * 2u, xib = (size_t)((ntok + tn - 1u) / tn) * tn * 4u;
+    const size_t wdb = tc_wd_bytes(tc_row_tiles(nrows), ncols), wib = (size_t)tc_row_tiles(nrows) * 4u;
+    Stage st;
+    if (!st.open(2u * Stage::pad(bytes) + Stage::pad(xb) + Stage::pad(ob) + Stage::pad(xsb) + Stage::pad(xib) + Stage::pad(wdb) + Stage::pad(wib) + Stage::pad(4u))) return 0;
+    uint8_t *raw = st.take(bytes), *planar = st.take(bytes), *wd = st.take(wdb);
+    float *xd = st.take<float>(xb), *od = st.take<float>(ob), *xinv = st.take<float>(xib), *winv = st.take<float>(wib);
+    __half *xs = st.take<__half>(xsb);
+    uint32_t *err = st.take<uint32_t>(4u);
+    cudaStream_t s = st.stream();
+    if (!st.upload(xd, x, xb)) return 0;
+    RC_CUDA(cudaMemsetAsync(err, 0, 4u, s));
+    if (!launch_tc_prep_x(xd, nullptr, ncols, ntok, ncols, tn, xs, xinv, s)) return 0;
+    if (!st.upload(raw, w, bytes) || !upload_matrix(type, nrows, ncols, raw, true, planar, nullptr, s)) return 0;
     TcArgs A{};
-    A.njobs = 1; A.ncols = ncols; A.ntok = ntok; A.xs = xs.as<__half>(); A.x_inv = xinv.as<float>(); A.err = err.as<uint32_t>();
-    A.wd = wd.as<uint8_t>(); A.w_inv = winv.as<float>();
-    A.job[0] = TcJob{planar.as<uint8_t>(), (uint64_t)nrows * (ncols / 256u), type, nrows, od.as<float>(), nrows, 0u};
+    A.njobs = 1; A.ncols = ncols; A.ntok = ntok; A.xs = xs; A.x_inv = xinv; A.err = err;
+    A.wd = wd; A.w_inv = winv;
+    A.job[0] = TcJob{planar, (uint64_t)nrows * (ncols / 256u), type, nrows, od, nrows, 0u};
     if (!launch_tc_gemm(A, tn, "tc_gemm", s)) return 0;
     uint32_t flag = 0;
-    RC_CUDA(cudaMemcpyAsync(&flag, err.p, 4u, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaMemcpyAsync(out, od.p, (size_t)ntok * nrows * 4u, cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaStreamSynchronize(s));
+    if (!st.download(out, od, ob) || !st.download(&flag, err, 4u) || !st.finish()) return 0;
     RC_REQUIRE(flag == 0u, "matmul_tc: a tensor-core stage never signalled completion (bounded wait ran out)");
     return 1;
 }
