@@ -44,6 +44,7 @@ int require_books(uint32_t ggml_type);
 // device pointers of the codebooks on the current device
 const uint8_t *books_iq2();
 const uint32_t *books_iq3s();
+bool books_iq3s_odd();       // every magnitude of the IQ3_S codebook is one of 1, 3, ..., 15 (what the 4-bit re-coding of the experts can hold)
 
 // Programmatic dependent launch: every kernel of the library is launched with the stream-serialisation attribute, so the
 // next kernel's blocks are scheduled (and run their prologue up to pdl_prologue's wait) while the previous kernel drains.

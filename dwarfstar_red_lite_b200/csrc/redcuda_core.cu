@@ -102,7 +102,7 @@ void DevMem::release() { if (p) { cudaFree(p); p = nullptr; bytes = 0; } }
 __device__ __align__(16) uint8_t d_iq2_grid[2048];
 __device__ __align__(16) uint32_t d_iq3s_grid[512];
 static std::mutex g_books_mu;
-static bool g_books_set[64] = {false};
+static bool g_books_set[64] = {false}, g_iq3s_odd[64] = {false};
 static const uint8_t *g_iq2_ptr[64] = {nullptr};
 static const uint32_t *g_iq3s_ptr[64] = {nullptr};
 
@@ -116,6 +116,7 @@ int require_books(uint32_t t) {
 }
 const uint8_t *books_iq2() { int dev = 0; cudaGetDevice(&dev); return g_iq2_ptr[dev & 63]; }
 const uint32_t *books_iq3s() { int dev = 0; cudaGetDevice(&dev); return g_iq3s_ptr[dev & 63]; }
+bool books_iq3s_odd() { int dev = 0; cudaGetDevice(&dev); return g_iq3s_odd[dev & 63]; }
 
 // ---- raw GGUF blocks -> planar ----
 __global__ void k_repack(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, uint32_t type, uint64_t nb, uint32_t units_per_block) {
@@ -644,6 +645,8 @@ int redcuda_set_codebooks(const uint8_t *iq2xxs_grid, uint32_t iq2xxs_bytes, con
     g_iq2_ptr[dev] = (const uint8_t *)p2;
     g_iq3s_ptr[dev] = (const uint32_t *)p3;
     g_books_set[dev] = true;
+    g_iq3s_odd[dev] = true;
+    for (uint32_t i = 0; i < 512u; ++i) if ((iq3s_grid[i] & 0xf1f1f1f1u) != 0x01010101u) g_iq3s_odd[dev] = false;
     return 1;
 }
 

@@ -293,6 +293,8 @@ struct redcuda_moe {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_quant = nullptr;
 };
 
+static uint32_t nib_fmt(uint32_t type) { return type == RC_IQ3_S ? NIB_IQ3 : NIB_IQ2; }
+static bool nib_type(uint32_t type) { return type == RC_IQ2_XXS || (type == RC_IQ3_S && books_iq3s_odd()); }
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // tensor-core path of the routed experts: IQ2_XXS gate/up/down with tile-able shapes
@@ -423,7 +425,7 @@ static int moe_launch_experts(redcuda_moe *m, bool gateup, uint32_t npairs, bool
         if (gateup) { if (!launch_tc_prep_rows(x, nullptr, x_stride, (npairs + x_div - 1u) / x_div, ncols, xd, xinv, s)) return 0; }
         else if (!launch_tc_prep_rows(x, m->tmp, x_stride, npairs, ncols, xd, xinv, s)) return 0;
         TcxArgs T{};
-        T.w[0] = gateup ? m->gate : m->down; T.w[1] = gateup ? m->up : nullptr; T.nmat = gateup ? 2u : 1u;
+        T.w[0] = gateup ? m->gate : m->down; T.w[1] = gateup ? m->up : nullptr; T.nmat = gateup ? 2u : 1u; T.fmt = nib_fmt(gateup ? m->d.type_gu : m->d.type_down);
         T.mat_bytes = gateup ? m->gu_bytes : m->down_bytes; T.nrows = nrows; T.ncols = ncols;
         T.expert_begin = m->d.expert_begin; T.n_local = m->d.expert_count;
         T.sorted = m->sorted; T.uexp = m->uexp; T.ustart = m->ustart; T.item_u = m->item_u; T.item_p0 = m->item_p0; T.n_items = m->n_items;
@@ -448,7 +450,7 @@ static int moe_launch_experts(redcuda_moe *m, bool gateup, uint32_t npairs, bool
         const uint32_t tok = moe_item_tokens(m, single_token, npairs);
         const uint32_t live = npairs < m->d.expert_count ? npairs : m->d.expert_count;
         const uint32_t max_items = single_token ? npairs : (npairs / tok + live < npairs ? npairs / tok + live : npairs);
-        if (m->nib) { M.item_tok = tok; M.work = m->work + (gateup ? 0 : 1); return launch_nib_experts(M, max_items, s); }
+        if (m->nib) { M.item_tok = tok; M.fmt = nib_fmt(gateup ? m->d.type_gu : m->d.type_down); M.work = m->work + (gateup ? 0 : 1); return launch_nib_experts(M, max_items, s); }
         return launch_moe_mma(M, max_items, tok, s);
     }
     MoeArgs A{};
@@ -529,10 +531,11 @@ static int moe_forward_fused1(redcuda_moe *m, const float *x, const float *logit
     M.w0 = m->gate; M.w1 = m->up; M.mat_bytes = m->gu_bytes; M.nb = m->gu_nb; M.nrows = m->d.ffn; M.ncols = m->d.hidden;
     M.expert_begin = m->d.expert_begin; M.n_local = m->d.expert_count; M.status = status_words();
     M.sorted = m->sorted; M.uexp = m->uexp; M.ustart = m->ustart; M.item_u = m->item_u; M.item_p0 = m->item_p0; M.n_items = m->n_items;
-    M.xq = nullptr; M.sx = nullptr; M.x_div = k; M.out = m->act; M.out_stride = m->d.ffn; M.item_tok = 1u; M.work = m->work; M.x_raw = x;
+    M.xq = nullptr; M.sx = nullptr; M.x_div = k; M.out = m->act; M.out_stride = m->d.ffn; M.item_tok = 1u; M.work = m->work; M.x_raw = x; M.fmt = nib_fmt(m->d.type_gu);
     if (!launch_nib_experts(M, k, s)) return 0;
     NibTailArgs D{};
     D.w_down = m->down; D.mat_bytes = m->down_bytes; D.nrows = m->d.hidden; D.ncols = m->d.ffn; D.expert_begin = m->d.expert_begin; D.n_local = m->d.expert_count;
+    D.fmt = nib_fmt(m->d.type_down);
     D.top_k = k; D.ids = m->ids; D.wk = m->wk; D.act = m->act; D.act_stride = m->d.ffn;
     D.sh_down = m->sh_down.base; D.sh_nb = m->sh_down.nb; D.sh_act = m->sh_act; D.scalar = m->scalar; D.resid = resid; D.out = out; D.status = status_words();
     return launch_nib_down_tail(D, s);
@@ -692,12 +695,12 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
         set_error("moe create: stream / event creation failed"); return bail();
     }
 
-    {   // RC_EXPERT_FMT: "nib4" keeps IQ2_XXS experts in the nibble layout (table-free decode, 2.09x the bytes), "iq2" in the
-        // planar GGUF bytes; unset = nib4 where the shapes allow it (measured on the 64-token batch: gate/up 105 -> 69 us,
+    {   // RC_EXPERT_FMT: "nib4" keeps IQ2_XXS / IQ3_S experts in the nibble layout (table-free decode, 2.09x / 1.25x the bytes),
+        // "iq2" in the planar GGUF bytes; unset = nib4 where the shapes allow it (measured on the 64-token batch: gate/up 105 -> 69 us,
         // down 74 -> 39 us per layer)
         const char *fmt = getenv("RC_EXPERT_FMT");
         const bool want = !(fmt && fmt[0] == 'i');
-        m->nib = want && d.type_gu == RC_IQ2_XXS && d.type_down == RC_IQ2_XXS && nib_shape_ok(d.ffn, d.hidden) && nib_shape_ok(d.hidden, d.ffn);
+        m->nib = want && nib_type(d.type_gu) && nib_type(d.type_down) && nib_shape_ok(d.ffn, d.hidden) && nib_shape_ok(d.hidden, d.ffn);
     }
     m->gu_bytes = m->nib ? nib_matrix_bytes(d.ffn, d.hidden) : rc_matrix_bytes(d.type_gu, d.ffn, d.hidden);
     m->down_bytes = m->nib ? nib_matrix_bytes(d.hidden, d.ffn) : rc_matrix_bytes(d.type_down, d.hidden, d.ffn);
@@ -726,9 +729,8 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
 
     // upload + planar repack; host sources go through a bounded staging buffer, expert by expert
     const bool dev = d.weights_on_device != 0;
-    DevMem scratch, planar_tmp;
+    DevMem scratch;
     const size_t raw_gu = rc_matrix_bytes(d.type_gu, d.ffn, d.hidden), raw_down = rc_matrix_bytes(d.type_down, d.hidden, d.ffn);
-    if (m->nib && !planar_tmp.alloc(raw_gu > raw_down ? raw_gu : raw_down)) return bail();
     const size_t big = raw_gu > raw_down ? raw_gu : raw_down;
     const size_t sc_b = big > shgu_b ? (big > shd_b ? big : shd_b) : (shgu_b > shd_b ? shgu_b : shd_b);
     if (!dev && !scratch.alloc(sc_b)) return bail();
@@ -738,17 +740,19 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
              upload_matrix(d.type_sh, d.ffn_sh, d.hidden, d.sh_gate, dev, W + o_shg, scratch.as<uint8_t>(), s) &&
              upload_matrix(d.type_sh, d.ffn_sh, d.hidden, d.sh_up, dev, W + o_shu, scratch.as<uint8_t>(), s) &&
              upload_matrix(d.type_sh, d.hidden, d.ffn_sh, d.sh_down, dev, W + o_shd, scratch.as<uint8_t>(), s);
-    // one expert matrix: raw GGUF rows -> planar (in place in the arena, or in a temporary when the arena holds the nibble layout)
-    auto put = [&](uint32_t type, uint32_t nrows, uint32_t ncols, const uint8_t *src, uint8_t *dst) -> int {
-        if (!m->nib) return upload_matrix(type, nrows, ncols, src, dev, dst, scratch.as<uint8_t>(), s);
-        return upload_matrix(type, nrows, ncols, src, dev, planar_tmp.as<uint8_t>(), scratch.as<uint8_t>(), s) &&
-               launch_nib_repack(planar_tmp.as<uint8_t>(), nrows, ncols, dst, s);
+    // expert matrices: GGUF rows -> planar, matrix by matrix, or -> the nibble layout, as many matrices at once as lie in device memory
+    auto put = [&](uint32_t type, uint32_t nrows, uint32_t ncols, size_t raw_bytes, const uint8_t *src, uint8_t *dst, uint64_t dst_bytes) -> int {
+        if (m->nib && dev) return launch_nib_repack(nib_fmt(type), src, (uint64_t)nrows * d.expert_count, ncols, dst, s);
+        for (uint32_t e = 0; e < d.expert_count; ++e) {
+            const uint8_t *se = src + (size_t)e * raw_bytes;
+            if (!m->nib) { if (!upload_matrix(type, nrows, ncols, se, dev, dst + (size_t)e * dst_bytes, scratch.as<uint8_t>(), s)) return 0; continue; }
+            RC_CUDA(cudaMemcpyAsync(scratch.p, se, raw_bytes, cudaMemcpyHostToDevice, s));
+            if (!launch_nib_repack(nib_fmt(type), scratch.as<uint8_t>(), nrows, ncols, dst + (size_t)e * dst_bytes, s)) return 0;
+        }
+        return 1;
     };
-    for (uint32_t e = 0; ok && e < d.expert_count; ++e) {
-        ok = put(d.type_gu, d.ffn, d.hidden, d.gate_exps + (size_t)e * raw_gu, m->gate + (size_t)e * m->gu_bytes) &&
-             put(d.type_gu, d.ffn, d.hidden, d.up_exps + (size_t)e * raw_gu, m->up + (size_t)e * m->gu_bytes) &&
-             put(d.type_down, d.hidden, d.ffn, d.down_exps + (size_t)e * raw_down, m->down + (size_t)e * m->down_bytes);
-    }
+    ok = ok && put(d.type_gu, d.ffn, d.hidden, raw_gu, d.gate_exps, m->gate, m->gu_bytes) && put(d.type_gu, d.ffn, d.hidden, raw_gu, d.up_exps, m->up, m->gu_bytes) &&
+         put(d.type_down, d.hidden, d.ffn, raw_down, d.down_exps, m->down, m->down_bytes);
     if (!ok) return bail();
 
     // workspace: this layer's own, or the caller's (shared by layers whose calls are ordered on one stream)

@@ -21,6 +21,7 @@ struct MmaArgs {
     uint32_t S, tiles_per_warp, item_tok, item_class;    // filled by launch_moe_mma
     float dw1, dw2;                // weights of digits 1 and 2 (2^bits, 4^bits), filled by launch_moe_mma
     uint32_t *work;                // nibble-layout kernels: the launch's unit counter, zeroed by the grouping kernel
+    uint32_t fmt;                  // nibble-layout kernels: NIB_IQ2 or NIB_IQ3
     const float *x_raw;            // nibble-layout gate/up of a single token: its fp32 activation row, quantised inside the kernel (xq / sx unused)
     uint32_t act_bits;             // digit width, filled by the launcher
 };
@@ -38,19 +39,22 @@ int launch_quant_act(const float *x, uint32_t x_stride, uint32_t rows, uint32_t 
 uint32_t mma_item_tokens(bool few_tokens, uint32_t npairs = 0u, uint32_t n_experts = 1u);
 // max_items = upper bound of work items (grid.y); item_tok: the size the items were cut with (2, 8 or 16)
 int launch_moe_mma(MmaArgs &A, uint32_t max_items, uint32_t item_tok, cudaStream_t s);
-// ---- nibble layout of IQ2_XXS expert matrices (redcuda_moe_nib.cu): 138 bytes per 256 weights, table-free decode ----
+// ---- nibble layout of IQ2_XXS / IQ3_S expert matrices (redcuda_moe_nib.cu): 138 bytes per 256 weights, table-free decode ----
 constexpr uint32_t NIB_BLOCK_BYTES = 138u;
+// what the 4-bit codes of a matrix mean (a template parameter of the kernels)
+constexpr uint32_t NIB_IQ2 = 0u, NIB_IQ3 = 1u;
 // one record = one 16-row tile x one 256-column block
 constexpr uint32_t NIB_SC_OFF = 2048u, NIB_D_OFF = 2176u, NIB_REC = 2208u;
-// byte offset of code word (t, kg) of row rr inside a record (16-byte pieces of odd rows pairwise swapped)
+// byte offset of code word (t, kg) of row rr inside a record (16-byte piece p of row rr is stored at p ^ (rr % 8))
 __host__ __device__ __forceinline__ uint32_t nib_code_off(uint32_t rr, uint32_t t, uint32_t kg) {
-    const uint32_t piece = (2u * t + (kg >> 2)) ^ (rr & 1u);
+    const uint32_t piece = (2u * t + (kg >> 2)) ^ (rr & 7u);
     return rr * 128u + piece * 16u + (kg & 3u) * 4u;
 }
 uint64_t nib_matrix_bytes(uint32_t nrows, uint32_t ncols);
 bool nib_shape_ok(uint32_t nrows, uint32_t ncols);
-// planar IQ2_XXS matrix -> nibble layout (dst: nib_matrix_bytes, 16-byte aligned)
-int launch_nib_repack(const uint8_t *planar, uint32_t nrows, uint32_t ncols, uint8_t *dst, cudaStream_t s);
+// GGUF rows of IQ2_XXS (NIB_IQ2) or IQ3_S (NIB_IQ3), one matrix or several in a row (nrows = all their rows) -> nibble layout
+// (dst: nib_matrix_bytes, 16-byte aligned)
+int launch_nib_repack(uint32_t fmt, const uint8_t *raw, uint64_t nrows, uint32_t ncols, uint8_t *dst, cudaStream_t s);
 // gate/up (A.w1 set) or down projection of the grouped pairs, work items of at most 8 pairs; persistent kernel
 int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s);
 // Single token, nibble layout: down projection of the token's top_k experts for one 16-row tile per block, the shared
@@ -65,6 +69,7 @@ struct NibTailArgs {
     const float *sh_act, *scalar, *resid;             // shared activation [ncols], its scalar gate [1], residual [nrows] or null
     float *out;
     float dw1, dw2; uint32_t bits;                    // filled by the launcher
+    uint32_t fmt;                                     // NIB_IQ2 or NIB_IQ3
     uint32_t *status;
 };
 bool nib_tail_ok(uint32_t top_k, uint32_t nrows, uint32_t ncols);

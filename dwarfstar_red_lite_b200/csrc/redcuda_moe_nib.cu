@@ -1,21 +1,26 @@
-// Routed IQ2_XXS experts in the "nibble" layout: a load-time re-coding whose decode needs no table in shared memory.
+// Routed IQ2_XXS and IQ3_S experts in the "nibble" layout: a load-time re-coding whose decode needs no table in shared memory.
 //
 // Why: IQ2_XXS stores 8 weights as one codebook index (8 bits) plus 7 sign bits; turning them into tensor-core operands
 // costs two dependent shared-memory lookups and ~10 integer instructions per 8 weights, and the expert kernels were
 // bound by instruction issue at a sixth of HBM speed (57 M warp instructions per gate/up launch of a 64-token batch).
 // Here every weight is re-coded once, at load, as a 4-bit code (bits 1:0 = which of the three codebook magnitudes
 // 8 / 25 / 43, bit 2 = sign); a lane then expands 4 weights into an int8 operand register with ONE instruction
-// (prmt against an 8-byte table held in two registers). Dequantised values are unchanged bit for bit
+// (prmt against an 8-byte table held in two registers). IQ3_S experts take the same layout (NIB_IQ3): their magnitudes are the
+// odd numbers 1 .. 15, so a signed weight is 2 n + 1 with n in -8 .. 7 and the code is n itself in two's complement; as the
+// high nibble of a byte with 8 below it, it IS the int8 operand 8 (2 n + 1) - one mask-and-or per 4 weights, and the block
+// scale d / 8 serves both formats. A layer of IQ3_S experts took 549 us for 24 tokens on the CUDA-core kernel, 136 here.
+// Dequantised values are unchanged bit for bit
 // (redcuda_nib_dequant_rows against rl_quant_dequant_row, native/redlite_native_quant_cpu.c:166-191). The price is bytes:
-// 138 per 256 weights instead of 66, i.e. 2.09x the HBM footprint and traffic of the routed experts.
+// 138 per 256 weights instead of 66 (IQ3_S: 110), i.e. 2.09x (1.25x) the HBM footprint and traffic of the routed experts.
 //
 // Layout of one expert matrix [nrows][ncols], bpr = ncols / 256 blocks per row: one contiguous RECORD of 2208 bytes per
 // (16-row tile, 256-column block), records ordered [tile][block], so that a warp fetches everything it needs for one
 // block of its tile with a single bulk copy:
 //   codes  @0     16 rows x 128 B; logical byte 32 t + 4 kg of a row = u32 word (t, kg) = the 8 weights 32 kg + 8 t .. +7
-//                 of the block, weight j in bits 4j+3..4j (a lane's 8 words are 32 contiguous bytes). The 16-byte
-//                 pieces of odd rows are stored pairwise swapped (piece p at p ^ 1): a record lands in shared memory
-//                 as it is, and with the swap the 16-byte reads of a quarter warp hit eight different bank groups
+//                 of the block, weight j in bits 4j+3..4j (NIB_IQ3: weights j and j + 4 in the low and high nibble of
+//                 byte j). Piece p (16 bytes) of row r is stored at p ^ (r % 8): a record lands in shared memory as it is,
+//                 and eight lanes that read the same piece of eight rows, or the pieces 2 t of two rows, hit eight
+//                 different bank groups
 //   scales @2048  16 rows x 8 B, byte kg = 2 s + 1, s the 4-bit scale of the 32-weight group
 //   d      @2176  16 fp16 block scales
 // Arithmetic is the integer tensor-core scheme of redcuda_moe_mma.cu (mma.sync m16n8k32 s8, activations as three
@@ -38,47 +43,68 @@
 #include "../../include/redcuda.h"
 
 #include <stdlib.h>
+#include <type_traits>
 
 namespace rc {
 
 uint64_t nib_matrix_bytes(uint32_t nrows, uint32_t ncols) { return (uint64_t)nrows * (ncols / 256u) * NIB_BLOCK_BYTES; }
 bool nib_shape_ok(uint32_t nrows, uint32_t ncols) { return nrows % 16u == 0 && (ncols == 256u || ncols == 512u || ncols == 1024u || ncols == 2048u); }
 
-// ---- planar IQ2_XXS -> nibble layout: one thread per (block, group kg, quarter t) ----
-__global__ void k_nib_repack(const uint8_t *__restrict__ planar, uint64_t nb, uint32_t nrows, uint32_t bpr, const uint8_t *__restrict__ iq2,
-                             uint8_t *__restrict__ dst) {
+// ---- GGUF rows of IQ2_XXS / IQ3_S -> nibble layout: one thread per (block, group kg, quarter t). Matrices that follow one
+// another in memory are repacked as one (their row counts are multiples of 16): a layer's 512 experts take one launch per
+// projection, where a planar repack and a recoding per matrix took 1024 ----
+template <uint32_t FMT>
+__global__ void k_nib_repack(const uint8_t *__restrict__ raw, uint64_t nb, uint32_t bpr, const RcBooks bk, uint8_t *__restrict__ dst) {
     pdl_prologue();
     const uint64_t total = nb * 32u;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t b = i >> 5;
         const uint32_t kg = ((uint32_t)i >> 2) & 7u, t = (uint32_t)i & 3u;
-        const uint32_t row = (uint32_t)(b / bpr), blk = (uint32_t)(b - (uint64_t)row * bpr);
-        const uint32_t auxg = *reinterpret_cast<const uint32_t *>(planar + b * 64u + kg * 8u), auxs = *reinterpret_cast<const uint32_t *>(planar + b * 64u + kg * 8u + 4u);
-        const uint8_t *gv = iq2 + ((auxg >> (8u * t)) & 255u) * 8u;
-        const uint32_t s8 = rc_sign8((auxs >> (7u * t)) & 127u);
-        uint32_t word = 0u;
+        const uint64_t row = b / bpr;
+        const uint32_t blk = (uint32_t)(b - row * bpr);
+        const uint8_t *bp = raw + b * (FMT == NIB_IQ2 ? 66u : 110u);
+        uint32_t word = 0u, s4;
+        if (FMT == NIB_IQ2) {
+            const unsigned short *q = reinterpret_cast<const unsigned short *>(bp + 2u + kg * 8u);
+            const uint32_t auxs = (uint32_t)q[2] | ((uint32_t)q[3] << 16);
+            const uint8_t *gv = bk.iq2 + (uint32_t)bp[2u + kg * 8u + t] * 8u;
+            const uint32_t s8 = rc_sign8((auxs >> (7u * t)) & 127u);
 #pragma unroll
-        for (uint32_t j = 0; j < 8u; ++j) {
-            const uint32_t m = gv[j] == 0x19u ? 1u : gv[j] == 0x2bu ? 2u : 0u;
-            word |= (m | (((s8 >> j) & 1u) << 2)) << (4u * j);
+            for (uint32_t j = 0; j < 8u; ++j) {
+                const uint32_t m = gv[j] == 0x19u ? 1u : gv[j] == 0x2bu ? 2u : 0u;
+                word |= (m | (((s8 >> j) & 1u) << 2)) << (4u * j);
+            }
+            s4 = auxs >> 28;
+        } else {
+            const uint8_t *qs = bp + 2u + 8u * kg + 2u * t;
+            const uint32_t qh = bp[66u + kg], sg = bp[74u + 4u * kg + t];
+            const uint32_t g[2] = {bk.iq3s[qs[0] | ((qh << (8u - 2u * t)) & 256u)], bk.iq3s[qs[1] | ((qh << (7u - 2u * t)) & 256u)]};
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; ++j) {
+                const int m = (int)((g[j >> 2] >> (8u * (j & 3u))) & 255u), v = (sg >> j) & 1u ? -m : m;       // 2 n + 1
+                word |= ((uint32_t)((v - 1) >> 1) & 15u) << (8u * (j & 3u) + 4u * (j >> 2));
+            }
+            s4 = ((uint32_t)bp[106u + (kg >> 1)] >> (4u * (kg & 1u))) & 15u;
         }
-        uint8_t *rec = dst + ((uint64_t)(row >> 4) * bpr + blk) * NIB_REC;
-        const uint32_t rr = row & 15u;
+        uint8_t *rec = dst + ((row >> 4) * bpr + blk) * NIB_REC;
+        const uint32_t rr = (uint32_t)row & 15u;
         *reinterpret_cast<uint32_t *>(rec + nib_code_off(rr, t, kg)) = word;
         if (t == 0u) {
-            rec[NIB_SC_OFF + rr * 8u + kg] = (uint8_t)(2u * (auxs >> 28) + 1u);
-            if (kg == 0u) *reinterpret_cast<unsigned short *>(rec + NIB_D_OFF + rr * 2u) = *reinterpret_cast<const unsigned short *>(planar + rc_iq2_d(nb) + b * 2u);
+            rec[NIB_SC_OFF + rr * 8u + kg] = (uint8_t)(2u * s4 + 1u);
+            if (kg == 0u) *reinterpret_cast<unsigned short *>(rec + NIB_D_OFF + rr * 2u) = *reinterpret_cast<const unsigned short *>(bp);
         }
     }
 }
 
-int launch_nib_repack(const uint8_t *planar, uint32_t nrows, uint32_t ncols, uint8_t *dst, cudaStream_t s) {
-    RC_REQUIRE(nib_shape_ok(nrows, ncols), "nibble layout: matrix %ux%u is not tileable (16 rows, 256/512/1024/2048 columns)", nrows, ncols);
-    RC_REQUIRE(((uintptr_t)dst & 15u) == 0 && ((uintptr_t)planar & 15u) == 0, "nibble layout: unaligned matrix");
-    const uint64_t nb = (uint64_t)nrows * (ncols / 256u), total = nb * 32u;
+int launch_nib_repack(uint32_t fmt, const uint8_t *raw, uint64_t nrows, uint32_t ncols, uint8_t *dst, cudaStream_t s) {
+    RC_REQUIRE(nrows % 16u == 0 && nib_shape_ok(16u, ncols), "nibble layout: %llu rows of %u columns are not tileable (16 rows, 256/512/1024/2048 columns)", (unsigned long long)nrows, ncols);
+    RC_REQUIRE(((uintptr_t)dst & 15u) == 0 && ((uintptr_t)raw & 1u) == 0, "nibble layout: unaligned matrix");
+    const uint64_t nb = nrows * (ncols / 256u), total = nb * 32u;
     const uint32_t grid = (uint32_t)((total + 255u) / 256u < 148u * 16u ? (total + 255u) / 256u : 148u * 16u);
     prof_begin("nib_repack", s);
-    RC_LAUNCH((k_nib_repack), grid ? grid : 1u, 256, 0, s, planar, nb, nrows, ncols / 256u, books_iq2(), dst);
+    const RcBooks bk{books_iq2(), books_iq3s()};
+    if (fmt == NIB_IQ2) RC_LAUNCH((k_nib_repack<NIB_IQ2>), grid ? grid : 1u, 256, 0, s, raw, nb, ncols / 256u, bk, dst);
+    else RC_LAUNCH((k_nib_repack<NIB_IQ3>), grid ? grid : 1u, 256, 0, s, raw, nb, ncols / 256u, bk, dst);
     prof_end(s);
     RC_LAUNCHED();
     return 1;
@@ -124,6 +150,9 @@ __device__ __forceinline__ uint32_t nb_prmt(uint32_t a, uint32_t b, uint32_t sel
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
     return d;
 }
+// the 8 codes of a word -> the int8 operands of weights 0..3 (lo) and 4..7 (hi)
+template <uint32_t FMT>
+__device__ __forceinline__ void nb_expand(uint32_t w, uint32_t &lo, uint32_t &hi);
 // one record into a ring slot: the copy engine signals the slot's mbarrier with the bytes it delivered
 __device__ __forceinline__ void nb_fetch(uint32_t dst, const void *src, uint32_t bar) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(NIB_REC) : "memory");
@@ -147,11 +176,20 @@ constexpr uint32_t NIB_WARPS = 8u;
 constexpr uint32_t NIB_STAGES_BATCH = 3u, NIB_STAGES_ONE = 8u;
 constexpr uint32_t NIB_TAB_POS = 0x002b1908u, NIB_TAB_NEG = 0x00d5e7f8u;      // bytes 8, 25, 43, 0 and -8, -25, -43, 0
 
+template <>
+__device__ __forceinline__ void nb_expand<NIB_IQ2>(uint32_t w, uint32_t &lo, uint32_t &hi) {
+    lo = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, w); hi = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, w >> 16);
+}
+template <>
+__device__ __forceinline__ void nb_expand<NIB_IQ3>(uint32_t w, uint32_t &lo, uint32_t &hi) {
+    lo = ((w << 4) & 0xf0f0f0f0u) | 0x08080808u; hi = (w & 0xf0f0f0f0u) | 0x08080808u;
+}
+
 // One warp: 16 rows x one 256-column block (a record in shared memory) against NT 8-column tiles of activation digits.
 // Bl: digits of column g of tile 0 at this block's first column + 8 t (tile n is n * 8 * BPITCH further).
-template <int NT, uint32_t BPITCH>
+template <uint32_t FMT, int NT, uint32_t BPITCH>
 __device__ __forceinline__ void nib_chunk(const uint8_t *st, const int8_t *Bl, uint32_t g, uint32_t t, const int (&z)[4], float (&out)[3][4]) {
-    const uint32_t o0 = g * 128u + ((2u * t) ^ (g & 1u)) * 16u, o1 = g * 128u + ((2u * t + 1u) ^ (g & 1u)) * 16u;   // rows g and g + 8 have the same parity
+    const uint32_t o0 = nib_code_off(g, t, 0u), o1 = nib_code_off(g, t, 4u);   // rows g and g + 8 have the same swizzle
     const uint4 qa0 = *reinterpret_cast<const uint4 *>(st + o0), qa1 = *reinterpret_cast<const uint4 *>(st + o1);
     const uint4 qb0 = *reinterpret_cast<const uint4 *>(st + 1024u + o0), qb1 = *reinterpret_cast<const uint4 *>(st + 1024u + o1);
     const uint2 sa = *reinterpret_cast<const uint2 *>(st + NIB_SC_OFF + g * 8u), sb = *reinterpret_cast<const uint2 *>(st + NIB_SC_OFF + (g + 8u) * 8u);
@@ -164,8 +202,9 @@ __device__ __forceinline__ void nib_chunk(const uint8_t *st, const int8_t *Bl, u
     for (int n = 0; n < NT; ++n) { blk[n][0] = blk[n][1] = blk[n][2] = blk[n][3] = 0; }
 #pragma unroll
     for (int kg = 0; kg < 8; ++kg) {
-        const uint32_t a0 = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, wa[kg]), a2 = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, wa[kg] >> 16);
-        const uint32_t a1 = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, wb[kg]), a3 = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, wb[kg] >> 16);
+        uint32_t a0, a1, a2, a3;
+        nb_expand<FMT>(wa[kg], a0, a2);
+        nb_expand<FMT>(wb[kg], a1, a3);
         const int sca = (int)nb_prmt(kg < 4 ? sa.x : sa.y, 0u, 0x4440u + (uint32_t)(kg & 3));
         const int scb = (int)nb_prmt(kg < 4 ? sb.x : sb.y, 0u, 0x4440u + (uint32_t)(kg & 3));
 #pragma unroll
@@ -225,7 +264,7 @@ __device__ __forceinline__ void nib_release(NibRing &R) {
 
 // All tiles of one unit for one warp, NT column tiles of digits in use (1: pairs packed into one tile, 3: a tile per digit).
 // vals[ti][.] = (row g, pair slot 0), (row g, pair slot 1), (row g + 8, slot 0), (row g + 8, slot 1), times the pair's scale.
-template <int NT, uint32_t BPR, uint32_t BPITCH, uint32_t TPW, uint32_t STAGES>
+template <uint32_t FMT, int NT, uint32_t BPR, uint32_t BPITCH, uint32_t TPW, uint32_t STAGES>
 __device__ __forceinline__ void nib_tiles(NibRing &R, const uint8_t *my_stage, const int8_t *Bbase, uint32_t tiles, uint32_t lane, uint32_t g, uint32_t t,
                                           const int (&z)[4], float dw1, float dw2, const float (&sxv)[2], float (&vals)[TPW][4]) {
     for (uint32_t ti = 0; ti < tiles; ++ti) {
@@ -235,7 +274,7 @@ __device__ __forceinline__ void nib_tiles(NibRing &R, const uint8_t *my_stage, c
         for (uint32_t c = 0; c < BPR; ++c) {
             nib_request<STAGES>(R, lane);
             const uint32_t slot = nib_acquire(R);
-            nib_chunk<NT, BPITCH>(my_stage + slot * NIB_REC, Bbase + c * 256u, g, t, z, out);
+            nib_chunk<FMT, NT, BPITCH>(my_stage + slot * NIB_REC, Bbase + c * 256u, g, t, z, out);
             nib_release<STAGES>(R);
         }
         float v[2][2];                 // [row half][pair slot]
@@ -259,7 +298,7 @@ __device__ __forceinline__ void nib_tiles(NibRing &R, const uint8_t *my_stage, c
 
 // GATEUP: warps 0-3 take the gate rows of 4 x TPW tiles, warps 4-7 the up rows of the same tiles; the up values cross a
 // small shared buffer and the gate warps store SiLU(gate) * up. Otherwise (down projection) 8 x TPW tiles per unit.
-template <bool GATEUP, uint32_t NCOLS, uint32_t STAGES>
+template <uint32_t FMT, bool GATEUP, uint32_t NCOLS, uint32_t STAGES>
 __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 2 : 1) k_nib_experts(const __grid_constant__ MmaArgs A) {
     pdl_prologue();
     extern __shared__ __align__(16) uint8_t smem[];
@@ -374,8 +413,8 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
         float vals[TPW][4];
         const uint32_t tiles = I.n / BPR;
         const int8_t *Bbase = Bs + (size_t)g * BPITCH + 8u * t;
-        if (packed) nib_tiles<1, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, tiles, lane, g, t, zero, A.dw1, A.dw2, sxv, vals);
-        else nib_tiles<3, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, tiles, lane, g, t, zero, A.dw1, A.dw2, sxv, vals);
+        if (packed) nib_tiles<FMT, 1, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, tiles, lane, g, t, zero, A.dw1, A.dw2, sxv, vals);
+        else nib_tiles<FMT, 3, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, tiles, lane, g, t, zero, A.dw1, A.dw2, sxv, vals);
         if (R.timed_out && lane == 0) { s_fail = 1u; if (A.status) A.status[ST_TIMEOUT] = 1u; }
         if (GATEUP) {
             if (is_up) for (uint32_t ti = 0; ti < tiles; ++ti) s_ex[ti][wslot][lane] = make_float4(vals[ti][0], vals[ti][1], vals[ti][2], vals[ti][3]);
@@ -417,7 +456,7 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
 // records arrive by bulk copy while the warp quantises expert k's activation row), the last two warps take the shared
 // expert's 16 rows (Q6_K, CUDA cores). Partial rows meet in shared memory and are summed in router order.
 constexpr uint32_t NIB_TAIL_MAX_K = 14u;
-template <uint32_t NCOLS>
+template <uint32_t FMT, uint32_t NCOLS>
 __global__ void __launch_bounds__((NIB_TAIL_MAX_K + 2u) * 32u) k_nib_down_tail(const __grid_constant__ NibTailArgs A) {
     pdl_prologue();
     extern __shared__ __align__(16) uint8_t smem[];
@@ -488,7 +527,7 @@ __global__ void __launch_bounds__((NIB_TAIL_MAX_K + 2u) * 32u) k_nib_down_tail(c
         int zero[4];
         asm volatile("mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;" : "=r"(zero[0]), "=r"(zero[1]), "=r"(zero[2]), "=r"(zero[3]));
         const int8_t *Bl = (g < 3u ? mine + g * BPITCH : zrow) + 8u * t;       // columns 0..2 = the pair's three digits, the rest of the tile is zero
-        if (live) for (uint32_t c = 0; c < BPR; ++c) nib_chunk<1, BPITCH>(my_rec + c * NIB_REC, Bl + c * 256u, g, t, zero, out);
+        if (live) for (uint32_t c = 0; c < BPR; ++c) nib_chunk<FMT, 1, BPITCH>(my_rec + c * NIB_REC, Bl + c * 256u, g, t, zero, out);
         const uint32_t src = (lane & ~3u) + 1u;
         const float x0 = __shfl_sync(0xffffffffu, out[0][0], src), x1 = __shfl_sync(0xffffffffu, out[0][2], src);
         if (t == 0u) {
@@ -531,9 +570,14 @@ int launch_nib_down_tail(NibTailArgs &A, cudaStream_t s) {
     const uint32_t threads = (A.top_k + 2u) * 32u, grid = A.nrows / 16u;
     prof_begin("moe_down_tail", s);
 #define RC_TAIL_LAUNCH(NC) do { \
-        RC_CUDA(cudaFuncSetAttribute(k_nib_down_tail<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        RC_LAUNCH((k_nib_down_tail<NC>), grid, threads, smem, s, A); } while (0)
-    if (A.ncols == 256u) RC_TAIL_LAUNCH(256u); else if (A.ncols == 512u) RC_TAIL_LAUNCH(512u); else RC_TAIL_LAUNCH(1024u);
+        RC_CUDA(cudaFuncSetAttribute(k_nib_down_tail<FMT, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        RC_LAUNCH((k_nib_down_tail<FMT, NC>), grid, threads, smem, s, A); } while (0)
+    auto launch = [&](auto fmt) -> int {
+        constexpr uint32_t FMT = decltype(fmt)::value;
+        if (A.ncols == 256u) RC_TAIL_LAUNCH(256u); else if (A.ncols == 512u) RC_TAIL_LAUNCH(512u); else RC_TAIL_LAUNCH(1024u);
+        return 1;
+    };
+    if (!(A.fmt == NIB_IQ2 ? launch(std::integral_constant<uint32_t, NIB_IQ2>{}) : launch(std::integral_constant<uint32_t, NIB_IQ3>{}))) return 0;
 #undef RC_TAIL_LAUNCH
     prof_end(s);
     RC_LAUNCHED();
@@ -560,8 +604,10 @@ int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s) {
     const size_t smem = nib_smem_bytes(A.ncols, stages);
     prof_begin(gateup ? "moe_gateup" : "moe_down", s);
 #define RC_NIB_LAUNCH(GU, NC, ST) do { \
-        RC_CUDA(cudaFuncSetAttribute(k_nib_experts<GU, NC, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        RC_LAUNCH((k_nib_experts<GU, NC, ST>), grid, NIB_WARPS * 32u, smem, s, A); } while (0)
+        RC_CUDA(cudaFuncSetAttribute(k_nib_experts<FMT, GU, NC, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        RC_LAUNCH((k_nib_experts<FMT, GU, NC, ST>), grid, NIB_WARPS * 32u, smem, s, A); } while (0)
+    auto launch = [&](auto fmt) -> int {
+    constexpr uint32_t FMT = decltype(fmt)::value;
     if (one) {
         if (A.ncols == 2048u) RC_NIB_LAUNCH(true, 2048u, NIB_STAGES_ONE); else if (A.ncols == 1024u) RC_NIB_LAUNCH(true, 1024u, NIB_STAGES_ONE);
         else if (A.ncols == 512u) RC_NIB_LAUNCH(true, 512u, NIB_STAGES_ONE); else RC_NIB_LAUNCH(true, 256u, NIB_STAGES_ONE);
@@ -572,6 +618,9 @@ int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s) {
         if (A.ncols == 2048u) RC_NIB_LAUNCH(false, 2048u, NIB_STAGES_BATCH); else if (A.ncols == 1024u) RC_NIB_LAUNCH(false, 1024u, NIB_STAGES_BATCH);
         else if (A.ncols == 512u) RC_NIB_LAUNCH(false, 512u, NIB_STAGES_BATCH); else RC_NIB_LAUNCH(false, 256u, NIB_STAGES_BATCH);
     }
+    return 1;
+    };
+    if (!(A.fmt == NIB_IQ2 ? launch(std::integral_constant<uint32_t, NIB_IQ2>{}) : launch(std::integral_constant<uint32_t, NIB_IQ3>{}))) return 0;
 #undef RC_NIB_LAUNCH
     prof_end(s);
     RC_LAUNCHED();
@@ -582,7 +631,7 @@ int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s) {
 
 using namespace rc;
 
-// Host-buffer check of the layout: raw IQ2_XXS GGUF rows -> planar -> nibble layout -> fp32. Must equal
+// Host-buffer check of the layout: raw IQ2_XXS GGUF rows -> nibble layout -> fp32. Must equal
 // redcuda_quant_dequant_rows (and rl_quant_dequant_row) bit for bit.
 extern "C" int redcuda_nib_dequant_rows(const uint8_t *rows, uint32_t nrows, uint32_t ncols, float *out) {
     if (!require_device() || !require_books(RC_IQ2_XXS)) return 0;
@@ -591,11 +640,11 @@ extern "C" int redcuda_nib_dequant_rows(const uint8_t *rows, uint32_t nrows, uin
     const uint64_t bytes = rc_matrix_bytes(RC_IQ2_XXS, nrows, ncols), nb = (uint64_t)nrows * (ncols / 256u);
     const size_t ob = (size_t)nrows * ncols * 4u, nibb = nib_matrix_bytes(nrows, ncols);
     Stage st;
-    if (!st.open(2u * Stage::pad(bytes) + Stage::pad(nibb) + Stage::pad(ob))) return 0;
-    uint8_t *raw = st.take(bytes), *planar = st.take(bytes), *nib = st.take(nibb);
+    if (!st.open(Stage::pad(bytes) + Stage::pad(nibb) + Stage::pad(ob))) return 0;
+    uint8_t *raw = st.take(bytes), *nib = st.take(nibb);
     float *o = st.take<float>(ob);
     cudaStream_t s = st.stream();
-    if (!st.upload(raw, rows, bytes) || !upload_matrix(RC_IQ2_XXS, nrows, ncols, raw, true, planar, nullptr, s) || !launch_nib_repack(planar, nrows, ncols, nib, s)) return 0;
+    if (!st.upload(raw, rows, bytes) || !launch_nib_repack(NIB_IQ2, raw, nrows, ncols, nib, s)) return 0;
     const uint64_t total = nb * 32u;
     RC_LAUNCH((k_nib_dequant), (unsigned)((total + 255u) / 256u < 4096u ? (total + 255u) / 256u : 4096u), 256, 0, s, nib, nb, nrows, ncols / 256u, o);
     RC_LAUNCHED();
