@@ -480,87 +480,78 @@ __global__ void __launch_bounds__(256) k_vec_sigmoid(const float *__restrict__ w
 
 // Router logits of a batch: logits[t][e] = (float) sum_k (double) x[t][k] * (double) w[e][k], F32 weights
 // (rl_quant_row_dot on an F32 row accumulates in double, native/redlite_native_quant_cpu.c:198-212, and the top-k that
-// follows must not depend on a summation order). The multi-token GEMV re-reads the matrix for every four tokens; this
-// is a small tiled fp64 GEMM instead: block = 32 tokens x 64 experts, K in tiles of 64 staged as doubles in shared
-// memory (the next tile is fetched into registers while the current one is multiplied); each of the 8 warps owns a
-// 16 x 16 tile of the result as 2 x 2 fragments of the fp64 tensor-core instruction (mma.sync.m8n8k4.f64: four 8-byte
-// shared loads per four instructions; the row pitch of 68 doubles keeps those loads conflict-free). Batches that do
-// not fill half of that tile take a block of 16 tokens x 32 experts with one fragment per warp.
-constexpr uint32_t RL_KT = 64u, RL_PITCH = RL_KT + 4u;
-template <uint32_t FR>            // fragments per warp and direction: block = 16 FR tokens x 32 FR experts
+// follows must not depend on a summation order), on the fp64 tensor-core instruction (mma.sync.m8n8k4.f64).
+// A small batch is bound by the length of the chain, a large one by the fp64 rate (64 FMA per SM and clock). So the eight
+// warps of a block split K, and every warp multiplies straight from global memory: a lane's A and B elements of four
+// successive instructions are one float4 (k order within 16 columns is the same permutation for both operands, and a sum
+// does not depend on it), which costs no shared-memory staging, no barrier per K tile and one conversion per element. The
+// eight partial tiles meet in shared memory once, in a fixed order. Block = 8 FT tokens x 8 FE experts.
+template <uint32_t FT, uint32_t FE>
 __global__ void __launch_bounds__(256) k_router_logits(const float *__restrict__ w, const float *__restrict__ x, uint32_t x_stride, uint32_t ntok,
                                                        uint32_t n_expert, uint32_t ncols, float *__restrict__ logits) {
     pdl_prologue();
-    constexpr uint32_t TT = 16u * FR, TE = 32u * FR;
-    extern __shared__ __align__(16) double rl_smem[];
-    double *xs = rl_smem, *ws = rl_smem + TT * RL_PITCH;
-    const uint32_t tid = threadIdx.x;
-    const uint32_t t0 = blockIdx.x * TT, e0 = blockIdx.y * TE;
-    // staging roles: a tile row is 64 floats = 16 float4; thread -> (row tid / 16 + 16 i, float4 tid % 16)
-    const uint32_t sr = tid >> 4, sc = (tid & 15u) * 4u;
-    constexpr uint32_t NW = TE / 16u, NX = TT / 16u;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 rw[NW], rx[NX];
-    auto fetch = [&](uint32_t k0) {
+    __shared__ double red[8][FT * FE * 64u];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, fr = lane >> 2, fk = lane & 3u;
+    const uint32_t t0 = blockIdx.x * 8u * FT, e0 = blockIdx.y * 8u * FE;
+    // lane -> A element (row lane / 4, k lane % 4), B element (k lane % 4, column lane / 4), C elements (row lane / 4, columns 2 (lane % 4), + 1);
+    // rows past the end repeat the last one, their results are not stored
+    const float *xp[FT], *wp[FE];
 #pragma unroll
-        for (uint32_t i = 0; i < NW; ++i) rw[i] = e0 + sr + 16u * i < n_expert ? __ldg(reinterpret_cast<const float4 *>(w + (size_t)(e0 + sr + 16u * i) * ncols + k0 + sc)) : zero;
+    for (uint32_t i = 0; i < FT; ++i) xp[i] = x + (size_t)min(t0 + 8u * i + fr, ntok - 1u) * x_stride + fk * 4u;
 #pragma unroll
-        for (uint32_t i = 0; i < NX; ++i) rx[i] = t0 + sr + 16u * i < ntok ? *reinterpret_cast<const float4 *>(x + (size_t)(t0 + sr + 16u * i) * x_stride + k0 + sc) : zero;
-    };
-    fetch(0u);
-    // warp -> (token group of 8 FR, expert group of 8 FR); lane -> A element (row lane/4, k lane%4), B element (k lane%4,
-    // column lane/4), C elements (row lane/4, columns 2*(lane%4), +1)
-    const uint32_t warp = tid >> 5, lane = tid & 31u, th = warp >> 2, eq = warp & 3u, fr = lane >> 2, fk = lane & 3u;
-    double acc[FR][FR][2];
+    for (uint32_t i = 0; i < FE; ++i) wp[i] = w + (size_t)min(e0 + 8u * i + fr, n_expert - 1u) * ncols + fk * 4u;
+    double acc[FT][FE][2];
 #pragma unroll
-    for (uint32_t i = 0; i < FR; ++i)
+    for (uint32_t i = 0; i < FT; ++i)
 #pragma unroll
-        for (uint32_t j = 0; j < FR; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    for (uint32_t k0 = 0; k0 < ncols; k0 += RL_KT) {
-        __syncthreads();                                   // the previous tile is no longer read
+        for (uint32_t j = 0; j < FE; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    const uint32_t n16 = ncols >> 4, c1 = n16 * (warp + 1u) / 8u;
+#pragma unroll 4
+    for (uint32_t c = n16 * warp / 8u; c < c1; ++c) {
+        float4 a[FT], b[FE];
 #pragma unroll
-        for (uint32_t i = 0; i < NW; ++i) { double *d = ws + (sr + 16u * i) * RL_PITCH + sc; d[0] = rw[i].x; d[1] = rw[i].y; d[2] = rw[i].z; d[3] = rw[i].w; }
+        for (uint32_t i = 0; i < FT; ++i) a[i] = *reinterpret_cast<const float4 *>(xp[i] + c * 16u);
 #pragma unroll
-        for (uint32_t i = 0; i < NX; ++i) { double *d = xs + (sr + 16u * i) * RL_PITCH + sc; d[0] = rx[i].x; d[1] = rx[i].y; d[2] = rx[i].z; d[3] = rx[i].w; }
-        __syncthreads();
-        if (k0 + RL_KT < ncols) fetch(k0 + RL_KT);
-        const double *a = xs + (th * 8u * FR + fr) * RL_PITCH + fk, *b = ws + (eq * 8u * FR + fr) * RL_PITCH + fk;
+        for (uint32_t i = 0; i < FE; ++i) b[i] = __ldg(reinterpret_cast<const float4 *>(wp[i] + c * 16u));
 #pragma unroll
-        for (uint32_t kk = 0; kk < RL_KT; kk += 4u) {
-            double av[FR], bv[FR];
+        for (uint32_t kk = 0; kk < 4u; ++kk) {
+            double av[FT], bv[FE];
 #pragma unroll
-            for (uint32_t i = 0; i < FR; ++i) { av[i] = a[i * 8u * RL_PITCH + kk]; bv[i] = b[i * 8u * RL_PITCH + kk]; }
+            for (uint32_t i = 0; i < FT; ++i) av[i] = (double)(kk == 0u ? a[i].x : kk == 1u ? a[i].y : kk == 2u ? a[i].z : a[i].w);
 #pragma unroll
-            for (uint32_t i = 0; i < FR; ++i)
+            for (uint32_t i = 0; i < FE; ++i) bv[i] = (double)(kk == 0u ? b[i].x : kk == 1u ? b[i].y : kk == 2u ? b[i].z : b[i].w);
 #pragma unroll
-                for (uint32_t j = 0; j < FR; ++j)
-                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]) : "d"(av[i]), "d"(bv[j]));
+            for (uint32_t i = 0; i < FT; ++i)
+#pragma unroll
+                for (uint32_t j = 0; j < FE; ++j)
+                    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]) : "d"(av[i]), "d"(bv[j]));
         }
     }
 #pragma unroll
-    for (uint32_t i = 0; i < FR; ++i)
+    for (uint32_t i = 0; i < FT; ++i)
 #pragma unroll
-        for (uint32_t j = 0; j < FR; ++j) {
-            const uint32_t t = t0 + (th * FR + i) * 8u + fr, e = e0 + (eq * FR + j) * 8u + 2u * fk;
-            if (t < ntok) {
-                if (e < n_expert) logits[(size_t)t * n_expert + e] = (float)acc[i][j][0];
-                if (e + 1u < n_expert) logits[(size_t)t * n_expert + e + 1u] = (float)acc[i][j][1];
-            }
-        }
+        for (uint32_t j = 0; j < FE; ++j) *reinterpret_cast<double2 *>(&red[warp][(i * FE + j) * 64u + lane * 2u]) = make_double2(acc[i][j][0], acc[i][j][1]);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < FT * FE * 64u; i += 256u) {
+        double s = 0.0;
+#pragma unroll
+        for (uint32_t v = 0; v < 8u; ++v) s += red[v][i];
+        const uint32_t f = i >> 6, r = (i & 63u) >> 3, col = i & 7u, t = t0 + (f / FE) * 8u + r, e = e0 + (f % FE) * 8u + col;
+        if (t < ntok && e < n_expert) logits[(size_t)t * n_expert + e] = (float)s;
+    }
 }
 
 int launch_router_logits(const float *w, const float *x, uint32_t x_stride, uint32_t ntok, uint32_t n_expert, uint32_t ncols, float *logits, cudaStream_t stream) {
-    RC_REQUIRE(ncols % RL_KT == 0 && x_stride % 4u == 0, "router logits: %u columns (stride %u) is not a multiple of %u", ncols, x_stride, RL_KT);
+    RC_REQUIRE(ncols % 16u == 0 && x_stride % 4u == 0, "router logits: %u columns (stride %u) is not a multiple of 16", ncols, x_stride);
     if (!ntok) return 1;
     prof_begin("moe_router_logits", stream);
-    if (ntok >= 256u && n_expert >= 64u) {
-        const size_t smem = (size_t)(32u + 64u) * RL_PITCH * sizeof(double);
-        RC_CUDA(cudaFuncSetAttribute(k_router_logits<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        RC_LAUNCH((k_router_logits<2>), dim3((ntok + 31u) / 32u, (n_expert + 63u) / 64u), 256, smem, stream, w, x, x_stride, ntok, n_expert, ncols, logits);
-    } else {
-        const size_t smem = (size_t)(16u + 32u) * RL_PITCH * sizeof(double);
-        RC_LAUNCH((k_router_logits<1>), dim3((ntok + 15u) / 16u, (n_expert + 31u) / 32u), 256, smem, stream, w, x, x_stride, ntok, n_expert, ncols, logits);
-    }
+    // the tile grows while the blocks still fill the chip about twice: a larger one converts and reads less per product
+    auto blocks = [&](uint32_t tt, uint32_t te) { return (uint64_t)((ntok + tt - 1u) / tt) * ((n_expert + te - 1u) / te); };
+#define RC_RL(FT, FE) RC_LAUNCH((k_router_logits<FT, FE>), dim3((ntok + 8u * FT - 1u) / (8u * FT), (n_expert + 8u * FE - 1u) / (8u * FE)), 256, 0, stream, w, x, x_stride, ntok, n_expert, ncols, logits)
+    if (ntok <= 8u) RC_RL(1u, 1u);
+    else if (blocks(16u, 8u) <= 296u) RC_RL(2u, 1u);
+    else RC_RL(2u, 2u);
+#undef RC_RL
     prof_end(stream);
     RC_LAUNCHED();
     return 1;

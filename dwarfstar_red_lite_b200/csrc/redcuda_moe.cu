@@ -185,12 +185,22 @@ __global__ void __launch_bounds__(256) k_moe_combine(const float *__restrict__ p
     const uint32_t r = (blockIdx.x * 256u + threadIdx.x) * 4u;
     if (r >= hidden) return;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t k = 0; k < top_k; ++k) {
-        const float wk = w[(size_t)t * top_k + k];
-        if (wk == 0.f) continue;           // also the mark of a pair that another shard computes: its row was never written
-        const size_t prow = pair_row ? pair_row[(size_t)t * top_k + k] : (size_t)t * top_k + k;   // where the pair's expert output sits
-        const float4 v = *reinterpret_cast<const float4 *>(pair_out + prow * hidden + r);
-        acc.x += wk * v.x; acc.y += wk * v.y; acc.z += wk * v.z; acc.w += wk * v.w;
+    // a token's rows are requested ten at a time, before the first is added: one round trip for the usual top-10 where a row
+    // per step made ten
+    for (uint32_t k0 = 0; k0 < top_k; k0 += 10u) {
+        float wk[10];
+        float4 v[10];
+#pragma unroll
+        for (uint32_t i = 0; i < 10u; ++i) wk[i] = k0 + i < top_k ? w[(size_t)t * top_k + k0 + i] : 0.f;
+#pragma unroll
+        for (uint32_t i = 0; i < 10u; ++i) {
+            if (wk[i] == 0.f) continue;    // also the mark of a pair that another shard computes: its row was never written
+            const size_t prow = pair_row ? pair_row[(size_t)t * top_k + k0 + i] : (size_t)t * top_k + k0 + i;   // where the pair's expert output sits
+            v[i] = *reinterpret_cast<const float4 *>(pair_out + prow * hidden + r);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 10u; ++i)
+            if (wk[i] != 0.f) { acc.x += wk[i] * v[i].x; acc.y += wk[i] * v[i].y; acc.z += wk[i] * v[i].z; acc.w += wk[i] * v[i].w; }
     }
     if (shared) {
         const float s = scalar ? scalar[t] : 1.0f;
@@ -365,7 +375,7 @@ static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with
         J.out_stride = stride; J.epi = epi;
     };
     if (with_router) {
-        // batches: the tiled fp64 GEMM (one pass over the router matrix per 16 tokens of a block, from shared memory)
+        // batches: the fp64 tensor-core kernel (6 tokens: 21 us with the GEMV of four tokens a pass)
         if (moe_router_tc(m, ntok)) {
             // opt-in: the logits as a split-fp16 product on the tcgen05 GEMM (see moe_router_tc)
             const uint32_t tn = tc_token_tile(ntok, tc_row_tiles(m->d.n_expert));
@@ -375,7 +385,7 @@ static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with
             T.wd = m->rt_wd; T.w_inv = m->rt_winv;
             T.job[0] = TcJob{m->router.base, 0u, RC_F32, m->d.n_expert, m->logits, m->d.n_expert, 0u};
             if (!launch_tc_gemm(T, tn, "moe_router_logits_tc", s)) return 0;
-        } else if (ntok >= 8u && m->router.type == RC_F32 && m->d.hidden % 64u == 0) {
+        } else if (ntok >= 2u && m->router.type == RC_F32) {
             if (!launch_router_logits((const float *)m->router.base, x, m->d.hidden, ntok, m->d.n_expert, m->d.hidden, m->logits, s)) return 0;
         } else add(m->router, nullptr, m->logits, m->d.n_expert, GEMV_STORE);
     }
