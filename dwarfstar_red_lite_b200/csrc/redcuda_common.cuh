@@ -61,17 +61,21 @@ __device__ __forceinline__ void pdl_prologue() {
     asm volatile("griddepcontrol.launch_dependents;" ::);
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// cluster_x: blocks along x that form a thread-block cluster (1: none)
 template <typename K, typename... Args>
-inline cudaError_t launch_kernel(int file_default, K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+inline cudaError_t launch_kernel(int file_default, uint32_t cluster_x, K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = (pdl_mode() < 0 ? file_default : pdl_mode()) ? 1 : 0;
-    cfg.attrs = at; cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster_x; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = cluster_x > 1u ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
-#define RC_LAUNCH(kernel, grid, block, smem, stream, ...) rc::launch_kernel(RC_PDL_DEFAULT, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)
+#define RC_LAUNCH(kernel, grid, block, smem, stream, ...) rc::launch_kernel(RC_PDL_DEFAULT, 1u, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)
+#define RC_LAUNCH_CLUSTER(cluster_x, kernel, grid, block, smem, stream, ...) rc::launch_kernel(RC_PDL_DEFAULT, cluster_x, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)
 #endif
 
 struct DevMem {

@@ -7,6 +7,7 @@
 //               registers, decayed, corrected and read out, then stored — one read and one write of the state,
 //               where the CPU path sweeps it four times
 //   k_dn_tail   per value head RMSNorm(core) * w * SiLU(z)
+//   k_dn_step   all three in one launch, the usual form: the kernels above serve state sizes and head ratios beyond it
 #include "redcuda_common.cuh"
 #include "redcuda_kernels.cuh"
 #include "redcuda_stage.cuh"
@@ -110,25 +111,36 @@ __global__ void k_dn_tail(DnDims D, const float *__restrict__ core, const float 
     out[idx] = x * inv * norm_w[i] * silu;
 }
 
-// Delta rule + gated RMSNorm of one value head in one block: grid (rank, batch), 8 warps, warp w owns the S / 8
-// consecutive state rows w * S / 8 ... Every lane first requests ALL of its rows (S / 8 rows x VPL floats: 64 registers
-// at S = 128), so a block has its whole 64 KB of state in flight at once — at batch 1 only `rank` blocks exist and each
-// must cover the memory latency by itself — then the rows are decayed, corrected, read out and stored one after the
-// other; q and k of the head are loaded once per lane instead of once per row. The head's S outputs meet in shared
-// memory, where the tail (k_dn_tail's arithmetic, unchanged) normalises and gates them: one launch less, and the
-// un-normalised outputs never travel through global memory.
-template <int VPL>
-__global__ void __launch_bounds__(256) k_dn_state_tail(DnDims D, const float *__restrict__ qk, const float *__restrict__ v,
-                                                       const float *__restrict__ beta, const float *__restrict__ gate, float *__restrict__ state,
-                                                       const float *__restrict__ z, const float *__restrict__ norm_w, float *__restrict__ out) {
+// The whole step of one value head in one block: grid (rank, batch), 8 warps, warp w owns the S / 8 consecutive state rows
+// w * S / 8 ... What bounds it is the state: one read and one write of 4 S^2 bytes per head (33.5 MB for 8 sequences of 32
+// heads of 128: 5.1 us at the copy rate). As separate kernels, preparation and state update took 13.7 us for them, because
+// the state was requested only after the preparation had ended. Here every lane first requests its conv windows and ALL
+// of its state rows (S / 8 rows x VPL floats: 64 registers at S = 128, the block's whole 64 KB in flight at once), and the
+// preparation (conv + SiLU, L2 norms, beta and gate: the arithmetic of k_dn_prep) runs while they arrive.
+// The value heads of one key head all need its q and k. Their blocks form a cluster: each computes q and k for itself, and
+// the first one moves the conv windows of the q / k channels on after all of them have read the old ones (cluster barrier).
+template <int VPL, uint32_t DC>            // DC: conv taps known at compile time (0: D.d_conv)
+__global__ void __launch_bounds__(256, 2) k_dn_step(DnDims D, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,
+                                                    const float *__restrict__ qkv, const float *__restrict__ ba, float *conv_state, float *__restrict__ state,
+                                                    const float *__restrict__ z, const float *__restrict__ norm_w, float *__restrict__ out) {
     pdl_prologue();
-    constexpr uint32_t S = VPL * 32u, RPW = S / 8u;
-    __shared__ float s_core[S];
-    __shared__ double red[8];
+    constexpr uint32_t S = VPL * 32u, RPW = S / 8u, TAPS = DC ? DC : 1u;
+    __shared__ float s_q[S], s_k[S], s_v[S], s_core[S], s_beta, s_gate;
+    __shared__ double red[8], red2[8];
     const uint32_t h = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t kh = h / (D.rank / D.groups);
-    const float *q = qk + ((size_t)seq * 2u * D.groups + kh) * S;
-    const float *k = qk + ((size_t)seq * 2u * D.groups + D.groups + kh) * S;
+    const uint32_t width = D.rank / D.groups, kh = h / width, first = h - kh * width == 0u, taps = DC ? DC : D.d_conv, ns = taps - 1u;
+    // conv channels of this thread: threads 0 .. S-1 the q channels, S .. 2S-1 the k channels of the key head; then 0 .. S-1 the head's v channels
+    const bool has_qk = tid < 2u * S, has_v = tid < S;
+    const uint32_t c_qk = (tid < S ? kh * S + tid : (D.groups + kh) * S + tid - S), c_v = 2u * D.groups * S + h * S + tid;
+    float *const cs_base = conv_state + (size_t)seq * D.channels * ns;
+    const float *const x_base = qkv + (size_t)seq * D.channels;
+    float wq[TAPS], kq[TAPS], wv[TAPS], kv_[TAPS];                 // window + new sample, and the taps
+    auto window = [&](uint32_t c, float (&w)[TAPS], float (&k)[TAPS]) {
+#pragma unroll
+        for (uint32_t j = 0; j < TAPS; ++j) { w[j] = j + 1u < TAPS ? cs_base[(size_t)c * ns + j] : x_base[c]; k[j] = conv_kernel[(size_t)c * taps + j]; }
+    };
+    if (DC && has_qk) window(c_qk, wq, kq);
+    if (DC && has_v) window(c_v, wv, kv_);
     float *rows = state + (((size_t)seq * D.rank + h) * S + (size_t)warp * RPW) * S;
     float m[RPW][VPL];
     // volatile asm keeps these loads where they are written: all of them are issued before the first row is worked on
@@ -138,18 +150,57 @@ __global__ void __launch_bounds__(256) k_dn_state_tail(DnDims D, const float *__
 #pragma unroll
         for (int t = 0; t < VPL; ++t) asm volatile("ld.global.f32 %0, [%1];" : "=f"(m[r][t]) : "l"(rows + (size_t)r * S + lane + 32 * t));
     __syncwarp();                      // a fixed point between the requests above and the shuffles below
+    auto conv_silu = [&](uint32_t c, const float (&w)[TAPS], const float (&k)[TAPS]) {
+        double acc = 0.0;
+        if (DC) {
+#pragma unroll
+            for (uint32_t j = 0; j < TAPS; ++j) acc += (double)w[j] * (double)k[j];
+        } else {
+            for (uint32_t j = 0; j < ns; ++j) acc += (double)cs_base[(size_t)c * ns + j] * (double)conv_kernel[(size_t)c * taps + j];
+            acc += (double)x_base[c] * (double)conv_kernel[(size_t)c * taps + ns];
+        }
+        return (float)(acc / (1.0 + exp(-acc)));
+    };
+    auto roll = [&](uint32_t c) {
+        float *cs = cs_base + (size_t)c * ns;
+        for (uint32_t j = 0; j + 1u < ns; ++j) cs[j] = cs[j + 1u];
+        cs[ns - 1u] = x_base[c];
+    };
+    const float y = has_qk ? conv_silu(c_qk, wq, kq) : 0.f;
+    __syncwarp();
+    if (width > 1u) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // this block has read the key head's windows
+    double ss = (double)y * (double)y;
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) red[warp] = ss;
+    if (has_v) { s_v[tid] = conv_silu(c_v, wv, kv_); roll(c_v); }
+    else if (tid == S || tid == S + 32u) {          // beta and gate: one thread each, in warps that have no v channels
+        const float *b = ba + (size_t)seq * 2u * D.rank + kh * 2u * width + (h - kh * width);
+        if (tid == S) s_beta = (float)sigmoid_stable((double)b[0]);
+        else s_gate = (float)(softplus_stable((double)b[width] + (double)dt_bias[h]) * (double)ssm_a[h]);
+    }
+    __syncthreads();
+    if (has_qk) {
+        const uint32_t w0 = tid < S ? 0u : S / 32u;
+        double tot = 0.0;
+        for (uint32_t w = 0; w < S / 32u; ++w) tot += red[w0 + w];
+        const double inv = 1.0 / fmax(sqrt(tot), (double)D.eps);
+        (tid < S ? s_q : s_k)[tid < S ? tid : tid - S] = (float)((double)y * inv);
+    }
+    __syncwarp();
+    if (width > 1u) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (first && has_qk) roll(c_qk);
+    __syncthreads();
     float qv[VPL], kv[VPL];
 #pragma unroll
-    for (int t = 0; t < VPL; ++t) { qv[t] = q[lane + 32 * t]; kv[t] = k[lane + 32 * t]; }
-    const float decay = expf(gate[(size_t)seq * D.rank + h]), bh = beta[(size_t)seq * D.rank + h], scale = 1.0f / sqrtf((float)S);
-    const float *vh = v + (size_t)seq * D.d_inner + (size_t)h * S + warp * RPW;
+    for (int t = 0; t < VPL; ++t) { qv[t] = s_q[lane + 32 * t]; kv[t] = s_k[lane + 32 * t]; }
+    const float decay = expf(s_gate), bh = s_beta, scale = 1.0f / sqrtf((float)S);
 #pragma unroll
     for (uint32_t r = 0; r < RPW; ++r) {
         float sum = 0.f;
 #pragma unroll
         for (int t = 0; t < VPL; ++t) { m[r][t] = m[r][t] * decay; sum += m[r][t] * kv[t]; }
         for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        const float delta = (vh[r] - sum) * bh;
+        const float delta = (s_v[warp * RPW + r] - sum) * bh;
         float o_acc = 0.f;
 #pragma unroll
         for (int t = 0; t < VPL; ++t) { m[r][t] += kv[t] * delta; o_acc += m[r][t] * qv[t]; rows[(size_t)r * S + lane + 32 * t] = m[r][t]; }
@@ -160,14 +211,14 @@ __global__ void __launch_bounds__(256) k_dn_state_tail(DnDims D, const float *__
     // gated RMSNorm over the head (the arithmetic of k_dn_tail)
     const size_t idx = (size_t)seq * D.d_inner + (size_t)h * S + tid;
     float x = 0.f, g = 0.f;
-    double ss = 0.0;
+    ss = 0.0;
     if (tid < S) { x = s_core[tid]; g = z[idx]; ss = (double)x * (double)x; }
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) red[warp] = ss;
+    if (lane == 0) red2[warp] = ss;
     __syncthreads();
     if (tid < S) {
         double tot = 0.0;
-        for (uint32_t w = 0; w < S / 32u; ++w) tot += red[w];
+        for (uint32_t w = 0; w < S / 32u; ++w) tot += red2[w];
         const float inv = 1.0f / sqrtf((float)(tot / (double)S) + D.eps);
         const float silu = g / (1.0f + expf(-g));
         out[idx] = x * inv * norm_w[tid] * silu;
@@ -787,28 +838,25 @@ int launch_deltanet(const DnDims &D, uint32_t batch, const float *conv_kernel, c
     RC_REQUIRE(D.rank && D.groups && D.rank % D.groups == 0 && D.d_inner == D.rank * D.S && D.channels == 2u * D.S * D.groups + D.d_inner && D.d_conv >= 2u,
                "deltanet: inconsistent dimensions");
     if (!batch) return 1;
+    // one launch where a head's state fits the registers of a block and the value heads of a key head fit a cluster; else three
+    const uint32_t width = D.rank / D.groups;
+    if (D.S <= 128u && width <= 8u) {
+        prof_begin("dn_step", s);
+        const dim3 gs(D.rank, batch);
+#define RC_DN_STEP(VPL, DC) RC_LAUNCH_CLUSTER(width, (k_dn_step<VPL, DC>), gs, 256, 0, s, D, conv_kernel, dt_bias, ssm_a, qkv, ba, conv_state, rec_state, z, norm_w, out)
+        if (D.S == 32u) { if (D.d_conv == 4u) RC_DN_STEP(1, 4u); else RC_DN_STEP(1, 0u); }
+        else if (D.S == 64u) { if (D.d_conv == 4u) RC_DN_STEP(2, 4u); else RC_DN_STEP(2, 0u); }
+        else { if (D.d_conv == 4u) RC_DN_STEP(4, 4u); else RC_DN_STEP(4, 0u); }
+#undef RC_DN_STEP
+        prof_end(s);
+        RC_LAUNCHED();
+        return 1;
+    }
     const dim3 gp(2u * D.groups + D.d_inner / D.S + 1u, batch);
     prof_begin("dn_prep", s);
     RC_LAUNCH((k_dn_prep), gp, D.S, 0, s, D, conv_kernel, dt_bias, ssm_a, qkv, ba, conv_state, qk, v, beta, gate);
     prof_end(s);
     RC_LAUNCHED();
-    // One block per (head, sequence) for state update + tail. Measured (16/32 heads of 128): batch 8 12.8 us against 16.5 us
-    // for the two-kernel form; a single sequence fills only 32 SMs that way and stays on the two-kernel form (7.3 against
-    // 7.9 us). RC_DN_FUSE=0 / 1 forces one or the other.
-    static const int fuse_env = getenv("RC_DN_FUSE") ? atoi(getenv("RC_DN_FUSE")) : -1;
-    const bool fuse = fuse_env < 0 ? batch >= 2u : fuse_env != 0;
-    if (fuse && D.S <= 128u) {
-        prof_begin("dn_state_tail", s);
-        const dim3 gs(D.rank, batch);
-        switch (D.S) {
-            case 32: RC_LAUNCH((k_dn_state_tail<1>), gs, 256, 0, s, D, qk, v, beta, gate, rec_state, z, norm_w, out); break;
-            case 64: RC_LAUNCH((k_dn_state_tail<2>), gs, 256, 0, s, D, qk, v, beta, gate, rec_state, z, norm_w, out); break;
-            default: RC_LAUNCH((k_dn_state_tail<4>), gs, 256, 0, s, D, qk, v, beta, gate, rec_state, z, norm_w, out); break;
-        }
-        prof_end(s);
-        RC_LAUNCHED();
-        return 1;
-    }
     prof_begin("dn_state", s);
     const uint64_t warps = (uint64_t)batch * D.rank * D.S;
     const uint32_t blocks = (uint32_t)((warps + 7u) / 8u);
