@@ -1,0 +1,245 @@
+// Single-token matrix-vector products (F32 / F16 / Q6_K rows): the dense projections, the LM head, the router logits with
+// the shared expert's gate / up and scalar gate of a decode step.
+//
+// What bounds it: HBM for the large matrices, the length of the dependent chain for the small ones. The general GEMV
+// (redcuda_core.cu) staged x in shared memory behind a barrier and read it back 16 bytes per four weights, turned every
+// 6-bit weight into a float with a conversion, and began a row's loads only after the previous row's sums. Here
+//   - a warp takes two rows of a 2048-column slice at a time, so that every 16 bytes of x read from shared memory serve both
+//     (x in registers instead, one row at a time, left 16 warps an SM: 80 us for a 151936 x 2048 matrix);
+//   - a 6-bit weight becomes a float by a byte permute into the mantissa of 2^23 and a packed subtraction, and two
+//     weights are multiplied by one packed FMA: 2.7 instructions a weight instead of about 5;
+//   - the first rows of resident weights are requested before the wait for the previous kernel (they do not depend on it);
+//   - rows wider than a slice are cut over the warps of the block, partial sums meet in shared memory in a fixed order.
+// Plain rows (router, scalar gate) are accumulated in double, as everywhere: they decide discrete outcomes.
+#include "redcuda_common.cuh"
+#include "redcuda_kernels.cuh"
+#include "redcuda_route.cuh"
+
+namespace rc {
+
+namespace {
+constexpr uint32_t G1_WARPS = 8u, G1_QCOLS = 2048u, G1_PCOLS = 512u;      // columns of one warp's slice: Q6_K, plain
+__host__ __device__ inline uint32_t g1_slices(uint32_t type, uint32_t ncols) { const uint32_t c = type == RC_Q6_K ? G1_QCOLS : G1_PCOLS; return (ncols + c - 1u) / c; }
+// warps that take different slices of the same rows; a slice count that does not divide the warps is walked by every warp
+__host__ __device__ inline uint32_t g1_slice_warps(uint32_t slices) { return slices <= G1_WARPS && G1_WARPS % slices == 0u ? slices : 1u; }
+// lanes per Q6_K row: the chunks of 64 columns of a short row, rounded up to a power of two
+__host__ __device__ inline uint32_t g1_lanes(uint32_t type, uint32_t ncols) {
+    if (type != RC_Q6_K) return 32u;
+    uint32_t l = 4u;
+    while (l < 32u && l < (ncols >> 6)) l <<= 1;
+    return l;
+}
+}  // namespace
+
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ uint64_t f2_pack(uint32_t lo, uint32_t hi) { return (uint64_t)lo | ((uint64_t)hi << 32); }
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+
+struct Q6Frag { uint4 a, b, h; uint2 sc; unsigned short d; };
+struct G1Tile { uint32_t row0, nvr, pair; bool resident; };      // nvr: rows of the tile, counted twice (w0, w1 in turn) for a gate / up pair
+
+// where column k of x sits in shared memory: eight lanes that read their 16 bytes of neighbouring chunks (k = 0, 16, 128, 144 of
+// two blocks) hit eight different bank groups
+__host__ __device__ __forceinline__ uint32_t g1_xi(uint32_t k) { return (k >> 8) * 268u + ((k >> 7) & 1u) * 136u + (k & 127u); }
+
+__device__ __forceinline__ void gemv1_q6k(const GemvJob &J, const G1Tile &T, const float *x, double *part, float *xs) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t cpr = J.ncols >> 6, bpr = J.ncols >> 8, S = g1_slices(RC_Q6_K, J.ncols), ws = g1_slice_warps(S), lpr = g1_lanes(RC_Q6_K, J.ncols), rw = 32u / lpr;
+    const uint32_t slot = lane / lpr, sub = lane % lpr, step = (G1_WARPS / ws) * rw, first = (warp / ws) * rw;
+    const uint64_t o_h = rc_q6_qh(J.nb), o_s = rc_q6_sc(J.nb), o_d = rc_q6_d(J.nb);
+    const uint64_t bias = f2_pack(__float_as_uint(-8388640.0f), __float_as_uint(-8388640.0f));      // 2^23 + 32
+    bool staged = false;
+    for (uint32_t sl = warp % ws; sl < S; sl += ws) {
+        const uint32_t c = sl * (G1_QCOLS / 64u) + sub;
+        const bool on = c < cpr;                                  // lanes past the row's end repeat its last chunk and add nothing
+        const uint32_t cc = on ? c : cpr - 1u, bcol = cc >> 2, half = (cc >> 1) & 1u, l0 = (cc & 1u) * 16u;
+        auto load = [&](uint32_t vr) {
+            vr = min(vr, T.nvr - 1u);
+            const uint8_t *w = T.pair && (vr & 1u) ? J.w1 : J.w0;
+            const uint64_t blk = (uint64_t)(T.row0 + (vr >> T.pair)) * bpr + bcol;
+            const uint8_t *wl = w + blk * 128u + half * 64u + l0;
+            Q6Frag f;
+            f.a = __ldg(reinterpret_cast<const uint4 *>(wl));
+            f.b = __ldg(reinterpret_cast<const uint4 *>(wl + 32u));
+            f.h = __ldg(reinterpret_cast<const uint4 *>(w + o_h + blk * 64u + half * 32u + l0));
+            f.sc = __ldg(reinterpret_cast<const uint2 *>(w + o_s + blk * 16u + half * 8u));
+            f.d = __ldg(reinterpret_cast<const unsigned short *>(w + o_d) + blk);
+            return f;
+        };
+        // two rows at a time: each 16 bytes of x read from shared memory serve both
+        Q6Frag f[2];
+        if (T.resident || staged) { f[0] = load(first + slot); f[1] = load(first + step + slot); }
+        if (!staged) {
+            staged = true;
+            pdl_wait();
+            for (uint32_t k = threadIdx.x * 4u; k < J.ncols; k += G1_WARPS * 128u) *reinterpret_cast<float4 *>(xs + g1_xi(k)) = *reinterpret_cast<const float4 *>(x + k);
+            if (!T.resident) { f[0] = load(first + slot); f[1] = load(first + step + slot); }
+            __syncthreads();
+        }
+        const float *xl = xs + bcol * 268u + half * 136u + l0;
+        for (uint32_t base = first; base < T.nvr; base += 2u * step) {
+            uint64_t s[2][4] = {{0u, 0u, 0u, 0u}, {0u, 0u, 0u, 0u}};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                uint32_t v[2][4];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const uint32_t a = w == 0 ? f[r].a.x : w == 1 ? f[r].a.y : w == 2 ? f[r].a.z : f[r].a.w, b = w == 0 ? f[r].b.x : w == 1 ? f[r].b.y : w == 2 ? f[r].b.z : f[r].b.w;
+                    const uint32_t h = w == 0 ? f[r].h.x : w == 1 ? f[r].h.y : w == 2 ? f[r].h.z : f[r].h.w;
+                    v[r][0] = (a & 0x0F0F0F0Fu) | ((h << 4) & 0x30303030u); v[r][1] = (b & 0x0F0F0F0Fu) | ((h << 2) & 0x30303030u);
+                    v[r][2] = ((a >> 4) & 0x0F0F0F0Fu) | (h & 0x30303030u); v[r][3] = ((b >> 4) & 0x0F0F0F0Fu) | ((h >> 2) & 0x30303030u);
+                }
+#pragma unroll
+                for (int qd = 0; qd < 4; ++qd) {
+                    const uint32_t m = 0x4B000000u;
+                    const ulonglong2 xv = *reinterpret_cast<const ulonglong2 *>(xl + 32u * qd + 4u * w);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const uint64_t w01 = f2_add(f2_pack(__byte_perm(v[r][qd], m, 0x7540), __byte_perm(v[r][qd], m, 0x7541)), bias);
+                        const uint64_t w23 = f2_add(f2_pack(__byte_perm(v[r][qd], m, 0x7542), __byte_perm(v[r][qd], m, 0x7543)), bias);
+                        s[r][qd] = f2_fma(w01, xv.x, s[r][qd]);
+                        s[r][qd] = f2_fma(w23, xv.y, s[r][qd]);
+                    }
+                }
+            }
+            float acc[2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float d = __half2float(__ushort_as_half(f[r].d));
+                // the four scales of this lane's runs of 16 sit in every other byte of its half block
+                const uint32_t q = l0 ? 8u : 0u;
+                const int sc[4] = {(int)(signed char)(f[r].sc.x >> q), (int)(signed char)(f[r].sc.x >> (q + 16u)), (int)(signed char)(f[r].sc.y >> q), (int)(signed char)(f[r].sc.y >> (q + 16u))};
+                acc[r] = 0.f;
+#pragma unroll
+                for (int qd = 0; qd < 4; ++qd) acc[r] += (d * (float)sc[qd]) * (__uint_as_float((uint32_t)s[r][qd]) + __uint_as_float((uint32_t)(s[r][qd] >> 32)));
+                if (!on) acc[r] = 0.f;
+            }
+            if (base + 2u * step < T.nvr) { f[0] = load(base + 2u * step + slot); f[1] = load(base + 3u * step + slot); }      // on the way during the reduction
+            for (uint32_t o = lpr >> 1; o; o >>= 1) { acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o); acc[1] += __shfl_xor_sync(0xffffffffu, acc[1], o); }
+            if (sub == 0u) {
+                if (base + slot < T.nvr) part[(base + slot) * S + sl] = (double)acc[0];
+                if (base + step + slot < T.nvr) part[(base + step + slot) * S + sl] = (double)acc[1];
+            }
+        }
+    }
+}
+
+template <bool HALF>
+__device__ __forceinline__ void gemv1_plain(const GemvJob &J, const G1Tile &T, const float *x, double *part) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t S = g1_slices(RC_F32, J.ncols), ws = g1_slice_warps(S), step = G1_WARPS / ws;
+    bool waited = false;
+    for (uint32_t sl = warp % ws; sl < S; sl += ws) {
+        const uint32_t k0 = sl * G1_PCOLS + lane * 4u;
+        float4 w[4], xv[4];
+        auto load = [&](uint32_t vr) {
+            const uint8_t *m = T.pair && (vr & 1u) ? J.w1 : J.w0;
+            const size_t row = (size_t)(T.row0 + (vr >> T.pair)) * J.ncols;
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i) {
+                const uint32_t k = k0 + 128u * i;
+                if (k >= J.ncols) { w[i] = make_float4(0.f, 0.f, 0.f, 0.f); continue; }
+                if (HALF) {
+                    const uint2 r = __ldg(reinterpret_cast<const uint2 *>(m + (row + k) * 2u));
+                    const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&r.x)), hi = __half22float2(*reinterpret_cast<const __half2 *>(&r.y));
+                    w[i] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                } else w[i] = __ldg(reinterpret_cast<const float4 *>(m + (row + k) * 4u));
+            }
+        };
+        uint32_t vr = warp / ws;
+        if (T.resident && vr < T.nvr) load(vr);
+        if (!waited) { pdl_wait(); waited = true; }
+        if (!T.resident && vr < T.nvr) load(vr);
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; ++i) {
+            const uint32_t k = k0 + 128u * i;
+            xv[i] = k < J.ncols ? *reinterpret_cast<const float4 *>(x + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        for (; vr < T.nvr; vr += step) {
+            double a0 = 0.0, a1 = 0.0;                    // two chains: the double FMA's latency is what a short row waits for
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i) {
+                a0 = fma((double)w[i].x, (double)xv[i].x, a0); a1 = fma((double)w[i].y, (double)xv[i].y, a1);
+                a0 = fma((double)w[i].z, (double)xv[i].z, a0); a1 = fma((double)w[i].w, (double)xv[i].w, a1);
+            }
+            if (vr + step < T.nvr) load(vr + step);
+            double acc = a0 + a1;
+            for (uint32_t o = 16u; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0u) part[vr * S + sl] = acc;
+        }
+    }
+    if (!waited) pdl_wait();
+}
+
+__global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1(const __grid_constant__ GemvArgs A) {
+    pdl_trigger();
+    extern __shared__ __align__(16) double g1_part[];      // [row of the tile (x 2 for a pair)][slice], behind it x
+    uint32_t j = 0;
+    while (j + 1u < A.njobs && blockIdx.x >= A.job[j + 1u].tile_begin) ++j;
+    const GemvJob &J = A.job[j];
+    const uint32_t row0 = (blockIdx.x - J.tile_begin) * J.rows_per_tile, nrow = min(J.rows_per_tile, J.nrows - row0), pair = J.epi == GEMV_PAIR_SILU ? 1u : 0u;
+    const G1Tile T{row0, nrow << pair, pair, A.resident != 0u};
+    if (J.type == RC_Q6_K) gemv1_q6k(J, T, A.x, g1_part, reinterpret_cast<float *>(g1_part + A.part_doubles));
+    else if (J.type == RC_F32) gemv1_plain<false>(J, T, A.x, g1_part);
+    else gemv1_plain<true>(J, T, A.x, g1_part);
+    __syncthreads();
+    const uint32_t S = g1_slices(J.type, J.ncols);
+    for (uint32_t r = threadIdx.x; r < nrow; r += G1_WARPS * 32u) {
+        const double *p = g1_part + (size_t)(r << pair) * S;
+        double s0 = 0.0, s1 = 0.0;
+        for (uint32_t i = 0; i < S; ++i) { s0 += p[i]; if (pair) s1 += p[S + i]; }
+        float v = (float)s0;
+        if (pair) v = (v / (1.0f + expf(-v))) * (float)s1;
+        else if (J.epi == GEMV_SIGMOID) v = 1.0f / (1.0f + expf(-v));
+        J.out[row0 + r] = v;
+    }
+    if (A.tail.ticket) route_tail(A.tail);
+}
+
+// One token and rows that k_gemv1 holds; the other block types stay with the general kernel.
+bool gemv1_ok(const GemvArgs &A) {
+    if (A.ntok != 1u || ((uintptr_t)A.x & 15u)) return false;
+    for (uint32_t j = 0; j < A.njobs; ++j) {
+        const uint32_t t = A.job[j].type;
+        if (t != RC_F32 && t != RC_F16 && t != RC_Q6_K) return false;
+        if (A.job[j].ncols > 8192u) return false;          // x in shared memory without the opt-in size
+    }
+    return true;
+}
+
+int launch_gemv1(GemvArgs &A, cudaStream_t stream) {
+    // Tiles of about equal bytes, three per SM (what the registers let reside), so that a launch is one wave whatever its jobs;
+    // at least one row per warp of the block, at most what 8 KB of partial sums hold.
+    uint64_t total = 0;
+    for (uint32_t j = 0; j < A.njobs; ++j) total += rc_matrix_bytes(A.job[j].type, A.job[j].nrows, A.job[j].ncols) << (A.job[j].epi == GEMV_PAIR_SILU ? 1 : 0);
+    const uint64_t target = (total + 443u) / 444u;
+    uint32_t tiles = 0;
+    size_t smem = 16u;
+    bool q6 = false;
+    for (uint32_t j = 0; j < A.njobs; ++j) {
+        GemvJob &J = A.job[j];
+        const uint32_t pair = J.epi == GEMV_PAIR_SILU ? 1u : 0u, S = g1_slices(J.type, J.ncols);
+        const uint32_t pass = G1_WARPS / g1_slice_warps(S) * (32u / g1_lanes(J.type, J.ncols)), grain = pass >> pair ? pass >> pair : 1u;
+        const uint64_t row = rc_row_bytes(J.type, J.ncols) << pair;
+        uint64_t rows = ((target + row - 1u) / row + grain - 1u) / grain * grain;
+        const uint32_t cap = 1024u / (S << pair);
+        if (rows > cap) rows = cap;
+        J.rows_per_tile = (uint32_t)rows;
+        J.tile_begin = tiles;
+        tiles += (J.nrows + J.rows_per_tile - 1u) / J.rows_per_tile;
+        const size_t need = (size_t)(J.rows_per_tile < J.nrows ? J.rows_per_tile : J.nrows) * (S << pair) * sizeof(double);
+        if (need > smem) smem = (need + 15u) / 16u * 16u;
+        q6 = q6 || J.type == RC_Q6_K;
+    }
+    A.part_doubles = (uint32_t)(smem / sizeof(double));
+    if (q6) smem += (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + 16u;
+    prof_begin(A.tag ? A.tag : "gemv", stream);
+    RC_LAUNCH((k_gemv1), tiles, G1_WARPS * 32u, smem, stream, A);
+    prof_end(stream);
+    RC_LAUNCHED();
+    return 1;
+}
+
+}  // namespace rc

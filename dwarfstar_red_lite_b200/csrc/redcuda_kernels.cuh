@@ -43,9 +43,13 @@ struct GemvArgs {
     const uint32_t *iq3s;
     const char *tag;           // name under which the launch is timed when profiling is on (host side only)
     RouteTail tail;
+    uint32_t part_doubles;     // filled by launch_gemv1
+    uint32_t resident;         // 1: the weights were in place before the stream's previous kernel began (they may be requested ahead of it)
 };
 
 int launch_gemv(GemvArgs &A, cudaStream_t stream);
+bool gemv1_ok(const GemvArgs &A);                            // single-token form (redcuda_gemv1.cu), taken by launch_gemv
+int launch_gemv1(GemvArgs &A, cudaStream_t stream);
 // group1 (ntok == 1 only, may be null): fill the grouping arrays in the same kernel; ids_mirror (may be null) gets a copy of the ids
 int launch_route(const float *logits_dev, uint32_t ntok, uint32_t n_expert, uint32_t top_k, uint32_t *ids_dev, float *weights_dev,
                  float *probs_dev, cudaStream_t stream, const RouteGroup1 *group1 = nullptr);

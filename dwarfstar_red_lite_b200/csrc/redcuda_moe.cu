@@ -367,7 +367,7 @@ static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with
                         const int8_t *xq = nullptr, const float *sx = nullptr, const RouteTail *tail = nullptr) {
     if (!xq) { xq = m->xq_x; sx = m->sx_x; }
     GemvArgs A{};
-    A.ntok = ntok; A.x = x; A.x_stride = m->d.hidden;
+    A.ntok = ntok; A.x = x; A.x_stride = m->d.hidden; A.resident = 1u;
     uint32_t j = 0;
     auto add = [&](const DMat &w0, const DMat *w1, float *out, uint32_t stride, uint32_t epi) {
         GemvJob &J = A.job[j++];
@@ -415,7 +415,7 @@ static int moe_shared_down(redcuda_moe *m, uint32_t ntok, cudaStream_t s) {
                               "moe_shared_down_mma", s);
     }
     GemvArgs A{};
-    A.ntok = ntok; A.x = m->sh_act; A.x_stride = m->d.ffn_sh; A.njobs = 1;
+    A.ntok = ntok; A.x = m->sh_act; A.x_stride = m->d.ffn_sh; A.njobs = 1; A.resident = 1u;
     GemvJob &J = A.job[0];
     J.w0 = m->sh_down.base; J.out = m->sh_out; J.nb = m->sh_down.nb; J.type = m->sh_down.type; J.nrows = m->sh_down.nrows; J.ncols = m->sh_down.ncols;
     J.out_stride = m->d.hidden; J.epi = GEMV_STORE;
