@@ -75,6 +75,7 @@ inline cudaError_t launch_kernel(int file_default, uint32_t cluster_x, K kernel,
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 #define RC_LAUNCH(kernel, grid, block, smem, stream, ...) rc::launch_kernel(RC_PDL_DEFAULT, 1u, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)
+#define RC_LAUNCH_PDL(kernel, grid, block, smem, stream, ...) rc::launch_kernel(1, 1u, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)      // whatever the file's default
 #define RC_LAUNCH_CLUSTER(cluster_x, kernel, grid, block, smem, stream, ...) rc::launch_kernel(RC_PDL_DEFAULT, cluster_x, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)
 #endif
 

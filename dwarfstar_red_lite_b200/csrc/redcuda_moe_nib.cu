@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr uint32_t BPR = NCOLS / 256u, TPW = BPR >= 8u ? 1u : 8u / BPR, WSLOTS = GATEUP ? 4u : 8u, UNIT_TILES = WSLOTS * TPW;
     constexpr uint32_t BPITCH = NCOLS + 32u, V16 = NCOLS / 16u;
+    constexpr bool ONE = STAGES == NIB_STAGES_ONE;        // the form of a single token: A.x_raw holds it
     __shared__ uint32_t s_unit[2];
     __shared__ volatile uint32_t s_fail;
     __shared__ __align__(8) uint64_t s_bar[NIB_WARPS][STAGES];
@@ -321,25 +322,39 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
 
     auto decode = [&](uint32_t unit, NibUnit &I) {
         const uint32_t item = unit / U, rb = unit - item * U;
-        const uint32_t u = A.item_u[item], p0 = A.item_p0[item];
-        uint32_t e = A.uexp[u] - A.expert_begin, nt = min(A.item_tok, A.ustart[u + 1u] - p0);
+        uint32_t e, nt;
+        if (ONE) { e = A.uexp[item] - A.expert_begin; nt = 1u; I.p0 = item; }       // single token: item = group = pair
+        else {
+            const uint32_t u = A.item_u[item], p0 = A.item_p0[item];
+            e = A.uexp[u] - A.expert_begin; nt = min(A.item_tok, A.ustart[u + 1u] - p0);
+            I.p0 = p0;
+        }
         if (e >= A.n_local) { if (A.status && tid == 0) A.status[ST_EXPERT_RANGE] = 1u; e = 0u; nt = 0u; }     // never index the arena with a foreign id
-        I.item = item; I.p0 = p0; I.nt = nt;
+        I.item = item; I.nt = nt;
         I.tile0 = rb * UNIT_TILES + wslot * TPW;
         const uint32_t tiles = I.tile0 >= ntile_rows ? 0u : min(TPW, ntile_rows - I.tile0);
         I.n = nt ? tiles * BPR : 0u;
         I.rec = wmat + (size_t)e * A.mat_bytes + (size_t)I.tile0 * BPR * NIB_REC;
     };
 
-    if (tid == 0) { s_unit[0] = atomicAdd(A.work, 1u); s_fail = 0u; }
+    // the units of a single token are few and equal: block b takes b, b + grid, ..., which saves the counter's round trip
+    if (tid == 0) { s_unit[0] = ONE ? blockIdx.x : atomicAdd(A.work, 1u); s_fail = 0u; }
     if (lane == 0) {
         for (uint32_t i = 0; i < STAGES; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(R.bar_s + 8u * i));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
+    uint32_t cur = s_unit[0], par = 0u, cur_item = 0xffffffffu;
+    uint32_t ahead = 0u;             // records of the CURRENT unit already requested (while the previous unit was multiplying)
+    NibUnit I{}, N{};
+    if (cur < total) decode(cur, I);
+    if (ONE) {                   // the first records are on their way while the block quantises the token
+        R.cur_src = I.rec; R.cur_rem = I.n;
+        while (ahead + 1u < STAGES && ahead < I.n) { nib_request<STAGES>(R, lane); ++ahead; }
+    }
     __shared__ float s_red[NIB_WARPS], s_sx;
-    if (A.x_raw) {
+    if (ONE) {
         // single token: every unit multiplies the same activation row, so the block turns it into digits itself (the
         // arithmetic of k_quant_act) — columns 0..2 of the one tile in use, columns 3..7 zero
         float mx = 0.f;
@@ -372,19 +387,15 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
         }
         __syncthreads();
     }
-    uint32_t cur = s_unit[0], par = 0u, cur_item = 0xffffffffu;
-    uint32_t ahead = 0u;             // records of the CURRENT unit already requested (while the previous unit was multiplying)
     int zero[4];                     // opaque to the compiler: four registers that stay zero, the accumulator input of every MMA
     asm volatile("mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;" : "=r"(zero[0]), "=r"(zero[1]), "=r"(zero[2]), "=r"(zero[3]));
-    NibUnit I{}, N{};
-    if (cur < total) decode(cur, I);
     while (cur < total) {
-        if (tid == 0) s_unit[par ^ 1u] = atomicAdd(A.work, 1u);
+        if (tid == 0) s_unit[par ^ 1u] = ONE ? cur + gridDim.x : atomicAdd(A.work, 1u);
         // this unit's stream; STAGES - 1 of its records are put in flight before the first read
         R.cur_src = I.rec + (size_t)ahead * NIB_REC; R.cur_rem = I.n - ahead; R.nxt_rem = 0u; R.nxt_taken = 0u;
         for (uint32_t i = ahead; i + 1u < STAGES; ++i) nib_request<STAGES>(R, lane);
         const bool packed = I.nt <= 2u;
-        if (!A.x_raw && I.item != cur_item) {    // activation digits of the item (every warp passed the barrier that ended the last unit)
+        if (!ONE && I.item != cur_item) {    // activation digits of the item (every warp passed the barrier that ended the last unit)
             const uint32_t ncolb = packed ? 8u : 24u;
             for (uint32_t i = tid; i < ncolb * V16; i += NIB_WARPS * 32u) {
                 const uint32_t col = i / V16, k = (i - col * V16) << 4;
@@ -403,7 +414,7 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
         for (uint32_t j = 0; j < 2u; ++j) {
             const uint32_t tk = packed ? (t >> 1) : 2u * t + j;
             ok[j] = packed ? (j == 0u && (t & 1u) == 0u && tk < I.nt) : tk < I.nt;
-            if (ok[j]) { prow[j] = A.sorted[I.p0 + tk]; sxv[j] = A.x_raw ? s_sx : A.sx[prow[j] / A.x_div]; }
+            if (ok[j]) { prow[j] = ONE ? I.p0 : A.sorted[I.p0 + tk]; sxv[j] = ONE ? s_sx : A.sx[prow[j] / A.x_div]; }
         }
         __syncthreads();             // digits and the next unit's number are in shared memory
         const uint32_t nxt = s_unit[par ^ 1u];
@@ -470,28 +481,30 @@ __global__ void __launch_bounds__((NIB_TAIL_MAX_K + 2u) * 32u) k_nib_down_tail(c
     float *xs = reinterpret_cast<float *>(zrow + BPITCH);                    // shared expert's activation, padded rows of redcuda_dot.cuh
     const uint32_t row0 = blockIdx.x * 16u;
 
-    for (uint32_t k = tid * 4u; k < BPITCH; k += blockDim.x * 4u) *reinterpret_cast<uint32_t *>(zrow + k) = 0u;
-    if (A.sh_down) for (uint32_t k = tid * 4u; k < NCOLS; k += blockDim.x * 4u) *reinterpret_cast<float4 *>(xs + xi(k)) = *reinterpret_cast<const float4 *>(A.sh_act + k);
-    if (tid < 16u) s_sh[tid] = 0.f;
-    if (warp < K && lane == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(nb_smem(&s_bar[warp])));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    __syncthreads();
+    // the warp's records are requested before anything else: the expert's id is the only thing they wait for
+    bool live = true;
+    uint8_t *my_rec = recs + warp * BPR * NIB_REC;
+    const uint32_t bar = nb_smem(&s_bar[warp < K ? warp : 0u]);
     if (warp < K) {
         uint32_t e = A.ids[warp] - A.expert_begin;
-        bool live = true;
         if (e >= A.n_local) { if (A.status && lane == 0) A.status[ST_EXPERT_RANGE] = 1u; e = 0u; live = false; }      // never index the arena with a foreign id
-        uint8_t *my_rec = recs + warp * BPR * NIB_REC;
-        const uint32_t bar = nb_smem(&s_bar[warp]);
         if (lane == 0) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar));
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             const uint8_t *src = A.w_down + (size_t)e * A.mat_bytes + (size_t)blockIdx.x * BPR * NIB_REC;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(BPR * NIB_REC) : "memory");
             for (uint32_t c = 0; c < BPR; ++c)
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                              :: "r"(nb_smem(my_rec + c * NIB_REC)), "l"(src + (size_t)c * NIB_REC), "r"(NIB_REC), "r"(bar) : "memory");
         }
+        __syncwarp();
+    }
+    for (uint32_t k = tid * 4u; k < BPITCH; k += blockDim.x * 4u) *reinterpret_cast<uint32_t *>(zrow + k) = 0u;
+    if (A.sh_down) for (uint32_t k = tid * 4u; k < NCOLS; k += blockDim.x * 4u) *reinterpret_cast<float4 *>(xs + xi(k)) = *reinterpret_cast<const float4 *>(A.sh_act + k);
+    if (tid < 16u) s_sh[tid] = 0.f;
+    __syncthreads();
+    if (warp < K) {
         // this expert's activation row -> digits (the arithmetic of k_quant_act), while the records are in flight
         const float *ar = A.act + (size_t)warp * A.act_stride;
         float v[PER_LANE];
@@ -568,6 +581,8 @@ int launch_nib_down_tail(NibTailArgs &A, cudaStream_t s) {
     const uint32_t bpr = A.ncols / 256u, bpitch = A.ncols + 32u;
     const size_t smem = (size_t)A.top_k * bpr * NIB_REC + (size_t)A.top_k * 3u * bpitch + bpitch + (size_t)x_padded(A.ncols) * 4u + 16u;
     const uint32_t threads = (A.top_k + 2u) * 32u, grid = A.nrows / 16u;
+    // launched plainly: ahead of time its blocks would gather on the SMs that the 80 gate / up blocks of a top-10 layer leave free
+    // (28.9 against 26.7 us a layer)
     prof_begin("moe_down_tail", s);
 #define RC_TAIL_LAUNCH(NC) do { \
         RC_CUDA(cudaFuncSetAttribute(k_nib_down_tail<FMT, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
@@ -598,14 +613,17 @@ int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s) {
     if (!sm_count) { int dev = 0; RC_CUDA(cudaGetDevice(&dev)); RC_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev)); }
     const uint32_t bpr = A.ncols / 256u, tpw = bpr >= 8u ? 1u : 8u / bpr, unit_tiles = (gateup ? 4u : 8u) * tpw;
     const uint64_t units = (uint64_t)max_items * ((A.nrows / 16u + unit_tiles - 1u) / unit_tiles);
-    const bool one = A.x_raw != nullptr;          // single token: deep rings, one block per SM
+    // single token: deep rings, one block per SM, and launched ahead of the previous kernel's end (a batch's blocks, two per SM for
+    // the whole launch, measured slower that way: a layer of 24 tokens 127 us against 119)
+    const bool one = A.x_raw != nullptr;
     const uint32_t per_sm = one ? 1u : 2u, stages = one ? NIB_STAGES_ONE : NIB_STAGES_BATCH;
     const uint32_t grid = (uint32_t)(units < per_sm * (uint64_t)sm_count ? (units ? units : 1u) : per_sm * (uint64_t)sm_count);
     const size_t smem = nib_smem_bytes(A.ncols, stages);
     prof_begin(gateup ? "moe_gateup" : "moe_down", s);
 #define RC_NIB_LAUNCH(GU, NC, ST) do { \
         RC_CUDA(cudaFuncSetAttribute(k_nib_experts<FMT, GU, NC, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        RC_LAUNCH((k_nib_experts<FMT, GU, NC, ST>), grid, NIB_WARPS * 32u, smem, s, A); } while (0)
+        if (one) RC_LAUNCH_PDL((k_nib_experts<FMT, GU, NC, ST>), grid, NIB_WARPS * 32u, smem, s, A); \
+        else RC_LAUNCH((k_nib_experts<FMT, GU, NC, ST>), grid, NIB_WARPS * 32u, smem, s, A); } while (0)
     auto launch = [&](auto fmt) -> int {
     constexpr uint32_t FMT = decltype(fmt)::value;
     if (one) {

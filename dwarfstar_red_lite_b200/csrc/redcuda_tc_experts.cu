@@ -61,37 +61,57 @@ __device__ __forceinline__ uint4 tcx_decode8(uint32_t word, uint32_t sc) {
 }
 
 // v[r][k] (optionally SiLU(a) * b) -> two fp16 digits per value, rows kept row-major: xd[r][digit][ncols]; x_inv[r]
-// undoes the row's power-of-two scale. grid = rows, block = 256
-__global__ void __launch_bounds__(256) k_tc_prep_rows(const float *__restrict__ a, const float *__restrict__ b, uint32_t stride, uint32_t ncols,
+// undoes the row's power-of-two scale. A warp per row, the row in its registers (8 values a lane and step of 256 columns):
+// the memory is what bounds it, and a block per row (two passes, 64 of 256 threads busy in the second) took 58 us where
+// 20480 rows of 512 move 126 MB. grid = rows / 8, block = 256; ncols a multiple of 256, at most 256 NCH
+template <uint32_t NCH>
+__global__ void __launch_bounds__(256) k_tc_prep_rows(const float *__restrict__ a, const float *__restrict__ b, uint32_t stride, uint32_t nrows, uint32_t ncols,
                                                       __half *__restrict__ xd, float *__restrict__ x_inv) {
     pdl_prologue();
-    __shared__ float red[8];
-    const uint32_t r = blockIdx.x, tid = threadIdx.x;
+    const uint32_t r = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (r >= nrows) return;
     const float *ar = a + (size_t)r * stride, *br = b ? b + (size_t)r * stride : nullptr;
+    float v[NCH][8];
     float mx = 0.f;
-    for (uint32_t k = tid; k < ncols; k += 256u) mx = fmaxf(mx, fabsf(br ? silu_mul(ar[k], br[k]) : ar[k]));
+#pragma unroll
+    for (uint32_t i = 0; i < NCH; ++i) {
+        const uint32_t k = i * 256u + lane * 8u;
+        if (k >= ncols) break;
+#pragma unroll
+        for (uint32_t h = 0; h < 2u; ++h) {
+            const float4 p = *reinterpret_cast<const float4 *>(ar + k + 4u * h);
+            v[i][4 * h] = p.x; v[i][4 * h + 1] = p.y; v[i][4 * h + 2] = p.z; v[i][4 * h + 3] = p.w;
+        }
+        if (br)
+#pragma unroll
+            for (uint32_t h = 0; h < 2u; ++h) {
+                const float4 q = *reinterpret_cast<const float4 *>(br + k + 4u * h);
+                v[i][4 * h] = silu_mul(v[i][4 * h], q.x); v[i][4 * h + 1] = silu_mul(v[i][4 * h + 1], q.y);
+                v[i][4 * h + 2] = silu_mul(v[i][4 * h + 2], q.z); v[i][4 * h + 3] = silu_mul(v[i][4 * h + 3], q.w);
+            }
+#pragma unroll
+        for (uint32_t j = 0; j < 8u; ++j) mx = fmaxf(mx, fabsf(v[i][j]));
+    }
     for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31u) == 0) red[tid >> 5] = mx;
-    __syncthreads();
-    mx = 0.f;
-    for (uint32_t w = 0; w < 8u; ++w) mx = fmaxf(mx, red[w]);
     int e = 0;
     if (mx > 0.f && mx < INFINITY) { int ex; frexpf(mx, &ex); e = 14 - ex; }     // max |v| * 2^e in [2^13, 2^14)
     e = e > 100 ? 100 : e < -100 ? -100 : e;
     const float sc = exp2f((float)e);
-    if (tid == 0) x_inv[r] = exp2f((float)-e);
+    if (lane == 0) x_inv[r] = exp2f((float)-e);
     __half *hi = xd + (size_t)r * 2u * ncols, *lo = hi + ncols;
-    for (uint32_t c = tid; c < ncols / 8u; c += 256u) {
+#pragma unroll
+    for (uint32_t i = 0; i < NCH; ++i) {
+        const uint32_t k = i * 256u + lane * 8u;
+        if (k >= ncols) break;
         __half h[8], l[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t k = c * 8u + j;
-            const float v = (br ? silu_mul(ar[k], br[k]) : ar[k]) * sc;
-            h[j] = __float2half_rn(v);
-            l[j] = __float2half_rn(v - __half2float(h[j]));
+        for (uint32_t j = 0; j < 8u; ++j) {
+            const float s = v[i][j] * sc;
+            h[j] = __float2half_rn(s);
+            l[j] = __float2half_rn(s - __half2float(h[j]));
         }
-        *reinterpret_cast<uint4 *>(hi + c * 8u) = *reinterpret_cast<const uint4 *>(h);
-        *reinterpret_cast<uint4 *>(lo + c * 8u) = *reinterpret_cast<const uint4 *>(l);
+        *reinterpret_cast<uint4 *>(hi + k) = *reinterpret_cast<const uint4 *>(h);
+        *reinterpret_cast<uint4 *>(lo + k) = *reinterpret_cast<const uint4 *>(l);
     }
 }
 
@@ -392,9 +412,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_experts(const __grid_const
 bool tcx_shape_ok(uint32_t nrows, uint32_t ncols) { return nrows % TC_M == 0 && nrows && (ncols == 256u || ncols == 512u || ncols == 1024u || ncols == 2048u); }
 
 int launch_tc_prep_rows(const float *a, const float *b, uint32_t stride, uint32_t nrows, uint32_t ncols, __half *xd, float *x_inv, cudaStream_t s) {
-    RC_REQUIRE(ncols % TC_KS == 0 && nrows, "tc experts: %u columns is not a multiple of %u, or no rows", ncols, TC_KS);
+    RC_REQUIRE(ncols % 256u == 0 && ncols && ncols <= 2048u && stride % 4u == 0 && nrows, "tc experts: rows of %u columns (stride %u) are not tileable, or no rows", ncols, stride);
     prof_begin(b ? "tcx_prep_act" : "tcx_prep_x", s);
-    RC_LAUNCH((k_tc_prep_rows), nrows, 256, 0, s, a, b, stride, ncols, xd, x_inv);
+    const uint32_t grid = (nrows + 7u) / 8u;
+    if (ncols <= 512u) RC_LAUNCH((k_tc_prep_rows<2>), grid, 256, 0, s, a, b, stride, nrows, ncols, xd, x_inv);
+    else RC_LAUNCH((k_tc_prep_rows<8>), grid, 256, 0, s, a, b, stride, nrows, ncols, xd, x_inv);
     prof_end(s);
     RC_LAUNCHED();
     return 1;
