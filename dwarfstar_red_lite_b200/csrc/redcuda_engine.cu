@@ -77,8 +77,21 @@ __global__ void __launch_bounds__(1024) k_rmsnorm(const float *__restrict__ x, c
     x += tok_off; normed += tok_off;
     if (branch) branch += tok_off;
     if (resid_out) resid_out += tok_off;
+    // a row of up to 4096 values stays in registers between the sum and the scaling, and the weights are on their way with it
+    constexpr uint32_t KEEP = 4u;
+    float keep[KEEP], wk[KEEP];
     double ss = 0.0;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+#pragma unroll
+    for (uint32_t j = 0; j < KEEP; ++j) {
+        const uint32_t i = threadIdx.x + j * 1024u;
+        if (i < n) { keep[j] = x[i]; if (branch) keep[j] = keep[j] + branch[i]; wk[j] = w[i]; }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < KEEP; ++j) {
+        const uint32_t i = threadIdx.x + j * 1024u;
+        if (i < n) { if (resid_out) resid_out[i] = keep[j]; ss += (double)keep[j] * (double)keep[j]; }
+    }
+    for (uint32_t i = threadIdx.x + KEEP * 1024u; i < n; i += 1024u) {
         float v = x[i];
         if (branch) v = v + branch[i];
         if (resid_out) resid_out[i] = v;
@@ -86,7 +99,12 @@ __global__ void __launch_bounds__(1024) k_rmsnorm(const float *__restrict__ x, c
     }
     const double tot = block_sum_d(ss, red);
     const double inv = 1.0 / sqrt(tot / (double)n + (double)eps);
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+#pragma unroll
+    for (uint32_t j = 0; j < KEEP; ++j) {
+        const uint32_t i = threadIdx.x + j * 1024u;
+        if (i < n) normed[i] = (float)((double)keep[j] * inv * (double)wk[j]);
+    }
+    for (uint32_t i = threadIdx.x + KEEP * 1024u; i < n; i += 1024u) {
         float v = x[i];
         if (branch) v = v + branch[i];
         normed[i] = (float)((double)v * inv * (double)w[i]);
@@ -139,7 +157,29 @@ __global__ void k_attn_prep(const float *__restrict__ qg, const float *__restric
     else kcache[((size_t)pos * n_kv + h) * hd + tid] = to_kv<KV>(outv);
 }
 
-// Split-K decode attention. grid = (n_kv, nsplit, tokens), block = 256 (8 warps); token z attends to positions <= pos_p[z]
+// VPL consecutive cache values of a lane, requested as one to two vector loads (their address is a multiple of their size)
+template <typename KV, int VPL>
+struct KvRaw {
+    static constexpr int BYTES = VPL * (int)sizeof(KV);
+    uint32_t w[BYTES / 4];
+    __device__ __forceinline__ void load(const KV *p) {
+        if constexpr (BYTES % 16 == 0) {
+#pragma unroll
+            for (int i = 0; i < BYTES / 16; ++i) { const uint4 v = reinterpret_cast<const uint4 *>(p)[i]; w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w; }
+        } else if constexpr (BYTES == 8) { const uint2 v = *reinterpret_cast<const uint2 *>(p); w[0] = v.x; w[1] = v.y; }
+        else w[0] = *reinterpret_cast<const uint32_t *>(p);
+    }
+    __device__ __forceinline__ void floats(float (&f)[VPL]) const {
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            if constexpr (sizeof(KV) == 4) f[i] = __uint_as_float(w[i]);
+            else f[i] = __half2float(__ushort_as_half((unsigned short)(w[i / 2] >> (16 * (i & 1)))));
+        }
+    }
+};
+
+// Split-K decode attention. The chain over a warp's positions bounds it (7 of them at 3500 positions): the rows of the next
+// position are requested before the current one is worked on, and a lane's part of a row is one vector load. grid = (n_kv, nsplit, tokens), block = 256 (8 warps); token z attends to positions <= pos_p[z]
 // (the K/V rows of a whole prefill chunk are appended before this runs, so the mask is the sequence length alone). Every block serves the G query heads of one
 // K/V head over a slice of positions (K and V rows are read once for all G heads); a warp takes every 8th position,
 // a lane VPL = head_dim/32 consecutive dimensions; online softmax per head. Partials: m, l and the accumulator.
@@ -164,11 +204,13 @@ __global__ void __launch_bounds__(256) k_attn_decode(const float *__restrict__ q
 #pragma unroll
         for (int i = 0; i < VPL; ++i) { q[g][i] = query[((size_t)kvh * G + g) * hd + lane * VPL + i] * scale; acc[g][i] = 0.f; }
     }
+    KvRaw<KV, VPL> kr, vr;
+    const size_t lane_off = (size_t)kvh * hd + lane * VPL, row = (size_t)n_kv * hd;
+    if (p_begin + warp < p_end) { kr.load(kcache + (p_begin + warp) * row + lane_off); vr.load(vcache + (p_begin + warp) * row + lane_off); }
     for (uint32_t p = p_begin + warp; p < p_end; p += 8u) {
-        const KV *kp = kcache + ((size_t)p * n_kv + kvh) * hd + lane * VPL, *vp = vcache + ((size_t)p * n_kv + kvh) * hd + lane * VPL;
         float kx[VPL], vx[VPL];
-#pragma unroll
-        for (int i = 0; i < VPL; ++i) { kx[i] = from_kv(kp[i]); vx[i] = from_kv(vp[i]); }
+        kr.floats(kx); vr.floats(vx);
+        if (p + 8u < p_end) { kr.load(kcache + (p + 8u) * row + lane_off); vr.load(vcache + (p + 8u) * row + lane_off); }
         float s[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) {

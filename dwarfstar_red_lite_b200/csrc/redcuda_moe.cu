@@ -524,7 +524,7 @@ static int moe_group(redcuda_moe *m, const uint32_t *pair_expert, uint32_t npair
     if (distinct && npairs <= 64u && !skip_foreign) {
         RC_LAUNCH((k_group_trivial), 1, 64, 0, s, pair_expert, npairs, m->sorted, m->uexp, m->ustart, m->n_unique, m->item_u, m->item_p0, m->n_items, m->work);
     } else {
-#define RC_GROUP(KEEP) RC_LAUNCH((k_group_pairs<KEEP>), 1, 1024, 0, s, pair_expert, npairs, m->d.expert_begin, m->d.expert_stride, skip_foreign ? 1u : 0u, m->d.expert_count, moe_item_tokens(m, false, npairs), m->sorted, m->uexp, m->ustart, m->n_unique, m->item_u, m->item_p0, m->n_items, m->bad, m->work, m->wait)
+#define RC_GROUP(KEEP) RC_LAUNCH_PDL_IF(npairs <= MOE_PDL_PAIRS, (k_group_pairs<KEEP>), 1, 1024, 0, s, pair_expert, npairs, m->d.expert_begin, m->d.expert_stride, skip_foreign ? 1u : 0u, m->d.expert_count, moe_item_tokens(m, false, npairs), m->sorted, m->uexp, m->ustart, m->n_unique, m->item_u, m->item_p0, m->n_items, m->bad, m->work, m->wait)
         if (npairs <= 3072u) RC_GROUP(3u); else RC_GROUP(20u);
 #undef RC_GROUP
     }
@@ -537,7 +537,7 @@ static int moe_combine(redcuda_moe *m, uint32_t ntok, const float *pair_out, con
                        float *out, cudaStream_t s) {
     const dim3 grid((m->d.hidden / 4u + 255u) / 256u, ntok);
     prof_begin("moe_combine", s);
-    RC_LAUNCH((k_moe_combine), grid, 256, 0, s, pair_out, wk, top_k, shared ? m->sh_out : nullptr, m->scalar, resid, out, m->d.hidden, nullptr);
+    RC_LAUNCH_PDL_IF(ntok * top_k <= MOE_PDL_PAIRS, (k_moe_combine), grid, 256, 0, s, pair_out, wk, top_k, shared ? m->sh_out : nullptr, m->scalar, resid, out, m->d.hidden, nullptr);
     prof_end(s);
     RC_LAUNCHED();
     return 1;
