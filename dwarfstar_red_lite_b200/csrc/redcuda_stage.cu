@@ -131,8 +131,10 @@ struct StageLease {
     uint8_t *dev = nullptr, *pin = nullptr;
     size_t dev_bytes = 0, pin_bytes = 0;
     std::vector<cudaEvent_t> events;
+    cudaEvent_t behind = nullptr;      // Stage::follow_default_stream
     ~StageLease() {
         for (cudaEvent_t e : events) cudaEventDestroy(e);
+        if (behind) cudaEventDestroy(behind);
         if (dev) cudaFree(dev);
         if (pin) cudaFreeHost(pin);
         if (s) cudaStreamDestroy(s);
@@ -181,7 +183,19 @@ int Stage::open(size_t device_bytes) {
         lease_->dev = m.as<uint8_t>(); lease_->dev_bytes = want;
         m.p = nullptr; m.bytes = 0;
     }
-    dev_ = lease_->dev; used_ = 0; pinned_used_ = 0;
+    dev_ = lease_->dev; used_ = 0; pinned_used_ = 0; followed_ = false;
+    return 1;
+}
+
+// The copy engine reads and writes pinned arrays by itself, and the caller may have copies of its own under way on them: one
+// that still fills an input, or one that still reads what is about to be overwritten. A call on such an array therefore starts
+// behind the default stream (and, with it, behind every stream that synchronises with it), as it did when it ran there.
+int Stage::follow_default_stream() {
+    if (followed_) return 1;
+    if (!lease_->behind) RC_CUDA(cudaEventCreateWithFlags(&lease_->behind, cudaEventDisableTiming));
+    RC_CUDA(cudaEventRecord(lease_->behind, cudaStreamLegacy));
+    RC_CUDA(cudaStreamWaitEvent(lease_->s, lease_->behind, 0));
+    followed_ = true;
     return 1;
 }
 
@@ -225,7 +239,11 @@ int Stage::drain_pinned() { RC_CUDA(cudaStreamSynchronize(lease_->s)); pinned_us
 int Stage::upload(void *dst_dev, const void *src_host, size_t bytes) {
     if (!bytes) return 1;
     cudaStream_t s = lease_->s;
-    if (host_is_pinned(src_host)) { RC_CUDA(cudaMemcpyAsync(dst_dev, src_host, bytes, cudaMemcpyHostToDevice, s)); return 1; }
+    if (host_is_pinned(src_host)) {
+        if (!follow_default_stream()) return 0;
+        RC_CUDA(cudaMemcpyAsync(dst_dev, src_host, bytes, cudaMemcpyHostToDevice, s));
+        return 1;
+    }
     const uint8_t *src = static_cast<const uint8_t *>(src_host);
     uint8_t *dst = static_cast<uint8_t *>(dst_dev);
     if (lease_->pin_bytes - pinned_used_ < bytes && lease_->pin_bytes < PINNED_MAX) {
@@ -260,7 +278,11 @@ int Stage::upload(void *dst_dev, const void *src_host, size_t bytes) {
 int Stage::download(void *dst_host, const void *src_dev, size_t bytes) {
     if (!bytes) return 1;
     cudaStream_t s = lease_->s;
-    if (host_is_pinned(dst_host)) { RC_CUDA(cudaMemcpyAsync(dst_host, src_dev, bytes, cudaMemcpyDeviceToHost, s)); return 1; }
+    if (host_is_pinned(dst_host)) {
+        if (!follow_default_stream()) return 0;
+        RC_CUDA(cudaMemcpyAsync(dst_host, src_dev, bytes, cudaMemcpyDeviceToHost, s));
+        return 1;
+    }
     uint8_t *dst = static_cast<uint8_t *>(dst_host);
     const uint8_t *src = static_cast<const uint8_t *>(src_dev);
     if (bytes > INLINE_MAX && lease_->pin_bytes < std::min(bytes, PINNED_MAX) && !stage_pinned(lease_, bytes)) return 0;

@@ -28,10 +28,12 @@ class Stage {
     cudaStream_t stream() const;
 
   private:
+    int follow_default_stream();
     int drain_pinned();      // waits until no copy reads or writes the pinned buffer any more
     StageLease *lease_ = nullptr;
     uint8_t *dev_ = nullptr;
     size_t used_ = 0, pinned_used_ = 0;
+    bool followed_ = false;
 };
 
 // Gives back every device and pinned buffer that idle leases keep (called when an allocation of the library fails)

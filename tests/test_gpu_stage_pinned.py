@@ -1,0 +1,46 @@
+"""Host-buffer calls on pinned arrays that copies of the default stream are still filling or still reading."""
+import numpy as np
+import pytest
+import torch
+
+import dwarfstar_red_lite_b200 as rc
+from dwarfstar_red_lite_b200 import synth
+
+pytestmark = pytest.mark.gpu
+NROWS, NCOLS = 64, 2048
+
+
+def _matvec(w, x_ptr, out_ptr, ntok=1):
+    lib = rc.lib()
+    assert lib.redcuda_quant_matvec(synth.Q6_K, w.ctypes.data, NROWS, NCOLS, x_ptr, ntok, out_ptr) == 1, lib.redcuda_last_error()
+
+
+@pytest.fixture(scope="module")
+def case():
+    rng = np.random.default_rng(2)
+    w = synth.quant_matrix(rng, synth.Q6_K, NROWS, NCOLS, 1e-3, 5e-3, (-64, 63))
+    x = rng.normal(0, 1, size=(1, NCOLS)).astype(np.float32)
+    # 256 MB in front of the copy that matters: milliseconds of work for the default stream
+    return w, x, rc.quant_matvec(synth.Q6_K, w, NROWS, NCOLS, x), torch.zeros(1 << 26, device="cuda"), torch.zeros(1 << 26).pin_memory()
+
+
+def test_input_still_being_filled(case):
+    w, x, want, big_dev, big_host = case
+    src, pinned, out = torch.from_numpy(x).cuda(), torch.zeros(1, NCOLS).pin_memory(), np.empty((1, NROWS), np.float32)
+    torch.cuda.synchronize()
+    big_host.copy_(big_dev, non_blocking=True)
+    pinned.copy_(src, non_blocking=True)
+    _matvec(w, pinned.data_ptr(), out.ctypes.data)
+    assert np.array_equal(out, want)
+
+
+def test_output_still_being_read(case):
+    w, x, want, big_dev, big_host = case
+    pinned, dst = torch.full((1, NROWS), 7.0).pin_memory(), torch.zeros(1, NROWS, device="cuda")
+    torch.cuda.synchronize()
+    big_dev.copy_(big_host, non_blocking=True)
+    dst.copy_(pinned, non_blocking=True)
+    _matvec(w, x.ctypes.data, pinned.data_ptr())
+    assert np.array_equal(pinned.numpy(), want)
+    torch.cuda.synchronize()
+    assert torch.all(dst == 7.0)
