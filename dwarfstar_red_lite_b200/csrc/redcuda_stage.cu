@@ -187,7 +187,7 @@ int Stage::open(size_t device_bytes) {
     return 1;
 }
 
-// The copy engine reads and writes pinned arrays by itself, and the caller may have copies of its own under way on them: one
+// The copy engine reads and writes such arrays by itself, and the caller may have copies of its own under way on them: one
 // that still fills an input, or one that still reads what is about to be overwritten. A call on such an array therefore starts
 // behind the default stream (and, with it, behind every stream that synchronises with it), as it did when it ran there.
 int Stage::follow_default_stream() {
@@ -227,11 +227,11 @@ static int stage_pinned(StageLease *l, size_t want) {
     l->pin_bytes = p;
     return 1;
 }
-// memory the copy engine can reach by itself
-static bool host_is_pinned(const void *p) {
+// memory the copy engine can reach by itself: pinned, managed, and device memory (a caller may hand in either kind of pointer)
+static bool dma_reaches(const void *p) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
-    return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
+    return a.type != cudaMemoryTypeUnregistered;
 }
 
 int Stage::drain_pinned() { RC_CUDA(cudaStreamSynchronize(lease_->s)); pinned_used_ = 0; return 1; }
@@ -239,9 +239,9 @@ int Stage::drain_pinned() { RC_CUDA(cudaStreamSynchronize(lease_->s)); pinned_us
 int Stage::upload(void *dst_dev, const void *src_host, size_t bytes) {
     if (!bytes) return 1;
     cudaStream_t s = lease_->s;
-    if (host_is_pinned(src_host)) {
+    if (dma_reaches(src_host)) {
         if (!follow_default_stream()) return 0;
-        RC_CUDA(cudaMemcpyAsync(dst_dev, src_host, bytes, cudaMemcpyHostToDevice, s));
+        RC_CUDA(cudaMemcpyAsync(dst_dev, src_host, bytes, cudaMemcpyDefault, s));
         return 1;
     }
     const uint8_t *src = static_cast<const uint8_t *>(src_host);
@@ -278,9 +278,9 @@ int Stage::upload(void *dst_dev, const void *src_host, size_t bytes) {
 int Stage::download(void *dst_host, const void *src_dev, size_t bytes) {
     if (!bytes) return 1;
     cudaStream_t s = lease_->s;
-    if (host_is_pinned(dst_host)) {
+    if (dma_reaches(dst_host)) {
         if (!follow_default_stream()) return 0;
-        RC_CUDA(cudaMemcpyAsync(dst_host, src_dev, bytes, cudaMemcpyDeviceToHost, s));
+        RC_CUDA(cudaMemcpyAsync(dst_host, src_dev, bytes, cudaMemcpyDefault, s));
         return 1;
     }
     uint8_t *dst = static_cast<uint8_t *>(dst_host);

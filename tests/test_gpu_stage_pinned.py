@@ -1,4 +1,5 @@
-"""Host-buffer calls on pinned arrays that copies of the default stream are still filling or still reading."""
+"""Host-buffer calls on arrays that are not ordinary host memory: pinned ones that copies of the default stream are still
+filling or still reading, and device memory."""
 import numpy as np
 import pytest
 import torch
@@ -44,3 +45,11 @@ def test_output_still_being_read(case):
     assert np.array_equal(pinned.numpy(), want)
     torch.cuda.synchronize()
     assert torch.all(dst == 7.0)
+
+
+def test_device_arrays(case):
+    w, x, want, _, _ = case
+    wd, xd, out = torch.from_numpy(w).cuda(), torch.from_numpy(x).cuda(), torch.zeros(1, NROWS, device="cuda")
+    lib = rc.lib()
+    assert lib.redcuda_quant_matvec(synth.Q6_K, wd.data_ptr(), NROWS, NCOLS, xd.data_ptr(), 1, out.data_ptr()) == 1, lib.redcuda_last_error()
+    assert np.array_equal(out.cpu().numpy(), want)
