@@ -552,6 +552,8 @@ int redcuda_set_codebooks(const uint8_t *iq2xxs_grid, uint32_t iq2xxs_bytes, con
     RC_CUDA(cudaGetSymbolAddress(&p2, d_iq2_grid));
     RC_CUDA(cudaGetSymbolAddress(&p3, d_iq3s_grid));
     if (!mma_set_luts(iq2xxs_grid)) return 0;
+    // a copy from pageable memory may still be on its way when it returns, and the calls that read the tables run on streams of their own
+    RC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     std::lock_guard<std::mutex> lk(g_books_mu);
     g_iq2_ptr[dev] = (const uint8_t *)p2;
     g_iq3s_ptr[dev] = (const uint32_t *)p3;

@@ -44,6 +44,8 @@ int kq_set_iq_tables(const uint32_t *iq3xxs, const uint64_t *iq2s, const int8_t 
     RC_CUDA(cudaGetSymbolAddress(&a, d_iq3xxs_grid));
     RC_CUDA(cudaGetSymbolAddress(&b, d_iq2s_grid));
     RC_CUDA(cudaGetSymbolAddress(&c, d_iq4nl));
+    // a copy from pageable memory may still be on its way when it returns, and the calls that read the tables run on streams of their own
+    RC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     std::lock_guard<std::mutex> lk(g_iq_mu);
     g_iq_tabs[dev].iq3xxs = (const uint32_t *)a; g_iq_tabs[dev].iq2s = (const uint64_t *)b; g_iq_tabs[dev].iq4nl = (const int8_t *)c;
     g_iq_tabs_set[dev] = true;
@@ -58,6 +60,7 @@ int kq_set_xs_tables(const int8_t *iq2xs, const int8_t *iq1m) {
     void *a = nullptr, *b = nullptr;
     RC_CUDA(cudaGetSymbolAddress(&a, d_iq2xs_grid));
     RC_CUDA(cudaGetSymbolAddress(&b, d_iq1m_grid));
+    RC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));      // as in kq_set_iq_tables
     std::lock_guard<std::mutex> lk(g_iq_mu);
     g_iq_tabs[dev].iq2xs = (const int8_t *)a; g_iq_tabs[dev].iq1m = (const int8_t *)b;
     g_xs_tabs_set[dev] = true;
