@@ -77,19 +77,16 @@ uint32_t act_digit_bits() {
 __global__ void __launch_bounds__(256) k_quant_act(const float *__restrict__ x, uint32_t x_stride, uint32_t ncols,
                                                    int8_t *__restrict__ xq, float *__restrict__ sx, uint32_t bits) {
     pdl_prologue();
-    __shared__ float red[8];
+    __shared__ uint32_t red[8];
     const uint32_t row = blockIdx.x, tid = threadIdx.x;
     const float *xr = x + (size_t)row * x_stride;
-    float mx = 0.f;
-    for (uint32_t k = tid * 4u; k < ncols; k += 1024u) {
-        const float4 v = *reinterpret_cast<const float4 *>(xr + k);
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-    }
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    uint32_t mx = 0u;
+    for (uint32_t k = tid * 4u; k < ncols; k += 1024u) mx = max(mx, act_mag4(*reinterpret_cast<const float4 *>(xr + k)));
+    mx = __reduce_max_sync(0xffffffffu, mx);
     if ((tid & 31u) == 0) red[tid >> 5] = mx;
     __syncthreads();
     mx = red[0];
-    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, red[w]);
+    for (int w = 1; w < 8; ++w) mx = max(mx, red[w]);
     const float QMAX = act_qmax(bits);
     const float scale = act_scale(mx, QMAX);
     const float inv = 1.0f / scale;

@@ -79,7 +79,11 @@ int launch_nib_down_tail(NibTailArgs &A, cudaStream_t s);
 // the three balanced digits of one activation and the row scale: the arithmetic of k_quant_act, shared with the kernels
 // that quantise a row themselves
 __device__ __forceinline__ float act_qmax(uint32_t bits) { return bits == 8u ? 8355711.0f : 1040000.0f; }    // largest value three digits hold: 127 * (65536 + 256 + 1), or just below 63.5 * 16384
-__device__ __forceinline__ float act_scale(float mx, float qmax) { return (mx > 0.f && mx < INFINITY) ? mx / qmax : 1.0f; }
+// |v| as bits: they order as the magnitudes do, with infinity and then NaN above every number
+__device__ __forceinline__ uint32_t act_mag(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t act_mag4(const float4 &v) { return max(max(act_mag(v.x), act_mag(v.y)), max(act_mag(v.z), act_mag(v.w))); }
+// mx: largest act_mag of the row. Digits cannot hold a non-finite value, so a row with one gets a NaN scale: its products are NaN.
+__device__ __forceinline__ float act_scale(uint32_t mx, float qmax) { return mx == 0u ? 1.0f : mx < 0x7f800000u ? __uint_as_float(mx) / qmax : __uint_as_float(0x7fffffffu); }
 __device__ __forceinline__ void act_digits(float f, float inv, float qmax, uint32_t bits, int &d0, int &d1, int &d2) {
     const int half = 1 << (bits - 1u), mask = (1 << bits) - 1;
     int iv = __float2int_rn(fminf(fmaxf(f * inv, -qmax), qmax));

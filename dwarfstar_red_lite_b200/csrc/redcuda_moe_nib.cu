@@ -353,20 +353,18 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
         R.cur_src = I.rec; R.cur_rem = I.n;
         while (ahead + 1u < STAGES && ahead < I.n) { nib_request<STAGES>(R, lane); ++ahead; }
     }
-    __shared__ float s_red[NIB_WARPS], s_sx;
+    __shared__ uint32_t s_red[NIB_WARPS];
+    __shared__ float s_sx;
     if (ONE) {
         // single token: every unit multiplies the same activation row, so the block turns it into digits itself (the
         // arithmetic of k_quant_act) — columns 0..2 of the one tile in use, columns 3..7 zero
-        float mx = 0.f;
-        for (uint32_t k = tid * 4u; k < NCOLS; k += NIB_WARPS * 128u) {
-            const float4 v = *reinterpret_cast<const float4 *>(A.x_raw + k);
-            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-        }
-        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        uint32_t mx = 0u;
+        for (uint32_t k = tid * 4u; k < NCOLS; k += NIB_WARPS * 128u) mx = max(mx, act_mag4(*reinterpret_cast<const float4 *>(A.x_raw + k)));
+        mx = __reduce_max_sync(0xffffffffu, mx);
         if (lane == 0) s_red[warp] = mx;
         __syncthreads();
         mx = s_red[0];
-        for (uint32_t w = 1; w < NIB_WARPS; ++w) mx = fmaxf(mx, s_red[w]);
+        for (uint32_t w = 1; w < NIB_WARPS; ++w) mx = max(mx, s_red[w]);
         const float qmax = act_qmax(A.act_bits), scale = act_scale(mx, qmax), inv = 1.0f / scale;
         if (tid == 0) s_sx = scale;
         for (uint32_t k = tid * 4u; k < NCOLS; k += NIB_WARPS * 128u) {
@@ -508,14 +506,14 @@ __global__ void __launch_bounds__((NIB_TAIL_MAX_K + 2u) * 32u) k_nib_down_tail(c
         // this expert's activation row -> digits (the arithmetic of k_quant_act), while the records are in flight
         const float *ar = A.act + (size_t)warp * A.act_stride;
         float v[PER_LANE];
-        float mx = 0.f;
+        uint32_t mx = 0u;
 #pragma unroll
         for (uint32_t i = 0; i < PER_LANE / 4u; ++i) {
             const float4 q = *reinterpret_cast<const float4 *>(ar + lane * 4u + 128u * i);
             v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
-            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
+            mx = max(mx, act_mag4(q));
         }
-        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mx = __reduce_max_sync(0xffffffffu, mx);
         const float qmax = act_qmax(A.bits), sx = act_scale(mx, qmax), inv = 1.0f / sx;
         int8_t *mine = digits + warp * 3u * BPITCH;
 #pragma unroll
