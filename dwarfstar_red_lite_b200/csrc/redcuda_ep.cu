@@ -15,7 +15,8 @@
 //   partial    this shard's experts over the pairs of ALL tokens that select them; the combine sums a token's local
 //              pairs and adds the shared-expert part to the rank's own tokens
 //   reduce     ncclReduceScatter(sum) of the partial outputs straight into the caller's output rows
-// Layers whose expert kernels take fp32 rows (non-IQ2_XXS experts) gather the fp32 rows instead of digits.
+// Layers whose expert kernels take fp32 rows, chunks that the tcgen05 expert kernel serves and layers with IQ3_S matrices (whose
+// four digits are as many bytes) gather the fp32 rows instead of digits.
 //
 // Two exchanges. NCCL (the fallback and A/B): the calls above. Peer memory (after redcuda_ep_attach_peers; ranks are
 // processes on one node whose exchange areas are mapped into each other with CUDA IPC): the all-gather becomes a push

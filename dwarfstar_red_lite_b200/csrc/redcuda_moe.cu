@@ -324,18 +324,31 @@ struct redcuda_moe {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_quant = nullptr;
 };
 
-static uint32_t nib_fmt(uint32_t type) { return type == RC_IQ3_S ? NIB_IQ3 : NIB_IQ2; }
+// Layers with IQ3_S matrices take their activations as wide digits: they ran on fp32 activations before the nibble layout held them,
+// and the 24-bit form per row is less than that (relative error of an expert's output against 64-bit sums, hidden 2048: fp32 1.6e-7 on any
+// row; three digits 3.1e-7 on Gaussian rows, 2.2e-6 with one element of 100, 4.7e-4 with a large one where the weights vanish; wide
+// digits 1.0e-7 on any). What it costs against three digits and the tcgen05 kernel, us a layer: 24 tokens 130 -> 128, 64 skewed 156 -> 168,
+// 300 391 -> 432, 2048 1235 -> 2159 (the fp32 kernel: 557, 1497, 2340, 11693).
+static bool moe_wide_types(const redcuda_moe_desc &d) { return d.type_gu == RC_IQ3_S || d.type_down == RC_IQ3_S; }
+static bool moe_wide(const redcuda_moe *m);
+static uint32_t nib_fmt(const redcuda_moe *m, uint32_t type) { return type == RC_IQ3_S ? NIB_IQ3 : moe_wide(m) ? NIB_IQ2W : NIB_IQ2; }
 static bool nib_type(uint32_t type) { return type == RC_IQ2_XXS || (type == RC_IQ3_S && books_iq3s_odd()); }
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// tensor-core path of the routed experts: IQ2_XXS gate/up/down with tile-able shapes
+static bool moe_wide(const redcuda_moe *m) { return m->nib && moe_wide_types(m->d); }
+// activation rows of the routed experts -> the digits that the layer's expert kernels read
+static int moe_quant_rows(const redcuda_moe *m, const float *x, uint32_t x_stride, uint32_t rows, uint32_t ncols, int8_t *xq, float *sx, cudaStream_t s) {
+    return moe_wide(m) ? launch_quant_act_wide(x, x_stride, rows, ncols, xq, sx, s) : launch_quant_act(x, x_stride, rows, ncols, xq, sx, s);
+}
+
+// integer tensor-core path of the routed experts: the nibble layout, or planar IQ2_XXS gate/up/down with tile-able shapes
 static bool moe_experts_mma(const redcuda_moe *m) {
     return m->nib || (m->use_mma && m->d.type_gu == RC_IQ2_XXS && m->d.type_down == RC_IQ2_XXS && m->d.hidden % 512u == 0 && m->d.ffn % 512u == 0);
 }
-// pairs per work item: the nibble-layout kernels take at most 8
+// pairs per work item: the nibble-layout kernels take at most 8, in the wide form 6
 static uint32_t moe_item_tokens(const redcuda_moe *m, bool single_token, uint32_t npairs) {
     if (m->tc_now && !single_token) return TCX_TN;
-    if (m->nib) return single_token ? 1u : 8u;
+    if (m->nib) return single_token ? 1u : moe_wide(m) ? NIB_WIDE_PAIRS : 8u;
     return mma_item_tokens(single_token, npairs, m->d.expert_count);
 }
 // Which expert kernels serve a call of npairs pairs (all_local: every pair belongs to this shard; otherwise the share
@@ -456,7 +469,7 @@ static int moe_launch_experts(redcuda_moe *m, bool gateup, uint32_t npairs, bool
         if (gateup) { if (!launch_tc_prep_rows(x, nullptr, x_stride, (npairs + x_div - 1u) / x_div, ncols, xd, xinv, s)) return 0; }
         else if (!launch_tc_prep_rows(x, m->tmp, x_stride, npairs, ncols, xd, xinv, s)) return 0;
         TcxArgs T{};
-        T.w[0] = gateup ? m->gate : m->down; T.w[1] = gateup ? m->up : nullptr; T.nmat = gateup ? 2u : 1u; T.fmt = nib_fmt(gateup ? m->d.type_gu : m->d.type_down);
+        T.w[0] = gateup ? m->gate : m->down; T.w[1] = gateup ? m->up : nullptr; T.nmat = gateup ? 2u : 1u;
         T.mat_bytes = gateup ? m->gu_bytes : m->down_bytes; T.nrows = nrows; T.ncols = ncols;
         T.expert_begin = m->d.expert_begin; T.n_local = m->d.expert_count;
         T.sorted = m->sorted; T.uexp = m->uexp; T.ustart = m->ustart; T.item_u = m->item_u; T.item_p0 = m->item_p0; T.n_items = m->n_items;
@@ -469,7 +482,7 @@ static int moe_launch_experts(redcuda_moe *m, bool gateup, uint32_t npairs, bool
     if (moe_experts_mma(m)) {
         int8_t *xq = gateup ? m->xq_x : m->xq_act;
         float *sx = gateup ? m->sx_x : m->sx_act;
-        if (!x_quantised && !launch_quant_act(x, x_stride, (npairs + x_div - 1u) / x_div, ncols, xq, sx, s)) return 0;
+        if (!x_quantised && !moe_quant_rows(m, x, x_stride, (npairs + x_div - 1u) / x_div, ncols, xq, sx, s)) return 0;
         const int8_t *xq_in = gateup && m->xq_ext ? m->xq_ext : xq;
         const float *sx_in = gateup && m->sx_ext ? m->sx_ext : sx;
         MmaArgs M{};
@@ -481,7 +494,7 @@ static int moe_launch_experts(redcuda_moe *m, bool gateup, uint32_t npairs, bool
         const uint32_t tok = moe_item_tokens(m, single_token, npairs);
         const uint32_t live = npairs < m->d.expert_count ? npairs : m->d.expert_count;
         const uint32_t max_items = single_token ? npairs : (npairs / tok + live < npairs ? npairs / tok + live : npairs);
-        if (m->nib) { M.item_tok = tok; M.fmt = nib_fmt(gateup ? m->d.type_gu : m->d.type_down); M.work = m->work + (gateup ? 0 : 1); return launch_nib_experts(M, max_items, s); }
+        if (m->nib) { M.item_tok = tok; M.fmt = nib_fmt(m, gateup ? m->d.type_gu : m->d.type_down); M.work = m->work + (gateup ? 0 : 1); return launch_nib_experts(M, max_items, s); }
         return launch_moe_mma(M, max_items, tok, s);
     }
     MoeArgs A{};
@@ -563,11 +576,11 @@ static int moe_forward_fused1(redcuda_moe *m, const float *x, const float *logit
     M.w0 = m->gate; M.w1 = m->up; M.mat_bytes = m->gu_bytes; M.nb = m->gu_nb; M.nrows = m->d.ffn; M.ncols = m->d.hidden;
     M.expert_begin = m->d.expert_begin; M.n_local = m->d.expert_count; M.status = status_words();
     M.sorted = m->sorted; M.uexp = m->uexp; M.ustart = m->ustart; M.item_u = m->item_u; M.item_p0 = m->item_p0; M.n_items = m->n_items;
-    M.xq = nullptr; M.sx = nullptr; M.x_div = k; M.out = m->act; M.out_stride = m->d.ffn; M.item_tok = 1u; M.work = m->work; M.x_raw = x; M.fmt = nib_fmt(m->d.type_gu);
+    M.xq = nullptr; M.sx = nullptr; M.x_div = k; M.out = m->act; M.out_stride = m->d.ffn; M.item_tok = 1u; M.work = m->work; M.x_raw = x; M.fmt = nib_fmt(m, m->d.type_gu);
     if (!launch_nib_experts(M, k, s)) return 0;
     NibTailArgs D{};
     D.w_down = m->down; D.mat_bytes = m->down_bytes; D.nrows = m->d.hidden; D.ncols = m->d.ffn; D.expert_begin = m->d.expert_begin; D.n_local = m->d.expert_count;
-    D.fmt = nib_fmt(m->d.type_down);
+    D.fmt = nib_fmt(m, m->d.type_down);
     D.top_k = k; D.ids = m->ids; D.wk = m->wk; D.act = m->act; D.act_stride = m->d.ffn;
     D.sh_down = m->sh_down.base; D.sh_nb = m->sh_down.nb; D.sh_act = m->sh_act; D.scalar = m->scalar; D.resid = resid; D.out = out; D.status = status_words();
     return launch_nib_down_tail(D, s);
@@ -580,7 +593,9 @@ static int moe_forward_on(redcuda_moe *m, uint32_t ntok, const float *x, const f
     const uint32_t k = m->d.top_k, npairs = ntok * k;
     moe_choose_path(m, npairs, true);
     // one quantisation of the token activations serves the routed gate/up and the shared gate/up
-    const bool xq = moe_experts_mma(m) || moe_shared_mma(m, ntok);
+    // (a wide layer has digits of its own for the routed experts: `wide` makes those, `xq` the shared expert's)
+    const bool wide = moe_wide(m);
+    const bool xq = wide ? moe_shared_mma(m, ntok) && !moe_shared_tc(m, ntok) : moe_experts_mma(m) || moe_shared_mma(m, ntok);
     // The shared expert needs nothing from the router, so it runs on a side stream next to the routed
     // experts and joins before the combine (both edges are events, so the fork is kept when the caller captures a graph).
     // With profiling on, everything stays on one stream so that per-kernel times are not overlapped.
@@ -588,18 +603,20 @@ static int moe_forward_on(redcuda_moe *m, uint32_t ntok, const float *x, const f
     // The quantisation of x leaves the critical path too: it opens the side stream (the shared expert's tensor-core
     // kernels, which read the digits as well, follow it there) and the main stream waits for it only before the
     // gate/up launch, behind the router GEMV, the selection and the grouping.
-    const bool quant_aside = fork && xq;
-    // the tcgen05 expert path keeps its fp16 digits where the int8 digits of the routed experts would go, so the int8
+    const bool quant_aside = fork && (xq || wide);
+    // the tcgen05 expert path and a wide layer keep their own digits where the int8 digits of the routed experts would go, so the
     // digits that the shared expert still reads move to the buffer of the stand-alone shared-expert call
-    int8_t *xqd = m->tc_now ? m->xq_own : m->xq_x;
-    float *sxd = m->tc_now ? m->sx_own : m->sx_x;
+    int8_t *xqd = m->tc_now || wide ? m->xq_own : m->xq_x;
+    float *sxd = m->tc_now || wide ? m->sx_own : m->sx_x;
+    if (wide && !quant_aside && !launch_quant_act_wide(x, m->d.hidden, ntok, m->d.hidden, m->xq_x, m->sx_x, s)) return 0;
     if (xq && !quant_aside && !launch_quant_act(x, m->d.hidden, ntok, m->d.hidden, xqd, sxd, s)) return 0;
     if (fork) {
         RC_CUDA(cudaEventRecord(m->ev_fork, s));
         RC_CUDA(cudaStreamWaitEvent(m->side, m->ev_fork, 0));
         if (quant_aside) {
-            if (!launch_quant_act(x, m->d.hidden, ntok, m->d.hidden, xqd, sxd, m->side)) return 0;
+            if (wide ? !launch_quant_act_wide(x, m->d.hidden, ntok, m->d.hidden, m->xq_x, m->sx_x, m->side) : !launch_quant_act(x, m->d.hidden, ntok, m->d.hidden, xqd, sxd, m->side)) return 0;
             RC_CUDA(cudaEventRecord(m->ev_quant, m->side));
+            if (wide && xq && !launch_quant_act(x, m->d.hidden, ntok, m->d.hidden, xqd, sxd, m->side)) return 0;
         }
         if (!moe_gemv_pre(m, ntok, x, false, true, xq, m->side, xqd, sxd) || !moe_shared_down(m, ntok, m->side)) return 0;
         RC_CUDA(cudaEventRecord(m->ev_join, m->side));
@@ -613,7 +630,7 @@ static int moe_forward_on(redcuda_moe *m, uint32_t ntok, const float *x, const f
         if (!moe_group(m, m->ids, npairs, ntok == 1u, s)) return 0;
     }
     if (quant_aside && !m->tc_now) RC_CUDA(cudaStreamWaitEvent(s, m->ev_quant, 0));
-    if (!moe_launch_experts(m, true, npairs, ntok == 1u, x, m->d.hidden, k, xq && moe_experts_mma(m), m->act, m->d.ffn, s)) return 0;
+    if (!moe_launch_experts(m, true, npairs, ntok == 1u, x, m->d.hidden, k, wide || (xq && moe_experts_mma(m)), m->act, m->d.ffn, s)) return 0;
     if (!fork && !moe_shared_down(m, ntok, s)) return 0;
     if (!moe_launch_experts(m, false, npairs, ntok == 1u, m->act, m->d.ffn, 1u, false, m->tmp, m->d.hidden, s)) return 0;
     if (fork) RC_CUDA(cudaStreamWaitEvent(s, m->ev_join, 0));
@@ -634,8 +651,9 @@ static size_t moe_ws_layout(const redcuda_moe_desc &d, redcuda_moe *m, uint8_t *
     put(r.sh_act, T * d.ffn_sh * 4u); put(r.sh_out, T * d.hidden * 4u); put(r.act, P * d.ffn * 4u); put(r.tmp, P * d.hidden * 4u);
     put(r.out, T * d.hidden * 4u); put(r.ids, P * 4u); put(r.sorted, P * 4u); put(r.uexp, (size_t)(d.expert_count + 1u) * 4u);
     put(r.ustart, (size_t)(d.expert_count + 2u) * 4u); put(r.n_unique, 16); put(r.bad, 16);
-    // digits of the routed experts' inputs: three int8 digits per value (mma.sync kernels) or two fp16 digits (tcgen05 kernel)
-    put(r.xq_x, P * 4u * d.hidden); put(r.sx_x, P * 4u); put(r.xq_act, P * 4u * d.ffn); put(r.sx_act, P * 4u);
+    // digits of the routed experts' inputs: three or four int8 digits per value (mma.sync kernels) or two fp16 digits (tcgen05 kernel)
+    const size_t sx_n = moe_wide_types(d) ? (d.hidden + 255u) / 256u : 1u, sa_n = moe_wide_types(d) ? (d.ffn + 255u) / 256u : 1u;     // scales of a row
+    put(r.xq_x, P * 4u * d.hidden); put(r.sx_x, P * 4u * sx_n); put(r.xq_act, P * 4u * d.ffn); put(r.sx_act, P * 4u * sa_n);
     put(r.xq_sh, T * 3u * d.ffn_sh); put(r.sx_sh, T * 4u); put(r.xq_own, T * 3u * d.hidden); put(r.sx_own, T * 4u);
     put(r.item_u, (P + 8u) * 4u); put(r.item_p0, (P + 8u) * 4u); put(r.n_items, 16); put(r.work, 16);
     put(r.sh_xs, tc_xs_halves((uint32_t)T, d.hidden > d.ffn_sh ? d.hidden : d.ffn_sh, 128u) * 2u); put(r.sh_xinv, (T + 128u) * 4u);
@@ -657,10 +675,11 @@ void moe_set_ids_mirror(redcuda_moe *m, uint32_t *dev_ptr) { m->ids_mirror = dev
 }
 namespace rc {
 // true when the routed experts read int8 activation digits (so a caller may quantise before an exchange and hand the digits in)
-// (for a call over ntok gathered tokens: the tcgen05 kernel of large chunks prepares its own fp16 digits from the fp32 rows)
+// (for a call over ntok gathered tokens: the tcgen05 kernel of large chunks prepares its own fp16 digits from the fp32 rows, and a layer
+// with wide digits takes the rows as well: its digits are as many bytes)
 bool moe_takes_digits(redcuda_moe *m, uint32_t ntok) {
     moe_choose_path(m, ntok * m->d.top_k, false);
-    return moe_experts_mma(m) && !m->tc_now;
+    return moe_experts_mma(m) && !m->tc_now && !moe_wide(m);
 }
 // The shard's experts over gathered tokens: x [ntok][hidden] fp32, or (when xq is given) its digits xq [ntok][3][hidden] with
 // scales sx [ntok]; ids / w [ntok][top_k] contiguous. out [ntok][hidden] as k_ep_combine defines it.
@@ -774,12 +793,12 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
              upload_matrix(d.type_sh, d.hidden, d.ffn_sh, d.sh_down, dev, W + o_shd, scratch.as<uint8_t>(), s);
     // expert matrices: GGUF rows -> planar, matrix by matrix, or -> the nibble layout, as many matrices at once as lie in device memory
     auto put = [&](uint32_t type, uint32_t nrows, uint32_t ncols, size_t raw_bytes, const uint8_t *src, uint8_t *dst, uint64_t dst_bytes) -> int {
-        if (m->nib && dev) return launch_nib_repack(nib_fmt(type), src, (uint64_t)nrows * d.expert_count, ncols, dst, s);
+        if (m->nib && dev) return launch_nib_repack(nib_fmt(m, type), src, (uint64_t)nrows * d.expert_count, ncols, dst, s);
         for (uint32_t e = 0; e < d.expert_count; ++e) {
             const uint8_t *se = src + (size_t)e * raw_bytes;
             if (!m->nib) { if (!upload_matrix(type, nrows, ncols, se, dev, dst + (size_t)e * dst_bytes, scratch.as<uint8_t>(), s)) return 0; continue; }
             RC_CUDA(cudaMemcpyAsync(scratch.p, se, raw_bytes, cudaMemcpyHostToDevice, s));
-            if (!launch_nib_repack(nib_fmt(type), scratch.as<uint8_t>(), nrows, ncols, dst + (size_t)e * dst_bytes, s)) return 0;
+            if (!launch_nib_repack(nib_fmt(m, type), scratch.as<uint8_t>(), nrows, ncols, dst + (size_t)e * dst_bytes, s)) return 0;
         }
         return 1;
     };
@@ -794,7 +813,8 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
     if (B) m->ws_shared = true;
     else { if (!m->ws.alloc(w)) return bail(); B = m->ws.as<uint8_t>(); }
     moe_ws_layout(d, m, B);
-    m->tc_ok = m->nib && tcx_shape_ok(d.ffn, d.hidden) && tcx_shape_ok(d.hidden, d.ffn);
+    // the tcgen05 expert kernel works on 22-bit digits and truncating accumulators (8.2e-7 against 64-bit sums): not for layers that had fp32
+    m->tc_ok = m->nib && !moe_wide(m) && tcx_shape_ok(d.ffn, d.hidden) && tcx_shape_ok(d.hidden, d.ffn);
     {   // RC_MOE_PATH=cuda keeps the IQ2_XXS experts on the CUDA-core kernels (A/B switch for profiling)
         const char *pth = getenv("RC_MOE_PATH");
         m->use_mma = !(pth && pth[0] == 'c');
@@ -888,7 +908,7 @@ int redcuda_moe_partial_device(redcuda_moe *m, uint32_t ntok, const float *x_dev
     const uint32_t k = m->d.top_k, npairs = ntok * k;
     moe_choose_path(m, npairs, false);
     const bool xq = moe_experts_mma(m) && !m->tc_now;
-    if (xq && !launch_quant_act(x_dev, x_stride, ntok, m->d.hidden, m->xq_x, m->sx_x, s)) return 0;
+    if (xq && !moe_quant_rows(m, x_dev, x_stride, ntok, m->d.hidden, m->xq_x, m->sx_x, s)) return 0;
     prof_begin("moe_mask_weights", s);
     RC_LAUNCH((k_mask_weights), (npairs + 255u) / 256u, 256, 0, s, ids_dev, weights_dev, ntok, k, meta_stride, m->d.expert_begin, m->d.expert_stride, m->d.expert_count, m->ids, m->wk);
     prof_end(s);

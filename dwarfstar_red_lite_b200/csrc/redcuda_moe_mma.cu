@@ -118,6 +118,38 @@ int launch_quant_act(const float *x, uint32_t x_stride, uint32_t rows, uint32_t 
     return 1;
 }
 
+// The wide form: one warp per row and 256-column block, 8 values a lane. xq[row][4][ncols], sx[row][ncols / 256]
+__global__ void __launch_bounds__(256) k_quant_act_wide(const float *__restrict__ x, uint32_t x_stride, uint32_t nblocks, uint32_t bpr,
+                                                        int8_t *__restrict__ xq, float *__restrict__ sx) {
+    pdl_prologue();
+    const uint32_t i = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (i >= nblocks) return;
+    const uint32_t row = i / bpr, b = i - row * bpr;
+    const float *xr = x + (size_t)row * x_stride + b * 256u + lane * 8u;
+    const float4 v0 = *reinterpret_cast<const float4 *>(xr), v1 = *reinterpret_cast<const float4 *>(xr + 4);
+    float up;
+    const float scale = actw_scale(__reduce_max_sync(0xffffffffu, max(act_mag4(v0), act_mag4(v1))), up);
+    if (lane == 0u) sx[i] = scale;
+    const uint32_t w0[4] = {actw_digits(v0.x, up), actw_digits(v0.y, up), actw_digits(v0.z, up), actw_digits(v0.w, up)};
+    const uint32_t w1[4] = {actw_digits(v1.x, up), actw_digits(v1.y, up), actw_digits(v1.z, up), actw_digits(v1.w, up)};
+    uint32_t p0[4], p1[4];
+    actw_planes(w0, p0); actw_planes(w1, p1);
+    int8_t *q = xq + (size_t)row * 4u * (bpr * 256u) + b * 256u + lane * 8u;
+#pragma unroll
+    for (uint32_t dg = 0; dg < 4u; ++dg) *reinterpret_cast<uint2 *>(q + (size_t)dg * (bpr * 256u)) = make_uint2(p0[dg], p1[dg]);
+}
+
+int launch_quant_act_wide(const float *x, uint32_t x_stride, uint32_t rows, uint32_t ncols, int8_t *xq, float *sx, cudaStream_t s) {
+    RC_REQUIRE(ncols % 256u == 0 && ncols && x_stride % 4u == 0, "quant_act: rows of %u columns (stride %u) are not blocks of 256", ncols, x_stride);
+    if (!rows) return 1;
+    const uint32_t nblocks = rows * (ncols / 256u);
+    prof_begin("moe_quant_act", s);
+    RC_LAUNCH((k_quant_act_wide), (nblocks + 7u) / 8u, 256, 0, s, x, x_stride, nblocks, ncols / 256u, xq, sx);
+    prof_end(s);
+    RC_LAUNCHED();
+    return 1;
+}
+
 // ---- small PTX wrappers ----
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);

@@ -13,15 +13,15 @@ struct MmaArgs {
     uint32_t *status;              // sticky status words (redcuda_common.cuh), may be null
     const uint32_t *sorted, *uexp, *ustart;              // pairs grouped by expert (k_group_pairs)
     const uint32_t *item_u, *item_p0, *n_items;          // work items: expert slot and first pair of up to `TOK` pairs
-    const int8_t *xq;              // activation digits [row][3][ncols]; row of pair p = p / x_div
-    const float *sx;               // activation scale per row
+    const int8_t *xq;              // activation digits [row][3][ncols] (wide form [row][4][ncols]); row of pair p = p / x_div
+    const float *sx;               // activation scale per row (wide form: per row and 256-column block)
     uint32_t x_div;
     float *out; uint32_t out_stride;                     // result row of pair p = out + p * out_stride
     const uint2 *lut_grid; const uint4 *lut_sign;        // filled by launch_moe_mma
     uint32_t S, tiles_per_warp, item_tok, item_class;    // filled by launch_moe_mma
     float dw1, dw2;                // weights of digits 1 and 2 (2^bits, 4^bits), filled by launch_moe_mma
     uint32_t *work;                // nibble-layout kernels: the launch's unit counter, zeroed by the grouping kernel
-    uint32_t fmt;                  // nibble-layout kernels: NIB_IQ2 or NIB_IQ3
+    uint32_t fmt;                  // nibble-layout kernels: NIB_IQ2, NIB_IQ3 or NIB_IQ2W
     const float *x_raw;            // nibble-layout gate/up of a single token: its fp32 activation row, quantised inside the kernel (xq / sx unused)
     uint32_t act_bits;             // digit width, filled by the launcher
 };
@@ -33,6 +33,8 @@ int mma_set_luts(const uint8_t *iq2_grid_host);
 uint32_t act_digit_bits();
 // x[rows][x_stride] (first ncols of each row) -> digits xq[rows][3][ncols] and scales sx[rows]
 int launch_quant_act(const float *x, uint32_t x_stride, uint32_t rows, uint32_t ncols, int8_t *xq, float *sx, cudaStream_t s);
+// the wide form: digits xq[rows][4][ncols] and scales sx[rows][ncols / 256]
+int launch_quant_act_wide(const float *x, uint32_t x_stride, uint32_t rows, uint32_t ncols, int8_t *xq, float *sx, cudaStream_t s);
 // Pairs one work item of the tensor-core expert kernel covers: 2 in the few-token configuration, 8 for a decode batch,
 // 16 when the experts see many pairs each (prefill chunks, expert-parallel shards): an expert's weights are decoded
 // once per item, so larger items halve that work where most experts would otherwise need two.
@@ -41,8 +43,11 @@ uint32_t mma_item_tokens(bool few_tokens, uint32_t npairs = 0u, uint32_t n_exper
 int launch_moe_mma(MmaArgs &A, uint32_t max_items, uint32_t item_tok, cudaStream_t s);
 // ---- nibble layout of IQ2_XXS / IQ3_S expert matrices (redcuda_moe_nib.cu): 138 bytes per 256 weights, table-free decode ----
 constexpr uint32_t NIB_BLOCK_BYTES = 138u;
-// what the 4-bit codes of a matrix mean (a template parameter of the kernels)
-constexpr uint32_t NIB_IQ2 = 0u, NIB_IQ3 = 1u;
+// What the 4-bit codes of a matrix mean and which digits its activations have (a template parameter of the kernels). NIB_IQ2:
+// three digits of 8 bits per value and one scale per row, as k_quant_act makes them. The other two are the wide form: four digits
+// and a power-of-two scale per 256-column block (k_quant_act_wide). NIB_IQ2W: IQ2_XXS codes of a layer whose other matrices are IQ3_S.
+constexpr uint32_t NIB_IQ2 = 0u, NIB_IQ3 = 1u, NIB_IQ2W = 2u;
+constexpr uint32_t NIB_WIDE_PAIRS = 6u;      // pairs of a work item in the wide form: four digits each fill the 24 columns of three tiles
 // one record = one 16-row tile x one 256-column block
 constexpr uint32_t NIB_SC_OFF = 2048u, NIB_D_OFF = 2176u, NIB_REC = 2208u;
 // byte offset of code word (t, kg) of row rr inside a record (16-byte piece p of row rr is stored at p ^ (rr % 8))
@@ -52,10 +57,10 @@ __host__ __device__ __forceinline__ uint32_t nib_code_off(uint32_t rr, uint32_t 
 }
 uint64_t nib_matrix_bytes(uint32_t nrows, uint32_t ncols);
 bool nib_shape_ok(uint32_t nrows, uint32_t ncols);
-// GGUF rows of IQ2_XXS (NIB_IQ2) or IQ3_S (NIB_IQ3), one matrix or several in a row (nrows = all their rows) -> nibble layout
+// GGUF rows of IQ2_XXS (NIB_IQ2, NIB_IQ2W) or IQ3_S (NIB_IQ3), one matrix or several in a row (nrows = all their rows) -> nibble layout
 // (dst: nib_matrix_bytes, 16-byte aligned)
 int launch_nib_repack(uint32_t fmt, const uint8_t *raw, uint64_t nrows, uint32_t ncols, uint8_t *dst, cudaStream_t s);
-// gate/up (A.w1 set) or down projection of the grouped pairs, work items of at most 8 pairs; persistent kernel
+// gate/up (A.w1 set) or down projection of the grouped pairs, work items of at most 8 pairs (wide form: NIB_WIDE_PAIRS); persistent kernel
 int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s);
 // Single token, nibble layout: down projection of the token's top_k experts for one 16-row tile per block, the shared
 // expert's down rows, and the tail out = resid + sum_k w_k * expert_k + shared * scalar, in router order — the fusion of
@@ -69,7 +74,7 @@ struct NibTailArgs {
     const float *sh_act, *scalar, *resid;             // shared activation [ncols], its scalar gate [1], residual [nrows] or null
     float *out;
     float dw1, dw2; uint32_t bits;                    // filled by the launcher
-    uint32_t fmt;                                     // NIB_IQ2 or NIB_IQ3
+    uint32_t fmt;                                     // NIB_IQ2, NIB_IQ3 or NIB_IQ2W
     uint32_t *status;
 };
 bool nib_tail_ok(uint32_t top_k, uint32_t nrows, uint32_t ncols);
@@ -90,6 +95,25 @@ __device__ __forceinline__ void act_digits(float f, float inv, float qmax, uint3
     d0 = ((iv + half) & mask) - half; iv = (iv - d0) >> bits;
     d1 = ((iv + half) & mask) - half; iv = (iv - d1) >> bits;
     d2 = iv;
+}
+
+// The wide form, for layers whose activations were multiplied in fp32 before they came to the digit kernels (IQ3_S). A 24-bit fixed
+// point per ROW loses the small elements of a row with a large one. Here a block of 256 columns, which a weight row scales by one d
+// as well, has a power-of-two scale that puts its largest magnitude into [2^29, 2^30): elements down to 2^-6 of that are exact and
+// the others are within 2^-31 of it, below the rounding of a single fp32 product with any weight of the block (their magnitudes
+// lie within a factor of 465). up: the multiplier; the returned scale undoes it. Blocks below 2^-97 keep fewer bits: their quantum
+// is 2^-127.
+__device__ __forceinline__ float actw_scale(uint32_t mx, float &up) {
+    const int e = min(29 - ((int)(mx >> 23) - 127), 126);
+    up = __uint_as_float((uint32_t)(e + 127) << 23);
+    return mx < 0x7f800000u ? __uint_as_float((uint32_t)(127 - e) << 23) : __uint_as_float(0x7fffffffu);
+}
+// byte i of a word: digit i of the value. Adding 128 to every digit makes all bytes non-negative, so that the carries resolve themselves.
+__device__ __forceinline__ uint32_t actw_digits(float f, float up) { return ((uint32_t)__float2int_rn(f * up) + 0x80808080u) ^ 0x80808080u; }
+// the digit words of four values -> plane[i] = digit i of the four
+__device__ __forceinline__ void actw_planes(const uint32_t (&w)[4], uint32_t (&plane)[4]) {
+    const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140), c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);
+    plane[0] = __byte_perm(a, b, 0x5410); plane[1] = __byte_perm(a, b, 0x7632); plane[2] = __byte_perm(c, d, 0x5410); plane[3] = __byte_perm(c, d, 0x7632);
 }
 #endif
 

@@ -25,6 +25,11 @@
 //   d      @2176  16 fp16 block scales
 // Arithmetic is the integer tensor-core scheme of redcuda_moe_mma.cu (mma.sync m16n8k32 s8, activations as three
 // balanced digits per value, s32 sums per 32-weight group scaled by the integer 2s+1, fp32 scaling by d/8 per block).
+// Layers with IQ3_S matrices take the wide form of the digits (actw_scale in redcuda_moe_mma.cuh): four per value and a scale per
+// 256-column block, applied with d / 8. On the CUDA-core kernel they had fp32 rows; relative errors of an expert's output against
+// 64-bit sums (hidden 2048, ffn 512, rows from Gaussian to one element of 10000): fp32 rows 1.3e-7 to 2.1e-7, wide digits 0.8e-7
+// to 1.2e-7. The fourth digit costs nothing where items hold one or two pairs, which fill one tile either way (24 tokens: 118 us a
+// layer with four, 120 with three).
 //
 // Kernel: persistent CTAs of 8 warps, two per SM. A unit of work = one work item (<= 8 pairs of one expert, cut by
 // k_group_pairs) x a block of rows; CTAs draw units from an atomic counter, so the routing skew never leaves SMs idle
@@ -33,7 +38,8 @@
 // boundaries). Waits on the mbarriers are bounded: a warp that gives up raises the status word and the CTA winds down.
 // Column layout of the digits: items of one or two pairs pack (pair, digit) into one 8-column tile (cols 3*pair+digit);
 // larger items use one tile per digit (col = 8*digit + pair), so a lane holds all three digits of its two pairs and the
-// epilogue needs no exchange.
+// epilogue needs no exchange. Wide form: col = 4*pair + digit, two pairs a tile and as many tiles as the item's pairs need (one to
+// three); the two lanes that hold a pair's digits exchange one sum each at the end of a tile.
 #define RC_PDL_DEFAULT 0
 #include "redcuda_common.cuh"
 #include "redcuda_dot.cuh"
@@ -62,9 +68,9 @@ __global__ void k_nib_repack(const uint8_t *__restrict__ raw, uint64_t nb, uint3
         const uint32_t kg = ((uint32_t)i >> 2) & 7u, t = (uint32_t)i & 3u;
         const uint64_t row = b / bpr;
         const uint32_t blk = (uint32_t)(b - row * bpr);
-        const uint8_t *bp = raw + b * (FMT == NIB_IQ2 ? 66u : 110u);
+        const uint8_t *bp = raw + b * (FMT == NIB_IQ3 ? 110u : 66u);
         uint32_t word = 0u, s4;
-        if (FMT == NIB_IQ2) {
+        if (FMT != NIB_IQ3) {
             const unsigned short *q = reinterpret_cast<const unsigned short *>(bp + 2u + kg * 8u);
             const uint32_t auxs = (uint32_t)q[2] | ((uint32_t)q[3] << 16);
             const uint8_t *gv = bk.iq2 + (uint32_t)bp[2u + kg * 8u + t] * 8u;
@@ -103,7 +109,7 @@ int launch_nib_repack(uint32_t fmt, const uint8_t *raw, uint64_t nrows, uint32_t
     const uint32_t grid = (uint32_t)((total + 255u) / 256u < 148u * 16u ? (total + 255u) / 256u : 148u * 16u);
     prof_begin("nib_repack", s);
     const RcBooks bk{books_iq2(), books_iq3s()};
-    if (fmt == NIB_IQ2) RC_LAUNCH((k_nib_repack<NIB_IQ2>), grid ? grid : 1u, 256, 0, s, raw, nb, ncols / 256u, bk, dst);
+    if (fmt != NIB_IQ3) RC_LAUNCH((k_nib_repack<NIB_IQ2>), grid ? grid : 1u, 256, 0, s, raw, nb, ncols / 256u, bk, dst);
     else RC_LAUNCH((k_nib_repack<NIB_IQ3>), grid ? grid : 1u, 256, 0, s, raw, nb, ncols / 256u, bk, dst);
     prof_end(s);
     RC_LAUNCHED();
@@ -181,23 +187,25 @@ __device__ __forceinline__ void nb_expand<NIB_IQ2>(uint32_t w, uint32_t &lo, uin
     lo = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, w); hi = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, w >> 16);
 }
 template <>
+__device__ __forceinline__ void nb_expand<NIB_IQ2W>(uint32_t w, uint32_t &lo, uint32_t &hi) { nb_expand<NIB_IQ2>(w, lo, hi); }
+template <>
 __device__ __forceinline__ void nb_expand<NIB_IQ3>(uint32_t w, uint32_t &lo, uint32_t &hi) {
     lo = ((w << 4) & 0xf0f0f0f0u) | 0x08080808u; hi = (w & 0xf0f0f0f0u) | 0x08080808u;
 }
 
 // One warp: 16 rows x one 256-column block (a record in shared memory) against NT 8-column tiles of activation digits.
 // Bl: digits of column g of tile 0 at this block's first column + 8 t (tile n is n * 8 * BPITCH further).
+// blk[n]: sums of rows g (0, 1) and g + 8 (2, 3), columns 2 t and 2 t + 1 of tile n; da, db: d / 8 of the two rows.
 template <uint32_t FMT, int NT, uint32_t BPITCH>
-__device__ __forceinline__ void nib_chunk(const uint8_t *st, const int8_t *Bl, uint32_t g, uint32_t t, const int (&z)[4], float (&out)[3][4]) {
+__device__ __forceinline__ void nib_sums(const uint8_t *st, const int8_t *Bl, uint32_t g, uint32_t t, const int (&z)[4], int (&blk)[NT][4], float &da, float &db) {
     const uint32_t o0 = nib_code_off(g, t, 0u), o1 = nib_code_off(g, t, 4u);   // rows g and g + 8 have the same swizzle
     const uint4 qa0 = *reinterpret_cast<const uint4 *>(st + o0), qa1 = *reinterpret_cast<const uint4 *>(st + o1);
     const uint4 qb0 = *reinterpret_cast<const uint4 *>(st + 1024u + o0), qb1 = *reinterpret_cast<const uint4 *>(st + 1024u + o1);
     const uint2 sa = *reinterpret_cast<const uint2 *>(st + NIB_SC_OFF + g * 8u), sb = *reinterpret_cast<const uint2 *>(st + NIB_SC_OFF + (g + 8u) * 8u);
-    const float da = 0.125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(st + NIB_D_OFF + g * 2u)));
-    const float db = 0.125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(st + NIB_D_OFF + (g + 8u) * 2u)));
+    da = 0.125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(st + NIB_D_OFF + g * 2u)));
+    db = 0.125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(st + NIB_D_OFF + (g + 8u) * 2u)));
     const uint32_t wa[8] = {qa0.x, qa0.y, qa0.z, qa0.w, qa1.x, qa1.y, qa1.z, qa1.w};
     const uint32_t wb[8] = {qb0.x, qb0.y, qb0.z, qb0.w, qb1.x, qb1.y, qb1.z, qb1.w};
-    int blk[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n) { blk[n][0] = blk[n][1] = blk[n][2] = blk[n][3] = 0; }
 #pragma unroll
@@ -216,11 +224,37 @@ __device__ __forceinline__ void nib_chunk(const uint8_t *st, const int8_t *Bl, u
             blk[n][2] += scb * d[2]; blk[n][3] += scb * d[3];
         }
     }
+}
+template <uint32_t FMT, int NT, uint32_t BPITCH>
+__device__ __forceinline__ void nib_chunk(const uint8_t *st, const int8_t *Bl, uint32_t g, uint32_t t, const int (&z)[4], float (&out)[3][4]) {
+    int blk[NT][4];
+    float da, db;
+    nib_sums<FMT, NT, BPITCH>(st, Bl, g, t, z, blk, da, db);
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         out[n][0] += da * (float)blk[n][0]; out[n][1] += da * (float)blk[n][1];
         out[n][2] += db * (float)blk[n][2]; out[n][3] += db * (float)blk[n][3];
     }
+}
+// The wide form: column 4 p + i is digit i of pair p, so lane t holds two digits of pair 2 n + t / 2 of tile n, the upper two where
+// t is odd. sx[n * 2 * SXP]: that pair's scale of this block. out[n]: rows g and g + 8.
+template <uint32_t FMT, int NT, uint32_t BPITCH, uint32_t SXP>
+__device__ __forceinline__ void nib_chunk_wide(const uint8_t *st, const int8_t *Bl, const float *sx, uint32_t g, uint32_t t, const int (&z)[4], float (&out)[NT][2]) {
+    int blk[NT][4];
+    float da, db;
+    nib_sums<FMT, NT, BPITCH>(st, Bl, g, t, z, blk, da, db);
+    const float up = t & 1u ? 65536.0f : 1.0f;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        const float w = sx[n * 2u * SXP] * up;              // a power of two, as da and db times it are without rounding
+        out[n][0] += (da * w) * fmaf(256.0f, (float)blk[n][1], (float)blk[n][0]);
+        out[n][1] += (db * w) * fmaf(256.0f, (float)blk[n][3], (float)blk[n][2]);
+    }
+}
+// a lane's row g and g + 8 sums of its two digits -> the full sum of row g (even t) or g + 8 (odd t)
+__device__ __forceinline__ float nib_pair_sum(float r0, float r1, uint32_t t) {
+    const float got = __shfl_xor_sync(0xffffffffu, t & 1u ? r0 : r1, 1);
+    return (t & 1u ? r1 : r0) + got;
 }
 
 struct NibUnit {
@@ -296,6 +330,25 @@ __device__ __forceinline__ void nib_tiles(NibRing &R, const uint8_t *my_stage, c
     }
 }
 
+// The wide form, NT = tiles in use (two pairs each). vals[ti][n] = row g (even t) or g + 8 (odd t) of pair 2 n + t / 2.
+template <uint32_t FMT, int NT, uint32_t BPR, uint32_t BPITCH, uint32_t TPW, uint32_t STAGES>
+__device__ __forceinline__ void nib_tiles_wide(NibRing &R, const uint8_t *my_stage, const int8_t *Bbase, const float *sx, uint32_t tiles, uint32_t lane, uint32_t g, uint32_t t,
+                                               const int (&z)[4], float (&vals)[TPW][4]) {
+    for (uint32_t ti = 0; ti < tiles; ++ti) {
+        float out[NT][2];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) out[n][0] = out[n][1] = 0.f;
+        for (uint32_t c = 0; c < BPR; ++c) {
+            nib_request<STAGES>(R, lane);
+            const uint32_t slot = nib_acquire(R);
+            nib_chunk_wide<FMT, NT, BPITCH, BPR>(my_stage + slot * NIB_REC, Bbase + c * 256u, sx + c, g, t, z, out);
+            nib_release<STAGES>(R);
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) vals[ti][n] = nib_pair_sum(out[n][0], out[n][1], t);
+    }
+}
+
 // GATEUP: warps 0-3 take the gate rows of 4 x TPW tiles, warps 4-7 the up rows of the same tiles; the up values cross a
 // small shared buffer and the gate warps store SiLU(gate) * up. Otherwise (down projection) 8 x TPW tiles per unit.
 template <uint32_t FMT, bool GATEUP, uint32_t NCOLS, uint32_t STAGES>
@@ -305,6 +358,8 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
     constexpr uint32_t BPR = NCOLS / 256u, TPW = BPR >= 8u ? 1u : 8u / BPR, WSLOTS = GATEUP ? 4u : 8u, UNIT_TILES = WSLOTS * TPW;
     constexpr uint32_t BPITCH = NCOLS + 32u, V16 = NCOLS / 16u;
     constexpr bool ONE = STAGES == NIB_STAGES_ONE;        // the form of a single token: A.x_raw holds it
+    constexpr bool WIDE = FMT != NIB_IQ2;
+    __shared__ float s_sxw[WIDE ? (ONE ? 1u : NIB_WIDE_PAIRS) * BPR : 1u];      // scales of the item's pairs and blocks
     __shared__ uint32_t s_unit[2];
     __shared__ volatile uint32_t s_fail;
     __shared__ __align__(8) uint64_t s_bar[NIB_WARPS][STAGES];
@@ -355,7 +410,24 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
     }
     __shared__ uint32_t s_red[NIB_WARPS];
     __shared__ float s_sx;
-    if (ONE) {
+    if (ONE && WIDE) {
+        // a warp per block of the row; columns 0..3 of the one tile in use, columns 4..7 zero
+        if (warp < BPR) {
+            const uint32_t k = warp * 256u + lane * 8u;
+            const float4 v0 = *reinterpret_cast<const float4 *>(A.x_raw + k), v1 = *reinterpret_cast<const float4 *>(A.x_raw + k + 4u);
+            float up;
+            const float scale = actw_scale(__reduce_max_sync(0xffffffffu, max(act_mag4(v0), act_mag4(v1))), up);
+            if (lane == 0) s_sxw[warp] = scale;
+            const uint32_t w0[4] = {actw_digits(v0.x, up), actw_digits(v0.y, up), actw_digits(v0.z, up), actw_digits(v0.w, up)};
+            const uint32_t w1[4] = {actw_digits(v1.x, up), actw_digits(v1.y, up), actw_digits(v1.z, up), actw_digits(v1.w, up)};
+            uint32_t p0[4], p1[4];
+            actw_planes(w0, p0); actw_planes(w1, p1);
+#pragma unroll
+            for (uint32_t col = 0u; col < 8u; ++col)
+                *reinterpret_cast<uint2 *>(Bs + col * BPITCH + k) = col < 4u ? make_uint2(p0[col & 3u], p1[col & 3u]) : make_uint2(0u, 0u);
+        }
+        __syncthreads();
+    } else if (ONE) {
         // single token: every unit multiplies the same activation row, so the block turns it into digits itself (the
         // arithmetic of k_quant_act) — columns 0..2 of the one tile in use, columns 3..7 zero
         uint32_t mx = 0u;
@@ -394,22 +466,36 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
         for (uint32_t i = ahead; i + 1u < STAGES; ++i) nib_request<STAGES>(R, lane);
         const bool packed = I.nt <= 2u;
         if (!ONE && I.item != cur_item) {    // activation digits of the item (every warp passed the barrier that ended the last unit)
-            const uint32_t ncolb = packed ? 8u : 24u;
+            const uint32_t ncolb = WIDE ? (I.nt + 1u) / 2u * 8u : packed ? 8u : 24u;
             for (uint32_t i = tid; i < ncolb * V16; i += NIB_WARPS * 32u) {
                 const uint32_t col = i / V16, k = (i - col * V16) << 4;
-                const uint32_t tk = packed ? col / 3u : (col & 7u), dg = packed ? col - 3u * (col / 3u) : (col >> 3);
+                const uint32_t tk = WIDE ? col >> 2 : packed ? col / 3u : (col & 7u), dg = WIDE ? col & 3u : packed ? col - 3u * (col / 3u) : (col >> 3);
                 uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (tk < I.nt) v = *reinterpret_cast<const uint4 *>(A.xq + ((size_t)(A.sorted[I.p0 + tk] / A.x_div) * 3u + dg) * NCOLS + k);
+                if (tk < I.nt) v = *reinterpret_cast<const uint4 *>(A.xq + ((size_t)(A.sorted[I.p0 + tk] / A.x_div) * (WIDE ? 4u : 3u) + dg) * NCOLS + k);
                 *reinterpret_cast<uint4 *>(Bs + (size_t)col * BPITCH + k) = v;
+            }
+            if (WIDE && tid < NIB_WIDE_PAIRS * BPR) {
+                const uint32_t tk = tid / BPR;
+                s_sxw[tid] = tk < I.nt ? A.sx[(size_t)(A.sorted[I.p0 + tk] / A.x_div) * BPR + (tid - tk * BPR)] : 0.f;
             }
             cur_item = I.item;
         }
-        // the pairs this lane stores: packed -> pair t/2 on even t; one tile per digit -> pairs 2t, 2t+1
-        uint32_t prow[2] = {0u, 0u};
+        // the pairs this lane stores: packed -> pair t/2 on even t; one tile per digit -> pairs 2t, 2t+1; wide -> pairs t/2, t/2 + 2, t/2 + 4
+        constexpr uint32_t NP = WIDE && !ONE ? NIB_WIDE_PAIRS / 2u : 2u;
+        uint32_t prow[NP];
         float sxv[2] = {0.f, 0.f};
-        bool ok[2];
+        bool ok[NP];
+        if (WIDE) {
+#pragma unroll
+            for (uint32_t j = 0; j < NP; ++j) {
+                const uint32_t tk = 2u * j + (t >> 1);
+                ok[j] = tk < I.nt;
+                prow[j] = ok[j] ? (ONE ? I.p0 : A.sorted[I.p0 + tk]) : 0u;
+            }
+        } else
 #pragma unroll
         for (uint32_t j = 0; j < 2u; ++j) {
+            prow[j] = 0u;
             const uint32_t tk = packed ? (t >> 1) : 2u * t + j;
             ok[j] = packed ? (j == 0u && (t & 1u) == 0u && tk < I.nt) : tk < I.nt;
             if (ok[j]) { prow[j] = ONE ? I.p0 : A.sorted[I.p0 + tk]; sxv[j] = ONE ? s_sx : A.sx[prow[j] / A.x_div]; }
@@ -422,7 +508,12 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
         float vals[TPW][4];
         const uint32_t tiles = I.n / BPR;
         const int8_t *Bbase = Bs + (size_t)g * BPITCH + 8u * t;
-        if (packed) nib_tiles<FMT, 1, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, tiles, lane, g, t, zero, A.dw1, A.dw2, sxv, vals);
+        if constexpr (WIDE) {
+            const float *sxw = s_sxw + (ONE ? 0u : (t >> 1) * BPR);
+            if (ONE || packed) nib_tiles_wide<FMT, 1, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, sxw, tiles, lane, g, t, zero, vals);
+            else if (I.nt <= 4u) nib_tiles_wide<FMT, 2, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, sxw, tiles, lane, g, t, zero, vals);
+            else nib_tiles_wide<FMT, 3, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, sxw, tiles, lane, g, t, zero, vals);
+        } else if (packed) nib_tiles<FMT, 1, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, tiles, lane, g, t, zero, A.dw1, A.dw2, sxv, vals);
         else nib_tiles<FMT, 3, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, tiles, lane, g, t, zero, A.dw1, A.dw2, sxv, vals);
         if (R.timed_out && lane == 0) { s_fail = 1u; if (A.status) A.status[ST_TIMEOUT] = 1u; }
         if (GATEUP) {
@@ -430,6 +521,10 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
         } else {
             for (uint32_t ti = 0; ti < tiles; ++ti) {
                 const uint32_t row = ((I.tile0 + ti) << 4) + g;
+                if (WIDE) {
+#pragma unroll
+                    for (uint32_t j = 0; j < NP; ++j) if (ok[j]) A.out[(size_t)prow[j] * A.out_stride + row + 8u * (t & 1u)] = vals[ti][j];
+                } else
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
                     if (ok[j]) {
@@ -445,6 +540,11 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
                 const float4 up = s_ex[ti][wslot][lane];
                 const float uv[4] = {up.x, up.y, up.z, up.w};
                 const uint32_t row = ((I.tile0 + ti) << 4) + g;
+                if (WIDE) {
+#pragma unroll
+                    for (uint32_t j = 0; j < NP; ++j)
+                        if (ok[j]) A.out[(size_t)prow[j] * A.out_stride + row + 8u * (t & 1u)] = (vals[ti][j] / (1.0f + expf(-vals[ti][j]))) * uv[j];
+                } else
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
                     if (ok[j]) {
@@ -469,13 +569,13 @@ template <uint32_t FMT, uint32_t NCOLS>
 __global__ void __launch_bounds__((NIB_TAIL_MAX_K + 2u) * 32u) k_nib_down_tail(const __grid_constant__ NibTailArgs A) {
     pdl_prologue();
     extern __shared__ __align__(16) uint8_t smem[];
-    constexpr uint32_t BPR = NCOLS / 256u, BPITCH = NCOLS + 32u, PER_LANE = NCOLS / 32u;
+    constexpr uint32_t BPR = NCOLS / 256u, BPITCH = NCOLS + 32u, PER_LANE = NCOLS / 32u, ND = FMT == NIB_IQ2 ? 3u : 4u;      // ND: digits of a value
     __shared__ __align__(8) uint64_t s_bar[NIB_TAIL_MAX_K];
     __shared__ float s_part[NIB_TAIL_MAX_K][16], s_sh[16];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u, K = A.top_k;
     uint8_t *recs = smem;                                                    // [K][BPR] records
-    int8_t *digits = reinterpret_cast<int8_t *>(smem + K * BPR * NIB_REC);   // [K][3][BPITCH]
-    int8_t *zrow = digits + K * 3u * BPITCH;                                 // one row of zeros: digit columns 3..7 of every tile
+    int8_t *digits = reinterpret_cast<int8_t *>(smem + K * BPR * NIB_REC);   // [K][ND][BPITCH]
+    int8_t *zrow = digits + K * ND * BPITCH;                                 // one row of zeros: the digit columns from ND on of every tile
     float *xs = reinterpret_cast<float *>(zrow + BPITCH);                    // shared expert's activation, padded rows of redcuda_dot.cuh
     const uint32_t row0 = blockIdx.x * 16u;
 
@@ -506,16 +606,31 @@ __global__ void __launch_bounds__((NIB_TAIL_MAX_K + 2u) * 32u) k_nib_down_tail(c
         // this expert's activation row -> digits (the arithmetic of k_quant_act), while the records are in flight
         const float *ar = A.act + (size_t)warp * A.act_stride;
         float v[PER_LANE];
-        uint32_t mx = 0u;
+        uint32_t mx = 0u, mxb[BPR];        // of the row, of its blocks
+#pragma unroll
+        for (uint32_t c = 0; c < BPR; ++c) mxb[c] = 0u;
 #pragma unroll
         for (uint32_t i = 0; i < PER_LANE / 4u; ++i) {
             const float4 q = *reinterpret_cast<const float4 *>(ar + lane * 4u + 128u * i);
             v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
-            mx = max(mx, act_mag4(q));
+            mx = max(mx, act_mag4(q)); mxb[i / 2u] = max(mxb[i / 2u], act_mag4(q));
         }
         mx = __reduce_max_sync(0xffffffffu, mx);
         const float qmax = act_qmax(A.bits), sx = act_scale(mx, qmax), inv = 1.0f / sx;
-        int8_t *mine = digits + warp * 3u * BPITCH;
+        int8_t *mine = digits + warp * ND * BPITCH;
+        float sxb[BPR];
+        if (ND == 4u) {
+#pragma unroll
+            for (uint32_t i = 0; i < PER_LANE / 4u; ++i) {
+                float up;
+                sxb[i / 2u] = actw_scale(i & 1u ? mxb[i / 2u] : (mxb[i / 2u] = __reduce_max_sync(0xffffffffu, mxb[i / 2u])), up);
+                const uint32_t w[4] = {actw_digits(v[4 * i], up), actw_digits(v[4 * i + 1], up), actw_digits(v[4 * i + 2], up), actw_digits(v[4 * i + 3], up)};
+                uint32_t pl[4];
+                actw_planes(w, pl);
+#pragma unroll
+                for (uint32_t dg = 0; dg < 4u; ++dg) *reinterpret_cast<uint32_t *>(mine + dg * BPITCH + lane * 4u + 128u * i) = pl[dg];
+            }
+        } else
 #pragma unroll
         for (uint32_t i = 0; i < PER_LANE / 4u; ++i) {
             uint32_t p0 = 0, p1 = 0, p2 = 0;
@@ -537,13 +652,22 @@ __global__ void __launch_bounds__((NIB_TAIL_MAX_K + 2u) * 32u) k_nib_down_tail(c
         for (int n = 0; n < 3; ++n) { out[n][0] = out[n][1] = out[n][2] = out[n][3] = 0.f; }
         int zero[4];
         asm volatile("mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;" : "=r"(zero[0]), "=r"(zero[1]), "=r"(zero[2]), "=r"(zero[3]));
-        const int8_t *Bl = (g < 3u ? mine + g * BPITCH : zrow) + 8u * t;       // columns 0..2 = the pair's three digits, the rest of the tile is zero
+        const int8_t *Bl = (g < ND ? mine + g * BPITCH : zrow) + 8u * t;       // columns 0 .. ND - 1 = the pair's digits, the rest of the tile is zero
+        if constexpr (ND == 4u) {
+            float ow[1][2] = {{0.f, 0.f}};
+            if (live)
+#pragma unroll
+                for (uint32_t c = 0; c < BPR; ++c) nib_chunk_wide<FMT, 1, BPITCH, 0u>(my_rec + c * NIB_REC, Bl + c * 256u, &sxb[c], g, t, zero, ow);
+            const float r = nib_pair_sum(ow[0][0], ow[0][1], t);
+            if (t < 2u) s_part[warp][g + 8u * t] = r;
+        } else {
         if (live) for (uint32_t c = 0; c < BPR; ++c) nib_chunk<FMT, 1, BPITCH>(my_rec + c * NIB_REC, Bl + c * 256u, g, t, zero, out);
         const uint32_t src = (lane & ~3u) + 1u;
         const float x0 = __shfl_sync(0xffffffffu, out[0][0], src), x1 = __shfl_sync(0xffffffffu, out[0][2], src);
         if (t == 0u) {
             s_part[warp][g] = (out[0][0] + A.dw1 * out[0][1] + A.dw2 * x0) * sx;
             s_part[warp][g + 8u] = (out[0][2] + A.dw1 * out[0][3] + A.dw2 * x1) * sx;
+        }
         }
     } else if (A.sh_down) {
         const uint32_t sw = warp - K;                                       // 0 or 1: rows 8 sw .. 8 sw + 7 of the tile
@@ -577,7 +701,7 @@ int launch_nib_down_tail(NibTailArgs &A, cudaStream_t s) {
     RC_REQUIRE(nib_tail_ok(A.top_k, A.nrows, A.ncols), "nibble down tail: top_k %u, %ux%u is not a shape it serves", A.top_k, A.nrows, A.ncols);
     A.bits = act_digit_bits(); A.dw1 = (float)(1u << A.bits); A.dw2 = A.dw1 * A.dw1;
     const uint32_t bpr = A.ncols / 256u, bpitch = A.ncols + 32u;
-    const size_t smem = (size_t)A.top_k * bpr * NIB_REC + (size_t)A.top_k * 3u * bpitch + bpitch + (size_t)x_padded(A.ncols) * 4u + 16u;
+    const size_t smem = (size_t)A.top_k * bpr * NIB_REC + (size_t)A.top_k * (A.fmt == NIB_IQ2 ? 3u : 4u) * bpitch + bpitch + (size_t)x_padded(A.ncols) * 4u + 16u;
     const uint32_t threads = (A.top_k + 2u) * 32u, grid = A.nrows / 16u;
     // launched plainly: ahead of time its blocks would gather on the SMs that the 80 gate / up blocks of a top-10 layer leave free
     // (28.9 against 26.7 us a layer)
@@ -590,7 +714,8 @@ int launch_nib_down_tail(NibTailArgs &A, cudaStream_t s) {
         if (A.ncols == 256u) RC_TAIL_LAUNCH(256u); else if (A.ncols == 512u) RC_TAIL_LAUNCH(512u); else RC_TAIL_LAUNCH(1024u);
         return 1;
     };
-    if (!(A.fmt == NIB_IQ2 ? launch(std::integral_constant<uint32_t, NIB_IQ2>{}) : launch(std::integral_constant<uint32_t, NIB_IQ3>{}))) return 0;
+    if (!(A.fmt == NIB_IQ2 ? launch(std::integral_constant<uint32_t, NIB_IQ2>{}) : A.fmt == NIB_IQ3 ? launch(std::integral_constant<uint32_t, NIB_IQ3>{})
+                           : launch(std::integral_constant<uint32_t, NIB_IQ2W>{}))) return 0;
 #undef RC_TAIL_LAUNCH
     prof_end(s);
     RC_LAUNCHED();
@@ -604,7 +729,7 @@ static size_t nib_smem_bytes(uint32_t ncols, uint32_t stages) { return (size_t)N
 int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s) {
     const bool gateup = A.w1 != nullptr;
     RC_REQUIRE(nib_shape_ok(A.nrows, A.ncols), "nibble experts: matrix %ux%u is not tileable", A.nrows, A.ncols);
-    RC_REQUIRE(A.work != nullptr && A.item_tok >= 1u && A.item_tok <= 8u, "nibble experts: work counter missing or items of %u pairs", A.item_tok);
+    RC_REQUIRE(A.work != nullptr && A.item_tok >= 1u && A.item_tok <= (A.fmt == NIB_IQ2 ? 8u : NIB_WIDE_PAIRS), "nibble experts: work counter missing or items of %u pairs", A.item_tok);
     A.act_bits = act_digit_bits(); A.dw1 = (float)(1u << A.act_bits); A.dw2 = A.dw1 * A.dw1;
     RC_REQUIRE(!A.x_raw || (gateup && A.item_tok == 1u), "nibble experts: in-kernel quantisation serves the gate/up of a single token");
     static int sm_count = 0;
@@ -636,7 +761,8 @@ int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s) {
     }
     return 1;
     };
-    if (!(A.fmt == NIB_IQ2 ? launch(std::integral_constant<uint32_t, NIB_IQ2>{}) : launch(std::integral_constant<uint32_t, NIB_IQ3>{}))) return 0;
+    if (!(A.fmt == NIB_IQ2 ? launch(std::integral_constant<uint32_t, NIB_IQ2>{}) : A.fmt == NIB_IQ3 ? launch(std::integral_constant<uint32_t, NIB_IQ3>{})
+                           : launch(std::integral_constant<uint32_t, NIB_IQ2W>{}))) return 0;
 #undef RC_NIB_LAUNCH
     prof_end(s);
     RC_LAUNCHED();

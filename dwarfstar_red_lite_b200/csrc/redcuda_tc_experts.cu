@@ -44,13 +44,10 @@ __device__ __forceinline__ uint32_t tcx_prmt(uint32_t a, uint32_t b, uint32_t se
 
 // 8 codes (one word) times the group's integer scale -> 8 exact fp16 values. A code selects a biased byte u = 128 + w;
 // 0x6400 | u is the fp16 number 1024 + u, and (1024 + u) * sc - 1152 * sc = w * sc with one rounding of an exact integer.
-// NIB_IQ3 codes are bytes already: 128 + 8 (2 n + 1) is the masked nibble with its top bit flipped and 8 below it.
-template <uint32_t FMT>
 __device__ __forceinline__ uint4 tcx_decode8(uint32_t word, uint32_t sc) {
     const __half2 hs = __half2half2(__ushort2half_rn((unsigned short)sc));
     const __half2 hb = __hmul2(hs, __float2half2_rn(-1152.0f));
-    const uint32_t b0 = FMT == NIB_IQ2 ? tcx_prmt(TCX_TAB_POS, TCX_TAB_NEG, word) : ((word << 4) & 0xf0f0f0f0u) ^ 0x88888888u;
-    const uint32_t b1 = FMT == NIB_IQ2 ? tcx_prmt(TCX_TAB_POS, TCX_TAB_NEG, word >> 16) : (word & 0xf0f0f0f0u) ^ 0x88888888u;
+    const uint32_t b0 = tcx_prmt(TCX_TAB_POS, TCX_TAB_NEG, word), b1 = tcx_prmt(TCX_TAB_POS, TCX_TAB_NEG, word >> 16);
     uint32_t h[4] = {tcx_prmt(b0, 0x64646464u, 0x5140u), tcx_prmt(b0, 0x64646464u, 0x5342u), tcx_prmt(b1, 0x64646464u, 0x5140u), tcx_prmt(b1, 0x64646464u, 0x5342u)};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -148,7 +145,7 @@ constexpr uint32_t TCX_NB = 3u;               // activation stage buffers
 constexpr uint32_t TCX_KS = 128u, TCX_SUBS = TCX_KS / TC_KS, TCX_SPB = 256u / TCX_KS;      // stage width, tiles per stage, stages per 256-column block
 constexpr uint32_t TCX_W_GATHER = 1u, TCX_N_GATHER = 2u, TCX_W_RAW = 3u, TCX_W_DECODE = 4u, TCX_N_DECODE = 8u, TCX_W_DRAIN = 12u;
 
-template <uint32_t FMT, int TN>
+template <int TN>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_experts(const __grid_constant__ TcxArgs A) {
     pdl_prologue();
     const uint32_t item = blockIdx.y;
@@ -345,10 +342,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_experts(const __grid_const
                 const uint8_t *rec = raw + (r >> 4) * NIB_REC;
                 const uint4 wd = *reinterpret_cast<const uint4 *>(rec + nib_code_off(rr, t, kg0));
                 const uint32_t sc4 = *reinterpret_cast<const uint32_t *>(rec + NIB_SC_OFF + rr * 8u + kg0);
-                *reinterpret_cast<uint4 *>(abuf + tcx_sw128(r, t)) = tcx_decode8<FMT>(wd.x, sc4 & 255u);
-                *reinterpret_cast<uint4 *>(abuf + tcx_sw128(r, t + 4u)) = tcx_decode8<FMT>(wd.y, (sc4 >> 8) & 255u);
-                *reinterpret_cast<uint4 *>(abuf + A_SUB + tcx_sw128(r, t)) = tcx_decode8<FMT>(wd.z, (sc4 >> 16) & 255u);
-                *reinterpret_cast<uint4 *>(abuf + A_SUB + tcx_sw128(r, t + 4u)) = tcx_decode8<FMT>(wd.w, sc4 >> 24);
+                *reinterpret_cast<uint4 *>(abuf + tcx_sw128(r, t)) = tcx_decode8(wd.x, sc4 & 255u);
+                *reinterpret_cast<uint4 *>(abuf + tcx_sw128(r, t + 4u)) = tcx_decode8(wd.y, (sc4 >> 8) & 255u);
+                *reinterpret_cast<uint4 *>(abuf + A_SUB + tcx_sw128(r, t)) = tcx_decode8(wd.z, (sc4 >> 16) & 255u);
+                *reinterpret_cast<uint4 *>(abuf + A_SUB + tcx_sw128(r, t + 4u)) = tcx_decode8(wd.w, sc4 >> 24);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // generic-proxy writes -> visible to the tensor core
             __syncwarp();
@@ -430,13 +427,8 @@ int launch_tc_experts(TcxArgs &A, uint32_t max_items, const char *tag, cudaStrea
     const size_t smem = 2u * (size_t)TCX_SUBS * TC_A_DIGIT + (size_t)TCX_NB * TCX_SUBS * 2u * TN * TC_KS * 2u + 2u * (size_t)TCX_RAW;
     const dim3 grid(A.nmat * (A.nrows / TC_M / tcx_tiles_per_cta(A.nrows, A.ncols)), max_items);
     prof_begin(tag, s);
-    if (A.fmt == NIB_IQ2) {
-        RC_CUDA(cudaFuncSetAttribute(k_tc_experts<NIB_IQ2, (int)TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        RC_LAUNCH((k_tc_experts<NIB_IQ2, (int)TN>), grid, TC_THREADS, smem, s, A);
-    } else {
-        RC_CUDA(cudaFuncSetAttribute(k_tc_experts<NIB_IQ3, (int)TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        RC_LAUNCH((k_tc_experts<NIB_IQ3, (int)TN>), grid, TC_THREADS, smem, s, A);
-    }
+    RC_CUDA(cudaFuncSetAttribute(k_tc_experts<(int)TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RC_LAUNCH((k_tc_experts<(int)TN>), grid, TC_THREADS, smem, s, A);
     prof_end(s);
     RC_LAUNCHED();
     return 1;

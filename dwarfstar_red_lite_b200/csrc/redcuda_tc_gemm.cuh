@@ -44,7 +44,6 @@ constexpr uint32_t TCX_TN = 64u;
 struct TcxArgs {
     const uint8_t *w[2];            // nibble-layout matrices of the shard: (gate, up) or (down, null)
     uint64_t mat_bytes;             // bytes of one expert matrix
-    uint32_t fmt;                   // NIB_IQ2 or NIB_IQ3
     uint32_t nmat, nrows, ncols;    // matrices in this launch (1 or 2), rows / columns of one expert matrix
     uint32_t expert_begin, n_local;
     const uint32_t *sorted, *uexp, *ustart, *item_u, *item_p0, *n_items;    // grouping (k_group_pairs)

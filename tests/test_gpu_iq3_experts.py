@@ -1,7 +1,8 @@
 """IQ3_S (and mixed IQ3_S / IQ2_XXS) experts in the 4-bit layout of the expert kernels, against the CPU oracle: one token,
-the pair-packing limits of a work item (1, 2, 3, 8, 9 pairs), a batch, and the tcgen05 chunk kernel. Bounds: the operands
-are exact integers, activations are 24-bit fixed point (22 bits on the chunk kernel) and everything else is fp32, so a
-layer output is good to a few 1e-6 of its range; 2e-5 leaves room for the order of the sums."""
+pair counts around the limits of a work item, a batch, and batches that IQ2_XXS layers would hand to the tcgen05 chunk kernel
+(layers with IQ3_S matrices stay on the integer kernels). Bounds: the operands are exact integers, activations are 32-bit fixed
+point per 256-column block and everything else is fp32, so a layer output is good to a few 1e-6 of its range; 2e-5 leaves room
+for the order of the sums."""
 import numpy as np
 import pytest
 
