@@ -111,27 +111,30 @@ __global__ void k_dn_tail(DnDims D, const float *__restrict__ core, const float 
     out[idx] = x * inv * norm_w[i] * silu;
 }
 
-// The whole step of one value head in one block: grid (rank, batch), 8 warps, warp w owns the S / 8 consecutive state rows
-// w * S / 8 ... What bounds it is the state: one read and one write of 4 S^2 bytes per head (33.5 MB for 8 sequences of 32
-// heads of 128: 5.1 us at the copy rate). As separate kernels, preparation and state update took 13.7 us for them, because
-// the state was requested only after the preparation had ended. Here every lane first requests its conv windows and ALL
-// of its state rows (S / 8 rows x VPL floats: 64 registers at S = 128, the block's whole 64 KB in flight at once), and the
-// preparation (conv + SiLU, L2 norms, beta and gate: the arithmetic of k_dn_prep) runs while they arrive.
+// The whole step in one launch: SPLIT blocks per value head, 8 warps each, a warp owns consecutive state rows. What bounds it is the
+// state: one read and one write of 4 S^2 bytes per head (33.5 MB for 8 sequences of 32 heads of 128: 5.1 us at the copy rate). As
+// separate kernels, preparation and state update took 13.7 us for them, because the state was requested only after the
+// preparation had ended. Here every lane first requests its conv windows and its state rows (RING of them a warp: with one block
+// per head of 128 that is 64 registers and the block's whole 64 KB in flight), and the preparation (conv + SiLU, L2 norms, beta and
+// gate: the arithmetic of k_dn_prep) runs while they arrive.
 // The value heads of one key head all need its q and k. Their blocks form a cluster: each computes q and k for itself, and
 // the first one moves the conv windows of the q / k channels on after all of them have read the old ones (cluster barrier).
-template <int VPL, uint32_t DC>            // DC: conv taps known at compile time (0: D.d_conv)
-__global__ void __launch_bounds__(256, 2) k_dn_step(DnDims D, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,
+// One block per head leaves most of the chip idle for a few sequences (a single one: 32 blocks). There 2 or 4 blocks share a
+// head's rows and pass each other their parts of the norm's sum; launch_deltanet has the rule and its times.
+// DC: conv taps known at compile time (0: D.d_conv); MINB: blocks per SM that the registers allow
+template <int VPL, uint32_t DC, uint32_t SPLIT, int MINB, uint32_t RING>
+__global__ void __launch_bounds__(256, MINB) k_dn_step(DnDims D, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,
                                                     const float *__restrict__ qkv, const float *__restrict__ ba, float *conv_state, float *__restrict__ state,
                                                     const float *__restrict__ z, const float *__restrict__ norm_w, float *__restrict__ out) {
     pdl_prologue();
-    constexpr uint32_t S = VPL * 32u, RPW = S / 8u, TAPS = DC ? DC : 1u;
-    __shared__ float s_q[S], s_k[S], s_v[S], s_core[S], s_beta, s_gate;
+    constexpr uint32_t S = VPL * 32u, SB = S / SPLIT, RPW = SB / 8u, TAPS = DC ? DC : 1u;        // SB: state rows of this block
+    __shared__ float s_q[S], s_k[S], s_v[SB], s_core[SB], s_beta, s_gate;
     __shared__ double red[8], red2[8];
-    const uint32_t h = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t width = D.rank / D.groups, kh = h / width, first = h - kh * width == 0u, taps = DC ? DC : D.d_conv, ns = taps - 1u;
-    // conv channels of this thread: threads 0 .. S-1 the q channels, S .. 2S-1 the k channels of the key head; then 0 .. S-1 the head's v channels
-    const bool has_qk = tid < 2u * S, has_v = tid < S;
-    const uint32_t c_qk = (tid < S ? kh * S + tid : (D.groups + kh) * S + tid - S), c_v = 2u * D.groups * S + h * S + tid;
+    const uint32_t h = blockIdx.x / SPLIT, part = blockIdx.x % SPLIT, seq = blockIdx.y, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t width = D.rank / D.groups, kh = h / width, first = h - kh * width == 0u && part == 0u, taps = DC ? DC : D.d_conv, ns = taps - 1u;
+    // conv channels of this thread: threads 0 .. S-1 the q channels, S .. 2S-1 the k channels of the key head; then 0 .. SB-1 the v channels of the block's rows
+    const bool has_qk = tid < 2u * S, has_v = tid < SB;
+    const uint32_t c_qk = (tid < S ? kh * S + tid : (D.groups + kh) * S + tid - S), c_v = 2u * D.groups * S + h * S + part * SB + tid;
     float *const cs_base = conv_state + (size_t)seq * D.channels * ns;
     const float *const x_base = qkv + (size_t)seq * D.channels;
     float wq[TAPS], kq[TAPS], wv[TAPS], kv_[TAPS];                 // window + new sample, and the taps
@@ -141,12 +144,12 @@ __global__ void __launch_bounds__(256, 2) k_dn_step(DnDims D, const float *__res
     };
     if (DC && has_qk) window(c_qk, wq, kq);
     if (DC && has_v) window(c_v, wv, kv_);
-    float *rows = state + (((size_t)seq * D.rank + h) * S + (size_t)warp * RPW) * S;
-    float m[RPW][VPL];
+    float *rows = state + (((size_t)seq * D.rank + h) * S + part * SB + (size_t)warp * RPW) * S;
+    float m[RING][VPL];
     // volatile asm keeps these loads where they are written: all of them are issued before the first row is worked on
     // (left to itself the compiler fetches each row just before its use, with one row in flight per warp)
 #pragma unroll
-    for (uint32_t r = 0; r < RPW; ++r)
+    for (uint32_t r = 0; r < RING; ++r)
 #pragma unroll
         for (int t = 0; t < VPL; ++t) asm volatile("ld.global.f32 %0, [%1];" : "=f"(m[r][t]) : "l"(rows + (size_t)r * S + lane + 32 * t));
     __syncwarp();                      // a fixed point between the requests above and the shuffles below
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(256, 2) k_dn_step(DnDims D, const float *__res
     };
     const float y = has_qk ? conv_silu(c_qk, wq, kq) : 0.f;
     __syncwarp();
-    if (width > 1u) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // this block has read the key head's windows
+    if (SPLIT > 1u || width > 1u) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // this block has read the key head's windows
     double ss = (double)y * (double)y;
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if (lane == 0) red[warp] = ss;
@@ -187,7 +190,7 @@ __global__ void __launch_bounds__(256, 2) k_dn_step(DnDims D, const float *__res
         (tid < S ? s_q : s_k)[tid < S ? tid : tid - S] = (float)((double)y * inv);
     }
     __syncwarp();
-    if (width > 1u) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (SPLIT > 1u || width > 1u) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (first && has_qk) roll(c_qk);
     __syncthreads();
     float qv[VPL], kv[VPL];
@@ -198,30 +201,50 @@ __global__ void __launch_bounds__(256, 2) k_dn_step(DnDims D, const float *__res
     for (uint32_t r = 0; r < RPW; ++r) {
         float sum = 0.f;
 #pragma unroll
-        for (int t = 0; t < VPL; ++t) { m[r][t] = m[r][t] * decay; sum += m[r][t] * kv[t]; }
+        for (int t = 0; t < VPL; ++t) { m[r % RING][t] = m[r % RING][t] * decay; sum += m[r % RING][t] * kv[t]; }
         for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         const float delta = (s_v[warp * RPW + r] - sum) * bh;
         float o_acc = 0.f;
 #pragma unroll
-        for (int t = 0; t < VPL; ++t) { m[r][t] += kv[t] * delta; o_acc += m[r][t] * qv[t]; rows[(size_t)r * S + lane + 32 * t] = m[r][t]; }
+        for (int t = 0; t < VPL; ++t) { m[r % RING][t] += kv[t] * delta; o_acc += m[r % RING][t] * qv[t]; rows[(size_t)r * S + lane + 32 * t] = m[r % RING][t]; }
+        if (r + RING < RPW) {
+#pragma unroll
+            for (int t = 0; t < VPL; ++t) asm volatile("ld.global.f32 %0, [%1];" : "=f"(m[r % RING][t]) : "l"(rows + (size_t)(r + RING) * S + lane + 32 * t));
+        }
         for (int o = 16; o; o >>= 1) o_acc += __shfl_xor_sync(0xffffffffu, o_acc, o);
         if (lane == 0) s_core[warp * RPW + r] = o_acc * scale;
     }
     __syncthreads();
     // gated RMSNorm over the head (the arithmetic of k_dn_tail)
-    const size_t idx = (size_t)seq * D.d_inner + (size_t)h * S + tid;
+    const size_t idx = (size_t)seq * D.d_inner + (size_t)h * S + part * SB + tid;
     float x = 0.f, g = 0.f;
     ss = 0.0;
-    if (tid < S) { x = s_core[tid]; g = z[idx]; ss = (double)x * (double)x; }
+    if (tid < SB) { x = s_core[tid]; g = z[idx]; ss = (double)x * (double)x; }
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) red2[warp] = ss;
-    __syncthreads();
-    if (tid < S) {
+    if (SPLIT == 1u) {
+        if (lane == 0) red2[warp] = ss;
+        __syncthreads();
+    } else {
+        // the head's sum of squares from all of its blocks: each hands its warps' parts to every block of the head
+        if (lane == 0 && warp < SB / 32u) {
+            const uint32_t at = (uint32_t)__cvta_generic_to_shared(&red2[part * (SB / 32u) + warp]), rank0 = (h - kh * width) * SPLIT;
+#pragma unroll
+            for (uint32_t p = 0; p < SPLIT; ++p) {
+                uint32_t peer;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(rank0 + p));
+                asm volatile("st.shared::cluster.f64 [%0], %1;" :: "r"(peer), "d"(ss) : "memory");
+            }
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    if (tid < SB) {
         double tot = 0.0;
         for (uint32_t w = 0; w < S / 32u; ++w) tot += red2[w];
         const float inv = 1.0f / sqrtf((float)(tot / (double)S) + D.eps);
         const float silu = g / (1.0f + expf(-g));
-        out[idx] = x * inv * norm_w[tid] * silu;
+        out[idx] = x * inv * norm_w[part * SB + tid] * silu;
     }
 }
 
@@ -842,11 +865,25 @@ int launch_deltanet(const DnDims &D, uint32_t batch, const float *conv_kernel, c
     const uint32_t width = D.rank / D.groups;
     if (D.S <= 128u && width <= 8u) {
         prof_begin("dn_step", s);
-        const dim3 gs(D.rank, batch);
-#define RC_DN_STEP(VPL, DC) RC_LAUNCH_CLUSTER(width, (k_dn_step<VPL, DC>), gs, 256, 0, s, D, conv_kernel, dt_bias, ssm_a, qkv, ba, conv_state, rec_state, z, norm_w, out)
-        if (D.S == 32u) { if (D.d_conv == 4u) RC_DN_STEP(1, 4u); else RC_DN_STEP(1, 0u); }
-        else if (D.S == 64u) { if (D.d_conv == 4u) RC_DN_STEP(2, 4u); else RC_DN_STEP(2, 0u); }
-        else { if (D.d_conv == 4u) RC_DN_STEP(4, 4u); else RC_DN_STEP(4, 0u); }
+#define RC_DN_STEP(VPL, SPLIT, MINB, RING) do { const dim3 gs(D.rank * SPLIT, batch); \
+        if (D.d_conv == 4u) RC_LAUNCH_CLUSTER(width * SPLIT, (k_dn_step<VPL, 4u, SPLIT, MINB, RING>), gs, 256, 0, s, D, conv_kernel, dt_bias, ssm_a, qkv, ba, conv_state, rec_state, z, norm_w, out); \
+        else RC_LAUNCH_CLUSTER(width * SPLIT, (k_dn_step<VPL, 0u, SPLIT, MINB, RING>), gs, 256, 0, s, D, conv_kernel, dt_bias, ssm_a, qkv, ba, conv_state, rec_state, z, norm_w, out); } while (0)
+        // Heads of 128: as many blocks per head as still fit the chip at once (3 blocks per SM with 4 or 8 rows a warp, 2 with 16) and
+        // a cluster (8 blocks), since a second wave costs more than idle SMs and every block repeats the preparation. us a step
+        // of 32 heads, graph-replayed, 1 / 3 / 4 / 6 / 8 / 10 sequences: 4 blocks 5.7 / 7.4 / 12.7 / 14.2 / 19.3 / 24.6, 2 blocks at
+        // 2 per SM 6.6 / 8.1 / 8.4 / 15.0 / 15.9 / 22.0, 2 blocks at 3 per SM 6.7 / 9.1 / 9.6 / 10.1 / 16.3 / 18.0, one block 7.7 / 10.2 / 10.8 /
+        // 11.4 / 11.9 / 18.5, one block at 3 per SM with half of its rows in flight 10.1 / 12.8 / 13.6 / 14.5 / 15.1 / 15.8 (the separate
+        // kernels: 7.7 / 8.8 / 10.9 / 11.1 / 12.8 / 15.4).
+        static int sms = 0;
+        if (!sms) { int dev = 0; RC_CUDA(cudaGetDevice(&dev)); RC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)); }
+        const uint64_t blocks = (uint64_t)D.rank * batch, two = 2u * (uint32_t)sms, three = 3u * (uint32_t)sms;
+        if (D.S == 32u) RC_DN_STEP(1, 1u, 2, 4u);
+        else if (D.S == 64u) RC_DN_STEP(2, 1u, 2, 8u);
+        else if (width <= 2u && 4u * blocks <= three) RC_DN_STEP(4, 4u, 2, 4u);
+        else if (width <= 4u && 2u * blocks <= two) RC_DN_STEP(4, 2u, 2, 8u);
+        else if (width <= 4u && 2u * blocks <= three) RC_DN_STEP(4, 2u, 3, 8u);
+        else if (blocks <= two) RC_DN_STEP(4, 1u, 2, 16u);
+        else RC_DN_STEP(4, 1u, 3, 8u);
 #undef RC_DN_STEP
         prof_end(s);
         RC_LAUNCHED();
