@@ -861,9 +861,13 @@ int launch_deltanet(const DnDims &D, uint32_t batch, const float *conv_kernel, c
     RC_REQUIRE(D.rank && D.groups && D.rank % D.groups == 0 && D.d_inner == D.rank * D.S && D.channels == 2u * D.S * D.groups + D.d_inner && D.d_conv >= 2u,
                "deltanet: inconsistent dimensions");
     if (!batch) return 1;
-    // one launch where a head's state fits the registers of a block and the value heads of a key head fit a cluster; else three
+    // one launch where a head's state fits the registers of a block and the value heads of a key head fit a cluster; else three.
+    // Three also where out lies in qkv or ba: only the separate kernels have read all of those before the first output is written.
     const uint32_t width = D.rank / D.groups;
-    if (D.S <= 128u && width <= 8u) {
+    auto overlap = [](const float *a, uint64_t na, const float *b, uint64_t nb) { return a < b + nb && b < a + na; };
+    const uint64_t n_out = (uint64_t)batch * D.d_inner;
+    const bool in_place = overlap(out, n_out, qkv, (uint64_t)batch * D.channels) || overlap(out, n_out, ba, (uint64_t)batch * 2u * D.rank);
+    if (D.S <= 128u && width <= 8u && !in_place) {
         prof_begin("dn_step", s);
 #define RC_DN_STEP(VPL, SPLIT, MINB, RING) do { const dim3 gs(D.rank * SPLIT, batch); \
         if (D.d_conv == 4u) RC_LAUNCH_CLUSTER(width * SPLIT, (k_dn_step<VPL, 4u, SPLIT, MINB, RING>), gs, 256, 0, s, D, conv_kernel, dt_bias, ssm_a, qkv, ba, conv_state, rec_state, z, norm_w, out); \

@@ -29,3 +29,35 @@ def test_blocks_per_head(groups, rank, batch, d_conv):
         # tolerances of the reference's stage tools (native/redlite_native_deltanet_state_cli.c:267-269); the output adds a norm over the head
         assert np.all(np.abs(rg[b] - rec[b]) <= 3e-6 + 3e-5 * np.abs(rec[b]))
         assert np.max(np.abs(out[b] - ref)) <= 2e-5 * np.max(np.abs(ref)) + 1e-7
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_output_in_the_input(batch):
+    """out may lie in qkv: every block's inputs are read before any output is written."""
+    import ctypes as C
+    import torch
+    from dwarfstar_red_lite_b200 import redcuda
+    S, groups, rank = 128, 16, 32
+    d_inner, channels = rank * S, 2 * S * groups + rank * S
+    g = torch.Generator(device="cuda")
+    g.manual_seed(batch)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    arr = [r(channels, 4) * 0.5, r(rank), -torch.exp(r(rank) * 0.5), 1.0 + 0.1 * r(S)]
+    P = redcuda.DeltanetParams(4, S, groups, rank, d_inner, channels, 1e-6, *[C.cast(a.data_ptr(), redcuda.f32p) for a in arr])
+    qkv, z, ba, conv, rec = r(batch, channels), r(batch, d_inner), r(batch, 2 * rank), r(batch, channels, 3), r(batch, rank, S, S) * 0.05
+    lib = rc.lib()
+
+    def step(inputs, out_ptr):
+        c, s = conv.clone(), rec.clone()
+        torch.cuda.synchronize()
+        assert lib.redcuda_deltanet_step_noalloc(C.byref(P), batch, inputs.data_ptr(), z.data_ptr(), ba.data_ptr(), c.data_ptr(), s.data_ptr(), out_ptr, None) == 1
+        torch.cuda.synchronize()
+        return c, s
+
+    out, buf = torch.empty(batch, d_inner, device="cuda"), qkv.clone()
+    c0, s0 = step(qkv, out.data_ptr())
+    c1, s1 = step(buf, buf.data_ptr())
+    got = buf.view(-1)[:batch * d_inner].view(batch, d_inner)
+    assert torch.equal(c0, c1)
+    # the forms differ in the order of a few 32-bit sums only
+    assert torch.allclose(s0, s1, rtol=3e-5, atol=3e-6) and torch.max(torch.abs(got - out)) <= 2e-5 * torch.max(torch.abs(out))
