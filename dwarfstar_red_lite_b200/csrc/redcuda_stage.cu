@@ -57,34 +57,40 @@ inline void copy_streaming(uint8_t *dst, const uint8_t *src, size_t n) {
 #endif
 }
 
-// One array cut into pieces. Threads claim pieces with `next`; piece i may be copied once `avail` > i (the pieces of a
-// download arrive one after the other) and done[i] is set when it has been.
+// One array cut into pieces. Threads claim them in order; piece i may be claimed once `avail` > i (the pieces of a download arrive one
+// after the other, and nobody waits for one with a claim on it) and done[i] is set when it has been copied.
 struct CopyBatch {
     uint8_t *dst; const uint8_t *src;
     size_t bytes, n;
     std::atomic<size_t> next{0}, avail{0};
-    std::atomic<bool> cancelled{false};
     std::vector<std::atomic<int>> done;
     CopyBatch(uint8_t *d, const uint8_t *s, size_t b) : dst(d), src(s), bytes(b), n((b + PIECE - 1) / PIECE), done(n) {}
     size_t piece(size_t i) const { return std::min(PIECE, bytes - i * PIECE); }
     bool exhausted() const { return next.load(std::memory_order_relaxed) >= n; }
-    // claims and copies one piece; false when none is left to claim
+    bool claimable() const { return next.load(std::memory_order_relaxed) < std::min(n, avail.load()); }
+    // claims and copies one piece; false when none can be claimed now
     bool step() {
-        const size_t i = next.fetch_add(1, std::memory_order_relaxed);
-        if (i >= n) return false;
-        while (avail.load(std::memory_order_acquire) <= i) cpu_relax();
-        if (!cancelled.load(std::memory_order_relaxed)) copy_streaming(dst + i * PIECE, src + i * PIECE, piece(i));
+        size_t i = next.load(std::memory_order_relaxed);
+        do {
+            if (i >= n || i >= avail.load(std::memory_order_acquire)) return false;
+        } while (!next.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
+        copy_streaming(dst + i * PIECE, src + i * PIECE, piece(i));
         done[i].store(1, std::memory_order_release);
         return true;
     }
-    void wait(size_t i) const { while (!done[i].load(std::memory_order_acquire)) cpu_relax(); }
+    // until piece i, claimed by another thread, has been copied: that thread may need this core to finish
+    void wait(size_t i) const {
+        for (int k = 0; !done[i].load(std::memory_order_acquire); ++k) { if (k < 4000) cpu_relax(); else std::this_thread::yield(); }
+    }
+    // no further claims; returns when nobody copies any more
+    void stop() { for (size_t i = 0, c = std::min(n, next.exchange(n)); i < c; ++i) wait(i); }
 };
 
 struct CopyPool {
     std::mutex mu;
     std::condition_variable cv;
     std::deque<std::shared_ptr<CopyBatch>> batches;
-    std::atomic<uint32_t> posted{0};
+    std::atomic<uint32_t> posted{0}, asleep{0};
     bool started = false;
 
     void start() {         // mu held
@@ -95,31 +101,45 @@ struct CopyPool {
             try { std::thread([this] { work(); }).detach(); } catch (...) { break; }      // fewer helpers: the caller copies what is left itself
         }
     }
+    // a batch with a piece to claim
     std::shared_ptr<CopyBatch> pick() {         // mu held
-        while (!batches.empty() && batches.front()->exhausted()) batches.pop_front();
-        return batches.empty() ? nullptr : batches.front();
+        for (auto it = batches.begin(); it != batches.end();) {
+            if ((*it)->exhausted()) { it = batches.erase(it); continue; }
+            if ((*it)->claimable()) return *it;
+            ++it;
+        }
+        return nullptr;
     }
     void work() {
         std::unique_lock<std::mutex> lk(mu);
         for (;;) {
             std::shared_ptr<CopyBatch> b = pick();
-            if (b) {
-                lk.unlock();
-                while (b->step()) {}
-                b.reset();
-                // calls follow one another closely: look for the next array for about as long as a wake-up takes before going to sleep
-                const uint32_t seen = posted.load(std::memory_order_relaxed);
-                for (int i = 0; i < 1500 && posted.load(std::memory_order_relaxed) == seen; ++i) cpu_relax();
-                lk.lock();
-                continue;
+            if (!b) {
+                asleep.fetch_add(1);
+                b = pick();             // what became claimable before wake() could see this thread asleep
+                if (!b) cv.wait(lk);
+                asleep.fetch_sub(1);
             }
-            cv.wait(lk);
+            if (!b) continue;
+            lk.unlock();
+            while (b->step()) {}
+            b.reset();
+            // pieces and calls follow one another closely: look for the next for about as long as a wake-up takes before going to sleep
+            const uint32_t seen = posted.load(std::memory_order_relaxed);
+            for (int i = 0; i < 1500 && posted.load(std::memory_order_relaxed) == seen; ++i) cpu_relax();
+            lk.lock();
         }
+    }
+    // pieces became claimable
+    void wake() {
+        posted.fetch_add(1);
+        if (!asleep.load()) return;
+        { std::lock_guard<std::mutex> lk(mu); }         // a thread counted asleep holds mu until it waits
+        cv.notify_all();
     }
     void post(const std::shared_ptr<CopyBatch> &b) {
         { std::lock_guard<std::mutex> lk(mu); start(); batches.push_back(b); }
-        posted.fetch_add(1, std::memory_order_relaxed);
-        cv.notify_all();
+        wake();
     }
 };
 CopyPool &copy_pool() { static CopyPool *p = new CopyPool(); return *p; }      // never destroyed: its threads outlive static destructors
@@ -305,16 +325,17 @@ int Stage::download(void *dst_host, const void *src_dev, size_t bytes) {
             at += n;
             continue;
         }
+        // the helpers are called when the first piece is there (until then they would have nothing to do but wait for the GPU)
         auto b = std::make_shared<CopyBatch>(dst + at, lease_->pin, n);
-        copy_pool().post(b);
         cudaError_t err = cudaSuccess;
         for (size_t i = 0; i < np && err == cudaSuccess; ++i) {
             err = cudaEventSynchronize(lease_->events[i]);
-            if (err == cudaSuccess) b->avail.store(i + 1, std::memory_order_release);
+            if (err != cudaSuccess) break;
+            b->avail.store(i + 1);
+            if (i == 0) copy_pool().post(b); else copy_pool().wake();
         }
-        if (err != cudaSuccess) { b->cancelled.store(true); b->avail.store(np, std::memory_order_release); }
-        while (b->step()) {}
-        for (size_t i = 0; i < np; ++i) b->wait(i);
+        if (err == cudaSuccess) while (b->step()) {}
+        b->stop();
         RC_CUDA(err);
         at += n;
     }

@@ -1,0 +1,67 @@
+"""CPU check of the host-buffer staging: csrc/redcuda_stage.cu compiled for the host against a fake CUDA runtime (stage_host_check.cpp)."""
+import ctypes as C
+import os
+import subprocess
+import threading
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA_INCLUDE = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+
+
+@pytest.fixture(scope="module")
+def so_path(tmp_path_factory):
+    if not os.path.exists(os.path.join(CUDA_INCLUDE, "cuda_runtime.h")):
+        pytest.skip("no CUDA headers")
+    so = str(tmp_path_factory.mktemp("stage") / "libstage.so")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", CUDA_INCLUDE, "-o", so, os.path.join(HERE, "stage_host_check.cpp"),
+                           "-x", "c++", os.path.join(HERE, "..", "dwarfstar_red_lite_b200", "csrc", "redcuda_stage.cu"), "-lpthread"])
+    return so
+
+
+@pytest.fixture(scope="module")
+def lib(so_path):
+    L = C.CDLL(so_path)
+    L.check_roundtrip.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t]
+    L.check_download_cpu.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+    L.check_download_cpu.restype = C.c_double
+    L.check_error.restype = C.c_char_p
+    return L
+
+
+def _bytes(n, seed=0):
+    return np.random.default_rng(seed).integers(0, 256, size=n, dtype=np.uint8), np.empty(n, np.uint8)
+
+
+@pytest.mark.parametrize("n", [1, 4095, 256 << 10, (256 << 10) + 1, (512 << 10) + 16, (9 << 20) + 7, 32 << 20, (32 << 20) + 16, (70 << 20) + 5])
+def test_roundtrip(lib, n):
+    """below and above the single-copy limit, several pieces, several rounds of the 32 MB pinned buffer in both directions"""
+    a, b = _bytes(n)
+    assert lib.check_roundtrip(a.ctypes.data, b.ctypes.data, n) == 1, lib.check_error()
+
+
+def test_roundtrip_from_several_threads(lib):
+    bad = []
+
+    def work(i):
+        for k, n in enumerate((3 << 20, 70000, 20 << 20, 900001)):
+            a, b = _bytes(n + i, seed=i * 4 + k)
+            if lib.check_roundtrip(a.ctypes.data, b.ctypes.data, n + i) != 1:
+                bad.append((i, n))
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+
+
+def test_helpers_sleep_while_the_gpu_works(lib):
+    """a download whose bytes are 400 ms away: the copying threads must not spend that time spinning"""
+    a, b = _bytes(8 << 20)
+    assert lib.check_roundtrip(a.ctypes.data, b.ctypes.data, a.size) == 1         # the threads are started
+    t = lib.check_download_cpu(a.ctypes.data, b.ctypes.data, a.size, 400)
+    assert 0.0 <= t < 0.2, t                                                       # one thread that spins throughout takes 0.4
