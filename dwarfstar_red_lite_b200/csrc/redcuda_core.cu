@@ -590,8 +590,9 @@ int redcuda_quant_dequant_rows(uint32_t type, const uint8_t *rows, uint32_t nrow
     const size_t n = (size_t)nrows * ncols;
     if (type == RC_F32) { memcpy(out, rows, n * 4u); return 1; }   // a copy, as in the reference (quant_cpu.c:159)
     Stage st;
-    if (!st.open(2u * Stage::pad(bytes) + Stage::pad(n * 4u))) return 0;
-    uint8_t *raw = st.take(bytes), *planar = st.take(bytes);
+    const bool quant = rc_is_quant(type);                          // F16 rows are read where they were uploaded
+    if (!st.open((quant ? 2u : 1u) * Stage::pad(bytes) + Stage::pad(n * 4u))) return 0;
+    uint8_t *raw = st.take(bytes), *planar = quant ? st.take(bytes) : nullptr;
     float *o = st.take<float>(n * 4u);
     cudaStream_t s = st.stream();
     if (!st.upload(raw, rows, bytes)) return 0;
@@ -617,11 +618,12 @@ int redcuda_quant_matvec(uint32_t type, const uint8_t *w, uint32_t nrows, uint32
     RC_REQUIRE(bytes, "matvec: %u columns is not a valid row length for type %u", ncols, type);
     const size_t xb = (size_t)ntok * ncols * 4u, ob = (size_t)ntok * nrows * 4u;
     Stage st;
-    if (!st.open(2u * Stage::pad(bytes) + Stage::pad(xb) + Stage::pad(ob))) return 0;
-    uint8_t *raw = st.take(bytes), *planar = st.take(bytes);
+    const bool quant = rc_is_quant(type);                          // F32 / F16 rows are read where they were uploaded
+    if (!st.open((quant ? 2u : 1u) * Stage::pad(bytes) + Stage::pad(xb) + Stage::pad(ob))) return 0;
+    uint8_t *raw = st.take(bytes), *planar = quant ? st.take(bytes) : raw;
     float *xd = st.take<float>(xb), *od = st.take<float>(ob);
     cudaStream_t s = st.stream();
-    if (!st.upload(xd, x, xb) || !st.upload(raw, w, bytes) || !upload_matrix(type, nrows, ncols, raw, true, planar, nullptr, s)) return 0;
+    if (!st.upload(xd, x, xb) || !st.upload(raw, w, bytes) || (quant && !upload_matrix(type, nrows, ncols, raw, true, planar, nullptr, s))) return 0;
     GemvArgs A{};
     A.njobs = 1; A.ntok = ntok; A.x = xd; A.x_stride = ncols;
     A.job[0].w0 = planar; A.job[0].w1 = nullptr; A.job[0].out = od; A.job[0].nb = (uint64_t)nrows * (ncols / 256u);

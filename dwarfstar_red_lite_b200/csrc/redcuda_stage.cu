@@ -4,6 +4,7 @@
 // upload itself 290 (one thread copies those bytes in 540, the link moves them in 180); matvec 64 x 256 of Q8_0 700 -> 34;
 // dequantisation of 8192 x 4096 values 39 -> 8.5 ms (bound by the page faults of the 134 MB it returns).
 #include "redcuda_stage.cuh"
+#include "../../include/redcuda.h"
 
 #include <string.h>
 #if defined(__x86_64__)
@@ -26,7 +27,8 @@ namespace {
 constexpr size_t PIECE = 512u << 10;             // a piece takes a core about 50 us and the link 10
 constexpr size_t INLINE_MAX = 256u << 10;        // below this waking a thread costs more than it saves
 constexpr size_t PINNED_MAX = 32u << 20;         // pinned bytes of a lease; larger arrays go through it in rounds
-constexpr size_t KEEP_DEVICE = 256u << 20;       // device bytes an idle lease may keep
+constexpr size_t KEEP_DEVICE = 256u << 20;       // device bytes that the idle leases of a device keep together
+constexpr size_t KEEP_PINNED = 64u << 20;        // pinned bytes that they keep together
 constexpr size_t KEEP_LEASES = 4;                // idle leases per device
 
 inline void cpu_relax() {
@@ -176,15 +178,18 @@ void stage_trim() {
 int Stage::open(size_t device_bytes) {
     int dev = 0;
     RC_CUDA(cudaGetDevice(&dev));
+    const bool own = device_bytes > KEEP_DEVICE;
     {
         std::lock_guard<std::mutex> lk(g_stage_mu);
         auto &v = stage_idle();
-        // the smallest idle lease that is large enough, else the largest (it grows)
+        // the smallest idle lease that is large enough, else the largest (it grows); a call whose area is not kept brings its own
+        // and takes the smallest, so that it uses up no warm one
+        const size_t want = own ? 0u : device_bytes;
         size_t best = v.size();
         for (size_t i = 0; i < v.size(); ++i) {
             if (v[i]->device != dev) continue;
             if (best == v.size()) { best = i; continue; }
-            const bool fits = v[i]->dev_bytes >= device_bytes, best_fits = v[best]->dev_bytes >= device_bytes;
+            const bool fits = v[i]->dev_bytes >= want, best_fits = v[best]->dev_bytes >= want;
             if (fits != best_fits ? fits : fits ? v[i]->dev_bytes < v[best]->dev_bytes : v[i]->dev_bytes > v[best]->dev_bytes) best = i;
         }
         if (best < v.size()) { lease_ = v[best]; v.erase(v.begin() + best); }
@@ -194,16 +199,22 @@ int Stage::open(size_t device_bytes) {
         lease_->device = dev;
         RC_CUDA(cudaStreamCreateWithFlags(&lease_->s, cudaStreamNonBlocking));
     }
-    if (lease_->dev_bytes < device_bytes) {
+    if (own) {
+        if (!own_.alloc(device_bytes)) {             // the lease's area may be what is missing
+            if (!lease_->dev) return 0;
+            cudaFree(lease_->dev); lease_->dev = nullptr; lease_->dev_bytes = 0;
+            if (!own_.alloc(device_bytes)) return 0;
+        }
+    } else if (lease_->dev_bytes < device_bytes) {
         if (lease_->dev) { cudaFree(lease_->dev); lease_->dev = nullptr; lease_->dev_bytes = 0; }
-        size_t want = pad(std::max<size_t>(device_bytes, 1u << 20));
-        if (want <= KEEP_DEVICE) { size_t p = 1u << 20; while (p < want) p <<= 1; want = p; }      // powers of two: a few growths, then none
+        size_t want = 1u << 20;
+        while (want < device_bytes) want <<= 1;      // powers of two: a few growths, then none
         DevMem m;
         if (!m.alloc(want)) return 0;
         lease_->dev = m.as<uint8_t>(); lease_->dev_bytes = want;
         m.p = nullptr; m.bytes = 0;
     }
-    dev_ = lease_->dev; used_ = 0; pinned_used_ = 0; followed_ = false;
+    dev_ = own ? own_.as<uint8_t>() : lease_->dev; used_ = 0; pinned_used_ = 0; followed_ = false;
     return 1;
 }
 
@@ -222,16 +233,24 @@ int Stage::follow_default_stream() {
 Stage::~Stage() {
     if (!lease_) return;
     cudaStreamSynchronize(lease_->s);        // after an error a copy may still be in flight
-    bool keep = lease_->s != nullptr && lease_->dev_bytes <= KEEP_DEVICE;
+    own_.release();
+    uint8_t *dev = nullptr, *pin = nullptr;  // what the idle leases may not keep
+    bool keep = lease_->s != nullptr;
     if (keep) {
         std::lock_guard<std::mutex> lk(g_stage_mu);
         auto &v = stage_idle();
-        size_t same = 0;
-        for (StageLease *l : v) same += l->device == lease_->device;
+        size_t same = 0, dev_sum = lease_->dev_bytes, pin_sum = lease_->pin_bytes;
+        for (StageLease *l : v) if (l->device == lease_->device) { ++same; dev_sum += l->dev_bytes; pin_sum += l->pin_bytes; }
         keep = same < KEEP_LEASES;
-        if (keep) v.push_back(lease_);
+        if (keep) {
+            if (dev_sum > KEEP_DEVICE) { dev = lease_->dev; lease_->dev = nullptr; lease_->dev_bytes = 0; }
+            if (pin_sum > KEEP_PINNED) { pin = lease_->pin; lease_->pin = nullptr; lease_->pin_bytes = 0; }
+            v.push_back(lease_);
+        }
     }
     if (!keep) delete lease_;
+    if (dev) cudaFree(dev);
+    if (pin) cudaFreeHost(pin);
 }
 
 cudaStream_t Stage::stream() const { return lease_->s; }
@@ -346,3 +365,5 @@ int Stage::download(void *dst_host, const void *src_dev, size_t bytes) {
 int Stage::finish() { RC_CUDA(cudaStreamSynchronize(lease_->s)); pinned_used_ = 0; return 1; }
 
 }  // namespace rc
+
+extern "C" int redcuda_trim(void) { rc::stage_trim(); return 1; }

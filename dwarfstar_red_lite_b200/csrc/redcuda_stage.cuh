@@ -31,12 +31,13 @@ class Stage {
     int follow_default_stream();
     int drain_pinned();      // waits until no copy reads or writes the pinned buffer any more
     StageLease *lease_ = nullptr;
+    DevMem own_;             // the device area of a call too large for a lease to keep
     uint8_t *dev_ = nullptr;
     size_t used_ = 0, pinned_used_ = 0;
     bool followed_ = false;
 };
 
-// Gives back every device and pinned buffer that idle leases keep (called when an allocation of the library fails)
+// Gives back every device and pinned buffer that idle leases keep (called when an allocation of the library fails, and by redcuda_trim)
 void stage_trim();
 
 }  // namespace rc

@@ -14,7 +14,7 @@ LIB_PATH = os.environ.get("REDCUDA_LIB") or os.path.join(HERE, "libredcuda.so") 
 u8p, f32p, u32p = C.POINTER(C.c_uint8), C.POINTER(C.c_float), C.POINTER(C.c_uint32)
 
 EXPORTS = [
-    "redcuda_abi_version", "redcuda_last_error", "redcuda_device_count", "redcuda_set_device", "redcuda_set_codebooks", "redcuda_set_codebooks_ext", "redcuda_set_codebooks_xs",
+    "redcuda_abi_version", "redcuda_last_error", "redcuda_device_count", "redcuda_set_device", "redcuda_trim", "redcuda_set_codebooks", "redcuda_set_codebooks_ext", "redcuda_set_codebooks_xs",
     "redcuda_quant_dequant_rows", "redcuda_nib_dequant_rows", "redcuda_quant_matvec", "redcuda_quant_matmul_tc", "redcuda_router_select_softmax_topk", "redcuda_deltanet_step",
     "redcuda_deltanet_step_noalloc",
     "redcuda_moe_create", "redcuda_moe_destroy", "redcuda_moe_resident_bytes", "redcuda_moe_forward",
@@ -123,6 +123,11 @@ def profile_report() -> dict:
 def _check(ok: int):
     if ok != 1:
         raise RedcudaError(lib().redcuda_last_error().decode(errors="replace"))
+
+
+def trim():
+    """Give back the device and pinned memory that the host-pointer calls keep between calls."""
+    _check(lib().redcuda_trim())
 
 
 def default_codebooks() -> tuple[np.ndarray, np.ndarray]:

@@ -33,6 +33,13 @@ const char *redcuda_last_error(void);
 int redcuda_device_count(void);
 int redcuda_set_device(int device);
 
+/* The host-pointer entry points keep their work areas between calls: per device at most 256 MB of device memory and 64 MB of
+ * pinned host memory, held by the library until an allocation of its own fails or until this call gives them back (also
+ * those of other devices). Calls that need more than 256 MB of device memory allocate and free theirs each time. Host arrays
+ * may be pageable, pinned or managed memory, or device memory; a call on arrays that are not pageable starts behind the work
+ * queued on the default stream. Always returns 1. */
+int redcuda_trim(void);
+
 /*
  * Codebooks of the IQ formats, supplied by the host exactly as the reference supplies its grids to the Metal pool
  * (iq2_xs_grid / iq1_m_grid arguments of redmetal_topk_pool_create, native/redmetal_topk.h:16-24):

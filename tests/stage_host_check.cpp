@@ -109,5 +109,17 @@ double check_download_cpu(const uint8_t *src, uint8_t *dst, size_t n, int delay_
     if (!st.download(dst, d, n) || !st.finish() || memcmp(src, dst, n)) return -1.0;
     return cpu_seconds() - t;
 }
+// work areas of several calls open at once, each of n bytes; then all of them end
+int check_open_many(size_t n, int calls) {
+    std::vector<rc::Stage *> v;
+    int ok = 1;
+    for (int i = 0; i < calls; ++i) { v.push_back(new rc::Stage()); ok &= v.back()->open(n); }
+    for (rc::Stage *s : v) delete s;
+    return ok;
+}
+size_t check_device_bytes() { return g_dev_bytes; }
+size_t check_pinned_bytes() { return g_pin_bytes; }
+int check_device_allocs() { return g_dev_allocs; }
+int check_pinned_allocs() { return g_pin_allocs; }
 const char *check_error() { return g_error.c_str(); }
 }

@@ -28,6 +28,8 @@ def lib(so_path):
     L.check_download_cpu.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
     L.check_download_cpu.restype = C.c_double
     L.check_error.restype = C.c_char_p
+    L.check_open_many.argtypes = [C.c_size_t, C.c_int]
+    L.check_device_bytes.restype = L.check_pinned_bytes.restype = C.c_size_t
     return L
 
 
@@ -65,3 +67,31 @@ def test_helpers_sleep_while_the_gpu_works(lib):
     assert lib.check_roundtrip(a.ctypes.data, b.ctypes.data, a.size) == 1         # the threads are started
     t = lib.check_download_cpu(a.ctypes.data, b.ctypes.data, a.size, 400)
     assert 0.0 <= t < 0.2, t                                                       # one thread that spins throughout takes 0.4
+
+
+def test_idle_memory_is_bounded_and_given_back(lib):
+    MB = 1 << 20
+    assert lib.check_open_many(200 * MB, 4) == 1
+    assert lib.check_device_bytes() <= 256 * MB
+    pairs = [_bytes(33 * MB, seed=i) for i in range(4)]
+    ts = [threading.Thread(target=lib.check_roundtrip, args=(a.ctypes.data, b.ctypes.data, a.size)) for a, b in pairs]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert all(np.array_equal(a, b) for a, b in pairs)
+    assert lib.check_device_bytes() <= 256 * MB and lib.check_pinned_bytes() <= 64 * MB
+    assert lib.redcuda_trim() == 1
+    assert lib.check_device_bytes() == 0 and lib.check_pinned_bytes() == 0
+
+
+def test_a_large_call_keeps_the_warm_areas(lib):
+    """a call above the kept size allocates its device area each time, but neither a stream's pinned buffer nor another call's area"""
+    MB = 1 << 20
+    lib.redcuda_trim()
+    small, large = _bytes(3 * MB), _bytes(300 * MB)
+    run = lambda p: lib.check_roundtrip(p[0].ctypes.data, p[1].ctypes.data, p[0].size)  # noqa: E731
+    assert run(small) == run(large) == run(small) == 1
+    dev, pin = lib.check_device_allocs(), lib.check_pinned_allocs()
+    assert run(large) == run(small) == run(large) == run(small) == 1
+    assert lib.check_device_allocs() == dev + 2 and lib.check_pinned_allocs() == pin
