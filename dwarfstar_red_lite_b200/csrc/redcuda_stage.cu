@@ -255,6 +255,8 @@ Stage::~Stage() {
 
 cudaStream_t Stage::stream() const { return lease_->s; }
 
+// Makes the pinned buffer at least `want` bytes large (PINNED_MAX at most). A host that has no pinned memory left is no error: the
+// lease is left without a buffer, and the caller leaves the array to the driver's own copy of pageable memory.
 static int stage_pinned(StageLease *l, size_t want) {
     want = std::min(PINNED_MAX, std::max<size_t>(want, 1u << 20));
     if (l->pin_bytes >= want) return 1;
@@ -262,7 +264,12 @@ static int stage_pinned(StageLease *l, size_t want) {
     while (p < want) p <<= 1;
     RC_CUDA(cudaStreamSynchronize(l->s));
     if (l->pin) { cudaFreeHost(l->pin); l->pin = nullptr; l->pin_bytes = 0; }
-    RC_CUDA(cudaMallocHost((void **)&l->pin, p));
+    if (cudaMallocHost((void **)&l->pin, p) != cudaSuccess) {
+        cudaGetLastError();
+        l->pin = nullptr;
+        stage_trim();                  // what idle leases keep may be what is missing
+        if (cudaMallocHost((void **)&l->pin, p) != cudaSuccess) { cudaGetLastError(); l->pin = nullptr; return 1; }
+    }
     l->pin_bytes = p;
     return 1;
 }
@@ -289,6 +296,7 @@ int Stage::upload(void *dst_dev, const void *src_host, size_t bytes) {
         const size_t want = pinned_used_ + bytes;
         if (!drain_pinned() || !stage_pinned(lease_, want)) return 0;
     }
+    if (!lease_->pin) { RC_CUDA(cudaMemcpyAsync(dst_dev, src_host, bytes, cudaMemcpyHostToDevice, s)); return 1; }
     for (size_t at = 0; at < bytes;) {
         if (pinned_used_ == lease_->pin_bytes && !drain_pinned()) return 0;
         const size_t n = std::min(bytes - at, lease_->pin_bytes - pinned_used_);
@@ -326,6 +334,12 @@ int Stage::download(void *dst_host, const void *src_dev, size_t bytes) {
     const uint8_t *src = static_cast<const uint8_t *>(src_dev);
     if (bytes > INLINE_MAX && lease_->pin_bytes < std::min(bytes, PINNED_MAX) && !stage_pinned(lease_, bytes)) return 0;
     if (!lease_->pin && !stage_pinned(lease_, bytes)) return 0;
+    if (!lease_->pin) {
+        RC_CUDA(cudaMemcpyAsync(dst_host, src_dev, bytes, cudaMemcpyDeviceToHost, s));
+        RC_CUDA(cudaStreamSynchronize(s));
+        pinned_used_ = 0;
+        return 1;
+    }
     for (size_t at = 0; at < bytes;) {
         const size_t n = std::min(bytes - at, lease_->pin_bytes), np = (n + PIECE - 1) / PIECE;
         // the device's copies are queued behind the uploads that still read the pinned buffer, so its start can be reused

@@ -117,6 +117,7 @@ int check_open_many(size_t n, int calls) {
     for (rc::Stage *s : v) delete s;
     return ok;
 }
+void check_pinned_fails(int on) { g_pin_fail = on; }
 size_t check_device_bytes() { return g_dev_bytes; }
 size_t check_pinned_bytes() { return g_pin_bytes; }
 int check_device_allocs() { return g_dev_allocs; }

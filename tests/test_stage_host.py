@@ -95,3 +95,16 @@ def test_a_large_call_keeps_the_warm_areas(lib):
     dev, pin = lib.check_device_allocs(), lib.check_pinned_allocs()
     assert run(large) == run(small) == run(large) == run(small) == 1
     assert lib.check_device_allocs() == dev + 2 and lib.check_pinned_allocs() == pin
+
+
+@pytest.mark.parametrize("n", [100, 9 << 20])
+def test_without_pinned_memory(lib, n):
+    """a host without pinned memory left: the driver copies the pageable arrays itself"""
+    a, b = _bytes(n)
+    lib.redcuda_trim()
+    lib.check_pinned_fails(1)
+    try:
+        assert lib.check_roundtrip(a.ctypes.data, b.ctypes.data, n) == 1, lib.check_error()
+    finally:
+        lib.check_pinned_fails(0)
+    assert lib.check_roundtrip(a.ctypes.data, b.ctypes.data, n) == 1, lib.check_error()
