@@ -163,19 +163,29 @@ struct StageLease {
     }
 };
 
+// The entry points have C linkage: what the containers above and below throw (a host without memory) ends a call with an error.
+template <class F>
+static int no_throw(F f) {
+    try { return f(); } catch (const std::exception &e) { set_error("host-buffer call: %s", e.what()); return 0; }
+}
+
 static std::mutex g_stage_mu;
 static std::vector<StageLease *> &stage_idle() { static std::vector<StageLease *> *v = new std::vector<StageLease *>(); return *v; }
 
 void stage_trim() {
     std::vector<StageLease *> drop;
-    { std::lock_guard<std::mutex> lk(g_stage_mu); drop.swap(stage_idle()); }
+    if (!no_throw([&] { std::lock_guard<std::mutex> lk(g_stage_mu); drop.swap(stage_idle()); return 1; })) return;
     int cur = 0;
     cudaGetDevice(&cur);
     for (StageLease *l : drop) { cudaSetDevice(l->device); delete l; }
     cudaSetDevice(cur);
 }
 
-int Stage::open(size_t device_bytes) {
+int Stage::open(size_t device_bytes) { return no_throw([&] { return open_or_throw(device_bytes); }); }
+int Stage::upload(void *dst_dev, const void *src_host, size_t bytes) { return no_throw([&] { return upload_or_throw(dst_dev, src_host, bytes); }); }
+int Stage::download(void *dst_host, const void *src_dev, size_t bytes) { return no_throw([&] { return download_or_throw(dst_host, src_dev, bytes); }); }
+
+int Stage::open_or_throw(size_t device_bytes) {
     int dev = 0;
     RC_CUDA(cudaGetDevice(&dev));
     const bool own = device_bytes > KEEP_DEVICE;
@@ -236,7 +246,7 @@ Stage::~Stage() {
     own_.release();
     uint8_t *dev = nullptr, *pin = nullptr;  // what the idle leases may not keep
     bool keep = lease_->s != nullptr;
-    if (keep) {
+    if (keep && no_throw([] { stage_idle(); return 1; })) {
         std::lock_guard<std::mutex> lk(g_stage_mu);
         auto &v = stage_idle();
         size_t same = 0, dev_sum = lease_->dev_bytes, pin_sum = lease_->pin_bytes;
@@ -245,7 +255,7 @@ Stage::~Stage() {
         if (keep) {
             if (dev_sum > KEEP_DEVICE) { dev = lease_->dev; lease_->dev = nullptr; lease_->dev_bytes = 0; }
             if (pin_sum > KEEP_PINNED) { pin = lease_->pin; lease_->pin = nullptr; lease_->pin_bytes = 0; }
-            v.push_back(lease_);
+            keep = no_throw([&] { v.push_back(lease_); return 1; }) != 0;
         }
     }
     if (!keep) delete lease_;
@@ -282,7 +292,7 @@ static bool dma_reaches(const void *p) {
 
 int Stage::drain_pinned() { RC_CUDA(cudaStreamSynchronize(lease_->s)); pinned_used_ = 0; return 1; }
 
-int Stage::upload(void *dst_dev, const void *src_host, size_t bytes) {
+int Stage::upload_or_throw(void *dst_dev, const void *src_host, size_t bytes) {
     if (!bytes) return 1;
     cudaStream_t s = lease_->s;
     if (dma_reaches(src_host)) {
@@ -322,7 +332,7 @@ int Stage::upload(void *dst_dev, const void *src_host, size_t bytes) {
 }
 
 // Returns with the bytes in dst_host (pageable memory) or with the copy queued (pinned memory)
-int Stage::download(void *dst_host, const void *src_dev, size_t bytes) {
+int Stage::download_or_throw(void *dst_host, const void *src_dev, size_t bytes) {
     if (!bytes) return 1;
     cudaStream_t s = lease_->s;
     if (dma_reaches(dst_host)) {

@@ -28,6 +28,9 @@ class Stage {
     cudaStream_t stream() const;
 
   private:
+    int open_or_throw(size_t device_bytes);
+    int upload_or_throw(void *dst_dev, const void *src_host, size_t bytes);
+    int download_or_throw(void *dst_host, const void *src_dev, size_t bytes);
     int follow_default_stream();
     int drain_pinned();      // waits until no copy reads or writes the pinned buffer any more
     StageLease *lease_ = nullptr;

@@ -39,18 +39,30 @@ void run_until(FakeStream *s, uint64_t event) {         // event 0: everything
 }
 }  // namespace
 
+// C++ allocations of this library: the k-th one of the marked thread fails
+static thread_local int t_fail_in = -1;
+void *operator new(size_t n) {
+    if (t_fail_in >= 0 && t_fail_in-- == 0) throw std::bad_alloc();
+    if (void *p = malloc(n ? n : 1)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void *p) noexcept { free(p); }
+void operator delete(void *p, size_t) noexcept { free(p); }
+struct NoFail { int keep = t_fail_in; NoFail() { t_fail_in = -1; } ~NoFail() { t_fail_in = keep; } };      // the fake runtime's own allocations
+
 extern "C" {
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
-cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = (cudaStream_t) new FakeStream(); return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { NoFail nf; *s = (cudaStream_t) new FakeStream(); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { delete (FakeStream *)s; return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { run_until((FakeStream *)s, 0); return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { *e = (cudaEvent_t)malloc(1); return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { free(e); return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    NoFail nf;
     std::lock_guard<std::mutex> lk(g_mu);
     g_event_stream[e] = (FakeStream *)s; g_event_id[e] = g_next_event;
     ((FakeStream *)s)->q.push_back(Op{nullptr, nullptr, 0, g_next_event++});
@@ -65,14 +77,16 @@ cudaError_t cudaEventSynchronize(cudaEvent_t e) {
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind, cudaStream_t s) {
+    NoFail nf;
     std::lock_guard<std::mutex> lk(g_mu);
     ((FakeStream *)s)->q.push_back(Op{dst, src, n, 0});
     return cudaSuccess;
 }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) { a->type = cudaMemoryTypeUnregistered; return cudaSuccess; }
-cudaError_t cudaMalloc(void **p, size_t n) { *p = malloc(n); std::lock_guard<std::mutex> lk(g_mu); g_dev[*p] = n; g_dev_bytes += n; ++g_dev_allocs; return cudaSuccess; }
+cudaError_t cudaMalloc(void **p, size_t n) { NoFail nf; *p = malloc(n); std::lock_guard<std::mutex> lk(g_mu); g_dev[*p] = n; g_dev_bytes += n; ++g_dev_allocs; return cudaSuccess; }
 cudaError_t cudaFree(void *p) { { std::lock_guard<std::mutex> lk(g_mu); g_dev_bytes -= g_dev[p]; g_dev.erase(p); } free(p); return cudaSuccess; }
 cudaError_t cudaMallocHost(void **p, size_t n) {
+    NoFail nf;
     std::lock_guard<std::mutex> lk(g_mu);
     if (g_pin_fail) return cudaErrorMemoryAllocation;
     *p = malloc(n); g_pin[*p] = n; g_pin_bytes += n; ++g_pin_allocs;
@@ -82,7 +96,7 @@ cudaError_t cudaFreeHost(void *p) { { std::lock_guard<std::mutex> lk(g_mu); g_pi
 }
 
 namespace rc {
-void set_error(const char *fmt, ...) { char b[512]; va_list ap; va_start(ap, fmt); vsnprintf(b, sizeof(b), fmt, ap); va_end(ap); g_error = b; }
+void set_error(const char *fmt, ...) { NoFail nf; char b[512]; va_list ap; va_start(ap, fmt); vsnprintf(b, sizeof(b), fmt, ap); va_end(ap); g_error = b; }
 std::atomic<uint64_t> g_launches{0};
 int DevMem::alloc(size_t n) { release(); if (cudaMalloc(&p, n) != cudaSuccess) return 0; bytes = n; return 1; }
 void DevMem::release() { if (p) { cudaFree(p); p = nullptr; bytes = 0; } }
@@ -116,6 +130,14 @@ int check_open_many(size_t n, int calls) {
     for (int i = 0; i < calls; ++i) { v.push_back(new rc::Stage()); ok &= v.back()->open(n); }
     for (rc::Stage *s : v) delete s;
     return ok;
+}
+// the same with the k-th C++ allocation of this thread failing; -1: none was left to fail
+int check_roundtrip_failing(const uint8_t *src, uint8_t *dst, size_t n, int k) {
+    t_fail_in = k;
+    const int ok = check_roundtrip(src, dst, n);
+    const bool failed = t_fail_in < 0;
+    t_fail_in = -1;
+    return failed ? ok : -1;
 }
 void check_pinned_fails(int on) { g_pin_fail = on; }
 size_t check_device_bytes() { return g_dev_bytes; }

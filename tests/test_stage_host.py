@@ -2,6 +2,7 @@
 import ctypes as C
 import os
 import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -108,3 +109,31 @@ def test_without_pinned_memory(lib, n):
     finally:
         lib.check_pinned_fails(0)
     assert lib.check_roundtrip(a.ctypes.data, b.ctypes.data, n) == 1, lib.check_error()
+
+
+_FAILING = """
+import ctypes as C, sys
+import numpy as np
+L = C.CDLL(sys.argv[1])
+L.check_roundtrip_failing.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+L.check_error.restype = C.c_char_p
+a = np.arange(3 << 20, dtype=np.uint8)
+b = np.empty_like(a)
+seen = set()
+for k in range(64):
+    L.redcuda_trim()
+    ok = L.check_roundtrip_failing(a.ctypes.data, b.ctypes.data, a.size, k)
+    if ok == -1:
+        break
+    assert ok in (0, 1) and (ok == 1 or L.check_error()), k
+    seen.add(ok)
+    assert L.check_roundtrip_failing(a.ctypes.data, b.ctypes.data, a.size, 1 << 30) == -1
+print("runs", k, "errors", 0 in seen)
+assert k >= 3 and 0 in seen
+"""
+
+
+def test_a_failing_allocation_ends_a_call_with_an_error(so_path):
+    """a process of its own: an exception that left a C entry point would end it"""
+    r = subprocess.run([sys.executable, "-c", _FAILING, so_path], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
