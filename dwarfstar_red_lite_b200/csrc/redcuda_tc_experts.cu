@@ -70,13 +70,15 @@ __global__ void __launch_bounds__(256) k_tc_prep_rows(const float *__restrict__ 
     const float *ar = a + (size_t)r * stride, *br = b ? b + (size_t)r * stride : nullptr;
     float v[NCH][8];
     float mx = 0.f;
+    const bool vec = ((size_t)ar & 15u) == 0u;       // a caller's rows may begin at any float (their stride is a multiple of four)
 #pragma unroll
     for (uint32_t i = 0; i < NCH; ++i) {
         const uint32_t k = i * 256u + lane * 8u;
         if (k >= ncols) break;
 #pragma unroll
         for (uint32_t h = 0; h < 2u; ++h) {
-            const float4 p = *reinterpret_cast<const float4 *>(ar + k + 4u * h);
+            const float *q = ar + k + 4u * h;
+            const float4 p = vec ? *reinterpret_cast<const float4 *>(q) : make_float4(q[0], q[1], q[2], q[3]);
             v[i][4 * h] = p.x; v[i][4 * h + 1] = p.y; v[i][4 * h + 2] = p.z; v[i][4 * h + 3] = p.w;
         }
         if (br)
