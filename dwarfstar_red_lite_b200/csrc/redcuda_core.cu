@@ -243,7 +243,6 @@ __global__ void __launch_bounds__(256) k_gemv(const __grid_constant__ GemvArgs A
             default: break;
         }
     }
-    if (NT == 1 && A.tail.ticket) route_tail(A.tail);
 }
 
 // Fill tile_begin / rows_per_tile of every job and launch. Jobs must share ncols (they read the same x rows).
@@ -260,6 +259,7 @@ int launch_gemv(GemvArgs &A, cudaStream_t stream) {
         total_rows += A.job[j].nrows;
     }
     if (gemv1_ok(A)) return launch_gemv1(A, stream);
+    RC_REQUIRE(!A.tail.ticket, "gemv: the routing tail needs F32 / F16 / Q6_K rows of at most 8192 columns and a 16-byte aligned vector");
     uint32_t lpr = 32u;
     while (lpr > (ncols >> 6)) lpr >>= 1;
     const uint32_t rows_per_pass = 8u * (32u / lpr);                 // rows one block covers per sweep of its 8 warps
