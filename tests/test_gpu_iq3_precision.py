@@ -73,6 +73,23 @@ def test_error_against_64_bit(tg, td, kind):
         assert _rel(got, _exact(layer, x, ids)) <= BOUND, ntok
 
 
+def test_block_scales_of_every_kind():
+    """negative, subnormal, zero and large fp16 block scales in turn"""
+    layer = _layer(synth.IQ3_S, synth.IQ3_S, 512, 256, 4, False)
+    scales = np.array([-0.01, 6e-8, 0.0, 0.5, 0.02, -3e-5], np.float16).view(np.uint8).reshape(-1, 2)
+    for m in (layer.gate, layer.up, layer.down):
+        b = m.reshape(-1, synth.BLOCK_BYTES[synth.IQ3_S])
+        b[:, 0:2] = scales[np.arange(b.shape[0]) % len(scales)]
+    x, rng = _rows("gauss", 9, 512)
+    ids = rng.integers(0, 4, size=9)
+    logits = np.full((9, 4), -10.0, np.float32)
+    logits[np.arange(9), ids] = 10.0
+    m = rc.MoeLayer(layer, max_tokens=9)
+    got = m.forward(x, logits_in=logits)
+    m.close()
+    assert _rel(got, _exact(layer, x, ids)) <= BOUND
+
+
 @pytest.mark.parametrize("hidden,ffn", [(256, 256), (512, 1024), (1024, 512)])
 @pytest.mark.parametrize("ntok", [1, 5, 30])
 def test_other_widths(hidden, ffn, ntok):

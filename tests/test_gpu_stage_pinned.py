@@ -1,5 +1,5 @@
 """Host-buffer calls on arrays that are not ordinary host memory: pinned ones that copies of the default stream are still
-filling or still reading, and device memory."""
+filling or still reading, device memory, and more rows than the pinned buffer of a call holds."""
 import numpy as np
 import pytest
 import torch
@@ -53,3 +53,14 @@ def test_device_arrays(case):
     lib = rc.lib()
     assert lib.redcuda_quant_matvec(synth.Q6_K, wd.data_ptr(), NROWS, NCOLS, xd.data_ptr(), 1, out.data_ptr()) == 1, lib.redcuda_last_error()
     assert np.array_equal(out.cpu().numpy(), want)
+
+
+def test_upload_of_several_rounds():
+    nrows, ncols = 9001, 4096                       # 39 MB of Q8_0 rows; the pinned buffer holds 32
+    rng = np.random.default_rng(5)
+    w = synth.quant_matrix(rng, synth.Q8_0, nrows, ncols, 1e-3, 5e-3)
+    x = rng.normal(0, 1, size=(1, ncols)).astype(np.float32)
+    got = rc.quant_matvec(synth.Q8_0, w, nrows, ncols, x)[0]
+    for r in (0, 1, 4000, 7700, 7711, nrows - 1):   # 32 MB end in row 7710
+        one = rc.quant_matvec(synth.Q8_0, w[r:r + 1], 1, ncols, x)[0, 0]
+        assert got[r] == one
