@@ -175,6 +175,7 @@ static std::vector<StageLease *> &stage_idle() { static std::vector<StageLease *
 void stage_trim() {
     std::vector<StageLease *> drop;
     if (!no_throw([&] { std::lock_guard<std::mutex> lk(g_stage_mu); drop.swap(stage_idle()); return 1; })) return;
+    if (drop.empty()) return;              // nothing kept: no device is touched (there may be none)
     int cur = 0;
     cudaGetDevice(&cur);
     for (StageLease *l : drop) { cudaSetDevice(l->device); delete l; }

@@ -52,7 +52,8 @@ struct NoFail { int keep = t_fail_in; NoFail() { t_fail_in = -1; } ~NoFail() { t
 
 extern "C" {
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+static int g_set_device = 0;
+cudaError_t cudaSetDevice(int) { ++g_set_device; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { NoFail nf; *s = (cudaStream_t) new FakeStream(); return cudaSuccess; }
@@ -140,6 +141,7 @@ int check_roundtrip_failing(const uint8_t *src, uint8_t *dst, size_t n, int k) {
     return failed ? ok : -1;
 }
 void check_pinned_fails(int on) { g_pin_fail = on; }
+int check_set_device_calls() { return g_set_device; }
 size_t check_device_bytes() { return g_dev_bytes; }
 size_t check_pinned_bytes() { return g_pin_bytes; }
 int check_device_allocs() { return g_dev_allocs; }

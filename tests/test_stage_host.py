@@ -84,6 +84,8 @@ def test_idle_memory_is_bounded_and_given_back(lib):
     assert lib.check_device_bytes() <= 256 * MB and lib.check_pinned_bytes() <= 64 * MB
     assert lib.redcuda_trim() == 1
     assert lib.check_device_bytes() == 0 and lib.check_pinned_bytes() == 0
+    calls = lib.check_set_device_calls()
+    assert lib.redcuda_trim() == 1 and lib.check_set_device_calls() == calls          # nothing kept: no device is touched
 
 
 def test_a_large_call_keeps_the_warm_areas(lib):
