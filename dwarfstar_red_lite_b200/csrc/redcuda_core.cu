@@ -348,8 +348,8 @@ __global__ void __launch_bounds__(256) k_route(const float *__restrict__ logits,
 }
 
 // Warp-per-token variant for n_expert <= 1024: the probabilities of a token live in the warp's registers (32 per lane
-// at most), every selection round is a register scan plus a 5-step shuffle argmax — no block barriers, so the k rounds
-// cost a few hundred dependent instructions instead of 2k barriers. Same arithmetic and tie rule as k_route.
+// at most), every selection round is an integer maximum over them and two warp reductions (redcuda_route.cuh) — no block
+// barriers. Same arithmetic and tie rule as k_route, and as there a non-finite softmax selects id 0 in every round.
 __global__ void __launch_bounds__(256) k_route_warp(const float *__restrict__ logits, uint32_t ntok, uint32_t n_expert, uint32_t top_k,
                                                     uint32_t *__restrict__ ids, float *__restrict__ weights, float *__restrict__ probs_out,
                                                     RouteGroup1 G, uint32_t *__restrict__ status) {

@@ -947,8 +947,8 @@ extern "C" int redcuda_deltanet_step(const redcuda_deltanet_params *p, uint32_t 
 // ---------------------------------------------------------------------------------------------------------------
 // Allocation-free variant of the DeltaNet step.
 //
-// The step needs scratch between its three kernels (normalised q/k, conv output v, beta, gate, un-normalised head
-// outputs). redcuda_deltanet_step allocates that scratch per call, which a caller cannot afford when it runs inside a
+// Where the step runs as three kernels (state size 256, more than eight value heads per key head, an output inside the inputs) it needs
+// scratch between them (normalised q/k, conv output v, beta, gate, un-normalised head outputs). redcuda_deltanet_step allocates that scratch per call, which a caller cannot afford when it runs inside a
 // serving loop that must never block on the allocator (cudaMalloc / cudaFree synchronise the whole device), or when
 // another runtime owns the device memory budget. For those callers the scratch lives in the array below, part of the
 // library image: every GPU that loads the library holds these 512 KiB until the process exits.
@@ -967,7 +967,7 @@ extern "C" int redcuda_deltanet_step_noalloc(const redcuda_deltanet_params *p, u
     RC_REQUIRE(p->conv_kernel && p->dt_bias && p->ssm_a && p->ssm_norm, "deltanet step (no-alloc): null parameter array");
     const DnDims D{p->d_conv, p->d_state, p->n_group, p->dt_rank, p->d_inner, p->channels, p->rms_eps};
     const uint64_t n_qk = (uint64_t)batch * 2u * D.groups * D.S, n_v = (uint64_t)batch * D.d_inner, n_r = (uint64_t)batch * D.rank;
-    const uint64_t need = n_qk + 2u * n_v + 2u * n_r;
+    const uint64_t need = n_qk + 2u * n_v + 2u * n_r;            // the limit is the call's, whichever form runs
     RC_REQUIRE(need <= RC_DN_SCRATCH_FLOATS,
                "deltanet step (no-alloc): batch %u with these dimensions needs %llu scratch floats, the built-in scratch holds %u; "
                "use a smaller batch or redcuda_deltanet_step", batch, (unsigned long long)need, RC_DN_SCRATCH_FLOATS);

@@ -122,13 +122,14 @@ int redcuda_deltanet_step(const redcuda_deltanet_params *p, uint32_t batch, cons
  * time: a serving loop with a latency budget (cudaMalloc / cudaFree stall the whole device), or a process in which
  * another runtime owns the device's memory budget and hands this library only the buffers it passes in. Every pointer
  * — the four arrays inside *p included — is DEVICE memory; the launches go to `stream` (cudaStream_t) and the call
- * returns without synchronising. The scratch between the kernels is a fixed array of 131,072 floats (512 KiB) inside
- * the library image, held by every GPU that loads the library until the process exits. A call needs
- * batch * (2 * n_group * d_state + 2 * d_inner + 2 * dt_rank) of them: 12,352 per sequence at the Qwen3-Next shape
- * (16 key / 32 value heads of 128), i.e. at most batch 10 there; larger requests fail with a message and launch
+ * returns without synchronising. A step is one launch for state sizes up to 128 with at most eight value heads per key head and an
+ * output outside the inputs; otherwise three kernels, whose scratch is a fixed array of 131,072 floats (512 KiB) inside
+ * the library image, held by every GPU that loads the library until the process exits. Every call is held to the batch that
+ * the three kernels would fit, batch * (2 * n_group * d_state + 2 * d_inner + 2 * dt_rank) floats: 12,352 per sequence at the
+ * Qwen3-Next shape (16 key / 32 value heads of 128), i.e. at most batch 10 there; larger requests fail with a message and launch
  * nothing. The call never calls cudaMalloc, cudaFree or any allocating routine. The first call on a device looks up
  * the array's device address (once, cached): make that first call before any stream capture begins. All calls share
- * the one array: two calls whose kernels overlap on the GPU (different streams, no ordering) race on it. Nothing in it
+ * the one array: two three-kernel calls that overlap on the GPU (different streams, no ordering) race on it. Nothing in it
  * needs clearing between calls — each call overwrites every value it later reads. */
 int redcuda_deltanet_step_noalloc(const redcuda_deltanet_params *p_device_arrays, uint32_t batch, const float *qkv_dev, const float *z_dev,
                                   const float *ba_dev, float *conv_state_dev, float *rec_state_dev, float *out_dev, void *stream);
