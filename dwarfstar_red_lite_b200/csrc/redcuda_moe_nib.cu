@@ -246,7 +246,7 @@ __device__ __forceinline__ void nib_chunk_wide(const uint8_t *st, const int8_t *
     const float up = t & 1u ? 65536.0f : 1.0f;
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
-        const float w = sx[n * 2u * SXP] * up;              // a power of two, as da and db times it are without rounding
+        const float w = sx[n * 2u * SXP] * up;              // a power of two: da * w and db * w are exact
         out[n][0] += (da * w) * fmaf(256.0f, (float)blk[n][1], (float)blk[n][0]);
         out[n][1] += (db * w) * fmaf(256.0f, (float)blk[n][3], (float)blk[n][2]);
     }
