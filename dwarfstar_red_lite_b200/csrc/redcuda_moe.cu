@@ -494,7 +494,7 @@ static int moe_launch_experts(redcuda_moe *m, bool gateup, uint32_t npairs, bool
         const uint32_t tok = moe_item_tokens(m, single_token, npairs);
         const uint32_t live = npairs < m->d.expert_count ? npairs : m->d.expert_count;
         const uint32_t max_items = single_token ? npairs : (npairs / tok + live < npairs ? npairs / tok + live : npairs);
-        if (m->nib) { M.item_tok = tok; M.fmt = nib_fmt(m, gateup ? m->d.type_gu : m->d.type_down); M.work = m->work + (gateup ? 0 : 1); return launch_nib_experts(M, max_items, s); }
+        if (m->nib) { M.item_tok = tok; M.fmt = nib_fmt(m, gateup ? m->d.type_gu : m->d.type_down); M.work = m->work + (gateup ? 0 : 1); return launch_nib_batch(M, max_items, s); }
         return launch_moe_mma(M, max_items, tok, s);
     }
     MoeArgs A{};
@@ -577,7 +577,7 @@ static int moe_forward_fused1(redcuda_moe *m, const float *x, const float *logit
     M.expert_begin = m->d.expert_begin; M.n_local = m->d.expert_count; M.status = status_words();
     M.sorted = m->sorted; M.uexp = m->uexp; M.ustart = m->ustart; M.item_u = m->item_u; M.item_p0 = m->item_p0; M.n_items = m->n_items;
     M.xq = nullptr; M.sx = nullptr; M.x_div = k; M.out = m->act; M.out_stride = m->d.ffn; M.item_tok = 1u; M.work = m->work; M.x_raw = x; M.fmt = nib_fmt(m, m->d.type_gu);
-    if (!launch_nib_experts(M, k, s)) return 0;
+    if (!launch_nib_one(M, k, s)) return 0;
     NibTailArgs D{};
     D.w_down = m->down; D.mat_bytes = m->down_bytes; D.nrows = m->d.hidden; D.ncols = m->d.ffn; D.expert_begin = m->d.expert_begin; D.n_local = m->d.expert_count;
     D.fmt = nib_fmt(m, m->d.type_down);

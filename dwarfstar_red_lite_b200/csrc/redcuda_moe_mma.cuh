@@ -20,7 +20,7 @@ struct MmaArgs {
     const uint2 *lut_grid; const uint4 *lut_sign;        // filled by launch_moe_mma
     uint32_t S, tiles_per_warp, item_tok, item_class;    // filled by launch_moe_mma
     float dw1, dw2;                // weights of digits 1 and 2 (2^bits, 4^bits), filled by launch_moe_mma
-    uint32_t *work;                // nibble-layout kernels: the launch's unit counter, zeroed by the grouping kernel
+    uint32_t *work;                // nibble-layout batch kernel: the launch's run counter, zeroed by the grouping kernel
     uint32_t fmt;                  // nibble-layout kernels: NIB_IQ2, NIB_IQ3 or NIB_IQ2W
     const float *x_raw;            // nibble-layout gate/up of a single token: its fp32 activation row, quantised inside the kernel (xq / sx unused)
     uint32_t act_bits;             // digit width, filled by the launcher
@@ -48,20 +48,29 @@ constexpr uint32_t NIB_BLOCK_BYTES = 138u;
 // and a power-of-two scale per 256-column block (k_quant_act_wide). NIB_IQ2W: IQ2_XXS codes of a layer whose other matrices are IQ3_S.
 constexpr uint32_t NIB_IQ2 = 0u, NIB_IQ3 = 1u, NIB_IQ2W = 2u;
 constexpr uint32_t NIB_WIDE_PAIRS = 6u;      // pairs of a work item in the wide form: four digits each fill the 24 columns of three tiles
-// one record = one 16-row tile x one 256-column block
+// One record = one 16-row tile x one 256-column block, laid out by the MMA fragments that a warp's lanes (g = lane / 4, t = lane % 4) take
+// from it: rows g and g + 8, code words (t, kg) of all eight 32-column groups kg.
 constexpr uint32_t NIB_SC_OFF = 2048u, NIB_D_OFF = 2176u, NIB_REC = 2208u;
-// byte offset of code word (t, kg) of row rr inside a record (16-byte piece p of row rr is stored at p ^ (rr % 8))
+// where the 16-byte pieces of a lane sit inside each of the record's four runs of 512 bytes (run 2 (row / 8) + kg / 4): a warp's load of
+// a run is contiguous, and from shared memory eight lanes (two rows, or the same t of eight rows) hit eight different bank groups
+__host__ __device__ __forceinline__ uint32_t nib_lane_off(uint32_t g, uint32_t t) { return (8u * t + (g ^ (2u * t))) * 16u; }
+// byte offset of code word (t, kg) of row rr inside a record
 __host__ __device__ __forceinline__ uint32_t nib_code_off(uint32_t rr, uint32_t t, uint32_t kg) {
-    const uint32_t piece = (2u * t + (kg >> 2)) ^ (rr & 7u);
-    return rr * 128u + piece * 16u + (kg & 3u) * 4u;
+    return (2u * (rr >> 3) + (kg >> 2)) * 512u + nib_lane_off(rr & 7u, t) + (kg & 3u) * 4u;
 }
+// byte offset of the scale of group kg and of d of row rr: rows g and g + 8 side by side
+__host__ __device__ __forceinline__ uint32_t nib_sc_off(uint32_t rr, uint32_t kg) { return NIB_SC_OFF + (rr & 7u) * 16u + (rr >> 3) * 8u + kg; }
+__host__ __device__ __forceinline__ uint32_t nib_d_off(uint32_t rr) { return NIB_D_OFF + (rr & 7u) * 4u + (rr >> 3) * 2u; }
 uint64_t nib_matrix_bytes(uint32_t nrows, uint32_t ncols);
 bool nib_shape_ok(uint32_t nrows, uint32_t ncols);
 // GGUF rows of IQ2_XXS (NIB_IQ2, NIB_IQ2W) or IQ3_S (NIB_IQ3), one matrix or several in a row (nrows = all their rows) -> nibble layout
 // (dst: nib_matrix_bytes, 16-byte aligned)
 int launch_nib_repack(uint32_t fmt, const uint8_t *raw, uint64_t nrows, uint32_t ncols, uint8_t *dst, cudaStream_t s);
-// gate/up (A.w1 set) or down projection of the grouped pairs, work items of at most 8 pairs (wide form: NIB_WIDE_PAIRS); persistent kernel
-int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s);
+// gate/up (A.w1 set) or down projection of the grouped pairs, work items of at most 8 pairs (wide form: NIB_WIDE_PAIRS), of which there are
+// at most max_items; persistent kernel (redcuda_moe_nib_batch.cu). A.work: its counter, zeroed by the grouping kernel
+int launch_nib_batch(MmaArgs &A, uint32_t max_items, cudaStream_t s);
+// gate/up of the top_k experts of a single token (A.x_raw), quantised inside the kernel
+int launch_nib_one(MmaArgs &A, uint32_t top_k, cudaStream_t s);
 // Single token, nibble layout: down projection of the token's top_k experts for one 16-row tile per block, the shared
 // expert's down rows, and the tail out = resid + sum_k w_k * expert_k + shared * scalar, in router order — the fusion of
 // redmetal_topk_down_tail (native/redmetal_topk.m:254-280). The act rows are quantised inside the kernel.

@@ -16,13 +16,11 @@
 // Layout of one expert matrix [nrows][ncols], bpr = ncols / 256 blocks per row: one contiguous RECORD of 2208 bytes per
 // (16-row tile, 256-column block), records ordered [tile][block], so that a warp fetches everything it needs for one
 // block of its tile with a single bulk copy:
-//   codes  @0     16 rows x 128 B; logical byte 32 t + 4 kg of a row = u32 word (t, kg) = the 8 weights 32 kg + 8 t .. +7
-//                 of the block, weight j in bits 4j+3..4j (NIB_IQ3: weights j and j + 4 in the low and high nibble of
-//                 byte j). Piece p (16 bytes) of row r is stored at p ^ (r % 8): a record lands in shared memory as it is,
-//                 and eight lanes that read the same piece of eight rows, or the pieces 2 t of two rows, hit eight
-//                 different bank groups
-//   scales @2048  16 rows x 8 B, byte kg = 2 s + 1, s the 4-bit scale of the 32-weight group
-//   d      @2176  16 fp16 block scales
+//   codes  @0     per row and 32-column group kg four words t of 8 weights 32 kg + 8 t .. +7 of the block, weight j in bits
+//                 4j+3..4j (NIB_IQ3: weights j and j + 4 in the low and high nibble of byte j); placed by nib_code_off so that a
+//                 warp's loads of them are contiguous in device memory and free of bank conflicts in shared memory
+//   scales @2048  16 rows x 8 B, byte kg = 2 s + 1, s the 4-bit scale of the 32-weight group (nib_sc_off)
+//   d      @2176  16 fp16 block scales (nib_d_off)
 // Arithmetic is the integer tensor-core scheme of redcuda_moe_mma.cu (mma.sync m16n8k32 s8, activations as three
 // balanced digits per value, s32 sums per 32-weight group scaled by the integer 2s+1, fp32 scaling by d/8 per block).
 // Layers with IQ3_S matrices take the wide form of the digits (actw_scale in redcuda_moe_mma.cuh): four per value and a scale per
@@ -31,20 +29,18 @@
 // to 1.2e-7. The fourth digit costs nothing where items hold one or two pairs, which fill one tile either way (24 tokens: 118 us a
 // layer with four, 120 with three).
 //
-// Kernel: persistent CTAs of 8 warps, two per SM. A unit of work = one work item (<= 8 pairs of one expert, cut by
-// k_group_pairs) x a block of rows; CTAs draw units from an atomic counter, so the routing skew never leaves SMs idle
-// and nothing is set up per unit except the item's activation digits in shared memory. Every warp streams its 16-row
-// tiles through a private ring of three records (one cp.async.bulk and one mbarrier each; the ring runs on across unit
-// boundaries). Waits on the mbarriers are bounded: a warp that gives up raises the status word and the CTA winds down.
-// Column layout of the digits: items of one or two pairs pack (pair, digit) into one 8-column tile (cols 3*pair+digit);
-// larger items use one tile per digit (col = 8*digit + pair), so a lane holds all three digits of its two pairs and the
-// epilogue needs no exchange. Wide form: col = 4*pair + digit, two pairs a tile and as many tiles as the item's pairs need (one to
+// Here: the re-coding and the two kernels of a single token (k_nib_one for gate/up, k_nib_down_tail); batches are in
+// redcuda_moe_nib_batch.cu. Every warp streams its 16-row tiles through a private ring of records (one cp.async.bulk and one mbarrier
+// each). Waits on the mbarriers are bounded: a warp that gives up raises the status word and the block winds down.
+// Column layout of the digits: items of up to four pairs pack two (pair, digit) triples into an 8-column tile (cols 3 * pair + digit);
+// larger items use one tile per digit (col = 8 * digit + pair), so a lane holds all three digits of its two pairs and the
+// epilogue needs no exchange. Wide form: col = 4 * pair + digit, two pairs a tile and as many tiles as the item's pairs need (one to
 // three); the two lanes that hold a pair's digits exchange one sum each at the end of a tile.
 #define RC_PDL_DEFAULT 0
 #include "redcuda_common.cuh"
 #include "redcuda_dot.cuh"
 #include "redcuda_kernels.cuh"
-#include "redcuda_moe_mma.cuh"
+#include "redcuda_nib.cuh"
 #include "redcuda_stage.cuh"
 #include "../../include/redcuda.h"
 
@@ -96,8 +92,8 @@ __global__ void k_nib_repack(const uint8_t *__restrict__ raw, uint64_t nb, uint3
         const uint32_t rr = (uint32_t)row & 15u;
         *reinterpret_cast<uint32_t *>(rec + nib_code_off(rr, t, kg)) = word;
         if (t == 0u) {
-            rec[NIB_SC_OFF + rr * 8u + kg] = (uint8_t)(2u * s4 + 1u);
-            if (kg == 0u) *reinterpret_cast<unsigned short *>(rec + NIB_D_OFF + rr * 2u) = *reinterpret_cast<const unsigned short *>(bp);
+            rec[nib_sc_off(rr, kg)] = (uint8_t)(2u * s4 + 1u);
+            if (kg == 0u) *reinterpret_cast<unsigned short *>(rec + nib_d_off(rr)) = *reinterpret_cast<const unsigned short *>(bp);
         }
     }
 }
@@ -127,8 +123,8 @@ __global__ void k_nib_dequant(const uint8_t *__restrict__ nib, uint64_t nb, uint
         const uint8_t *rec = nib + ((uint64_t)(row >> 4) * bpr + blk) * NIB_REC;
         const uint32_t rr = row & 15u;
         const uint32_t word = *reinterpret_cast<const uint32_t *>(rec + nib_code_off(rr, t, kg));
-        const uint32_t scb = rec[NIB_SC_OFF + rr * 8u + kg];
-        const float d = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(rec + NIB_D_OFF + rr * 2u)));
+        const uint32_t scb = rec[nib_sc_off(rr, kg)];
+        const float d = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(rec + nib_d_off(rr))));
         const float db = d * (0.5f + (float)((scb - 1u) >> 1)) * 0.25f;
         float *o = out + ((uint64_t)row * bpr + blk) * 256u + kg * 32u + t * 8u;
 #pragma unroll
@@ -140,132 +136,12 @@ __global__ void k_nib_dequant(const uint8_t *__restrict__ nib, uint64_t nb, uint
     }
 }
 
-// ---- small PTX wrappers ----
-__device__ __forceinline__ uint32_t nb_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// z: four registers that hold zero for the whole kernel, the accumulator input of every MMA (each 32-weight group gets
-// its own exact s32 product sum, scaled by the group's integer scale afterwards)
-__device__ __forceinline__ void nb_mma(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, const int (&z)[4]) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(z[0]), "r"(z[1]), "r"(z[2]), "r"(z[3]));
-}
-// byte permute with the selector taken as it is (the intrinsic masks bit 3 of every selector nibble first, one more
-// instruction per use; the 4-bit codes never set it)
-__device__ __forceinline__ uint32_t nb_prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
-// the 8 codes of a word -> the int8 operands of weights 0..3 (lo) and 4..7 (hi)
-template <uint32_t FMT>
-__device__ __forceinline__ void nb_expand(uint32_t w, uint32_t &lo, uint32_t &hi);
-// one record into a ring slot: the copy engine signals the slot's mbarrier with the bytes it delivered
-__device__ __forceinline__ void nb_fetch(uint32_t dst, const void *src, uint32_t bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(NIB_REC) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(dst), "l"(src), "r"(NIB_REC), "r"(bar) : "memory");
-}
-constexpr uint32_t NIB_SPIN_LIMIT = 1u << 22;      // polls of the (itself time-limited) try_wait: far beyond any real wait
-__device__ __forceinline__ bool nb_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < NIB_SPIN_LIMIT; ++i) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
 constexpr uint32_t NIB_WARPS = 8u;
-// records in flight per warp: 3 for batches (two blocks per SM), 8 for a single token (few units, one block per SM: a
-// warp requests its whole tile at once, one HBM round trip instead of three)
-constexpr uint32_t NIB_STAGES_BATCH = 3u, NIB_STAGES_ONE = 8u;
-constexpr uint32_t NIB_TAB_POS = 0x002b1908u, NIB_TAB_NEG = 0x00d5e7f8u;      // bytes 8, 25, 43, 0 and -8, -25, -43, 0
+constexpr uint32_t NIB_STAGES = 8u;       // records in flight per warp: a warp requests its whole tile of 2048 columns at once, one HBM round trip
 
-template <>
-__device__ __forceinline__ void nb_expand<NIB_IQ2>(uint32_t w, uint32_t &lo, uint32_t &hi) {
-    lo = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, w); hi = nb_prmt(NIB_TAB_POS, NIB_TAB_NEG, w >> 16);
-}
-template <>
-__device__ __forceinline__ void nb_expand<NIB_IQ2W>(uint32_t w, uint32_t &lo, uint32_t &hi) { nb_expand<NIB_IQ2>(w, lo, hi); }
-template <>
-__device__ __forceinline__ void nb_expand<NIB_IQ3>(uint32_t w, uint32_t &lo, uint32_t &hi) {
-    lo = ((w << 4) & 0xf0f0f0f0u) | 0x08080808u; hi = (w & 0xf0f0f0f0u) | 0x08080808u;
-}
-
-// One warp: 16 rows x one 256-column block (a record in shared memory) against NT 8-column tiles of activation digits.
-// Bl: digits of column g of tile 0 at this block's first column + 8 t (tile n is n * 8 * BPITCH further).
-// blk[n]: sums of rows g (0, 1) and g + 8 (2, 3), columns 2 t and 2 t + 1 of tile n; da, db: d / 8 of the two rows.
-template <uint32_t FMT, int NT, uint32_t BPITCH>
-__device__ __forceinline__ void nib_sums(const uint8_t *st, const int8_t *Bl, uint32_t g, uint32_t t, const int (&z)[4], int (&blk)[NT][4], float &da, float &db) {
-    const uint32_t o0 = nib_code_off(g, t, 0u), o1 = nib_code_off(g, t, 4u);   // rows g and g + 8 have the same swizzle
-    const uint4 qa0 = *reinterpret_cast<const uint4 *>(st + o0), qa1 = *reinterpret_cast<const uint4 *>(st + o1);
-    const uint4 qb0 = *reinterpret_cast<const uint4 *>(st + 1024u + o0), qb1 = *reinterpret_cast<const uint4 *>(st + 1024u + o1);
-    const uint2 sa = *reinterpret_cast<const uint2 *>(st + NIB_SC_OFF + g * 8u), sb = *reinterpret_cast<const uint2 *>(st + NIB_SC_OFF + (g + 8u) * 8u);
-    da = 0.125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(st + NIB_D_OFF + g * 2u)));
-    db = 0.125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(st + NIB_D_OFF + (g + 8u) * 2u)));
-    const uint32_t wa[8] = {qa0.x, qa0.y, qa0.z, qa0.w, qa1.x, qa1.y, qa1.z, qa1.w};
-    const uint32_t wb[8] = {qb0.x, qb0.y, qb0.z, qb0.w, qb1.x, qb1.y, qb1.z, qb1.w};
-#pragma unroll
-    for (int n = 0; n < NT; ++n) { blk[n][0] = blk[n][1] = blk[n][2] = blk[n][3] = 0; }
-#pragma unroll
-    for (int kg = 0; kg < 8; ++kg) {
-        uint32_t a0, a1, a2, a3;
-        nb_expand<FMT>(wa[kg], a0, a2);
-        nb_expand<FMT>(wb[kg], a1, a3);
-        const int sca = (int)nb_prmt(kg < 4 ? sa.x : sa.y, 0u, 0x4440u + (uint32_t)(kg & 3));
-        const int scb = (int)nb_prmt(kg < 4 ? sb.x : sb.y, 0u, 0x4440u + (uint32_t)(kg & 3));
-#pragma unroll
-        for (int n = 0; n < NT; ++n) {
-            const uint2 bf = *reinterpret_cast<const uint2 *>(Bl + (uint32_t)n * 8u * BPITCH + (uint32_t)kg * 32u);
-            int d[4];
-            nb_mma(d, a0, a1, a2, a3, bf.x, bf.y, z);
-            blk[n][0] += sca * d[0]; blk[n][1] += sca * d[1];
-            blk[n][2] += scb * d[2]; blk[n][3] += scb * d[3];
-        }
-    }
-}
-template <uint32_t FMT, int NT, uint32_t BPITCH>
-__device__ __forceinline__ void nib_chunk(const uint8_t *st, const int8_t *Bl, uint32_t g, uint32_t t, const int (&z)[4], float (&out)[3][4]) {
-    int blk[NT][4];
-    float da, db;
-    nib_sums<FMT, NT, BPITCH>(st, Bl, g, t, z, blk, da, db);
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-        out[n][0] += da * (float)blk[n][0]; out[n][1] += da * (float)blk[n][1];
-        out[n][2] += db * (float)blk[n][2]; out[n][3] += db * (float)blk[n][3];
-    }
-}
-// The wide form: column 4 p + i is digit i of pair p, so lane t holds two digits of pair 2 n + t / 2 of tile n, the upper two where
-// t is odd. sx[n * 2 * SXP]: that pair's scale of this block. out[n]: rows g and g + 8.
-template <uint32_t FMT, int NT, uint32_t BPITCH, uint32_t SXP>
-__device__ __forceinline__ void nib_chunk_wide(const uint8_t *st, const int8_t *Bl, const float *sx, uint32_t g, uint32_t t, const int (&z)[4], float (&out)[NT][2]) {
-    int blk[NT][4];
-    float da, db;
-    nib_sums<FMT, NT, BPITCH>(st, Bl, g, t, z, blk, da, db);
-    const float up = t & 1u ? 65536.0f : 1.0f;
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-        const float w = sx[n * 2u * SXP] * up;              // a power of two: da * w and db * w are exact
-        out[n][0] += (da * w) * fmaf(256.0f, (float)blk[n][1], (float)blk[n][0]);
-        out[n][1] += (db * w) * fmaf(256.0f, (float)blk[n][3], (float)blk[n][2]);
-    }
-}
-// a lane's row g and g + 8 sums of its two digits -> the full sum of row g (even t) or g + 8 (odd t)
-__device__ __forceinline__ float nib_pair_sum(float r0, float r1, uint32_t t) {
-    const float got = __shfl_xor_sync(0xffffffffu, t & 1u ? r0 : r1, 1);
-    return (t & 1u ? r1 : r0) + got;
-}
-
-struct NibUnit {
-    const uint8_t *rec;        // first record of this warp's tiles in the unit (records of a tile, then of the next tile, are contiguous)
-    uint32_t item, p0, nt;     // work item, its first pair in sorted[], its pairs
-    uint32_t tile0, n;         // first 16-row tile of this warp and the number of records it streams in the unit
-};
-
-// A warp's private ring of STAGES record slots. Records are requested in stream order: first the rest of the
-// current unit (cur_*), then the first ones of the next unit (nxt_*), so the ring never drains at a unit boundary.
-// Between two reads exactly one request is made, which keeps STAGES - 1 records in flight behind the one being read.
+// A warp's private ring of record slots. Records are requested in stream order: first the rest of the current unit (cur_*), then the
+// first ones of the next unit (nxt_*), so the ring never drains at a unit boundary. Between two reads exactly one request is made,
+// which keeps NIB_STAGES - 1 records in flight behind the one being read.
 struct NibRing {
     uint32_t stage_s, bar_s;           // shared-memory addresses of slot 0 and of its mbarrier
     uint32_t prod, cons, phase;        // next slot to fill / to read; bit s = parity the next read of slot s waits for
@@ -273,14 +149,13 @@ struct NibRing {
     uint32_t cur_rem, nxt_rem, nxt_taken;
     uint32_t timed_out;
 };
-template <uint32_t STAGES>
 __device__ __forceinline__ void nib_request(NibRing &R, uint32_t lane) {
     const uint8_t *src;
     if (R.cur_rem) { src = R.cur_src; R.cur_src += NIB_REC; --R.cur_rem; }
     else if (R.nxt_rem) { src = R.nxt_src; R.nxt_src += NIB_REC; --R.nxt_rem; ++R.nxt_taken; }
     else return;
     if (lane == 0) nb_fetch(R.stage_s + R.prod * NIB_REC, src, R.bar_s + 8u * R.prod);
-    R.prod = R.prod + 1u == STAGES ? 0u : R.prod + 1u;
+    R.prod = R.prod + 1u == NIB_STAGES ? 0u : R.prod + 1u;
 }
 // waits for the oldest record; returns its slot. After a wait ran out no further wait is attempted (the results of the
 // launch are void: the caller raises the status word).
@@ -289,128 +164,95 @@ __device__ __forceinline__ uint32_t nib_acquire(NibRing &R) {
     if (!R.timed_out && !nb_wait(R.bar_s + 8u * slot, (R.phase >> slot) & 1u)) R.timed_out = 1u;
     return slot;
 }
-template <uint32_t STAGES>
 __device__ __forceinline__ void nib_release(NibRing &R) {
     __syncwarp();                      // every lane has read the slot: it may be refilled
     R.phase ^= 1u << R.cons;
-    R.cons = R.cons + 1u == STAGES ? 0u : R.cons + 1u;
+    R.cons = R.cons + 1u == NIB_STAGES ? 0u : R.cons + 1u;
 }
 
-// All tiles of one unit for one warp, NT column tiles of digits in use (1: pairs packed into one tile, 3: a tile per digit).
-// vals[ti][.] = (row g, pair slot 0), (row g, pair slot 1), (row g + 8, slot 0), (row g + 8, slot 1), times the pair's scale.
-template <uint32_t FMT, int NT, uint32_t BPR, uint32_t BPITCH, uint32_t TPW, uint32_t STAGES>
-__device__ __forceinline__ void nib_tiles(NibRing &R, const uint8_t *my_stage, const int8_t *Bbase, uint32_t tiles, uint32_t lane, uint32_t g, uint32_t t,
-                                          const int (&z)[4], float dw1, float dw2, const float (&sxv)[2], float (&vals)[TPW][4]) {
+// A unit's tiles for one warp. vals[ti][0], [1] = rows g and g + 8 on the lanes t == 0 (three digits: times the token's scale sx), or
+// vals[ti][0] = row g (t == 0) or g + 8 (t == 1) in the wide form, whose block scales are sxw.
+template <uint32_t FMT, uint32_t BPR, uint32_t BPITCH, uint32_t TPW>
+__device__ __forceinline__ void nib_tiles(NibRing &R, const uint8_t *my_stage, const int8_t *Bbase, const float *sxw, uint32_t tiles, uint32_t lane, uint32_t g, uint32_t t,
+                                          const int (&z)[4], float dw1, float dw2, float sx, float (&vals)[TPW][2]) {
     for (uint32_t ti = 0; ti < tiles; ++ti) {
-        float out[3][4];
-#pragma unroll
-        for (int n = 0; n < 3; ++n) { out[n][0] = out[n][1] = out[n][2] = out[n][3] = 0.f; }
+        float out[3][4], ow[1][2] = {{0.f, 0.f}};
+        out[0][0] = out[0][1] = out[0][2] = out[0][3] = 0.f;
         for (uint32_t c = 0; c < BPR; ++c) {
-            nib_request<STAGES>(R, lane);
+            nib_request(R, lane);
             const uint32_t slot = nib_acquire(R);
-            nib_chunk<FMT, NT, BPITCH>(my_stage + slot * NIB_REC, Bbase + c * 256u, g, t, z, out);
-            nib_release<STAGES>(R);
+            if constexpr (FMT != NIB_IQ2) nib_chunk_wide<FMT, 1, BPITCH, BPR>(my_stage + slot * NIB_REC, Bbase + c * 256u, sxw + c, g, t, z, ow);
+            else nib_chunk<FMT, 1, BPITCH>(my_stage + slot * NIB_REC, Bbase + c * 256u, g, t, z, out);
+            nib_release(R);
         }
-        float v[2][2];                 // [row half][pair slot]
-        if (NT == 1) {
-            const uint32_t src = (lane & ~3u) + 1u;
-            const float x0 = __shfl_sync(0xffffffffu, out[0][0], src), y0 = __shfl_sync(0xffffffffu, out[0][1], src);
-            const float x1 = __shfl_sync(0xffffffffu, out[0][2], src), y1 = __shfl_sync(0xffffffffu, out[0][3], src);
-            // t == 0: pair 0 = cols 0, 1 (own) and 2 (lane t = 1); t == 2: pair 1 = col 3 (lane t = 1) and cols 4, 5 (own)
-            v[0][0] = t == 0u ? out[0][0] + dw1 * out[0][1] + dw2 * x0 : y0 + dw1 * out[0][0] + dw2 * out[0][1];
-            v[1][0] = t == 0u ? out[0][2] + dw1 * out[0][3] + dw2 * x1 : y1 + dw1 * out[0][2] + dw2 * out[0][3];
-            v[0][1] = v[1][1] = 0.f;
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) v[h][j] = out[0][2 * h + j] + dw1 * out[1][2 * h + j] + dw2 * out[2][2 * h + j];
+        if (FMT != NIB_IQ2) vals[ti][0] = nib_pair_sum(ow[0][0], ow[0][1], t);
+        else {
+            const uint32_t src = (lane & ~3u) + 1u;      // digits 0 and 1 are the columns of lane t = 0, digit 2 is lane t = 1's first
+            const float x0 = __shfl_sync(0xffffffffu, out[0][0], src), x1 = __shfl_sync(0xffffffffu, out[0][2], src);
+            vals[ti][0] = (out[0][0] + dw1 * out[0][1] + dw2 * x0) * sx; vals[ti][1] = (out[0][2] + dw1 * out[0][3] + dw2 * x1) * sx;
         }
-        vals[ti][0] = v[0][0] * sxv[0]; vals[ti][1] = v[0][1] * sxv[1]; vals[ti][2] = v[1][0] * sxv[0]; vals[ti][3] = v[1][1] * sxv[1];
     }
 }
 
-// The wide form, NT = tiles in use (two pairs each). vals[ti][n] = row g (even t) or g + 8 (odd t) of pair 2 n + t / 2.
-template <uint32_t FMT, int NT, uint32_t BPR, uint32_t BPITCH, uint32_t TPW, uint32_t STAGES>
-__device__ __forceinline__ void nib_tiles_wide(NibRing &R, const uint8_t *my_stage, const int8_t *Bbase, const float *sx, uint32_t tiles, uint32_t lane, uint32_t g, uint32_t t,
-                                               const int (&z)[4], float (&vals)[TPW][4]) {
-    for (uint32_t ti = 0; ti < tiles; ++ti) {
-        float out[NT][2];
-#pragma unroll
-        for (int n = 0; n < NT; ++n) out[n][0] = out[n][1] = 0.f;
-        for (uint32_t c = 0; c < BPR; ++c) {
-            nib_request<STAGES>(R, lane);
-            const uint32_t slot = nib_acquire(R);
-            nib_chunk_wide<FMT, NT, BPITCH, BPR>(my_stage + slot * NIB_REC, Bbase + c * 256u, sx + c, g, t, z, out);
-            nib_release<STAGES>(R);
-        }
-#pragma unroll
-        for (int n = 0; n < NT; ++n) vals[ti][n] = nib_pair_sum(out[n][0], out[n][1], t);
-    }
-}
-
-// GATEUP: warps 0-3 take the gate rows of 4 x TPW tiles, warps 4-7 the up rows of the same tiles; the up values cross a
-// small shared buffer and the gate warps store SiLU(gate) * up. Otherwise (down projection) 8 x TPW tiles per unit.
-template <uint32_t FMT, bool GATEUP, uint32_t NCOLS, uint32_t STAGES>
-__global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 2 : 1) k_nib_experts(const __grid_constant__ MmaArgs A) {
+// Gate/up with SiLU * mul of a single token's experts: blocks of 8 warps take units of 4 x TPW tiles; warps 0-3 the gate rows, warps
+// 4-7 the up rows of the same tiles; the up values cross a small shared buffer and the gate warps store SiLU(gate) * up. The token is
+// quantised in the kernel, while the first records arrive.
+template <uint32_t FMT, uint32_t NCOLS>
+__global__ void __launch_bounds__(NIB_WARPS * 32u, 1) k_nib_one(const __grid_constant__ MmaArgs A) {
     pdl_prologue();
     extern __shared__ __align__(16) uint8_t smem[];
-    constexpr uint32_t BPR = NCOLS / 256u, TPW = BPR >= 8u ? 1u : 8u / BPR, WSLOTS = GATEUP ? 4u : 8u, UNIT_TILES = WSLOTS * TPW;
-    constexpr uint32_t BPITCH = NCOLS + 32u, V16 = NCOLS / 16u;
-    constexpr bool ONE = STAGES == NIB_STAGES_ONE;        // the form of a single token: A.x_raw holds it
+    constexpr uint32_t BPR = NCOLS / 256u, TPW = BPR >= 8u ? 1u : 8u / BPR, UNIT_TILES = 4u * TPW, BPITCH = NCOLS + 32u;
     constexpr bool WIDE = FMT != NIB_IQ2;
-    __shared__ float s_sxw[WIDE ? (ONE ? 1u : NIB_WIDE_PAIRS) * BPR : 1u];      // scales of the item's pairs and blocks
-    __shared__ uint32_t s_unit[2];
+    __shared__ float s_sxw[WIDE ? BPR : 1u];      // scales of the token's blocks
     __shared__ volatile uint32_t s_fail;
-    __shared__ __align__(8) uint64_t s_bar[NIB_WARPS][STAGES];
-    __shared__ __align__(16) float4 s_ex[GATEUP ? TPW : 1u][4][32];
+    __shared__ __align__(8) uint64_t s_bar[NIB_WARPS][NIB_STAGES];
+    __shared__ float2 s_ex[TPW][4][32];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
-    uint8_t *my_stage = smem + warp * (STAGES * NIB_REC);
-    int8_t *Bs = reinterpret_cast<int8_t *>(smem + NIB_WARPS * STAGES * NIB_REC);
+    uint8_t *my_stage = smem + warp * (NIB_STAGES * NIB_REC);
+    int8_t *Bs = reinterpret_cast<int8_t *>(smem + NIB_WARPS * NIB_STAGES * NIB_REC);
     const uint32_t ntile_rows = A.nrows >> 4, U = (ntile_rows + UNIT_TILES - 1u) / UNIT_TILES;
     const uint32_t total = *A.n_items * U;
-    const bool is_up = GATEUP && warp >= 4u;
-    const uint32_t wslot = GATEUP ? (warp & 3u) : warp;
+    const bool is_up = warp >= 4u;
+    const uint32_t wslot = warp & 3u;
     const uint8_t *wmat = is_up ? A.w1 : A.w0;
     NibRing R{};
     R.stage_s = nb_smem(my_stage); R.bar_s = nb_smem(&s_bar[warp][0]);
 
-    auto decode = [&](uint32_t unit, NibUnit &I) {
-        const uint32_t item = unit / U, rb = unit - item * U;
-        uint32_t e, nt;
-        if (ONE) { e = A.uexp[item] - A.expert_begin; nt = 1u; I.p0 = item; }       // single token: item = group = pair
-        else {
-            const uint32_t u = A.item_u[item], p0 = A.item_p0[item];
-            e = A.uexp[u] - A.expert_begin; nt = min(A.item_tok, A.ustart[u + 1u] - p0);
-            I.p0 = p0;
-        }
-        if (e >= A.n_local) { if (A.status && tid == 0) A.status[ST_EXPERT_RANGE] = 1u; e = 0u; nt = 0u; }     // never index the arena with a foreign id
-        I.item = item; I.nt = nt;
+    struct Unit {
+        const uint8_t *rec;        // first record of this warp's tiles in the unit (records of a tile, then of the next tile, are contiguous)
+        uint32_t item;             // = the pair
+        uint32_t tile0, n;         // first 16-row tile of this warp and the number of records it streams in the unit
+    };
+    auto decode = [&](uint32_t unit, Unit &I) {
+        const uint32_t rb = unit % U;
+        I.item = unit / U;
+        uint32_t e = A.uexp[I.item] - A.expert_begin;
+        const bool ok = e < A.n_local;
+        if (!ok) { if (A.status && tid == 0) A.status[ST_EXPERT_RANGE] = 1u; e = 0u; }     // never index the arena with a foreign id
         I.tile0 = rb * UNIT_TILES + wslot * TPW;
         const uint32_t tiles = I.tile0 >= ntile_rows ? 0u : min(TPW, ntile_rows - I.tile0);
-        I.n = nt ? tiles * BPR : 0u;
+        I.n = ok ? tiles * BPR : 0u;
         I.rec = wmat + (size_t)e * A.mat_bytes + (size_t)I.tile0 * BPR * NIB_REC;
     };
 
-    // the units of a single token are few and equal: block b takes b, b + grid, ..., which saves the counter's round trip
-    if (tid == 0) { s_unit[0] = ONE ? blockIdx.x : atomicAdd(A.work, 1u); s_fail = 0u; }
+    // the units are few and equal: block b takes b, b + grid, ...
+    if (tid == 0) s_fail = 0u;
     if (lane == 0) {
-        for (uint32_t i = 0; i < STAGES; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(R.bar_s + 8u * i));
+        for (uint32_t i = 0; i < NIB_STAGES; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(R.bar_s + 8u * i));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
-    uint32_t cur = s_unit[0], par = 0u, cur_item = 0xffffffffu;
+    uint32_t cur = blockIdx.x;
     uint32_t ahead = 0u;             // records of the CURRENT unit already requested (while the previous unit was multiplying)
-    NibUnit I{}, N{};
+    Unit I{}, N{};
     if (cur < total) decode(cur, I);
-    if (ONE) {                   // the first records are on their way while the block quantises the token
-        R.cur_src = I.rec; R.cur_rem = I.n;
-        while (ahead + 1u < STAGES && ahead < I.n) { nib_request<STAGES>(R, lane); ++ahead; }
-    }
+    // the first records are on their way while the block quantises the token
+    R.cur_src = I.rec; R.cur_rem = I.n;
+    while (ahead + 1u < NIB_STAGES && ahead < I.n) { nib_request(R, lane); ++ahead; }
     __shared__ uint32_t s_red[NIB_WARPS];
-    __shared__ float s_sx;
-    if (ONE && WIDE) {
+    float sx = 1.0f;
+    if (WIDE) {
         // a warp per block of the row; columns 0..3 of the one tile in use, columns 4..7 zero
         if (warp < BPR) {
             const uint32_t k = warp * 256u + lane * 8u;
@@ -426,10 +268,9 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
             for (uint32_t col = 0u; col < 8u; ++col)
                 *reinterpret_cast<uint2 *>(Bs + col * BPITCH + k) = col < 4u ? make_uint2(p0[col & 3u], p1[col & 3u]) : make_uint2(0u, 0u);
         }
-        __syncthreads();
-    } else if (ONE) {
-        // single token: every unit multiplies the same activation row, so the block turns it into digits itself (the
-        // arithmetic of k_quant_act) — columns 0..2 of the one tile in use, columns 3..7 zero
+    } else {
+        // every unit multiplies the same activation row, so the block turns it into digits itself (the arithmetic of
+        // k_quant_act): columns 0..2 of the one tile in use, columns 3..7 zero
         uint32_t mx = 0u;
         for (uint32_t k = tid * 4u; k < NCOLS; k += NIB_WARPS * 128u) mx = max(mx, act_mag4(*reinterpret_cast<const float4 *>(A.x_raw + k)));
         mx = __reduce_max_sync(0xffffffffu, mx);
@@ -437,8 +278,7 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
         __syncthreads();
         mx = s_red[0];
         for (uint32_t w = 1; w < NIB_WARPS; ++w) mx = max(mx, s_red[w]);
-        const float qmax = act_qmax(A.act_bits), scale = act_scale(mx, qmax), inv = 1.0f / scale;
-        if (tid == 0) s_sx = scale;
+        const float qmax = act_qmax(A.act_bits), inv = 1.0f / (sx = act_scale(mx, qmax));
         for (uint32_t k = tid * 4u; k < NCOLS; k += NIB_WARPS * 128u) {
             const float4 v = *reinterpret_cast<const float4 *>(A.x_raw + k);
             const float f[4] = {v.x, v.y, v.z, v.w};
@@ -455,108 +295,36 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, STAGES == NIB_STAGES_BATCH ? 
 #pragma unroll
             for (uint32_t col = 3u; col < 8u; ++col) *reinterpret_cast<uint32_t *>(Bs + col * BPITCH + k) = 0u;
         }
-        __syncthreads();
     }
+    __syncthreads();
     int zero[4];                     // opaque to the compiler: four registers that stay zero, the accumulator input of every MMA
     asm volatile("mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;" : "=r"(zero[0]), "=r"(zero[1]), "=r"(zero[2]), "=r"(zero[3]));
     while (cur < total) {
-        if (tid == 0) s_unit[par ^ 1u] = ONE ? cur + gridDim.x : atomicAdd(A.work, 1u);
-        // this unit's stream; STAGES - 1 of its records are put in flight before the first read
+        const uint32_t nxt = cur + gridDim.x;
+        // this unit's stream; NIB_STAGES - 1 of its records are put in flight before the first read
         R.cur_src = I.rec + (size_t)ahead * NIB_REC; R.cur_rem = I.n - ahead; R.nxt_rem = 0u; R.nxt_taken = 0u;
-        for (uint32_t i = ahead; i + 1u < STAGES; ++i) nib_request<STAGES>(R, lane);
-        const bool packed = I.nt <= 2u;
-        if (!ONE && I.item != cur_item) {    // activation digits of the item (every warp passed the barrier that ended the last unit)
-            const uint32_t ncolb = WIDE ? (I.nt + 1u) / 2u * 8u : packed ? 8u : 24u;
-            for (uint32_t i = tid; i < ncolb * V16; i += NIB_WARPS * 32u) {
-                const uint32_t col = i / V16, k = (i - col * V16) << 4;
-                const uint32_t tk = WIDE ? col >> 2 : packed ? col / 3u : (col & 7u), dg = WIDE ? col & 3u : packed ? col - 3u * (col / 3u) : (col >> 3);
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (tk < I.nt) v = *reinterpret_cast<const uint4 *>(A.xq + ((size_t)(A.sorted[I.p0 + tk] / A.x_div) * (WIDE ? 4u : 3u) + dg) * NCOLS + k);
-                *reinterpret_cast<uint4 *>(Bs + (size_t)col * BPITCH + k) = v;
-            }
-            if (WIDE && tid < NIB_WIDE_PAIRS * BPR) {
-                const uint32_t tk = tid / BPR;
-                s_sxw[tid] = tk < I.nt ? A.sx[(size_t)(A.sorted[I.p0 + tk] / A.x_div) * BPR + (tid - tk * BPR)] : 0.f;
-            }
-            cur_item = I.item;
-        }
-        // the pairs this lane stores: packed -> pair t/2 on even t; one tile per digit -> pairs 2t, 2t+1; wide -> pairs t/2, t/2 + 2, t/2 + 4
-        constexpr uint32_t NP = WIDE && !ONE ? NIB_WIDE_PAIRS / 2u : 2u;
-        uint32_t prow[NP];
-        float sxv[2] = {0.f, 0.f};
-        bool ok[NP];
-        if (WIDE) {
-#pragma unroll
-            for (uint32_t j = 0; j < NP; ++j) {
-                const uint32_t tk = 2u * j + (t >> 1);
-                ok[j] = tk < I.nt;
-                prow[j] = ok[j] ? (ONE ? I.p0 : A.sorted[I.p0 + tk]) : 0u;
-            }
-        } else
-#pragma unroll
-        for (uint32_t j = 0; j < 2u; ++j) {
-            prow[j] = 0u;
-            const uint32_t tk = packed ? (t >> 1) : 2u * t + j;
-            ok[j] = packed ? (j == 0u && (t & 1u) == 0u && tk < I.nt) : tk < I.nt;
-            if (ok[j]) { prow[j] = ONE ? I.p0 : A.sorted[I.p0 + tk]; sxv[j] = ONE ? s_sx : A.sx[prow[j] / A.x_div]; }
-        }
-        __syncthreads();             // digits and the next unit's number are in shared memory
-        const uint32_t nxt = s_unit[par ^ 1u];
-        const bool nv = nxt < total;
-        if (nv) { decode(nxt, N); if (I.n + 1u >= STAGES) { R.nxt_src = N.rec; R.nxt_rem = N.n; } }     // a unit shorter than the ring does not look ahead
-
-        float vals[TPW][4];
+        for (uint32_t i = ahead; i + 1u < NIB_STAGES; ++i) nib_request(R, lane);
+        if (nxt < total) { decode(nxt, N); if (I.n + 1u >= NIB_STAGES) { R.nxt_src = N.rec; R.nxt_rem = N.n; } }     // a unit shorter than the ring does not look ahead
+        float vals[TPW][2];
         const uint32_t tiles = I.n / BPR;
-        const int8_t *Bbase = Bs + (size_t)g * BPITCH + 8u * t;
-        if constexpr (WIDE) {
-            const float *sxw = s_sxw + (ONE ? 0u : (t >> 1) * BPR);
-            if (ONE || packed) nib_tiles_wide<FMT, 1, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, sxw, tiles, lane, g, t, zero, vals);
-            else if (I.nt <= 4u) nib_tiles_wide<FMT, 2, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, sxw, tiles, lane, g, t, zero, vals);
-            else nib_tiles_wide<FMT, 3, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, sxw, tiles, lane, g, t, zero, vals);
-        } else if (packed) nib_tiles<FMT, 1, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, tiles, lane, g, t, zero, A.dw1, A.dw2, sxv, vals);
-        else nib_tiles<FMT, 3, BPR, BPITCH, TPW, STAGES>(R, my_stage, Bbase, tiles, lane, g, t, zero, A.dw1, A.dw2, sxv, vals);
+        nib_tiles<FMT, BPR, BPITCH, TPW>(R, my_stage, Bs + (size_t)g * BPITCH + 8u * t, s_sxw, tiles, lane, g, t, zero, A.dw1, A.dw2, sx, vals);
         if (R.timed_out && lane == 0) { s_fail = 1u; if (A.status) A.status[ST_TIMEOUT] = 1u; }
-        if (GATEUP) {
-            if (is_up) for (uint32_t ti = 0; ti < tiles; ++ti) s_ex[ti][wslot][lane] = make_float4(vals[ti][0], vals[ti][1], vals[ti][2], vals[ti][3]);
-        } else {
+        if (is_up) for (uint32_t ti = 0; ti < tiles; ++ti) s_ex[ti][wslot][lane] = make_float2(vals[ti][0], vals[ti][1]);
+        __syncthreads();             // up values are in s_ex
+        const bool fail = s_fail != 0u;
+        if (!is_up && t < (WIDE ? 2u : 1u)) {
             for (uint32_t ti = 0; ti < tiles; ++ti) {
-                const uint32_t row = ((I.tile0 + ti) << 4) + g;
-                if (WIDE) {
-#pragma unroll
-                    for (uint32_t j = 0; j < NP; ++j) if (ok[j]) A.out[(size_t)prow[j] * A.out_stride + row + 8u * (t & 1u)] = vals[ti][j];
-                } else
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    if (ok[j]) {
-                        A.out[(size_t)prow[j] * A.out_stride + row] = vals[ti][j];
-                        A.out[(size_t)prow[j] * A.out_stride + row + 8u] = vals[ti][2 + j];
-                    }
+                const float2 up = s_ex[ti][wslot][lane];
+                float *o = A.out + (size_t)I.item * A.out_stride + ((I.tile0 + ti) << 4) + g;
+                const float g0 = vals[ti][0], g1 = vals[ti][1];
+                if (WIDE) o[8u * t] = (g0 / (1.0f + expf(-g0))) * up.x;
+                else { o[0] = (g0 / (1.0f + expf(-g0))) * up.x; o[8] = (g1 / (1.0f + expf(-g1))) * up.y; }
             }
         }
-        __syncthreads();             // the unit is done in every warp: up values are in s_ex, the digits may be replaced
-        const bool fail = s_fail != 0u;      // written only between the two barriers of a unit, read only here: every warp sees the same value
-        if (GATEUP && !is_up) {
-            for (uint32_t ti = 0; ti < tiles; ++ti) {
-                const float4 up = s_ex[ti][wslot][lane];
-                const float uv[4] = {up.x, up.y, up.z, up.w};
-                const uint32_t row = ((I.tile0 + ti) << 4) + g;
-                if (WIDE) {
-#pragma unroll
-                    for (uint32_t j = 0; j < NP; ++j)
-                        if (ok[j]) A.out[(size_t)prow[j] * A.out_stride + row + 8u * (t & 1u)] = (vals[ti][j] / (1.0f + expf(-vals[ti][j]))) * uv[j];
-                } else
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    if (ok[j]) {
-                        const float g0 = vals[ti][j], g1 = vals[ti][2 + j];
-                        A.out[(size_t)prow[j] * A.out_stride + row] = (g0 / (1.0f + expf(-g0))) * uv[j];
-                        A.out[(size_t)prow[j] * A.out_stride + row + 8u] = (g1 / (1.0f + expf(-g1))) * uv[2 + j];
-                    }
-            }
-        }
-        if (fail) break;             // some warp's copy never arrived (status word raised): stop drawing units
+        if (nxt < total) __syncthreads();      // s_ex and s_fail have been read (the same for every thread of the block)
+        if (fail) break;             // some warp's copy never arrived (status word raised): no further unit
         ahead = R.nxt_taken;
-        cur = nxt; I = N; par ^= 1u;
+        cur = nxt; I = N;
     }
 }
 
@@ -722,44 +490,26 @@ int launch_nib_down_tail(NibTailArgs &A, cudaStream_t s) {
     return 1;
 }
 
-static size_t nib_smem_bytes(uint32_t ncols, uint32_t stages) { return (size_t)NIB_WARPS * stages * NIB_REC + 24u * (size_t)(ncols + 32u); }
-
-// A.w0 / A.w1: nibble-layout expert matrices (gate and up, or down and nullptr); A.work: the unit counter of this launch
-// (zeroed by the grouping kernel); items are cut with at most 8 pairs. max_items bounds the number of work items.
-int launch_nib_experts(MmaArgs &A, uint32_t max_items, cudaStream_t s) {
-    const bool gateup = A.w1 != nullptr;
+// A.w0 / A.w1: nibble-layout gate and up matrices of the experts, A.x_raw the token's row
+int launch_nib_one(MmaArgs &A, uint32_t top_k, cudaStream_t s) {
     RC_REQUIRE(nib_shape_ok(A.nrows, A.ncols), "nibble experts: matrix %ux%u is not tileable", A.nrows, A.ncols);
-    RC_REQUIRE(A.work != nullptr && A.item_tok >= 1u && A.item_tok <= (A.fmt == NIB_IQ2 ? 8u : NIB_WIDE_PAIRS), "nibble experts: work counter missing or items of %u pairs", A.item_tok);
+    RC_REQUIRE(A.x_raw && A.w1 && A.item_tok == 1u, "nibble experts: in-kernel quantisation serves the gate/up of a single token");
     A.act_bits = act_digit_bits(); A.dw1 = (float)(1u << A.act_bits); A.dw2 = A.dw1 * A.dw1;
-    RC_REQUIRE(!A.x_raw || (gateup && A.item_tok == 1u), "nibble experts: in-kernel quantisation serves the gate/up of a single token");
     static int sm_count = 0;
     if (!sm_count) { int dev = 0; RC_CUDA(cudaGetDevice(&dev)); RC_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev)); }
-    const uint32_t bpr = A.ncols / 256u, tpw = bpr >= 8u ? 1u : 8u / bpr, unit_tiles = (gateup ? 4u : 8u) * tpw;
-    const uint64_t units = (uint64_t)max_items * ((A.nrows / 16u + unit_tiles - 1u) / unit_tiles);
-    // single token: deep rings, one block per SM, and launched ahead of the previous kernel's end (a batch's blocks, two per SM for
-    // the whole launch, measured slower that way: a layer of 24 tokens 127 us against 119)
-    const bool one = A.x_raw != nullptr;
-    const uint32_t per_sm = one ? 1u : 2u, stages = one ? NIB_STAGES_ONE : NIB_STAGES_BATCH;
-    const uint32_t grid = (uint32_t)(units < per_sm * (uint64_t)sm_count ? (units ? units : 1u) : per_sm * (uint64_t)sm_count);
-    const size_t smem = nib_smem_bytes(A.ncols, stages);
-    prof_begin(gateup ? "moe_gateup" : "moe_down", s);
-#define RC_NIB_LAUNCH(GU, NC, ST) do { \
-        RC_CUDA(cudaFuncSetAttribute(k_nib_experts<FMT, GU, NC, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        if (one) RC_LAUNCH_PDL((k_nib_experts<FMT, GU, NC, ST>), grid, NIB_WARPS * 32u, smem, s, A); \
-        else RC_LAUNCH((k_nib_experts<FMT, GU, NC, ST>), grid, NIB_WARPS * 32u, smem, s, A); } while (0)
+    const uint32_t bpr = A.ncols / 256u, unit_tiles = 4u * (bpr >= 8u ? 1u : 8u / bpr);
+    const uint64_t units = (uint64_t)top_k * ((A.nrows / 16u + unit_tiles - 1u) / unit_tiles);
+    const uint32_t grid = (uint32_t)(units < (uint64_t)sm_count ? (units ? units : 1u) : (uint64_t)sm_count);
+    const size_t smem = (size_t)NIB_WARPS * NIB_STAGES * NIB_REC + 8u * (size_t)(A.ncols + 32u);
+    prof_begin("moe_gateup", s);
+    // launched ahead of the previous kernel's end
+#define RC_NIB_LAUNCH(NC) do { \
+        RC_CUDA(cudaFuncSetAttribute(k_nib_one<FMT, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        RC_LAUNCH_PDL((k_nib_one<FMT, NC>), grid, NIB_WARPS * 32u, smem, s, A); } while (0)
     auto launch = [&](auto fmt) -> int {
-    constexpr uint32_t FMT = decltype(fmt)::value;
-    if (one) {
-        if (A.ncols == 2048u) RC_NIB_LAUNCH(true, 2048u, NIB_STAGES_ONE); else if (A.ncols == 1024u) RC_NIB_LAUNCH(true, 1024u, NIB_STAGES_ONE);
-        else if (A.ncols == 512u) RC_NIB_LAUNCH(true, 512u, NIB_STAGES_ONE); else RC_NIB_LAUNCH(true, 256u, NIB_STAGES_ONE);
-    } else if (gateup) {
-        if (A.ncols == 2048u) RC_NIB_LAUNCH(true, 2048u, NIB_STAGES_BATCH); else if (A.ncols == 1024u) RC_NIB_LAUNCH(true, 1024u, NIB_STAGES_BATCH);
-        else if (A.ncols == 512u) RC_NIB_LAUNCH(true, 512u, NIB_STAGES_BATCH); else RC_NIB_LAUNCH(true, 256u, NIB_STAGES_BATCH);
-    } else {
-        if (A.ncols == 2048u) RC_NIB_LAUNCH(false, 2048u, NIB_STAGES_BATCH); else if (A.ncols == 1024u) RC_NIB_LAUNCH(false, 1024u, NIB_STAGES_BATCH);
-        else if (A.ncols == 512u) RC_NIB_LAUNCH(false, 512u, NIB_STAGES_BATCH); else RC_NIB_LAUNCH(false, 256u, NIB_STAGES_BATCH);
-    }
-    return 1;
+        constexpr uint32_t FMT = decltype(fmt)::value;
+        if (A.ncols == 2048u) RC_NIB_LAUNCH(2048u); else if (A.ncols == 1024u) RC_NIB_LAUNCH(1024u); else if (A.ncols == 512u) RC_NIB_LAUNCH(512u); else RC_NIB_LAUNCH(256u);
+        return 1;
     };
     if (!(A.fmt == NIB_IQ2 ? launch(std::integral_constant<uint32_t, NIB_IQ2>{}) : A.fmt == NIB_IQ3 ? launch(std::integral_constant<uint32_t, NIB_IQ3>{})
                            : launch(std::integral_constant<uint32_t, NIB_IQ2W>{}))) return 0;

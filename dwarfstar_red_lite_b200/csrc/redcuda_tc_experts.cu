@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_experts(const __grid_const
     }
     for (uint32_t i = tid; i < TC_M * nblk; i += TC_THREADS) {     // block scales of the CTA's rows: s_d[tile * bpr + block][row of the tile]
         const uint32_t cb = i / TC_M, r = i - cb * TC_M, tile = cb / bpr, c = cb - tile * bpr;
-        s_d[cb][r] = 0.125f * __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(wrec + ((uint64_t)(tile * 8u + (r >> 4)) * bpr + c) * NIB_REC + NIB_D_OFF + (r & 15u) * 2u))));
+        s_d[cb][r] = 0.125f * __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(wrec + ((uint64_t)(tile * 8u + (r >> 4)) * bpr + c) * NIB_REC + nib_d_off(r & 15u)))));
     }
     if (tid == 0) {
         fail = 0u;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_experts(const __grid_const
                 const uint32_t r = q * 64u + dw * 8u + (lane >> 2), rr = r & 15u;
                 const uint8_t *rec = raw + (r >> 4) * NIB_REC;
                 const uint4 wd = *reinterpret_cast<const uint4 *>(rec + nib_code_off(rr, t, kg0));
-                const uint32_t sc4 = *reinterpret_cast<const uint32_t *>(rec + NIB_SC_OFF + rr * 8u + kg0);
+                const uint32_t sc4 = *reinterpret_cast<const uint32_t *>(rec + nib_sc_off(rr, kg0));
                 *reinterpret_cast<uint4 *>(abuf + tcx_sw128(r, t)) = tcx_decode8(wd.x, sc4 & 255u);
                 *reinterpret_cast<uint4 *>(abuf + tcx_sw128(r, t + 4u)) = tcx_decode8(wd.y, (sc4 >> 8) & 255u);
                 *reinterpret_cast<uint4 *>(abuf + A_SUB + tcx_sw128(r, t)) = tcx_decode8(wd.z, (sc4 >> 16) & 255u);
