@@ -58,8 +58,8 @@ __host__ __device__ __forceinline__ uint32_t nib_lane_off(uint32_t g, uint32_t t
 __host__ __device__ __forceinline__ uint32_t nib_code_off(uint32_t rr, uint32_t t, uint32_t kg) {
     return (2u * (rr >> 3) + (kg >> 2)) * 512u + nib_lane_off(rr & 7u, t) + (kg & 3u) * 4u;
 }
-// byte offset of the scale of group kg and of d of row rr: rows g and g + 8 side by side
-__host__ __device__ __forceinline__ uint32_t nib_sc_off(uint32_t rr, uint32_t kg) { return NIB_SC_OFF + (rr & 7u) * 16u + (rr >> 3) * 8u + kg; }
+// byte offset of the scale of group kg and of d of row rr: those of four groups together, rows g and g + 8 side by side
+__host__ __device__ __forceinline__ uint32_t nib_sc_off(uint32_t rr, uint32_t kg) { return NIB_SC_OFF + (kg >> 2) * 64u + (rr & 7u) * 8u + (rr >> 3) * 4u + (kg & 3u); }
 __host__ __device__ __forceinline__ uint32_t nib_d_off(uint32_t rr) { return NIB_D_OFF + (rr & 7u) * 4u + (rr >> 3) * 2u; }
 uint64_t nib_matrix_bytes(uint32_t nrows, uint32_t ncols);
 bool nib_shape_ok(uint32_t nrows, uint32_t ncols);

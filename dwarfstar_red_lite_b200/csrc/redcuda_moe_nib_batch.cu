@@ -39,13 +39,19 @@ __device__ __forceinline__ uint4 nbb_ldg(const uint8_t *p) {
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
+__device__ __forceinline__ uint2 nbb_ldg2(const uint8_t *p) {
+    uint2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ uint32_t nbb_ldg1(const uint8_t *p) {
     uint32_t v;
     asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
-// A lane's part of the two records of a step. q[m][h][i]: codes of row g + 8 h, 32-column groups 4 i .. 4 i + 3, of record m.
-struct NbbFrag { uint4 q[2][2][2], sc[2]; uint32_t d[2]; };
+// A lane's part of the two records of a step. q[m][h][i]: codes of row g + 8 h, 32-column groups 4 i .. 4 i + 3, of record m; sc[m][i]: the
+// scales of these groups, rows g and g + 8; d[m]: d of the two rows. Every piece is loaded again for the next step once it is used up.
+struct NbbFrag { uint4 q[2][2][2]; uint2 sc[2][2]; uint32_t d[2]; };
 // Half i (four groups) of the two records against NT tiles of digits: the exact s32 products of a group times its integer scale, added up
 // in blk[m][n]: rows g (0, 1) and g + 8 (2, 3), columns 2 t and 2 t + 1 of tile n.
 template <uint32_t FMT, int NT, uint32_t BPITCH>
@@ -62,8 +68,8 @@ __device__ __forceinline__ void nbb_half(const NbbFrag &F, const int i, const in
             uint32_t a0, a1, a2, a3;
             nb_expand<FMT>(wa, a0, a2);
             nb_expand<FMT>(wb, a1, a3);
-            const int sa = (int)nb_prmt(i ? F.sc[m].y : F.sc[m].x, 0u, 0x4440u + (uint32_t)kk);
-            const int sb = (int)nb_prmt(i ? F.sc[m].w : F.sc[m].z, 0u, 0x4440u + (uint32_t)kk);
+            const int sa = (int)nb_prmt(F.sc[m][i].x, 0u, 0x4440u + (uint32_t)kk);
+            const int sb = (int)nb_prmt(F.sc[m][i].y, 0u, 0x4440u + (uint32_t)kk);
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 int p[4];
@@ -94,10 +100,10 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
     __shared__ NbbSeg s_seg[2];
     __shared__ float s_sxw[2][WIDE ? NIB_WIDE_PAIRS * BPR : 1u];       // wide: scales of the item's pairs and blocks
     __shared__ uint32_t s_taken[2], s_left[2], s_run[2];               // pieces drawn, warps that are through with the buffer; what is left of the block's run
-    __shared__ __align__(8) uint64_t s_full[2];
+    __shared__ __align__(8) uint64_t s_told[2], s_full[2];             // the part's description is in s_seg; its pairs and digits are there as well
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
     int8_t *digits = reinterpret_cast<int8_t *>(smem);
-    const uint32_t full_s = nb_smem(&s_full[0]);
+    const uint32_t full_s = nb_smem(&s_full[0]), told_s = nb_smem(&s_told[0]);
     const uint32_t ntile = A.nrows >> 4, npair = GATEUP ? ntile : (ntile + 1u) / 2u, PPI = (npair + TPP - 1u) / TPP;     // tile pairs and pieces of an item
     const uint32_t total = *A.n_items * PPI, share = (total + gridDim.x - 1u) / gridDim.x;
     bool failed = false;
@@ -118,27 +124,30 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
             if (lane == 0) k = gridDim.x + atomicAdd(A.work, 1u);
             run_of(__shfl_sync(0xffffffffu, k, 0), lo, hi);
         }
-        uint32_t nt = 0u, row = 0u, count = 0u, item = 0u;
+        uint32_t nt = 0u, row = 0u, count = 0u, p0 = 0u;
         if (lo < hi) {
-            item = lo / PPI;
-            const uint32_t first = lo - item * PPI, u = A.item_u[item], p0 = A.item_p0[item];
+            const uint32_t item = lo / PPI, first = lo - item * PPI, u = A.item_u[item];
+            p0 = A.item_p0[item];
             uint32_t e = A.uexp[u] - A.expert_begin;
             nt = min(A.item_tok, A.ustart[u + 1u] - p0);
             if (e >= A.n_local) { if (A.status && lane == 0) A.status[ST_EXPERT_RANGE] = 1u; e = 0u; nt = 0u; }      // never index the arena with a foreign id
             count = min(PPI - first, hi - lo);
-            if (lane < nt) { row = A.sorted[p0 + lane]; S.row[lane] = row; }
-            if (!WIDE && lane < nt) S.sx[lane] = A.sx[row / A.x_div];
             if (lane == 0) { S.rec = A.w0 + (size_t)e * A.mat_bytes; S.first = first; S.nt = nt; }
         }
-        row /= A.x_div;
+        __syncwarp();                // every lane has read the run
+        // the description first: it lets the warps request weights while the pairs are looked up and their digits copied
+        if (lane == 0) {
+            S.count = count; s_run[0] = lo + count; s_run[1] = hi; s_taken[buf] = 0u; s_left[buf] = 0u;
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(told_s + 8u * buf) : "memory");
+        }
+        if (lane < nt) { row = A.sorted[p0 + lane]; S.row[lane] = row; row /= A.x_div; }
+        if (!WIDE && lane < nt) S.sx[lane] = A.sx[row];
         if (WIDE)
 #pragma unroll
             for (uint32_t i0 = 0u; i0 < NIB_WIDE_PAIRS * BPR; i0 += 32u) {
                 const uint32_t i = i0 + lane, r = __shfl_sync(0xffffffffu, row, i / BPR & 31u);
                 if (i < NIB_WIDE_PAIRS * BPR) s_sxw[buf][i] = i / BPR < nt ? A.sx[(size_t)r * BPR + i % BPR] : 0.f;
             }
-        __syncwarp();                // every lane has read the run
-        if (lane == 0) { S.count = count; s_run[0] = lo + count; s_run[1] = hi; s_taken[buf] = 0u; s_left[buf] = 0u; }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(full_s + 8u * buf), "r"(nt * ND * NCOLS) : "memory");
@@ -152,7 +161,10 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
     };
 
     if (tid == 0) {
-        for (uint32_t i = 0; i < 2u; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(full_s + 8u * i));
+        for (uint32_t i = 0; i < 2u; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(told_s + 8u * i));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(full_s + 8u * i));
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         uint32_t lo, hi;
@@ -160,17 +172,21 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
         s_run[0] = lo; s_run[1] = hi;
     }
     __syncthreads();
-    if (warp == 0) { fill(0u); __syncwarp(); fill(1u); }
-
     // ---- the warp's pieces ----
     struct Piece { const uint8_t *rec; uint32_t pair0, steps; };
     const size_t to_up = GATEUP ? (size_t)(A.w1 - A.w0) : 0u;
     uint32_t seg = 0u;                                   // the warp draws from item part seg, seg + 1, ... (buffer seg % 2)
-    auto seg_full = [&](uint32_t k, bool block) {        // are the part's description and digits in shared memory?
-        const uint32_t bar = full_s + 8u * (k & 1u), par = (k >> 1) & 1u;
-        if (block) { if (!failed) failed = !__all_sync(0xffffffffu, nb_wait(bar, par)); return !failed; }
+    auto wait_for = [&](uint32_t bars, uint32_t k) {      // part k's description (told_s) or digits (full_s)
+        if (!failed) failed = !__all_sync(0xffffffffu, nb_wait(bars + 8u * (k & 1u), (k >> 1) & 1u));
+        return !failed;
+    };
+    // the first two parts; the second by the warp that a small batch has least work for
+    if (warp == 0) fill(0u);
+    else if (warp == NBB_WARPS - 1u && wait_for(told_s, 0u)) fill(1u);
+    __syncwarp();
+    auto told = [&](uint32_t k) {                        // is part k's description there already?
         uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(done) : "r"(bar), "r"(par) : "memory");
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(done) : "r"(told_s + 8u * (k & 1u)), "r"((k >> 1) & 1u) : "memory");
         return __all_sync(0xffffffffu, done != 0u) != 0;
     };
     auto draw = [&](uint32_t k, Piece &P) {              // a piece of part k, or false: the part has none left
@@ -199,22 +215,25 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
             b = a + (2u * (P.pair0 + q) + 1u < ntile ? BPR * NIB_REC : 0u);      // an odd last tile is taken twice and stored once
         }
     };
-    const uint32_t lane_code = nib_lane_off(g, t), lane_sc = NIB_SC_OFF + g * 16u, lane_d = NIB_D_OFF + g * 4u;
+    const uint32_t lane_code = nib_lane_off(g, t), lane_sc = NIB_SC_OFF + g * 8u, lane_d = NIB_D_OFF + g * 4u;
     NbbFrag F;
     auto load_half = [&](const int i, const uint8_t *a, const uint8_t *b) {
+        F.sc[0][i] = nbb_ldg2(a + lane_sc + 64 * i); F.sc[1][i] = nbb_ldg2(b + lane_sc + 64 * i);
         F.q[0][0][i] = nbb_ldg(a + lane_code + 512 * i); F.q[0][1][i] = nbb_ldg(a + lane_code + 1024 + 512 * i);
         F.q[1][0][i] = nbb_ldg(b + lane_code + 512 * i); F.q[1][1][i] = nbb_ldg(b + lane_code + 1024 + 512 * i);
     };
+    auto load_d = [&](const uint8_t *a, const uint8_t *b) { F.d[0] = nbb_ldg1(a + lane_d); F.d[1] = nbb_ldg1(b + lane_d); };
     int zero[4];                     // opaque to the compiler: four registers that stay zero, the accumulator input of every MMA
     asm volatile("mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;" : "=r"(zero[0]), "=r"(zero[1]), "=r"(zero[2]), "=r"(zero[3]));
 
     Piece P{}, N{};
+    uint32_t digits_of = 0xffffffffu;    // the part whose digits this warp has waited for
     bool have = false, more = true;  // N holds the next piece, whose first step is in F; there may be one
     for (;;) {
         if (have) P = N;
         else {
             for (;;) {
-                if (!seg_full(seg, true)) break;
+                if (!wait_for(told_s, seg)) break;
                 if (s_seg[seg & 1u].count == 0u) { more = false; break; }
                 if (draw(seg, P)) break;
                 leave(seg); ++seg;
@@ -222,20 +241,22 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
             if (failed || !more) break;
             const uint8_t *a, *b;
             place(P, 0u, a, b);
-            load_half(0, a, b); load_half(1, a, b);
-            F.sc[0] = nbb_ldg(a + lane_sc); F.sc[1] = nbb_ldg(b + lane_sc); F.d[0] = nbb_ldg1(a + lane_d); F.d[1] = nbb_ldg1(b + lane_d);
+            load_half(0, a, b); load_half(1, a, b); load_d(a, b);
         }
         have = false;
+        if (digits_of != seg) { if (!wait_for(full_s, seg)) break; digits_of = seg; }
         const uint32_t cur = seg, buf = seg & 1u;
         const NbbSeg &S = s_seg[buf];
         const uint32_t nt = S.nt;
-        // The next piece is drawn when its first step is due: from this item part or, if the block has it already, from the next (never from
-        // the one behind that: its buffer is this part's).
+        // The next piece is drawn when its first step is due: from this item part or, if the block has it already, from the next
+        // (never from the one behind that: its buffer is this part's).
         auto draw_next = [&]() {
             if (!more) return;
-            if (draw(cur, N)) { have = true; return; }
-            seg = cur + 1u;
-            if (!seg_full(seg, false)) return;
+            if (seg == cur) {
+                if (draw(cur, N)) { have = true; return; }
+                seg = cur + 1u;
+            }
+            if (!told(seg)) return;
             if (s_seg[seg & 1u].count == 0u) more = false; else have = draw(seg, N);
         };
         const int8_t *Bl = digits + (buf * NBB_COLS + g) * BPITCH + 8u * t;
@@ -250,17 +271,16 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
                     for (int n = 0; n < NT; ++n)
 #pragma unroll
                         for (int j = 0; j < (WIDE ? 2 : 4); ++j) out[m][n][j] = 0.f;
+#pragma unroll 1
                 for (uint32_t c = 0u; c < BPR; ++c, ++s) {
+                    if (s + 1u == P.steps) draw_next();
                     const uint8_t *a, *b;            // the step behind this one; where none is known, this piece's first records are read again
-                    if (s + 1u < P.steps) place(P, s + 1u, a, b);
-                    else { draw_next(); if (have) place(N, 0u, a, b); else place(P, 0u, a, b); }
+                    if (s + 1u < P.steps) place(P, s + 1u, a, b); else if (have) place(N, 0u, a, b); else place(P, 0u, a, b);
                     int blk[2][NT][4];
 #pragma unroll
                     for (int m = 0; m < 2; ++m)
 #pragma unroll
                         for (int n = 0; n < NT; ++n) blk[m][n][0] = blk[m][n][1] = blk[m][n][2] = blk[m][n][3] = 0;
-                    const uint4 sc0 = nbb_ldg(a + lane_sc), sc1 = nbb_ldg(b + lane_sc);
-                    const uint32_t d0 = nbb_ldg1(a + lane_d), d1 = nbb_ldg1(b + lane_d);
                     nbb_half<FMT, NT, BPITCH>(F, 0, Bl + c * 256u, zero, blk);
                     load_half(0, a, b);
                     nbb_half<FMT, NT, BPITCH>(F, 1, Bl + c * 256u, zero, blk);
@@ -271,7 +291,7 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
                         const __half2 h = *reinterpret_cast<const __half2 *>(&F.d[m]);
                         d[m][0] = 0.125f * __low2float(h); d[m][1] = 0.125f * __high2float(h);
                     }
-                    F.sc[0] = sc0; F.sc[1] = sc1; F.d[0] = d0; F.d[1] = d1;
+                    load_d(a, b);
 #pragma unroll
                     for (int m = 0; m < 2; ++m)
 #pragma unroll

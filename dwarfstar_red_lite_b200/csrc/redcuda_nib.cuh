@@ -62,8 +62,8 @@ __device__ __forceinline__ void nib_sums(const uint8_t *st, const int8_t *Bl, ui
     const uint32_t o = nib_lane_off(g, t);
     const uint4 qa0 = *reinterpret_cast<const uint4 *>(st + o), qa1 = *reinterpret_cast<const uint4 *>(st + 512u + o);
     const uint4 qb0 = *reinterpret_cast<const uint4 *>(st + 1024u + o), qb1 = *reinterpret_cast<const uint4 *>(st + 1536u + o);
-    const uint4 sab = *reinterpret_cast<const uint4 *>(st + NIB_SC_OFF + g * 16u);
-    const uint2 sa = make_uint2(sab.x, sab.y), sb = make_uint2(sab.z, sab.w);
+    const uint2 s0 = *reinterpret_cast<const uint2 *>(st + NIB_SC_OFF + g * 8u), s1 = *reinterpret_cast<const uint2 *>(st + NIB_SC_OFF + 64u + g * 8u);
+    const uint2 sa = make_uint2(s0.x, s1.x), sb = make_uint2(s0.y, s1.y);
     const __half2 dab = *reinterpret_cast<const __half2 *>(st + NIB_D_OFF + g * 4u);
     da = 0.125f * __low2float(dab); db = 0.125f * __high2float(dab);
     const uint32_t wa[8] = {qa0.x, qa0.y, qa0.z, qa0.w, qa1.x, qa1.y, qa1.z, qa1.w};
