@@ -10,12 +10,15 @@
 //               exactly in s32 (|.| < 2^25), the result and digit 0 converted to fp32 and accumulated with the fp32
 //               scale d*sc
 //
-// Block = 8 warps = MS matrices x KS column splits x TGB groups of 8 tokens, for one tile of 16 rows; partial sums meet
-// in shared memory, where the epilogue (plain store or SiLU(gate)*up) is applied.
+// Block = one tile of 16 rows (of one matrix, or of a gate / up pair) x TGB groups of 8 tokens; its 8 warps split the columns KS ways in
+// units of 128 and take a token group each. Weights and digits of up to 2048 columns are staged in shared memory by bulk copies, a row
+// each, at pitches that keep the fragment loads free of bank conflicts. (Loaded straight from global memory, 4 bytes a lane from eight
+// rows 1024 bytes apart, the kernel was bound by the L1 tag rate: 88 cycles an SM for every 16 columns of 8 tokens.)
+// Partial sums meet in shared memory, where the epilogue (plain store or SiLU(gate)*up) is applied.
 #define RC_PDL_DEFAULT 0
 #include "redcuda_common.cuh"
 #include "redcuda_kernels.cuh"
-#include "redcuda_moe_mma.cuh"
+#include "redcuda_nib.cuh"
 
 namespace rc {
 
@@ -32,77 +35,149 @@ struct Q6Args {
     uint32_t nrows, ncols, ntok;
     const int8_t *xq; const float *sx;      // digits [ntok][3][ncols], scale per token
     float *out; uint32_t out_stride;        // out[token * out_stride + row]
-    uint32_t pair_silu;                     // 1: out = SiLU(w[0].x) * (w[1].x)
-    uint32_t MS, KS;                        // matrices and column splits per block (8 % (MS*KS) == 0)
+    uint32_t *status;
+    uint32_t KS;                            // column splits (8 % KS == 0); 8 / KS token groups per block
     uint32_t bits; float dw1;               // digit width and 2^bits
 };
+constexpr uint32_t Q6M_PANEL = 2048u;       // columns staged at a time
+// bytes of a staged panel of pc columns: 16 rows of a matrix, 8 tokens
+__host__ __device__ constexpr uint32_t q6m_a_bytes(uint32_t pc) { return 16u * (pc / 2u + 16u + pc / 4u + 16u + pc / 16u + 16u); }
+__host__ __device__ constexpr uint32_t q6m_b_bytes(uint32_t pc) { return 24u * (pc + 16u); }
 
-__global__ void __launch_bounds__(256) k_q6k_mma(const __grid_constant__ Q6Args A) {
+template <uint32_t MS>
+__global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Args A) {
     pdl_prologue();
-    __shared__ float part[8][16][8];        // per warp: 16 rows x 8 tokens
+    extern __shared__ __align__(16) uint8_t q6m_smem[];
+    __shared__ float part[MS][8][16][8];    // per matrix and warp: 16 rows x 8 tokens
+    __shared__ float s_d[MS][16][Q6M_PANEL / 256u];
+    __shared__ __align__(8) uint64_t s_bar;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
-    const uint32_t MS = A.MS, KS = A.KS, TGB = 8u / (MS * KS);
-    const uint32_t mat = warp % MS, ks = (warp / MS) % KS, tgl = warp / (MS * KS);
+    const uint32_t KS = A.KS, TGB = 8u / KS, ks = warp % KS, tgl = warp / KS;
     const uint32_t tg = blockIdx.y * TGB + tgl;                 // group of 8 tokens
-    const uint32_t row0 = blockIdx.x * 16u, bpr = A.ncols >> 8, nsteps = A.ncols >> 4;
-    const uint32_t s_begin = ks * (nsteps / KS), s_end = s_begin + nsteps / KS;
-    const uint8_t *base = A.w[mat];
-    const uint64_t nb = A.nb;
-    const uint32_t tok = tg * 8u + g;                           // this lane's B column
-    const bool tok_ok = tok < A.ntok;
-    const int8_t *xrow = A.xq + (size_t)(tok_ok ? tok : 0u) * 3u * A.ncols + 4u * t;
-    float out[4] = {0.f, 0.f, 0.f, 0.f};
+    const uint32_t row0 = blockIdx.x * 16u, bpr = A.ncols >> 8;
+    const uint32_t tok_first = blockIdx.y * TGB * 8u, ntok_b = min(TGB * 8u, A.ntok - tok_first);     // the block's tokens
+    const uint32_t pcmax = min(A.ncols, Q6M_PANEL), a_bytes = q6m_a_bytes(pcmax);
+    const uint32_t ql_pitch = pcmax / 2u + 16u, qh_pitch = pcmax / 4u + 16u, sc_pitch = pcmax / 16u + 16u, b_pitch = pcmax + 16u;
+    uint8_t *b_base = q6m_smem + MS * a_bytes;
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    float out[MS][4];
+#pragma unroll
+    for (uint32_t m = 0; m < MS; ++m) out[m][0] = out[m][1] = out[m][2] = out[m][3] = 0.f;
     int z[4];
     asm volatile("mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;" : "=r"(z[0]), "=r"(z[1]), "=r"(z[2]), "=r"(z[3]));
-    if (tg * 8u < A.ntok) {
-#pragma unroll 8
-        for (uint32_t s = s_begin; s < s_end; ++s) {
-            const uint32_t b = s >> 4, grp = s & 15u, h = grp >> 3, q = (grp >> 1) & 3u, i = grp & 1u;
-            uint32_t a[2];
-            float scl[2];
-#pragma unroll
-            for (int hr = 0; hr < 2; ++hr) {
-                const uint64_t blk = (uint64_t)(row0 + hr * 8u + g) * bpr + b;
-                const uint32_t ql = __ldg(reinterpret_cast<const uint32_t *>(base + blk * 128u + 64u * h + 32u * (q & 1u) + 16u * i + 4u * t));
-                const uint32_t qh = __ldg(reinterpret_cast<const uint32_t *>(base + rc_q6_qh(nb) + blk * 64u + 32u * h + 16u * i + 4u * t));
-                const int sc = (int)(signed char)__ldg(base + rc_q6_sc(nb) + blk * 16u + grp);
-                const float d = __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(base + rc_q6_d(nb)) + blk)));
-                const uint32_t v = ((ql >> (4u * (q >> 1))) & 0x0F0F0F0Fu) | (((qh >> (2u * q)) & 0x03030303u) << 4);
-                const uint32_t u = v ^ 0x20202020u;            // 6-bit two's complement of (value - 32)
-                a[hr] = u + (u & 0x20202020u) * 6u;             // sign-extend every byte to 8 bits (bits 6,7 were clear: no carry)
-                scl[hr] = d * (float)sc;
+    bool ok = true;
+    uint32_t parity = 0u;
+    for (uint32_t blk0 = 0u; blk0 < bpr; blk0 += Q6M_PANEL / 256u, parity ^= 1u) {
+        const uint32_t nblk = min(bpr - blk0, Q6M_PANEL / 256u), pc = nblk * 256u;
+        __syncthreads();                     // the barrier is ready; the panel before this one has been read
+        if (tid == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(MS * 16u * (pc / 2u + pc / 4u + pc / 16u) + ntok_b * 3u * pc) : "memory");
+        __syncthreads();
+        for (uint32_t i = tid; i < MS * 48u + ntok_b * 3u; i += 256u) {
+            const uint8_t *src;
+            uint8_t *dst;
+            uint32_t n;
+            if (i < MS * 48u) {
+                const uint32_t m = i / 48u, j = i - m * 48u, plane = j >> 4, r = j & 15u;
+                const uint64_t blk = (uint64_t)(row0 + r) * bpr + blk0;
+                uint8_t *am = q6m_smem + m * a_bytes;
+                if (plane == 0u) { src = A.w[m] + blk * 128u; dst = am + r * ql_pitch; n = pc / 2u; }
+                else if (plane == 1u) { src = A.w[m] + rc_q6_qh(A.nb) + blk * 64u; dst = am + 16u * ql_pitch + r * qh_pitch; n = pc / 4u; }
+                else { src = A.w[m] + rc_q6_sc(A.nb) + blk * 16u; dst = am + 16u * (ql_pitch + qh_pitch) + r * sc_pitch; n = pc / 16u; }
+            } else {                         // tokens beyond the batch leave their columns as they are: a column of the product depends on no other
+                const uint32_t j = i - MS * 48u;
+                src = reinterpret_cast<const uint8_t *>(A.xq) + ((size_t)tok_first * 3u + j) * A.ncols + blk0 * 256u; dst = b_base + j * b_pitch; n = pc;
             }
-            int d0[4], d1[4], d2[4];
-            const uint32_t b0 = tok_ok ? __ldg(reinterpret_cast<const uint32_t *>(xrow + 16u * s)) : 0u;
-            const uint32_t b1 = tok_ok ? __ldg(reinterpret_cast<const uint32_t *>(xrow + A.ncols + 16u * s)) : 0u;
-            const uint32_t b2 = tok_ok ? __ldg(reinterpret_cast<const uint32_t *>(xrow + 2u * A.ncols + 16u * s)) : 0u;
-            mma_s8_k16(d0, a[0], a[1], b0, z);
-            mma_s8_k16(d1, a[0], a[1], b1, z);
-            mma_s8_k16(d2, a[0], a[1], b2, z);
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n), "r"(bar) : "memory");
+        }
+        for (uint32_t i = tid; i < MS * 16u * nblk; i += 256u) {
+            const uint32_t m = i / (16u * nblk), j = i - m * 16u * nblk, r = j / nblk, c = j - r * nblk;
+            s_d[m][r][c] = __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(A.w[m] + rc_q6_d(A.nb)) + (uint64_t)(row0 + r) * bpr + blk0 + c)));
+        }
+        __syncthreads();                     // s_d
+        if (ok) ok = nb_wait(bar, parity);
+        if (!ok || tg * 8u >= A.ntok) continue;
+        const uint8_t *xb = b_base + (tgl * 8u + g) * 3u * b_pitch + 4u * t;
+        for (uint32_t u = ks; u < 2u * nblk; u += KS) {
+            const uint32_t b = u >> 1, h = u & 1u;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int hi = d1[c] + (d2[c] << A.bits);                 // 8-bit digits: the full recombination would leave s32
-                out[c] += scl[c >> 1] * fmaf(A.dw1, (float)hi, (float)d0[c]);
+            for (uint32_t i = 0; i < 2u; ++i) {
+                uint32_t bx[4][3];
+#pragma unroll
+                for (uint32_t q = 0; q < 4u; ++q)
+#pragma unroll
+                    for (uint32_t dg = 0; dg < 3u; ++dg) bx[q][dg] = *reinterpret_cast<const uint32_t *>(xb + dg * b_pitch + b * 256u + h * 128u + 32u * q + 16u * i);
+#pragma unroll
+                for (uint32_t m = 0; m < MS; ++m) {
+                    const uint8_t *am = q6m_smem + m * a_bytes;
+                    uint32_t ql[2][2], qh[2];
+                    float d[2];
+                    uint2 sc[2];
+#pragma unroll
+                    for (uint32_t hr = 0; hr < 2u; ++hr) {
+                        const uint32_t r = g + 8u * hr;
+                        const uint8_t *lp = am + r * ql_pitch + b * 128u + 64u * h + 16u * i + 4u * t;
+                        ql[hr][0] = *reinterpret_cast<const uint32_t *>(lp); ql[hr][1] = *reinterpret_cast<const uint32_t *>(lp + 32u);
+                        qh[hr] = *reinterpret_cast<const uint32_t *>(am + 16u * ql_pitch + r * qh_pitch + b * 64u + 32u * h + 16u * i + 4u * t);
+                        sc[hr] = *reinterpret_cast<const uint2 *>(am + 16u * (ql_pitch + qh_pitch) + r * sc_pitch + b * 16u + 8u * h);
+                        d[hr] = s_d[m][r][b];
+                    }
+#pragma unroll
+                    for (uint32_t q = 0; q < 4u; ++q) {
+                        uint32_t a[2];
+                        float scl[2];
+#pragma unroll
+                        for (uint32_t hr = 0; hr < 2u; ++hr) {
+                            const uint32_t v = ((ql[hr][q & 1u] >> (4u * (q >> 1))) & 0x0F0F0F0Fu) | (((qh[hr] >> (2u * q)) & 0x03030303u) << 4);
+                            const uint32_t x = v ^ 0x20202020u;            // 6-bit two's complement of (value - 32)
+                            a[hr] = x + (x & 0x20202020u) * 6u;             // sign-extend every byte to 8 bits (bits 6,7 were clear: no carry)
+                            scl[hr] = d[hr] * (float)(int)(signed char)((q < 2u ? sc[hr].x : sc[hr].y) >> (16u * (q & 1u) + 8u * i));
+                        }
+                        int d0[4], d1[4], d2[4];
+                        mma_s8_k16(d0, a[0], a[1], bx[q][0], z);
+                        mma_s8_k16(d1, a[0], a[1], bx[q][1], z);
+                        mma_s8_k16(d2, a[0], a[1], bx[q][2], z);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const int hi = d1[c] + (d2[c] << A.bits);                 // 8-bit digits: the full recombination would leave s32
+                            out[m][c] += scl[c >> 1] * fmaf(A.dw1, (float)hi, (float)d0[c]);
+                        }
+                    }
+                }
             }
         }
-        // accumulator columns 2t, 2t+1 of this lane are tokens tg*8 + 2t, +1
-        const uint32_t tk0 = tg * 8u + 2u * t;
-        const float s0 = tk0 < A.ntok ? A.sx[tk0] : 0.f, s1 = tk0 + 1u < A.ntok ? A.sx[tk0 + 1u] : 0.f;
-        out[0] *= s0; out[1] *= s1; out[2] *= s0; out[3] *= s1;
     }
-    part[warp][g][2u * t] = out[0]; part[warp][g][2u * t + 1u] = out[1];
-    part[warp][g + 8u][2u * t] = out[2]; part[warp][g + 8u][2u * t + 1u] = out[3];
+    // accumulator columns 2t, 2t+1 of this lane are tokens tg*8 + 2t, +1
+    const uint32_t tk0 = tg * 8u + 2u * t;
+    const float s0 = tk0 < A.ntok ? A.sx[tk0] : 0.f, s1 = tk0 + 1u < A.ntok ? A.sx[tk0 + 1u] : 0.f;
+#pragma unroll
+    for (uint32_t m = 0; m < MS; ++m) {
+        part[m][warp][g][2u * t] = out[m][0] * s0; part[m][warp][g][2u * t + 1u] = out[m][1] * s1;
+        part[m][warp][g + 8u][2u * t] = out[m][2] * s0; part[m][warp][g + 8u][2u * t + 1u] = out[m][3] * s1;
+    }
+    if (!ok) {                               // a copy never came: the results are void; it is given as long again before the block may end
+        if (A.status) A.status[ST_TIMEOUT] = 1u;
+        nb_wait(bar, parity ^ 1u);
+    }
     __syncthreads();
     // epilogue: TGB token groups x 16 rows x 8 tokens
     for (uint32_t idx = tid; idx < TGB * 128u; idx += 256u) {
         const uint32_t tl = idx >> 7, row = (idx >> 3) & 15u, c = idx & 7u;
         const uint32_t tkn = (blockIdx.y * TGB + tl) * 8u + c;
         if (tkn >= A.ntok || row0 + row >= A.nrows) continue;
-        float val[2] = {0.f, 0.f};
-        for (uint32_t m = 0; m < MS; ++m)
-            for (uint32_t k = 0; k < KS; ++k) val[m] += part[(tl * KS + k) * MS + m][row][c];
+        float val[MS];
+#pragma unroll
+        for (uint32_t m = 0; m < MS; ++m) {
+            val[m] = 0.f;
+            for (uint32_t k = 0; k < KS; ++k) val[m] += part[m][tl * KS + k][row][c];
+        }
         float v = val[0];
-        if (A.pair_silu) v = (val[0] / (1.0f + expf(-val[0]))) * val[1];
+        if (MS == 2u) v = (val[0] / (1.0f + expf(-val[0]))) * val[MS - 1u];
         A.out[(size_t)tkn * A.out_stride + row0 + row] = v;
     }
 }
@@ -114,19 +189,21 @@ int launch_q6k_mma(const uint8_t *w0, const uint8_t *w1, uint64_t nb, uint32_t n
     if (!ntok) return 1;
     Q6Args A{};
     A.w[0] = w0; A.w[1] = w1 ? w1 : w0; A.nb = nb; A.nrows = nrows; A.ncols = ncols; A.ntok = ntok; A.xq = xq; A.sx = sx;
-    A.out = out; A.out_stride = out_stride; A.pair_silu = w1 ? 1u : 0u;
-    A.MS = w1 ? 2u : 1u;
+    A.out = out; A.out_stride = out_stride; A.status = status_words();
     A.bits = act_digit_bits(); A.dw1 = (float)(1u << A.bits);
-    const uint32_t nsteps = ncols / 16u, tgroups = (ntok + 7u) / 8u, tiles = nrows / 16u;
-    // column splits while the launch would leave SMs idle and every split keeps >= 16 steps
-    uint32_t KS = 1u;
-    while (A.MS * KS * 2u <= 8u && (nsteps / (KS * 2u)) >= 16u && nsteps % (KS * 2u) == 0 &&
-           (uint64_t)tiles * ((tgroups + 8u / (A.MS * KS) - 1u) / (8u / (A.MS * KS))) < 148u * 2u) KS <<= 1;
-    A.KS = KS;
-    const uint32_t TGB = 8u / (A.MS * KS);
-    const dim3 grid(tiles, (tgroups + TGB - 1u) / TGB);
+    const uint32_t units = ncols / 128u, tgroups = (ntok + 7u) / 8u, pc = ncols < Q6M_PANEL ? ncols : Q6M_PANEL;
+    A.KS = units >= 8u ? 8u : units >= 4u ? 4u : 2u;
+    const uint32_t TGB = 8u / A.KS, ms = w1 ? 2u : 1u;
+    const size_t smem = (size_t)ms * q6m_a_bytes(pc) + (size_t)TGB * q6m_b_bytes(pc);
+    const dim3 grid(nrows / 16u, (tgroups + TGB - 1u) / TGB);
     prof_begin(tag, s);
-    RC_LAUNCH((k_q6k_mma), grid, 256, 0, s, A);
+    if (w1) {
+        RC_CUDA(cudaFuncSetAttribute(k_q6k_mma<2u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        RC_LAUNCH((k_q6k_mma<2u>), grid, 256, smem, s, A);
+    } else {
+        RC_CUDA(cudaFuncSetAttribute(k_q6k_mma<1u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        RC_LAUNCH((k_q6k_mma<1u>), grid, 256, smem, s, A);
+    }
     prof_end(s);
     RC_LAUNCHED();
     return 1;
