@@ -121,9 +121,9 @@ __device__ __forceinline__ uint64_t tcx_desc_sw128(uint32_t addr) {
     return (uint64_t)((addr >> 4) & 0x3fffu) | (1ull << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 __device__ __forceinline__ uint32_t tcx_sw128(uint32_t r, uint32_t c) { return r * 128u + ((c ^ (r & 7u)) << 4); }
-// 128-row tiles one CTA works through: as many as keep it at 8 blocks of 256 columns (and divide the matrix)
-__host__ __device__ uint32_t tcx_tiles_per_cta(uint32_t nrows, uint32_t ncols) {
-    uint32_t tpc = 2048u / ncols;
+// 128-row tiles one CTA works through: `blocks` 256-column blocks of them, as far as that divides the matrix
+__host__ __device__ uint32_t tcx_tiles_per_cta(uint32_t nrows, uint32_t ncols, uint32_t blocks) {
+    uint32_t tpc = blocks * 256u / ncols;
     const uint32_t rtiles = nrows / 128u;
     tpc = tpc < 1u ? 1u : tpc;
     while (tpc > 1u && rtiles % tpc) tpc >>= 1;
@@ -162,7 +162,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_experts(const __grid_const
     __shared__ volatile uint32_t fail;               // a bounded wait ran out: every role stops at its next wait
     __shared__ uint32_t s_row[TN], s_pair[TN];       // activation row and pair of every token slot of the item (TCX_DEAD beyond its pairs)
     __shared__ float s_xinv[TN];
-    __shared__ float s_d[8][TC_M];                   // d / 8 of every row for every 256-column block (at most 8 blocks)
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
 
     const uint32_t u = A.item_u[item], p0 = A.item_p0[item], pe = A.ustart[u + 1u];
@@ -172,9 +171,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_experts(const __grid_const
         if (tid == 0 && A.status) A.status[ST_EXPERT_RANGE] = 1u;
         return;
     }
-    // A CTA takes tpc consecutive 128-row tiles of one matrix, one after the other, so that 8 blocks of 256 columns pass
+    // A CTA takes tpc consecutive 128-row tiles of one matrix, one after the other, so that A.cta_blocks blocks of 256 columns pass
     // through it whatever the row length: the set-up and the pipeline fill are paid once per CTA, not once per short row.
-    const uint32_t bpr = A.ncols >> 8, kstage = A.ncols / TCX_KS, tpc = tcx_tiles_per_cta(A.nrows, A.ncols);
+    const uint32_t bpr = A.ncols >> 8, kstage = A.ncols / TCX_KS, tpc = tcx_tiles_per_cta(A.nrows, A.ncols, A.cta_blocks);
     const uint32_t groups = A.nrows / TC_M / tpc, mat = blockIdx.x / groups, rt0 = (blockIdx.x - mat * groups) * tpc;
     const uint32_t nstage = tpc * kstage, nblk = tpc * bpr;           // stages and 256-column blocks of the whole CTA
     const uint8_t *wrec = A.w[mat] + (uint64_t)e * A.mat_bytes + (uint64_t)(rt0 * 8u) * bpr * NIB_REC;    // record (16-row tile 8 rt0 + j, block c) at (j * bpr + c) * NIB_REC
@@ -184,10 +183,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_experts(const __grid_const
         uint32_t row = TCX_DEAD, pair = TCX_DEAD; float inv = 0.f;
         if (tid < nt) { pair = A.sorted[p0 + tid]; row = pair / A.x_div; inv = A.x_inv[row]; }
         s_row[tid] = row; s_pair[tid] = pair; s_xinv[tid] = inv;
-    }
-    for (uint32_t i = tid; i < TC_M * nblk; i += TC_THREADS) {     // block scales of the CTA's rows: s_d[tile * bpr + block][row of the tile]
-        const uint32_t cb = i / TC_M, r = i - cb * TC_M, tile = cb / bpr, c = cb - tile * bpr;
-        s_d[cb][r] = 0.125f * __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(wrec + ((uint64_t)(tile * 8u + (r >> 4)) * bpr + c) * NIB_REC + nib_d_off(r & 15u)))));
     }
     if (tid == 0) {
         fail = 0u;
@@ -364,12 +359,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_experts(const __grid_const
 #pragma unroll
         for (uint32_t j = 0; j < (uint32_t)TN; ++j) acc[j] = 0.f;
         bool ok = true;
+        // d / 8 of this thread's row, a block ahead
+        auto scale_of = [&](uint32_t blk) {
+            const uint32_t r = qlane + lane, tile = blk / bpr, c = blk - tile * bpr;
+            return 0.125f * __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(wrec + ((uint64_t)(tile * 8u + (r >> 4)) * bpr + c) * NIB_REC + nib_d_off(r & 15u)))));
+        };
+        float dnext = scale_of(0u);
         for (uint32_t blk = 0; blk < nblk && ok; ++blk) {
+            const float dsc = dnext;
+            if (blk + 1u < nblk) dnext = scale_of(blk + 1u);
             ok = wait_idle(&acc_full[blk & 1u], (blk >> 1) & 1u);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             
-            const float dsc = s_d[blk][qlane + lane];
             const uint32_t base = tmem + (qlane << 16) + (blk & 1u) * 2u * (uint32_t)TN;
 #pragma unroll
             for (uint32_t cc = 0; cc < (uint32_t)TN; cc += 16u) {
@@ -427,7 +429,10 @@ int launch_tc_experts(TcxArgs &A, uint32_t max_items, const char *tag, cudaStrea
     RC_REQUIRE(max_items <= 65535u, "tc experts: %u work items exceed the grid", max_items);
     constexpr uint32_t TN = TCX_TN;
     const size_t smem = 2u * (size_t)TCX_SUBS * TC_A_DIGIT + (size_t)TCX_NB * TCX_SUBS * 2u * TN * TC_KS * 2u + 2u * (size_t)TCX_RAW;
-    const dim3 grid(A.nmat * (A.nrows / TC_M / tcx_tiles_per_cta(A.nrows, A.ncols)), max_items);
+    // Blocks of 256 columns per CTA: setting a CTA up and draining it takes 5 us, a block 1.2, and one CTA fits an SM. So a CTA takes as many
+    // as leave every SM six CTAs or more.
+    for (A.cta_blocks = 32u; A.cta_blocks > 8u && (uint64_t)max_items * A.nmat * (A.nrows / TC_M / tcx_tiles_per_cta(A.nrows, A.ncols, A.cta_blocks)) < 148u * 6u;) A.cta_blocks >>= 1;
+    const dim3 grid(A.nmat * (A.nrows / TC_M / tcx_tiles_per_cta(A.nrows, A.ncols, A.cta_blocks)), max_items);
     prof_begin(tag, s);
     RC_CUDA(cudaFuncSetAttribute(k_tc_experts<(int)TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     RC_LAUNCH((k_tc_experts<(int)TN>), grid, TC_THREADS, smem, s, A);

@@ -52,6 +52,7 @@ struct TcxArgs {
     uint32_t x_div;                 // activation row of pair p = p / x_div
     float *out[2];                  // out[m][p * out_stride + row]
     uint32_t out_stride;
+    uint32_t cta_blocks;            // filled by launch_tc_experts
     uint32_t *err, *status;         // timeout flag of the launch; sticky status words (may be null)
 };
 // v[r][k] = b ? SiLU(a[r][k]) * b[r][k] : a[r][k]  ->  fp16 digits xd[r][2][ncols] and x_inv[r]
