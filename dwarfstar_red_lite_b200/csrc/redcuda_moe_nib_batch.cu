@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
     int8_t *digits = reinterpret_cast<int8_t *>(smem);
     const uint32_t full_s = nb_smem(&s_full[0]), told_s = nb_smem(&s_told[0]);
-    const uint32_t ntile = A.nrows >> 4, npair = GATEUP ? ntile : (ntile + 1u) / 2u, PPI = (npair + TPP - 1u) / TPP;     // tile pairs and pieces of an item
+    const uint32_t ntile = A.nrows >> 4, npair = GATEUP ? ntile : ntile / 2u, PPI = (npair + TPP - 1u) / TPP;     // tile pairs and pieces of an item
     const uint32_t total = *A.n_items * PPI, share = (total + gridDim.x - 1u) / gridDim.x;
     bool failed = false;
 
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
         else {
             const uint32_t q = s / BPR;
             a = P.rec + (size_t)(s + q * BPR) * NIB_REC;
-            b = a + (2u * (P.pair0 + q) + 1u < ntile ? BPR * NIB_REC : 0u);      // an odd last tile is taken twice and stored once
+            b = a + BPR * NIB_REC;
         }
     };
     const uint32_t lane_code = nib_lane_off(g, t), lane_sc = NIB_SC_OFF + g * 8u, lane_d = NIB_D_OFF + g * 4u;
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
                 auto store = [&](uint32_t pr, uint32_t r, float v0, float v1) {
                     float *o = A.out + (size_t)S.row[pr] * A.out_stride + row0 + r;
                     if (GATEUP) *o = (v0 / (1.0f + expf(-v0))) * v1;
-                    else { o[0] = v0; if (2u * pair + 1u < ntile) o[16] = v1; }
+                    else { o[0] = v0; o[16] = v1; }
                 };
 #pragma unroll
                 for (int n = 0; n < (PACKED || WIDE ? NT : 1); ++n) {
@@ -368,11 +368,12 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
 int launch_nib_batch(MmaArgs &A, uint32_t max_items, cudaStream_t s) {
     const bool gateup = A.w1 != nullptr;
     RC_REQUIRE(nib_shape_ok(A.nrows, A.ncols), "nibble experts: matrix %ux%u is not tileable", A.nrows, A.ncols);
+    RC_REQUIRE(gateup || A.nrows % 32u == 0, "nibble experts: %u rows of down are not pairs of tiles", A.nrows);      // (every size the layout takes as columns is)
     RC_REQUIRE(A.work != nullptr && A.item_tok >= 1u && A.item_tok <= (A.fmt == NIB_IQ2 ? 8u : NIB_WIDE_PAIRS), "nibble experts: work counter missing or items of %u pairs", A.item_tok);
     A.act_bits = act_digit_bits(); A.dw1 = (float)(1u << A.act_bits); A.dw2 = A.dw1 * A.dw1;
     static int sm_count = 0;
     if (!sm_count) { int dev = 0; RC_CUDA(cudaGetDevice(&dev)); RC_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev)); }
-    const uint32_t tiles = A.nrows / 16u, pairs = gateup ? tiles : (tiles + 1u) / 2u, tpp = nbb_pairs(A.ncols);
+    const uint32_t tiles = A.nrows / 16u, pairs = gateup ? tiles : tiles / 2u, tpp = nbb_pairs(A.ncols);
     const uint64_t pieces = (uint64_t)max_items * ((pairs + tpp - 1u) / tpp);
     const uint32_t grid = (uint32_t)(pieces < (uint64_t)sm_count ? (pieces ? pieces : 1u) : (uint64_t)sm_count);
     prof_begin(gateup ? "moe_gateup" : "moe_down", s);
