@@ -10,10 +10,10 @@
 //               exactly in s32 (|.| < 2^25), the result and digit 0 converted to fp32 and accumulated with the fp32
 //               scale d*sc
 //
-// Block = one tile of 16 rows (of one matrix, or of a gate / up pair) x TGB groups of 8 tokens; its 8 warps split the columns KS ways in
-// units of 128 and take a token group each. Weights and digits of up to 2048 columns are staged in shared memory by bulk copies, a row
-// each, at pitches that keep the fragment loads free of bank conflicts. (Loaded straight from global memory, 4 bytes a lane from eight
-// rows 1024 bytes apart, the kernel was bound by the L1 tag rate: 88 cycles an SM for every 16 columns of 8 tokens.)
+// Block = 8 warps = MS matrices x KS column splits x TGB groups of 8 tokens, for one tile of 16 rows. Weights and digits of a panel of
+// columns are staged in shared memory by bulk copies, a row each, at pitches that keep the fragment loads free of bank conflicts.
+// (Loaded straight from global memory, 4 bytes a lane from eight rows 1024 bytes apart, the kernel was bound by the L1 tag rate: 88
+// cycles an SM for every 16 columns of 8 tokens. Shared expert of 64 tokens: 26 + 13 us then.)
 // Partial sums meet in shared memory, where the epilogue (plain store or SiLU(gate)*up) is applied.
 #define RC_PDL_DEFAULT 0
 #include "redcuda_common.cuh"
@@ -36,27 +36,28 @@ struct Q6Args {
     const int8_t *xq; const float *sx;      // digits [ntok][3][ncols], scale per token
     float *out; uint32_t out_stride;        // out[token * out_stride + row]
     uint32_t *status;
-    uint32_t KS;                            // column splits (8 % KS == 0); 8 / KS token groups per block
+    uint32_t MS, KS, panel;                 // matrices and column splits per block (8 % (MS * KS) == 0), columns staged at a time
     uint32_t bits; float dw1;               // digit width and 2^bits
 };
-constexpr uint32_t Q6M_PANEL = 2048u;       // columns staged at a time
+constexpr uint32_t Q6M_PANEL = 4096u;       // most columns staged at a time
 // bytes of a staged panel of pc columns: 16 rows of a matrix, 8 tokens
 __host__ __device__ constexpr uint32_t q6m_a_bytes(uint32_t pc) { return 16u * (pc / 2u + 16u + pc / 4u + 16u + pc / 16u + 16u); }
 __host__ __device__ constexpr uint32_t q6m_b_bytes(uint32_t pc) { return 24u * (pc + 16u); }
 
-template <uint32_t MS>
 __global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Args A) {
     pdl_prologue();
     extern __shared__ __align__(16) uint8_t q6m_smem[];
-    __shared__ float part[MS][8][16][8];    // per matrix and warp: 16 rows x 8 tokens
-    __shared__ float s_d[MS][16][Q6M_PANEL / 256u];
+    __shared__ float part[8][16][8];        // per warp: 16 rows x 8 tokens
+    __shared__ float s_d[2][16][Q6M_PANEL / 256u];
     __shared__ __align__(8) uint64_t s_bar;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
-    const uint32_t KS = A.KS, TGB = 8u / KS, ks = warp % KS, tgl = warp / KS;
+    const uint32_t MS = A.MS, KS = A.KS, TGB = 8u / (MS * KS);
+    const uint32_t mat = warp % MS, ks = (warp / MS) % KS, tgl = warp / (MS * KS);
     const uint32_t tg = blockIdx.y * TGB + tgl;                 // group of 8 tokens
     const uint32_t row0 = blockIdx.x * 16u, bpr = A.ncols >> 8;
     const uint32_t tok_first = blockIdx.y * TGB * 8u, ntok_b = min(TGB * 8u, A.ntok - tok_first);     // the block's tokens
-    const uint32_t pcmax = min(A.ncols, Q6M_PANEL), a_bytes = q6m_a_bytes(pcmax);
+    const uint32_t u_begin = ks * (2u * bpr / KS), u_end = u_begin + 2u * bpr / KS;                   // the warp's runs of 128 columns
+    const uint32_t pcmax = A.panel, a_bytes = q6m_a_bytes(pcmax);
     const uint32_t ql_pitch = pcmax / 2u + 16u, qh_pitch = pcmax / 4u + 16u, sc_pitch = pcmax / 16u + 16u, b_pitch = pcmax + 16u;
     uint8_t *b_base = q6m_smem + MS * a_bytes;
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
@@ -65,15 +66,13 @@ __global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Ar
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    float out[MS][4];
-#pragma unroll
-    for (uint32_t m = 0; m < MS; ++m) out[m][0] = out[m][1] = out[m][2] = out[m][3] = 0.f;
+    float out[4] = {0.f, 0.f, 0.f, 0.f};
     int z[4];
     asm volatile("mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;" : "=r"(z[0]), "=r"(z[1]), "=r"(z[2]), "=r"(z[3]));
     bool ok = true;
     uint32_t parity = 0u;
-    for (uint32_t blk0 = 0u; blk0 < bpr; blk0 += Q6M_PANEL / 256u, parity ^= 1u) {
-        const uint32_t nblk = min(bpr - blk0, Q6M_PANEL / 256u), pc = nblk * 256u;
+    for (uint32_t blk0 = 0u; blk0 < bpr; blk0 += pcmax / 256u, parity ^= 1u) {
+        const uint32_t nblk = min(bpr - blk0, pcmax / 256u), pc = nblk * 256u;
         __syncthreads();                     // the barrier is ready; the panel before this one has been read
         if (tid == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(MS * 16u * (pc / 2u + pc / 4u + pc / 16u) + ntok_b * 3u * pc) : "memory");
         __syncthreads();
@@ -102,64 +101,55 @@ __global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Ar
         __syncthreads();                     // s_d
         if (ok) ok = nb_wait(bar, parity);
         if (!ok || tg * 8u >= A.ntok) continue;
-        const uint8_t *xb = b_base + (tgl * 8u + g) * 3u * b_pitch + 4u * t;
-        for (uint32_t u = ks; u < 2u * nblk; u += KS) {
-            const uint32_t b = u >> 1, h = u & 1u;
+        const uint8_t *xb = b_base + (tgl * 8u + g) * 3u * b_pitch + 4u * t, *am = q6m_smem + mat * a_bytes;
+        for (uint32_t u = max(u_begin, 2u * blk0); u < min(u_end, 2u * (blk0 + nblk)); ++u) {
+            const uint32_t b = (u >> 1) - blk0, h = u & 1u;
+            uint32_t ql[2][2][2], qh[2][2];       // [row g / g + 8][columns 0..15 / 16..31 of a run of 32][runs 0, 2 / 1, 3]
+            float d[2];
+            uint2 sc[2];
 #pragma unroll
-            for (uint32_t i = 0; i < 2u; ++i) {
-                uint32_t bx[4][3];
+            for (uint32_t hr = 0; hr < 2u; ++hr) {
+                const uint32_t r = g + 8u * hr;
 #pragma unroll
-                for (uint32_t q = 0; q < 4u; ++q)
+                for (uint32_t i = 0; i < 2u; ++i) {
+                    const uint8_t *lp = am + r * ql_pitch + b * 128u + 64u * h + 16u * i + 4u * t;
+                    ql[hr][i][0] = *reinterpret_cast<const uint32_t *>(lp); ql[hr][i][1] = *reinterpret_cast<const uint32_t *>(lp + 32u);
+                    qh[hr][i] = *reinterpret_cast<const uint32_t *>(am + 16u * ql_pitch + r * qh_pitch + b * 64u + 32u * h + 16u * i + 4u * t);
+                }
+                sc[hr] = *reinterpret_cast<const uint2 *>(am + 16u * (ql_pitch + qh_pitch) + r * sc_pitch + b * 16u + 8u * h);
+                d[hr] = s_d[mat][r][b];
+            }
 #pragma unroll
-                    for (uint32_t dg = 0; dg < 3u; ++dg) bx[q][dg] = *reinterpret_cast<const uint32_t *>(xb + dg * b_pitch + b * 256u + h * 128u + 32u * q + 16u * i);
+            for (uint32_t q = 0; q < 4u; ++q)
 #pragma unroll
-                for (uint32_t m = 0; m < MS; ++m) {
-                    const uint8_t *am = q6m_smem + m * a_bytes;
-                    uint32_t ql[2][2], qh[2];
-                    float d[2];
-                    uint2 sc[2];
+                for (uint32_t i = 0; i < 2u; ++i) {
+                    const uint8_t *xp = xb + b * 256u + h * 128u + 32u * q + 16u * i;
+                    uint32_t a[2];
+                    float scl[2];
 #pragma unroll
                     for (uint32_t hr = 0; hr < 2u; ++hr) {
-                        const uint32_t r = g + 8u * hr;
-                        const uint8_t *lp = am + r * ql_pitch + b * 128u + 64u * h + 16u * i + 4u * t;
-                        ql[hr][0] = *reinterpret_cast<const uint32_t *>(lp); ql[hr][1] = *reinterpret_cast<const uint32_t *>(lp + 32u);
-                        qh[hr] = *reinterpret_cast<const uint32_t *>(am + 16u * ql_pitch + r * qh_pitch + b * 64u + 32u * h + 16u * i + 4u * t);
-                        sc[hr] = *reinterpret_cast<const uint2 *>(am + 16u * (ql_pitch + qh_pitch) + r * sc_pitch + b * 16u + 8u * h);
-                        d[hr] = s_d[m][r][b];
+                        const uint32_t v = ((ql[hr][i][q & 1u] >> (4u * (q >> 1))) & 0x0F0F0F0Fu) | (((qh[hr][i] >> (2u * q)) & 0x03030303u) << 4);
+                        const uint32_t x = v ^ 0x20202020u;            // 6-bit two's complement of (value - 32)
+                        a[hr] = x + (x & 0x20202020u) * 6u;             // sign-extend every byte to 8 bits (bits 6,7 were clear: no carry)
+                        scl[hr] = d[hr] * (float)(int)(signed char)((q < 2u ? sc[hr].x : sc[hr].y) >> (16u * (q & 1u) + 8u * i));
                     }
+                    int d0[4], d1[4], d2[4];
+                    mma_s8_k16(d0, a[0], a[1], *reinterpret_cast<const uint32_t *>(xp), z);
+                    mma_s8_k16(d1, a[0], a[1], *reinterpret_cast<const uint32_t *>(xp + b_pitch), z);
+                    mma_s8_k16(d2, a[0], a[1], *reinterpret_cast<const uint32_t *>(xp + 2u * b_pitch), z);
 #pragma unroll
-                    for (uint32_t q = 0; q < 4u; ++q) {
-                        uint32_t a[2];
-                        float scl[2];
-#pragma unroll
-                        for (uint32_t hr = 0; hr < 2u; ++hr) {
-                            const uint32_t v = ((ql[hr][q & 1u] >> (4u * (q >> 1))) & 0x0F0F0F0Fu) | (((qh[hr] >> (2u * q)) & 0x03030303u) << 4);
-                            const uint32_t x = v ^ 0x20202020u;            // 6-bit two's complement of (value - 32)
-                            a[hr] = x + (x & 0x20202020u) * 6u;             // sign-extend every byte to 8 bits (bits 6,7 were clear: no carry)
-                            scl[hr] = d[hr] * (float)(int)(signed char)((q < 2u ? sc[hr].x : sc[hr].y) >> (16u * (q & 1u) + 8u * i));
-                        }
-                        int d0[4], d1[4], d2[4];
-                        mma_s8_k16(d0, a[0], a[1], bx[q][0], z);
-                        mma_s8_k16(d1, a[0], a[1], bx[q][1], z);
-                        mma_s8_k16(d2, a[0], a[1], bx[q][2], z);
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const int hi = d1[c] + (d2[c] << A.bits);                 // 8-bit digits: the full recombination would leave s32
-                            out[m][c] += scl[c >> 1] * fmaf(A.dw1, (float)hi, (float)d0[c]);
-                        }
+                    for (int c = 0; c < 4; ++c) {
+                        const int hi = d1[c] + (d2[c] << A.bits);                 // 8-bit digits: the full recombination would leave s32
+                        out[c] += scl[c >> 1] * fmaf(A.dw1, (float)hi, (float)d0[c]);
                     }
                 }
-            }
         }
     }
     // accumulator columns 2t, 2t+1 of this lane are tokens tg*8 + 2t, +1
     const uint32_t tk0 = tg * 8u + 2u * t;
     const float s0 = tk0 < A.ntok ? A.sx[tk0] : 0.f, s1 = tk0 + 1u < A.ntok ? A.sx[tk0 + 1u] : 0.f;
-#pragma unroll
-    for (uint32_t m = 0; m < MS; ++m) {
-        part[m][warp][g][2u * t] = out[m][0] * s0; part[m][warp][g][2u * t + 1u] = out[m][1] * s1;
-        part[m][warp][g + 8u][2u * t] = out[m][2] * s0; part[m][warp][g + 8u][2u * t + 1u] = out[m][3] * s1;
-    }
+    part[warp][g][2u * t] = out[0] * s0; part[warp][g][2u * t + 1u] = out[1] * s1;
+    part[warp][g + 8u][2u * t] = out[2] * s0; part[warp][g + 8u][2u * t + 1u] = out[3] * s1;
     if (!ok) {                               // a copy never came: the results are void; it is given as long again before the block may end
         if (A.status) A.status[ST_TIMEOUT] = 1u;
         nb_wait(bar, parity ^ 1u);
@@ -170,14 +160,11 @@ __global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Ar
         const uint32_t tl = idx >> 7, row = (idx >> 3) & 15u, c = idx & 7u;
         const uint32_t tkn = (blockIdx.y * TGB + tl) * 8u + c;
         if (tkn >= A.ntok || row0 + row >= A.nrows) continue;
-        float val[MS];
-#pragma unroll
-        for (uint32_t m = 0; m < MS; ++m) {
-            val[m] = 0.f;
-            for (uint32_t k = 0; k < KS; ++k) val[m] += part[m][tl * KS + k][row][c];
-        }
+        float val[2] = {0.f, 0.f};
+        for (uint32_t m = 0; m < MS; ++m)
+            for (uint32_t k = 0; k < KS; ++k) val[m] += part[(tl * KS + k) * MS + m][row][c];
         float v = val[0];
-        if (MS == 2u) v = (val[0] / (1.0f + expf(-val[0]))) * val[MS - 1u];
+        if (MS == 2u) v = (val[0] / (1.0f + expf(-val[0]))) * val[1];
         A.out[(size_t)tkn * A.out_stride + row0 + row] = v;
     }
 }
@@ -191,19 +178,21 @@ int launch_q6k_mma(const uint8_t *w0, const uint8_t *w1, uint64_t nb, uint32_t n
     A.w[0] = w0; A.w[1] = w1 ? w1 : w0; A.nb = nb; A.nrows = nrows; A.ncols = ncols; A.ntok = ntok; A.xq = xq; A.sx = sx;
     A.out = out; A.out_stride = out_stride; A.status = status_words();
     A.bits = act_digit_bits(); A.dw1 = (float)(1u << A.bits);
-    const uint32_t units = ncols / 128u, tgroups = (ntok + 7u) / 8u, pc = ncols < Q6M_PANEL ? ncols : Q6M_PANEL;
-    A.KS = units >= 8u ? 8u : units >= 4u ? 4u : 2u;
-    const uint32_t TGB = 8u / A.KS, ms = w1 ? 2u : 1u;
-    const size_t smem = (size_t)ms * q6m_a_bytes(pc) + (size_t)TGB * q6m_b_bytes(pc);
-    const dim3 grid(nrows / 16u, (tgroups + TGB - 1u) / TGB);
+    A.MS = w1 ? 2u : 1u;
+    const uint32_t nsteps = ncols / 16u, tgroups = (ntok + 7u) / 8u, tiles = nrows / 16u;
+    // column splits while the launch would leave SMs or warps idle and every split keeps 256 columns or more (whole runs of 128)
+    uint32_t KS = 1u;
+    while (A.MS * KS * 2u <= 8u && nsteps / (KS * 2u) >= 16u && nsteps % (KS * 16u) == 0 &&
+           ((uint64_t)tiles * ((tgroups + 8u / (A.MS * KS) - 1u) / (8u / (A.MS * KS))) < 148u * 2u || tgroups < 8u / (A.MS * KS))) KS <<= 1;
+    A.KS = KS;
+    const uint32_t TGB = 8u / (A.MS * KS), groups = TGB < tgroups ? TGB : tgroups;      // groups of tokens that a block really has
+    auto bytes = [&](uint32_t pc) { return (size_t)A.MS * q6m_a_bytes(pc) + (size_t)groups * q6m_b_bytes(pc); };
+    for (A.panel = ncols < Q6M_PANEL ? ncols : Q6M_PANEL; bytes(A.panel) > 216u * 1024u;) A.panel = (A.panel / 2u + 255u) / 256u * 256u;
+    const size_t smem = bytes(A.panel);
+    const dim3 grid(tiles, (tgroups + TGB - 1u) / TGB);
     prof_begin(tag, s);
-    if (w1) {
-        RC_CUDA(cudaFuncSetAttribute(k_q6k_mma<2u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        RC_LAUNCH((k_q6k_mma<2u>), grid, 256, smem, s, A);
-    } else {
-        RC_CUDA(cudaFuncSetAttribute(k_q6k_mma<1u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        RC_LAUNCH((k_q6k_mma<1u>), grid, 256, smem, s, A);
-    }
+    RC_CUDA(cudaFuncSetAttribute(k_q6k_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RC_LAUNCH((k_q6k_mma), grid, 256, smem, s, A);
     prof_end(s);
     RC_LAUNCHED();
     return 1;
