@@ -406,10 +406,17 @@ __global__ void __launch_bounds__(256) k_vec_sigmoid(const float *__restrict__ w
 // successive instructions are one float4 (k order within 16 columns is the same permutation for both operands, and a sum
 // does not depend on it), which costs no shared-memory staging, no barrier per K tile and one conversion per element. The
 // eight partial tiles meet in shared memory once, in a fixed order. Block = 8 FT tokens x 8 FE experts.
-template <uint32_t FT, uint32_t FE>
+// a load that stays where it is written
+__device__ __forceinline__ float4 ldg_now(const float *p) {
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+constexpr uint32_t RL_ALL = 16u;      // steps of 16 columns of a warp's eighth of a row of 2048
+template <uint32_t FT, uint32_t FE, bool ALL>
 __global__ void __launch_bounds__(256) k_router_logits(const float *__restrict__ w, const float *__restrict__ x, uint32_t x_stride, uint32_t ntok,
                                                        uint32_t n_expert, uint32_t ncols, float *__restrict__ logits) {
-    pdl_prologue();
+    if (ALL) asm volatile("griddepcontrol.launch_dependents;" ::); else pdl_prologue();
     __shared__ double red[8][FT * FE * 64u];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, fr = lane >> 2, fk = lane & 3u;
     const uint32_t t0 = blockIdx.x * 8u * FT, e0 = blockIdx.y * 8u * FE;
@@ -425,14 +432,8 @@ __global__ void __launch_bounds__(256) k_router_logits(const float *__restrict__
     for (uint32_t i = 0; i < FT; ++i)
 #pragma unroll
         for (uint32_t j = 0; j < FE; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    const uint32_t n16 = ncols >> 4, c1 = n16 * (warp + 1u) / 8u;
-#pragma unroll 4
-    for (uint32_t c = n16 * warp / 8u; c < c1; ++c) {
-        float4 a[FT], b[FE];
-#pragma unroll
-        for (uint32_t i = 0; i < FT; ++i) a[i] = *reinterpret_cast<const float4 *>(xp[i] + c * 16u);
-#pragma unroll
-        for (uint32_t i = 0; i < FE; ++i) b[i] = __ldg(reinterpret_cast<const float4 *>(wp[i] + c * 16u));
+    const uint32_t n16 = ncols >> 4, c0 = n16 * warp / 8u, c1 = n16 * (warp + 1u) / 8u;
+    auto multiply = [&](const float4 (&a)[FT], const float4 (&b)[FE]) {
 #pragma unroll
         for (uint32_t kk = 0; kk < 4u; ++kk) {
             double av[FT], bv[FE];
@@ -445,6 +446,35 @@ __global__ void __launch_bounds__(256) k_router_logits(const float *__restrict__
 #pragma unroll
                 for (uint32_t j = 0; j < FE; ++j)
                     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]) : "d"(av[i]), "d"(bv[j]));
+        }
+    };
+    if constexpr (ALL) {
+        // a small batch: the warp's whole share of the weights is requested at once, ahead of the wait for the kernel that writes x
+        float4 b[RL_ALL][FE];                // a step beyond the share repeats the last one of the row and is not multiplied
+#pragma unroll
+        for (uint32_t c = 0; c < RL_ALL; ++c)
+#pragma unroll
+            for (uint32_t i = 0; i < FE; ++i) b[c][i] = ldg_now(wp[i] + min(c0 + c, n16 - 1u) * 16u);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+        for (uint32_t c4 = 0; c4 < RL_ALL; c4 += 4u) {
+            float4 a[4][FT];
+#pragma unroll
+            for (uint32_t c = 0; c < 4u; ++c)
+#pragma unroll
+                for (uint32_t i = 0; i < FT; ++i) a[c][i] = *reinterpret_cast<const float4 *>(xp[i] + min(c0 + c4 + c, n16 - 1u) * 16u);
+#pragma unroll
+            for (uint32_t c = 0; c < 4u; ++c) if (c0 + c4 + c < c1) multiply(a[c], b[c4 + c]);
+        }
+    } else {
+#pragma unroll 4
+        for (uint32_t c = c0; c < c1; ++c) {
+            float4 a[FT], b[FE];
+#pragma unroll
+            for (uint32_t i = 0; i < FT; ++i) a[i] = *reinterpret_cast<const float4 *>(xp[i] + c * 16u);
+#pragma unroll
+            for (uint32_t i = 0; i < FE; ++i) b[i] = __ldg(reinterpret_cast<const float4 *>(wp[i] + c * 16u));
+            multiply(a, b);
         }
     }
 #pragma unroll
@@ -467,10 +497,12 @@ int launch_router_logits(const float *w, const float *x, uint32_t x_stride, uint
     prof_begin("moe_router_logits", stream);
     // the tile grows while the blocks still fill the chip about twice: a larger one converts and reads less per product
     auto blocks = [&](uint32_t tt, uint32_t te) { return (uint64_t)((ntok + tt - 1u) / tt) * ((n_expert + te - 1u) / te); };
-#define RC_RL(FT, FE) RC_LAUNCH((k_router_logits<FT, FE>), dim3((ntok + 8u * FT - 1u) / (8u * FT), (n_expert + 8u * FE - 1u) / (8u * FE)), 256, 0, stream, w, x, x_stride, ntok, n_expert, ncols, logits)
-    if (ntok <= 8u) RC_RL(1u, 1u);
-    else if (blocks(16u, 8u) <= 296u) RC_RL(2u, 1u);
-    else RC_RL(2u, 2u);
+    // up to two blocks per SM the loads of a warp's whole share go out together (ALL): HBM is waited for once instead of once per four steps
+    const bool all = ncols <= 128u * RL_ALL;
+#define RC_RL(FT, FE, ALL) RC_LAUNCH((k_router_logits<FT, FE, ALL>), dim3((ntok + 8u * FT - 1u) / (8u * FT), (n_expert + 8u * FE - 1u) / (8u * FE)), 256, 0, stream, w, x, x_stride, ntok, n_expert, ncols, logits)
+    if (ntok <= 8u) { if (all) RC_RL(1u, 1u, true); else RC_RL(1u, 1u, false); }
+    else if (blocks(16u, 8u) <= 296u) { if (all) RC_RL(2u, 1u, true); else RC_RL(2u, 1u, false); }
+    else RC_RL(2u, 2u, false);
 #undef RC_RL
     prof_end(stream);
     RC_LAUNCHED();
