@@ -8,7 +8,7 @@
 // (prmt against an 8-byte table held in two registers). IQ3_S experts take the same layout (NIB_IQ3): their magnitudes are the
 // odd numbers 1 .. 15, so a signed weight is 2 n + 1 with n in -8 .. 7 and the code is n itself in two's complement; as the
 // high nibble of a byte with 8 below it, it IS the int8 operand 8 (2 n + 1) - one mask-and-or per 4 weights, and the block
-// scale d / 8 serves both formats. A layer of IQ3_S experts took 549 us for 24 tokens on the CUDA-core kernel, 136 here.
+// scale d / 8 serves both formats. A layer of IQ3_S experts took 549 us for 24 tokens on the CUDA-core kernel, 109 here.
 // Dequantised values are unchanged bit for bit
 // (redcuda_nib_dequant_rows against rl_quant_dequant_row, native/redlite_native_quant_cpu.c:166-191). The price is bytes:
 // 138 per 256 weights instead of 66 (IQ3_S: 110), i.e. 2.09x (1.25x) the HBM footprint and traffic of the routed experts.
