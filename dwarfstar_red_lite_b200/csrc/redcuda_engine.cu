@@ -25,6 +25,7 @@
 namespace rc {
 
 const uint32_t *moe_last_ids_device(const redcuda_moe *m);   // redcuda_moe.cu
+int moe_forward_norm1(redcuda_moe *m, const float *x, const GemvNorm &N, const float *resid, float *out, cudaStream_t s);      // see redcuda_moe.cu
 void moe_set_ids_mirror(redcuda_moe *m, uint32_t *dev_ptr);   // a single token's router ids are also written to dev_ptr
 size_t moe_workspace_bytes(const redcuda_moe_desc *d);
 // expert parallelism: which contiguous share of every layer's experts the engines opened next will hold
@@ -68,8 +69,10 @@ __device__ __forceinline__ double block_sum_d(double v, double *red) {
     return t;
 }
 
-// normed = RMSNorm(x [+ branch]) * w (engine_cpu.c:96-101, 418-424); resid_out (optional) = x + branch. One block per token.
-__global__ void __launch_bounds__(1024) k_rmsnorm(const float *__restrict__ x, const float *__restrict__ branch, const float *__restrict__ w,
+// normed = RMSNorm(x [+ branch]) * w (engine_cpu.c:96-101, 418-424); resid_out (optional) = x + branch. One block of THREADS per token: 1024 where the token is
+// alone, its row is the chain; 256 for the rows of a chunk, where the barriers of one block are hidden by the others of its SM.
+template <uint32_t THREADS>
+__global__ void __launch_bounds__(THREADS) k_rmsnorm(const float *__restrict__ x, const float *__restrict__ branch, const float *__restrict__ w,
                                                   uint32_t n, float eps, float *__restrict__ resid_out, float *__restrict__ normed) {
     pdl_prologue();
     __shared__ double red[32];
@@ -78,20 +81,20 @@ __global__ void __launch_bounds__(1024) k_rmsnorm(const float *__restrict__ x, c
     if (branch) branch += tok_off;
     if (resid_out) resid_out += tok_off;
     // a row of up to 4096 values stays in registers between the sum and the scaling, and the weights are on their way with it
-    constexpr uint32_t KEEP = 4u;
+    constexpr uint32_t KEEP = 4096u / THREADS;
     float keep[KEEP], wk[KEEP];
     double ss = 0.0;
 #pragma unroll
     for (uint32_t j = 0; j < KEEP; ++j) {
-        const uint32_t i = threadIdx.x + j * 1024u;
+        const uint32_t i = threadIdx.x + j * THREADS;
         if (i < n) { keep[j] = x[i]; if (branch) keep[j] = keep[j] + branch[i]; wk[j] = w[i]; }
     }
 #pragma unroll
     for (uint32_t j = 0; j < KEEP; ++j) {
-        const uint32_t i = threadIdx.x + j * 1024u;
+        const uint32_t i = threadIdx.x + j * THREADS;
         if (i < n) { if (resid_out) resid_out[i] = keep[j]; ss += (double)keep[j] * (double)keep[j]; }
     }
-    for (uint32_t i = threadIdx.x + KEEP * 1024u; i < n; i += 1024u) {
+    for (uint32_t i = threadIdx.x + KEEP * THREADS; i < n; i += THREADS) {
         float v = x[i];
         if (branch) v = v + branch[i];
         if (resid_out) resid_out[i] = v;
@@ -101,10 +104,10 @@ __global__ void __launch_bounds__(1024) k_rmsnorm(const float *__restrict__ x, c
     const double inv = 1.0 / sqrt(tot / (double)n + (double)eps);
 #pragma unroll
     for (uint32_t j = 0; j < KEEP; ++j) {
-        const uint32_t i = threadIdx.x + j * 1024u;
+        const uint32_t i = threadIdx.x + j * THREADS;
         if (i < n) normed[i] = (float)((double)keep[j] * inv * (double)wk[j]);
     }
-    for (uint32_t i = threadIdx.x + KEEP * 1024u; i < n; i += 1024u) {
+    for (uint32_t i = threadIdx.x + KEEP * THREADS; i < n; i += THREADS) {
         float v = x[i];
         if (branch) v = v + branch[i];
         normed[i] = (float)((double)v * inv * (double)w[i]);
@@ -376,13 +379,26 @@ static void eng_err(char *error, size_t cap, const char *msg) { if (error && cap
 #define ENG_RC(call) do { if (!(call)) { eng_err(error, cap, redcuda_last_error()); return 0; } } while (0)
 #define ENG_CUDA(expr) do { cudaError_t e_ = (expr); if (e_ != cudaSuccess) { ENG_FAIL("%s failed: %s", #expr, cudaGetErrorString(e_)); } } while (0)
 
-static int eng_gemv(rl_engine *e, const DMat *mats, float *const *outs, uint32_t n, const float *x, const char *tag) {
+static void eng_rmsnorm(rl_engine *e, uint32_t ntok, const float *x, const GemvNorm &N) {
+    prof_begin(N.branch ? "resid_rmsnorm" : "rmsnorm", e->stream);
+    if (ntok < 148u) RC_LAUNCH((k_rmsnorm<1024u>), ntok, 1024, 0, e->stream, x, N.branch, N.w, e->info.hidden, N.eps, N.resid, N.normed);
+    else RC_LAUNCH((k_rmsnorm<256u>), ntok, 256, 0, e->stream, x, N.branch, N.w, e->info.hidden, N.eps, N.resid, N.normed);
+    prof_end(e->stream);
+    g_launches.fetch_add(1);
+}
+
+// norm (may be null): the input is RMSNorm(x [+ branch]) * w, computed by the GEMV where it can be and by a kernel before it where not
+static int eng_gemv(rl_engine *e, const DMat *mats, float *const *outs, uint32_t n, const float *x, const char *tag, const GemvNorm *norm = nullptr) {
     GemvArgs A{};
     A.njobs = n; A.ntok = 1; A.x = x; A.x_stride = mats[0].ncols; A.tag = tag; A.resident = 1u;
     for (uint32_t j = 0; j < n; ++j) {
         GemvJob &J = A.job[j];
         J.w0 = mats[j].base; J.w1 = nullptr; J.out = outs[j]; J.nb = mats[j].nb; J.type = mats[j].type; J.nrows = mats[j].nrows; J.ncols = mats[j].ncols;
         J.out_stride = mats[j].nrows; J.epi = GEMV_STORE;
+    }
+    if (norm) {
+        A.norm = *norm;
+        if (!gemv1_norm_ok(A)) { A.norm = GemvNorm{}; A.x = norm->normed; eng_rmsnorm(e, 1u, x, *norm); }
     }
     return launch_gemv(A, e->stream);
 }
@@ -448,14 +464,11 @@ static int eng_step_device(rl_engine *e, bool want_logits, char *error, size_t c
     const DnDims D{in.d_conv, in.d_state, in.n_group, in.dt_rank, in.d_inner, in.channels, in.rms_eps};
     for (uint32_t l = 0; l < in.n_layer; ++l) {
         const EngLayer &L = e->layers[l];
-        prof_begin("rmsnorm", s);
-        RC_LAUNCH((k_rmsnorm), 1, 1024, 0, s, x, nullptr, L.attn_norm, in.hidden, in.rms_eps, nullptr, e->normed);
-        prof_end(s);
-        g_launches.fetch_add(1);
+        const GemvNorm attn_norm{L.attn_norm, nullptr, in.rms_eps, nullptr, e->normed}, post_norm{L.post_norm, e->branch, in.rms_eps, e->resid, e->normed};
         if (L.recurrent) {
             const DMat mats[3] = {L.qkv, L.z, L.ba};
             float *outs[3] = {e->qkv, e->z, e->ba};
-            ENG_RC(eng_gemv(e, mats, outs, 3, e->normed, "dn_proj_gemv"));
+            ENG_RC(eng_gemv(e, mats, outs, 3, x, "dn_proj_gemv", &attn_norm));
             ENG_RC(launch_deltanet(D, 1u, L.conv_k, L.dt, L.a, L.ssm_norm, e->qkv, e->z, e->ba, e->conv + (size_t)L.ridx * (in.d_conv - 1u) * in.channels,
                                    e->rec + (size_t)L.ridx * in.dt_rank * in.d_state * in.d_state, e->dn_qk, e->dn_v, e->dn_beta, e->dn_gate, e->dn_core, e->ng, s));
             float *o1[1] = {e->branch};
@@ -463,33 +476,33 @@ static int eng_step_device(rl_engine *e, bool want_logits, char *error, size_t c
         } else {
             const DMat mats[3] = {L.q, L.k, L.v};
             float *outs[3] = {e->qg, e->kraw, e->vraw};
-            ENG_RC(eng_gemv(e, mats, outs, 3, e->normed, "attn_proj_gemv"));
+            ENG_RC(eng_gemv(e, mats, outs, 3, x, "attn_proj_gemv", &attn_norm));
             if (e->kv_half) { if (!eng_attention<__half>(e, L, 1u, e->pos_d, error, cap)) return 0; }
             else { if (!eng_attention<float>(e, L, 1u, e->pos_d, error, cap)) return 0; }
             float *o1[1] = {e->branch};
             ENG_RC(eng_gemv(e, &L.o, o1, 1, e->gated, "attn_out_gemv"));
         }
-        prof_begin("resid_rmsnorm", s);
-        RC_LAUNCH((k_rmsnorm), 1, 1024, 0, s, x, e->branch, L.post_norm, in.hidden, in.rms_eps, e->resid, e->normed);
-        prof_end(s);
-        g_launches.fetch_add(1);
         float *xo = e->layer_out_d + (size_t)l * in.hidden;
         if (e->ep_world > 1) {
+            eng_rmsnorm(e, 1u, x, post_norm);
             ENG_RC(redcuda_ep_layer_forward_n(e->ep, L.moe, 1u, e->normed, nullptr, e->resid, xo, s));
             ENG_CUDA(cudaMemcpyAsync(e->router_ids_d + (size_t)l * RL_ENGINE_MAX_TOPK, redcuda_ep_last_ids_device(e->ep), in.top_k * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-        } else
-        ENG_RC(redcuda_moe_forward_device(L.moe, 1u, e->normed, nullptr, e->resid, xo, s));      // its router kernel also fills router_ids_d (mirror set at open)
+        } else {                                             // its router kernel also fills router_ids_d (mirror set at open)
+            const int done = moe_forward_norm1(L.moe, x, post_norm, e->resid, xo, s);
+            ENG_RC(done);
+            if (done < 0) {
+                eng_rmsnorm(e, 1u, x, post_norm);
+                ENG_RC(redcuda_moe_forward_device(L.moe, 1u, e->normed, nullptr, e->resid, xo, s));
+            }
+        }
         if (e->ep_world == 1 && in.n_expert > 1024u) ENG_CUDA(cudaMemcpyAsync(e->router_ids_d + (size_t)l * RL_ENGINE_MAX_TOPK, moe_last_ids_device(L.moe), in.top_k * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
         x = xo;
     }
-    prof_begin("rmsnorm", s);
-    RC_LAUNCH((k_rmsnorm), 1, 1024, 0, s, x, nullptr, e->output_norm, in.hidden, in.rms_eps, nullptr, e->final_norm_d);
-    prof_end(s);
-    g_launches.fetch_add(1);
+    const GemvNorm output_norm{e->output_norm, nullptr, in.rms_eps, nullptr, e->final_norm_d};
     if (want_logits) {
         float *o1[1] = {e->logits_d};
-        ENG_RC(eng_gemv(e, &e->output, o1, 1, e->final_norm_d, "lm_head_gemv"));
-    }
+        ENG_RC(eng_gemv(e, &e->output, o1, 1, x, "lm_head_gemv", &output_norm));
+    } else eng_rmsnorm(e, 1u, x, output_norm);
     RC_LAUNCH((k_advance), 1, 32, 0, s, e->pos_d);
     g_launches.fetch_add(1);
     ENG_CUDA(cudaGetLastError());
@@ -556,10 +569,7 @@ static int eng_prefill_chunk(rl_engine *e, uint32_t n, bool want_logits, char *e
     const float *x = e->bx[0];
     for (uint32_t l = 0; l < in.n_layer; ++l) {
         const EngLayer &L = e->layers[l];
-        prof_begin("rmsnorm", s);
-        RC_LAUNCH((k_rmsnorm), n, 1024, 0, s, x, nullptr, L.attn_norm, in.hidden, in.rms_eps, nullptr, e->normed);
-        prof_end(s);
-        g_launches.fetch_add(1);
+        eng_rmsnorm(e, n, x, GemvNorm{L.attn_norm, nullptr, in.rms_eps, nullptr, e->normed});
         if (L.recurrent) {
             const DMat mats[3] = {L.qkv, L.z, L.ba};
             float *outs[3] = {e->qkv, e->z, e->ba};
@@ -577,10 +587,7 @@ static int eng_prefill_chunk(rl_engine *e, uint32_t n, bool want_logits, char *e
             float *o1[1] = {e->branch};
             ENG_RC(eng_proj(e, &L.o, o1, 1, e->gated, n, "attn_out"));
         }
-        prof_begin("resid_rmsnorm", s);
-        RC_LAUNCH((k_rmsnorm), n, 1024, 0, s, x, e->branch, L.post_norm, in.hidden, in.rms_eps, e->resid, e->normed);
-        prof_end(s);
-        g_launches.fetch_add(1);
+        eng_rmsnorm(e, n, x, GemvNorm{L.post_norm, e->branch, in.rms_eps, e->resid, e->normed});
         float *xo = e->bx[(l + 1u) & 1u];
         if (e->ep_world > 1) ENG_RC(redcuda_ep_layer_forward_n(e->ep, L.moe, n, e->normed, nullptr, e->resid, xo, s));
         else ENG_RC(redcuda_moe_forward_device(L.moe, n, e->normed, nullptr, e->resid, xo, s));
@@ -588,14 +595,11 @@ static int eng_prefill_chunk(rl_engine *e, uint32_t n, bool want_logits, char *e
         ENG_CUDA(cudaMemcpyAsync(e->layer_out_d + (size_t)l * in.hidden, xo + last * in.hidden, in.hidden * 4u, cudaMemcpyDeviceToDevice, s));
         x = xo;
     }
-    prof_begin("rmsnorm", s);
-    RC_LAUNCH((k_rmsnorm), 1, 1024, 0, s, x + last * in.hidden, nullptr, e->output_norm, in.hidden, in.rms_eps, nullptr, e->final_norm_d);
-    prof_end(s);
-    g_launches.fetch_add(1);
+    const GemvNorm output_norm{e->output_norm, nullptr, in.rms_eps, nullptr, e->final_norm_d};
     if (want_logits) {
         float *o1[1] = {e->logits_d};
-        ENG_RC(eng_gemv(e, &e->output, o1, 1, e->final_norm_d, "lm_head_gemv"));
-    }
+        ENG_RC(eng_gemv(e, &e->output, o1, 1, x + last * in.hidden, "lm_head_gemv", &output_norm));
+    } else eng_rmsnorm(e, 1u, x + last * in.hidden, output_norm);
     ENG_CUDA(cudaGetLastError());
     e->position += n;
     return 1;

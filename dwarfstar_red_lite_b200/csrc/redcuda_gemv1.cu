@@ -44,7 +44,56 @@ struct G1Tile { uint32_t row0, nvr, pair; bool resident; };      // nvr: rows of
 // two blocks) hit eight different bank groups
 __host__ __device__ __forceinline__ uint32_t g1_xi(uint32_t k) { return (k >> 8) * 268u + ((k >> 7) & 1u) * 136u + (k & 127u); }
 
-__device__ __forceinline__ void gemv1_q6k(const GemvJob &J, const G1Tile &T, const float *x, double *part, float *xs) {
+// x into shared memory, by every thread of the block; with a norm, normalised on the way. A kernel of its own for it (one block) took 4.6 us
+// of a decoding step's chain twice a layer; here it is about one, most of it while the first weights arrive. ncols at most G1_NCOLS then.
+constexpr uint32_t G1_NCOLS = 2048u;
+template <bool NORM>
+__device__ __forceinline__ void gemv1_stage(const GemvArgs &A, uint32_t ncols, float *xs) {
+    if (!NORM) {
+        for (uint32_t k = threadIdx.x * 4u; k < ncols; k += G1_WARPS * 128u) *reinterpret_cast<float4 *>(xs + g1_xi(k)) = *reinterpret_cast<const float4 *>(A.x + k);
+        return;
+    }
+    __shared__ double red[G1_WARPS];
+    constexpr uint32_t N = G1_NCOLS / (G1_WARPS * 128u);
+    float4 v[N], w[N];
+    double ss = 0.0;
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) {
+        const uint32_t k = threadIdx.x * 4u + j * G1_WARPS * 128u;
+        v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k >= ncols) continue;
+        v[j] = *reinterpret_cast<const float4 *>(A.x + k);
+        w[j] = __ldg(reinterpret_cast<const float4 *>(A.norm.w + k));
+        if (A.norm.branch) {
+            const float4 b = *reinterpret_cast<const float4 *>(A.norm.branch + k);
+            v[j].x += b.x; v[j].y += b.y; v[j].z += b.z; v[j].w += b.w;
+        }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) ss += (double)v[j].x * (double)v[j].x + (double)v[j].y * (double)v[j].y + (double)v[j].z * (double)v[j].z + (double)v[j].w * (double)v[j].w;
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    double tot = 0.0;
+#pragma unroll
+    for (uint32_t i = 0; i < G1_WARPS; ++i) tot += red[i];
+    const double inv = 1.0 / sqrt(tot / (double)ncols + (double)A.norm.eps);
+#pragma unroll
+    for (uint32_t j = 0; j < N; ++j) {
+        const uint32_t k = threadIdx.x * 4u + j * G1_WARPS * 128u;
+        if (k >= ncols) continue;
+        const float4 n = make_float4((float)((double)v[j].x * inv * (double)w[j].x), (float)((double)v[j].y * inv * (double)w[j].y),
+                                     (float)((double)v[j].z * inv * (double)w[j].z), (float)((double)v[j].w * inv * (double)w[j].w));
+        *reinterpret_cast<float4 *>(xs + g1_xi(k)) = n;
+        if (blockIdx.x == 0u) {
+            *reinterpret_cast<float4 *>(A.norm.normed + k) = n;
+            if (A.norm.resid) *reinterpret_cast<float4 *>(A.norm.resid + k) = v[j];
+        }
+    }
+}
+
+template <bool NORM>
+__device__ __forceinline__ void gemv1_q6k(const GemvArgs &A, const GemvJob &J, const G1Tile &T, double *part, float *xs) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t cpr = J.ncols >> 6, bpr = J.ncols >> 8, S = g1_slices(RC_Q6_K, J.ncols), ws = g1_slice_warps(S), lpr = g1_lanes(RC_Q6_K, J.ncols), rw = 32u / lpr;
     const uint32_t slot = lane / lpr, sub = lane % lpr, step = (G1_WARPS / ws) * rw, first = (warp / ws) * rw;
@@ -74,7 +123,7 @@ __device__ __forceinline__ void gemv1_q6k(const GemvJob &J, const G1Tile &T, con
         if (!staged) {
             staged = true;
             pdl_wait();
-            for (uint32_t k = threadIdx.x * 4u; k < J.ncols; k += G1_WARPS * 128u) *reinterpret_cast<float4 *>(xs + g1_xi(k)) = *reinterpret_cast<const float4 *>(x + k);
+            gemv1_stage<NORM>(A, J.ncols, xs);
             if (!T.resident) { f[0] = load(first + slot); f[1] = load(first + step + slot); }
             __syncthreads();
         }
@@ -126,8 +175,8 @@ __device__ __forceinline__ void gemv1_q6k(const GemvJob &J, const G1Tile &T, con
     }
 }
 
-template <bool HALF>
-__device__ __forceinline__ void gemv1_plain(const GemvJob &J, const G1Tile &T, const float *x, double *part) {
+template <bool NORM, bool HALF>
+__device__ __forceinline__ void gemv1_plain(const GemvArgs &A, const GemvJob &J, const G1Tile &T, double *part, float *xs) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t S = g1_slices(RC_F32, J.ncols), ws = g1_slice_warps(S), step = G1_WARPS / ws;
     bool waited = false;
@@ -150,12 +199,16 @@ __device__ __forceinline__ void gemv1_plain(const GemvJob &J, const G1Tile &T, c
         };
         uint32_t vr = warp / ws;
         if (T.resident && vr < T.nvr) load(vr);
-        if (!waited) { pdl_wait(); waited = true; }
+        if (!waited) {
+            pdl_wait();
+            waited = true;
+            if (NORM) { gemv1_stage<NORM>(A, J.ncols, xs); __syncthreads(); }      // every warp has a slice, so all of them come here
+        }
         if (!T.resident && vr < T.nvr) load(vr);
 #pragma unroll
         for (uint32_t i = 0; i < 4u; ++i) {
             const uint32_t k = k0 + 128u * i;
-            xv[i] = k < J.ncols ? *reinterpret_cast<const float4 *>(x + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xv[i] = k < J.ncols ? *reinterpret_cast<const float4 *>(NORM ? xs + g1_xi(k) : A.x + k) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         for (; vr < T.nvr; vr += step) {
             double a0 = 0.0, a1 = 0.0;                    // two chains: the double FMA's latency is what a short row waits for
@@ -173,6 +226,7 @@ __device__ __forceinline__ void gemv1_plain(const GemvJob &J, const G1Tile &T, c
     if (!waited) pdl_wait();
 }
 
+template <bool NORM>
 __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1(const __grid_constant__ GemvArgs A) {
     pdl_trigger();
     extern __shared__ __align__(16) double g1_part[];      // [row of the tile (x 2 for a pair)][slice], behind it x
@@ -181,9 +235,10 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1(const __grid_consta
     const GemvJob &J = A.job[j];
     const uint32_t row0 = (blockIdx.x - J.tile_begin) * J.rows_per_tile, nrow = min(J.rows_per_tile, J.nrows - row0), pair = J.epi == GEMV_PAIR_SILU ? 1u : 0u;
     const G1Tile T{row0, nrow << pair, pair, A.resident != 0u};
-    if (J.type == RC_Q6_K) gemv1_q6k(J, T, A.x, g1_part, reinterpret_cast<float *>(g1_part + A.part_doubles));
-    else if (J.type == RC_F32) gemv1_plain<false>(J, T, A.x, g1_part);
-    else gemv1_plain<true>(J, T, A.x, g1_part);
+    float *xs = reinterpret_cast<float *>(g1_part + A.part_doubles);
+    if (J.type == RC_Q6_K) gemv1_q6k<NORM>(A, J, T, g1_part, xs);
+    else if (J.type == RC_F32) gemv1_plain<NORM, false>(A, J, T, g1_part, xs);
+    else gemv1_plain<NORM, true>(A, J, T, g1_part, xs);
     __syncthreads();
     const uint32_t S = g1_slices(J.type, J.ncols);
     for (uint32_t r = threadIdx.x; r < nrow; r += G1_WARPS * 32u) {
@@ -209,7 +264,14 @@ bool gemv1_ok(const GemvArgs &A) {
     return true;
 }
 
+bool gemv1_norm_ok(const GemvArgs &A) {
+    for (uint32_t j = 0; j < A.njobs; ++j) if (A.job[j].ncols != A.job[0].ncols || A.job[j].ncols % 4u) return false;
+    auto al = [](const void *p) { return ((uintptr_t)p & 15u) == 0u; };
+    return gemv1_ok(A) && A.job[0].ncols <= G1_NCOLS && A.norm.normed && al(A.norm.w) && al(A.norm.branch) && al(A.norm.resid) && al(A.norm.normed);
+}
+
 int launch_gemv1(GemvArgs &A, cudaStream_t stream) {
+    RC_REQUIRE(!A.norm.w || gemv1_norm_ok(A), "gemv: this input cannot be normalised on the way");
     // Tiles of about equal bytes, three per SM (what the registers let reside), so that a launch is one wave whatever its jobs;
     // at least one row per warp of the block, at most what 8 KB of partial sums hold.
     uint64_t total = 0;
@@ -234,9 +296,10 @@ int launch_gemv1(GemvArgs &A, cudaStream_t stream) {
         q6 = q6 || J.type == RC_Q6_K;
     }
     A.part_doubles = (uint32_t)(smem / sizeof(double));
-    if (q6) smem += (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + 16u;
+    if (q6 || A.norm.w) smem += (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + 16u;
     prof_begin(A.tag ? A.tag : "gemv", stream);
-    RC_LAUNCH((k_gemv1), tiles, G1_WARPS * 32u, smem, stream, A);
+    if (A.norm.w) RC_LAUNCH((k_gemv1<true>), tiles, G1_WARPS * 32u, smem, stream, A);
+    else RC_LAUNCH((k_gemv1<false>), tiles, G1_WARPS * 32u, smem, stream, A);
     prof_end(stream);
     RC_LAUNCHED();
     return 1;

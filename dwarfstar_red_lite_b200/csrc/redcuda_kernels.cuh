@@ -33,6 +33,9 @@ struct RouteTail {
     uint32_t *status;
 };
 
+// The input of a single-token GEMV as RMSNorm(x [+ branch]) * w, computed by every block for itself: normed and resid (may be null) are
+// written by one of them. w null: x as it is.
+struct GemvNorm { const float *w, *branch; float eps; float *resid, *normed; };
 #define RC_MAX_JOBS 6u
 struct GemvArgs {
     GemvJob job[RC_MAX_JOBS];
@@ -43,12 +46,14 @@ struct GemvArgs {
     const uint32_t *iq3s;
     const char *tag;           // name under which the launch is timed when profiling is on (host side only)
     RouteTail tail;
+    GemvNorm norm;             // only where gemv1_norm_ok
     uint32_t part_doubles;     // filled by launch_gemv1
     uint32_t resident;         // 1: the weights were in place before the stream's previous kernel began (they may be requested ahead of it)
 };
 
 int launch_gemv(GemvArgs &A, cudaStream_t stream);
 bool gemv1_ok(const GemvArgs &A);                            // single-token form (redcuda_gemv1.cu), taken by launch_gemv
+bool gemv1_norm_ok(const GemvArgs &A);                       // the form that also normalises its input
 int launch_gemv1(GemvArgs &A, cudaStream_t stream);
 // group1 (ntok == 1 only, may be null): fill the grouping arrays in the same kernel; ids_mirror (may be null) gets a copy of the ids
 int launch_route(const float *logits_dev, uint32_t ntok, uint32_t n_expert, uint32_t top_k, uint32_t *ids_dev, float *weights_dev,

@@ -327,8 +327,8 @@ struct redcuda_moe {
 // Layers with IQ3_S matrices take their activations as wide digits: they ran on fp32 activations before the nibble layout held them,
 // and the 24-bit form per row is less than that (relative error of an expert's output against 64-bit sums, hidden 2048: fp32 1.6e-7 on any
 // row; three digits 3.1e-7 on Gaussian rows, 2.2e-6 with one element of 100, 4.7e-4 with a large one where the weights vanish; wide
-// digits 1.0e-7 on any). What it costs against three digits and the tcgen05 kernel, us a layer: 24 tokens 130 -> 128, 64 skewed 156 -> 168,
-// 300 391 -> 432, 2048 1235 -> 2159 (the fp32 kernel: 557, 1497, 2340, 11693).
+// digits 1.0e-7 on any). A layer of 24 tokens takes 109 us, of 2048 1714 (the fp32
+// kernel: 557 and 11693).
 static bool moe_wide_types(const redcuda_moe_desc &d) { return d.type_gu == RC_IQ3_S || d.type_down == RC_IQ3_S; }
 static bool moe_wide(const redcuda_moe *m);
 static uint32_t nib_fmt(const redcuda_moe *m, uint32_t type) { return type == RC_IQ3_S ? NIB_IQ3 : moe_wide(m) ? NIB_IQ2W : NIB_IQ2; }
@@ -354,8 +354,9 @@ static uint32_t moe_item_tokens(const redcuda_moe *m, bool single_token, uint32_
 // Which expert kernels serve a call of npairs pairs (all_local: every pair belongs to this shard; otherwise the share
 // expert_count / n_expert of them): the tcgen05 kernel works on items of up to 64 pairs of one expert and decodes an
 // expert's weights once per item, so it needs experts that see many pairs each (prefill chunks of 2048 tokens: 40 pairs
-// per expert). RC_MOE_TC_MIN = pairs per expert from which it is used (default 32; 0 = never). Measured on 2048-token
-// chunks: gate/up 0.86 ms against 1.00 ms for the mma.sync kernels with items of 8 pairs, down 0.45 against 0.41 ms.
+// per expert). RC_MOE_TC_MIN = pairs per expert from which it is used (default 32; 0 = never): its error against
+// 64-bit sums is 8.9e-7 where the integer kernels have 3.7e-7, so it takes over only where it gains much. A layer of 1400 tokens takes 965 us
+// on the integer kernels, one of 1700 990 on this.
 static void moe_choose_path(redcuda_moe *m, uint32_t npairs, bool all_local) {
     const char *v = getenv("RC_MOE_TC_MIN");
     const uint32_t min_avg = v ? (uint32_t)atoi(v) : 32u;
@@ -398,7 +399,7 @@ static int moe_shared_tc_gemm(redcuda_moe *m, uint32_t ntok, const float *x, con
 
 // x_quantised: xq_x / sx_x already hold the digits of x
 static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with_router, bool with_shared, bool x_quantised, cudaStream_t s,
-                        const int8_t *xq = nullptr, const float *sx = nullptr, const RouteTail *tail = nullptr) {
+                        const int8_t *xq = nullptr, const float *sx = nullptr, const RouteTail *tail = nullptr, const GemvNorm *norm = nullptr) {
     if (!xq) { xq = m->xq_x; sx = m->sx_x; }
     GemvArgs A{};
     A.ntok = ntok; A.x = x; A.x_stride = m->d.hidden; A.resident = 1u;
@@ -438,6 +439,7 @@ static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with
     A.njobs = j;
     A.tag = "moe_pre_gemv";
     if (tail) A.tail = *tail;
+    if (norm) A.norm = *norm;
     return launch_gemv(A, s);
 }
 
@@ -565,13 +567,15 @@ static bool moe_fused1_ok(const redcuda_moe *m) {
     return want && m->nib && m->d.type_sh == RC_Q6_K && m->d.n_expert <= 1024u && nib_tail_ok(m->d.top_k, m->d.hidden, m->d.ffn) &&
            m->d.ffn_sh == m->d.ffn;
 }
-static int moe_forward_fused1(redcuda_moe *m, const float *x, const float *logits_in, const float *resid, float *out, cudaStream_t s) {
+// norm (may be null): the token is RMSNorm(x [+ branch]) * w, which the first kernel computes and leaves in norm->normed (and norm->resid) for the others
+static int moe_forward_fused1(redcuda_moe *m, const float *x, const float *logits_in, const float *resid, float *out, cudaStream_t s, const GemvNorm *norm = nullptr) {
     const uint32_t k = m->d.top_k;
     RouteTail T{};
     T.ticket = m->ticket; T.logits = logits_in ? logits_in : m->logits; T.n_expert = m->d.n_expert; T.top_k = k; T.ids = m->ids; T.weights = m->wk;
     T.G = RouteGroup1{m->sorted, m->uexp, m->ustart, m->n_unique, m->item_u, m->item_p0, m->n_items, m->ids_mirror, m->work};
     T.status = status_words();
-    if (!moe_gemv_pre(m, 1u, x, logits_in == nullptr, true, false, s, nullptr, nullptr, &T)) return 0;
+    if (!moe_gemv_pre(m, 1u, x, logits_in == nullptr, true, false, s, nullptr, nullptr, &T, norm)) return 0;
+    if (norm) x = norm->normed;
     MmaArgs M{};
     M.w0 = m->gate; M.w1 = m->up; M.mat_bytes = m->gu_bytes; M.nb = m->gu_nb; M.nrows = m->d.ffn; M.ncols = m->d.hidden;
     M.expert_begin = m->d.expert_begin; M.n_local = m->d.expert_count; M.status = status_words();
@@ -637,6 +641,18 @@ static int moe_forward_on(redcuda_moe *m, uint32_t ntok, const float *x, const f
     return moe_combine(m, ntok, m->tmp, m->wk, k, true, resid, out, s);
 }
 
+namespace rc {
+// One token whose input is RMSNorm(x + N.branch) * N.w: 1 done, 0 failed, -1 this layer has no kernel that normalises its input (the
+// caller does it). resid: N.resid or another row.
+int moe_forward_norm1(redcuda_moe *m, const float *x, const GemvNorm &N, const float *resid, float *out, cudaStream_t s) {
+    if (!moe_fused1_ok(m) || m->router.type != RC_F32 || m->sh_gate_inp.type != RC_F32) return -1;
+    GemvArgs A{};
+    A.ntok = 1u; A.x = x; A.njobs = 1u; A.norm = N;
+    A.job[0].type = RC_F32; A.job[0].ncols = m->d.hidden;
+    if (!gemv1_norm_ok(A)) return -1;
+    return moe_forward_fused1(m, x, nullptr, resid, out, s, &N);
+}
+}
 // Carves the workspace of a layer out of B (m and B null: only the size is computed). Every piece is 256-byte aligned.
 static size_t moe_ws_layout(const redcuda_moe_desc &d, redcuda_moe *m, uint8_t *B) {
     const size_t T = d.max_tokens, P = T * d.top_k;
