@@ -53,24 +53,19 @@ __device__ __forceinline__ void gemv1_stage(const GemvArgs &A, uint32_t ncols, f
         for (uint32_t k = threadIdx.x * 4u; k < ncols; k += G1_WARPS * 128u) *reinterpret_cast<float4 *>(xs + g1_xi(k)) = *reinterpret_cast<const float4 *>(A.x + k);
         return;
     }
+    // the row waits in shared memory for its sum: the first weights hold the registers
     __shared__ double red[G1_WARPS];
-    constexpr uint32_t N = G1_NCOLS / (G1_WARPS * 128u);
-    float4 v[N], w[N];
     double ss = 0.0;
-#pragma unroll
-    for (uint32_t j = 0; j < N; ++j) {
-        const uint32_t k = threadIdx.x * 4u + j * G1_WARPS * 128u;
-        v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (k >= ncols) continue;
-        v[j] = *reinterpret_cast<const float4 *>(A.x + k);
-        w[j] = __ldg(reinterpret_cast<const float4 *>(A.norm.w + k));
+    for (uint32_t k = threadIdx.x * 4u; k < ncols; k += G1_WARPS * 128u) {
+        float4 v = *reinterpret_cast<const float4 *>(A.x + k);
         if (A.norm.branch) {
             const float4 b = *reinterpret_cast<const float4 *>(A.norm.branch + k);
-            v[j].x += b.x; v[j].y += b.y; v[j].z += b.z; v[j].w += b.w;
+            v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
         }
+        *reinterpret_cast<float4 *>(xs + g1_xi(k)) = v;
+        if (blockIdx.x == 0u && A.norm.resid) *reinterpret_cast<float4 *>(A.norm.resid + k) = v;
+        ss += (double)v.x * (double)v.x + (double)v.y * (double)v.y + (double)v.z * (double)v.z + (double)v.w * (double)v.w;
     }
-#pragma unroll
-    for (uint32_t j = 0; j < N; ++j) ss += (double)v[j].x * (double)v[j].x + (double)v[j].y * (double)v[j].y + (double)v[j].z * (double)v[j].z + (double)v[j].w * (double)v[j].w;
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = ss;
     __syncthreads();
@@ -78,17 +73,12 @@ __device__ __forceinline__ void gemv1_stage(const GemvArgs &A, uint32_t ncols, f
 #pragma unroll
     for (uint32_t i = 0; i < G1_WARPS; ++i) tot += red[i];
     const double inv = 1.0 / sqrt(tot / (double)ncols + (double)A.norm.eps);
-#pragma unroll
-    for (uint32_t j = 0; j < N; ++j) {
-        const uint32_t k = threadIdx.x * 4u + j * G1_WARPS * 128u;
-        if (k >= ncols) continue;
-        const float4 n = make_float4((float)((double)v[j].x * inv * (double)w[j].x), (float)((double)v[j].y * inv * (double)w[j].y),
-                                     (float)((double)v[j].z * inv * (double)w[j].z), (float)((double)v[j].w * inv * (double)w[j].w));
+    for (uint32_t k = threadIdx.x * 4u; k < ncols; k += G1_WARPS * 128u) {
+        const float4 v = *reinterpret_cast<const float4 *>(xs + g1_xi(k)), w = __ldg(reinterpret_cast<const float4 *>(A.norm.w + k));
+        const float4 n = make_float4((float)((double)v.x * inv * (double)w.x), (float)((double)v.y * inv * (double)w.y),
+                                     (float)((double)v.z * inv * (double)w.z), (float)((double)v.w * inv * (double)w.w));
         *reinterpret_cast<float4 *>(xs + g1_xi(k)) = n;
-        if (blockIdx.x == 0u) {
-            *reinterpret_cast<float4 *>(A.norm.normed + k) = n;
-            if (A.norm.resid) *reinterpret_cast<float4 *>(A.norm.resid + k) = v[j];
-        }
+        if (blockIdx.x == 0u) *reinterpret_cast<float4 *>(A.norm.normed + k) = n;
     }
 }
 
