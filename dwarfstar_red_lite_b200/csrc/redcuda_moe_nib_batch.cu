@@ -223,6 +223,16 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
         F.q[1][0][i] = nbb_ldg(b + lane_code + 512 * i); F.q[1][1][i] = nbb_ldg(b + lane_code + 1024 + 512 * i);
     };
     auto load_d = [&](const uint8_t *a, const uint8_t *b) { F.d[0] = nbb_ldg1(a + lane_d); F.d[1] = nbb_ldg1(b + lane_d); };
+    // A fragment is loaded half a step before its use, which a few warps on an SM cannot hide from HBM: where fewer than half of a block's
+    // warps get a piece, the piece's records, which lie together, are sent for in L2 at once. us a layer without and with: 2 tokens (5 pieces
+    // a block) 52.1 and 50.4, but 3 tokens (7) 48.5 and 49.7, 6 (13) 56.4 and 60.0.
+    auto send_for = [&](const Piece &P) {
+        if (lane == 0) {
+            const uint32_t bytes = P.steps * NIB_REC;
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(P.rec), "r"(GATEUP ? bytes : 2u * bytes) : "memory");
+            if (GATEUP) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(P.rec + to_up), "r"(bytes) : "memory");
+        }
+    };
     int zero[4];                     // opaque to the compiler: four registers that stay zero, the accumulator input of every MMA
     asm volatile("mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;" : "=r"(zero[0]), "=r"(zero[1]), "=r"(zero[2]), "=r"(zero[3]));
 
@@ -242,6 +252,7 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
             const uint8_t *a, *b;
             place(P, 0u, a, b);
             load_half(0, a, b); load_half(1, a, b); load_d(a, b);
+            if (2u * share < NBB_WARPS) send_for(P);
         }
         have = false;
         if (digits_of != seg) { if (!wait_for(full_s, seg)) break; digits_of = seg; }
