@@ -397,9 +397,11 @@ static int moe_shared_tc_gemm(redcuda_moe *m, uint32_t ntok, const float *x, con
     return launch_tc_gemm(A, tn, tag, s);
 }
 
-// x_quantised: xq_x / sx_x already hold the digits of x
+// x_quantised: xq_x / sx_x already hold the digits of x. norm (one token): x is normalised on the way; -1 with nothing launched where a
+// kernel would take part that reads x as it is
 static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with_router, bool with_shared, bool x_quantised, cudaStream_t s,
                         const int8_t *xq = nullptr, const float *sx = nullptr, const RouteTail *tail = nullptr, const GemvNorm *norm = nullptr) {
+    if (norm && (moe_router_tc(m, ntok) || moe_shared_tc(m, ntok))) return -1;
     if (!xq) { xq = m->xq_x; sx = m->sx_x; }
     GemvArgs A{};
     A.ntok = ntok; A.x = x; A.x_stride = m->d.hidden; A.resident = 1u;
@@ -574,7 +576,8 @@ static int moe_forward_fused1(redcuda_moe *m, const float *x, const float *logit
     T.ticket = m->ticket; T.logits = logits_in ? logits_in : m->logits; T.n_expert = m->d.n_expert; T.top_k = k; T.ids = m->ids; T.weights = m->wk;
     T.G = RouteGroup1{m->sorted, m->uexp, m->ustart, m->n_unique, m->item_u, m->item_p0, m->n_items, m->ids_mirror, m->work};
     T.status = status_words();
-    if (!moe_gemv_pre(m, 1u, x, logits_in == nullptr, true, false, s, nullptr, nullptr, &T, norm)) return 0;
+    const int pre = moe_gemv_pre(m, 1u, x, logits_in == nullptr, true, false, s, nullptr, nullptr, &T, norm);
+    if (pre != 1) return pre;
     if (norm) x = norm->normed;
     MmaArgs M{};
     M.w0 = m->gate; M.w1 = m->up; M.mat_bytes = m->gu_bytes; M.nb = m->gu_nb; M.nrows = m->d.ffn; M.ncols = m->d.hidden;
