@@ -401,7 +401,7 @@ static int moe_shared_tc_gemm(redcuda_moe *m, uint32_t ntok, const float *x, con
 // kernel would take part that reads x as it is
 static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with_router, bool with_shared, bool x_quantised, cudaStream_t s,
                         const int8_t *xq = nullptr, const float *sx = nullptr, const RouteTail *tail = nullptr, const GemvNorm *norm = nullptr) {
-    if (norm && (moe_router_tc(m, ntok) || moe_shared_tc(m, ntok))) return -1;
+    if (norm && moe_router_tc(m, ntok)) return -1;
     if (!xq) { xq = m->xq_x; sx = m->sx_x; }
     GemvArgs A{};
     A.ntok = ntok; A.x = x; A.x_stride = m->d.hidden; A.resident = 1u;
@@ -567,7 +567,7 @@ static int moe_combine(redcuda_moe *m, uint32_t ntok, const float *pair_out, con
 static bool moe_fused1_ok(const redcuda_moe *m) {
     static const bool want = !(getenv("RC_MOE_FUSE1") && atoi(getenv("RC_MOE_FUSE1")) == 0);     // A/B switch
     return want && m->nib && m->d.type_sh == RC_Q6_K && m->d.n_expert <= 1024u && nib_tail_ok(m->d.top_k, m->d.hidden, m->d.ffn) &&
-           m->d.ffn_sh == m->d.ffn;
+           m->d.ffn_sh == m->d.ffn && !moe_shared_tc(m, 1u);       // the third launch takes SiLU(gate) * up, which the tcgen05 form leaves to its down projection
 }
 // norm (may be null): the token is RMSNorm(x [+ branch]) * w, which the first kernel computes and leaves in norm->normed (and norm->resid) for the others
 static int moe_forward_fused1(redcuda_moe *m, const float *x, const float *logits_in, const float *resid, float *out, cudaStream_t s, const GemvNorm *norm = nullptr) {

@@ -1,5 +1,5 @@
-"""A decoding step with the opt-in router logits on the tcgen05 GEMM, from the first token on: that kernel reads the normalised row, which no
-kernel before it may be left out to make."""
+"""A decoding step with the router logits (opt-in) or the shared expert on the tcgen05 GEMM from the first token on: the first reads the
+normalised row, which no kernel before it may be left out to make; the second leaves SiLU(gate) * up to its down projection."""
 import numpy as np
 import pytest
 
@@ -9,7 +9,7 @@ from dwarfstar_red_lite_b200.engine import Engine
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("switch", ["RC_ROUTER_TC_MIN"])
+@pytest.mark.parametrize("switch", ["RC_ROUTER_TC_MIN", "RC_SH_TC_MIN"])
 def test_step_with_a_tensor_core_form_from_one_token(tmp_path, switch, monkeypatch):
     dims = synth.tiny_model_dims(n_layer=4, type_shared=synth.Q6_K)
     path = str(tmp_path / "tiny.gguf")
