@@ -19,6 +19,7 @@
 #include "redcuda_common.cuh"
 #include "redcuda_kernels.cuh"
 #include "redcuda_nib.cuh"
+#include "redcuda_q6k_panels.cuh"
 
 namespace rc {
 
@@ -39,10 +40,9 @@ struct Q6Args {
     uint32_t MS, KS, panel;                 // matrices and column splits per block (8 % (MS * KS) == 0), columns staged at a time
     uint32_t bits; float dw1;               // digit width and 2^bits
 };
-constexpr uint32_t Q6M_PANEL = 4096u;       // most columns staged at a time
-// bytes of a staged panel of pc columns: 16 rows of a matrix, 8 tokens
-__host__ __device__ constexpr uint32_t q6m_a_bytes(uint32_t pc) { return 16u * (pc / 2u + 16u + pc / 4u + 16u + pc / 16u + 16u); }
-__host__ __device__ constexpr uint32_t q6m_b_bytes(uint32_t pc) { return 24u * (pc + 16u); }
+// the steps of q6m_panels, as the kernel's lambdas
+template <class S, class W, class M> struct Q6Panels { S send; W arrived; M multiply; };
+template <class S, class W, class M> Q6Panels(S, W, M) -> Q6Panels<S, W, M>;
 
 __global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Args A) {
     pdl_prologue();
@@ -69,10 +69,8 @@ __global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Ar
     float out[4] = {0.f, 0.f, 0.f, 0.f};
     int z[4];
     asm volatile("mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;" : "=r"(z[0]), "=r"(z[1]), "=r"(z[2]), "=r"(z[3]));
-    bool ok = true;
-    uint32_t parity = 0u;
-    for (uint32_t blk0 = 0u; blk0 < bpr; blk0 += pcmax / 256u, parity ^= 1u) {
-        const uint32_t nblk = min(bpr - blk0, pcmax / 256u), pc = nblk * 256u;
+    auto send = [&](uint32_t blk0, uint32_t nblk) {
+        const uint32_t pc = nblk * 256u;
         __syncthreads();                     // the barrier is ready; the panel before this one has been read
         if (tid == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(MS * 16u * (pc / 2u + pc / 4u + pc / 16u) + ntok_b * 3u * pc) : "memory");
         __syncthreads();
@@ -98,9 +96,10 @@ __global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Ar
             const uint32_t m = i / (16u * nblk), j = i - m * 16u * nblk, r = j / nblk, c = j - r * nblk;
             s_d[m][r][c] = __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(A.w[m] + rc_q6_d(A.nb)) + (uint64_t)(row0 + r) * bpr + blk0 + c)));
         }
-        __syncthreads();                     // s_d
-        if (ok) ok = nb_wait(bar, parity);
-        if (!ok || tg * 8u >= A.ntok) continue;
+    };
+    auto arrived = [&](uint32_t parity) { return __syncthreads_and(nb_wait(bar, parity)) != 0; };      // its block barrier also publishes s_d
+    auto multiply = [&](uint32_t blk0, uint32_t nblk) {
+        if (tg * 8u >= A.ntok) return;
         const uint8_t *xb = b_base + (tgl * 8u + g) * 3u * b_pitch + 4u * t, *am = q6m_smem + mat * a_bytes;
         for (uint32_t u = max(u_begin, 2u * blk0); u < min(u_end, 2u * (blk0 + nblk)); ++u) {
             const uint32_t b = (u >> 1) - blk0, h = u & 1u;
@@ -144,16 +143,15 @@ __global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Ar
                     }
                 }
         }
-    }
+    };
+    Q6Panels steps{send, arrived, multiply};
+    const bool ok = q6m_panels(steps, bpr, pcmax / 256u);
     // accumulator columns 2t, 2t+1 of this lane are tokens tg*8 + 2t, +1
     const uint32_t tk0 = tg * 8u + 2u * t;
     const float s0 = tk0 < A.ntok ? A.sx[tk0] : 0.f, s1 = tk0 + 1u < A.ntok ? A.sx[tk0 + 1u] : 0.f;
     part[warp][g][2u * t] = out[0] * s0; part[warp][g][2u * t + 1u] = out[1] * s1;
     part[warp][g + 8u][2u * t] = out[2] * s0; part[warp][g + 8u][2u * t + 1u] = out[3] * s1;
-    if (!ok) {                               // a copy never came: the results are void; it is given as long again before the block may end
-        if (A.status) A.status[ST_TIMEOUT] = 1u;
-        nb_wait(bar, parity ^ 1u);
-    }
+    if (!ok && tid == 0 && A.status) A.status[ST_TIMEOUT] = 1u;      // a copy never came: the results are void
     __syncthreads();
     // epilogue: TGB token groups x 16 rows x 8 tokens
     for (uint32_t idx = tid; idx < TGB * 128u; idx += 256u) {
@@ -178,21 +176,13 @@ int launch_q6k_mma(const uint8_t *w0, const uint8_t *w1, uint64_t nb, uint32_t n
     A.w[0] = w0; A.w[1] = w1 ? w1 : w0; A.nb = nb; A.nrows = nrows; A.ncols = ncols; A.ntok = ntok; A.xq = xq; A.sx = sx;
     A.out = out; A.out_stride = out_stride; A.status = status_words();
     A.bits = act_digit_bits(); A.dw1 = (float)(1u << A.bits);
-    A.MS = w1 ? 2u : 1u;
-    const uint32_t nsteps = ncols / 16u, tgroups = (ntok + 7u) / 8u, tiles = nrows / 16u;
-    // column splits while the launch would leave SMs or warps idle and every split keeps 256 columns or more (whole runs of 128)
-    uint32_t KS = 1u;
-    while (A.MS * KS * 2u <= 8u && nsteps / (KS * 2u) >= 16u && nsteps % (KS * 16u) == 0 &&
-           ((uint64_t)tiles * ((tgroups + 8u / (A.MS * KS) - 1u) / (8u / (A.MS * KS))) < 148u * 2u || tgroups < 8u / (A.MS * KS))) KS <<= 1;
-    A.KS = KS;
-    const uint32_t TGB = 8u / (A.MS * KS), groups = TGB < tgroups ? TGB : tgroups;      // groups of tokens that a block really has
-    auto bytes = [&](uint32_t pc) { return (size_t)A.MS * q6m_a_bytes(pc) + (size_t)groups * q6m_b_bytes(pc); };
-    for (A.panel = ncols < Q6M_PANEL ? ncols : Q6M_PANEL; bytes(A.panel) > 216u * 1024u;) A.panel = (A.panel / 2u + 255u) / 256u * 256u;
-    const size_t smem = bytes(A.panel);
-    const dim3 grid(tiles, (tgroups + TGB - 1u) / TGB);
+    const Q6Plan P = q6m_plan(w1 != nullptr, nrows, ncols, ntok);
+    A.MS = P.MS; A.KS = P.KS; A.panel = P.panel;
+    const uint32_t tok_block = 8u * (8u / (P.MS * P.KS));
+    const dim3 grid(nrows / 16u, (ntok + tok_block - 1u) / tok_block);
     prof_begin(tag, s);
-    RC_CUDA(cudaFuncSetAttribute(k_q6k_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    RC_LAUNCH((k_q6k_mma), grid, 256, smem, s, A);
+    RC_CUDA(cudaFuncSetAttribute(k_q6k_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
+    RC_LAUNCH((k_q6k_mma), grid, 256, P.smem, s, A);
     prof_end(s);
     RC_LAUNCHED();
     return 1;
