@@ -413,8 +413,10 @@ __device__ __forceinline__ float4 ldg_now(const float *p) {
     return v;
 }
 constexpr uint32_t RL_ALL = 16u;      // steps of 16 columns of a warp's eighth of a row of 2048
+// (x is not __restrict__: a load that the compiler may take for one of constant memory could move ahead of the wait in the middle of the ALL
+// form, and the kernel before this one may write x. Without it the loads stay behind the wait's memory clobber.)
 template <uint32_t FT, uint32_t FE, bool ALL>
-__global__ void __launch_bounds__(256) k_router_logits(const float *__restrict__ w, const float *__restrict__ x, uint32_t x_stride, uint32_t ntok,
+__global__ void __launch_bounds__(256) k_router_logits(const float *__restrict__ w, const float *x, uint32_t x_stride, uint32_t ntok,
                                                        uint32_t n_expert, uint32_t ncols, float *__restrict__ logits) {
     if (ALL) asm volatile("griddepcontrol.launch_dependents;" ::); else pdl_prologue();
     __shared__ double red[8][FT * FE * 64u];
