@@ -398,6 +398,12 @@ __global__ void __launch_bounds__(256) k_vec_sigmoid(const float *__restrict__ w
     }
 }
 
+// a load that stays where it is written (one of the non-coherent path may be moved behind a wait)
+__device__ __forceinline__ float4 ldg_now(const float *p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 // Router logits of a batch: logits[t][e] = (float) sum_k (double) x[t][k] * (double) w[e][k], F32 weights
 // (rl_quant_row_dot on an F32 row accumulates in double, native/redlite_native_quant_cpu.c:198-212, and the top-k that
 // follows must not depend on a summation order), on the fp64 tensor-core instruction (mma.sync.m8n8k4.f64).
@@ -406,16 +412,10 @@ __global__ void __launch_bounds__(256) k_vec_sigmoid(const float *__restrict__ w
 // successive instructions are one float4 (k order within 16 columns is the same permutation for both operands, and a sum
 // does not depend on it), which costs no shared-memory staging, no barrier per K tile and one conversion per element. The
 // eight partial tiles meet in shared memory once, in a fixed order. Block = 8 FT tokens x 8 FE experts.
-// a load that stays where it is written
-__device__ __forceinline__ float4 ldg_now(const float *p) {
-    float4 v;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
-constexpr uint32_t RL_ALL = 16u;      // steps of 16 columns of a warp's eighth of a row of 2048
-// (x is not __restrict__: a load that the compiler may take for one of constant memory could move ahead of the wait in the middle of the ALL
-// form, and the kernel before this one may write x. Without it the loads stay behind the wait's memory clobber.)
-template <uint32_t FT, uint32_t FE, bool ALL>
+// (x is not __restrict__: a load that the compiler may take for one of constant memory could move ahead of the wait in the middle of the form
+// that requests its weights first, and the kernel before this one may write x. Without it the loads stay behind the wait's memory clobber.)
+// ALL: the steps of 16 columns of a warp's eighth of a row, whose weights it requests together; 0: by steps
+template <uint32_t FT, uint32_t FE, uint32_t ALL>
 __global__ void __launch_bounds__(256) k_router_logits(const float *__restrict__ w, const float *x, uint32_t x_stride, uint32_t ntok,
                                                        uint32_t n_expert, uint32_t ncols, float *__restrict__ logits) {
     if (ALL) asm volatile("griddepcontrol.launch_dependents;" ::); else pdl_prologue();
@@ -452,21 +452,22 @@ __global__ void __launch_bounds__(256) k_router_logits(const float *__restrict__
     };
     if constexpr (ALL) {
         // a small batch: the warp's whole share of the weights is requested at once, ahead of the wait for the kernel that writes x
-        float4 b[RL_ALL][FE];                // a step beyond the share repeats the last one of the row and is not multiplied
+        float4 b[ALL][FE];
 #pragma unroll
-        for (uint32_t c = 0; c < RL_ALL; ++c)
+        for (uint32_t c = 0; c < ALL; ++c)
 #pragma unroll
-            for (uint32_t i = 0; i < FE; ++i) b[c][i] = ldg_now(wp[i] + min(c0 + c, n16 - 1u) * 16u);
+            for (uint32_t i = 0; i < FE; ++i) b[c][i] = ldg_now(wp[i] + (c0 + c) * 16u);
         asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
-        for (uint32_t c4 = 0; c4 < RL_ALL; c4 += 4u) {
-            float4 a[4][FT];
+        for (uint32_t c4 = 0; c4 < ALL; c4 += 4u) {
+            constexpr uint32_t N = ALL < 4u ? ALL : 4u;
+            float4 a[N][FT];
 #pragma unroll
-            for (uint32_t c = 0; c < 4u; ++c)
+            for (uint32_t c = 0; c < N; ++c)
 #pragma unroll
-                for (uint32_t i = 0; i < FT; ++i) a[c][i] = *reinterpret_cast<const float4 *>(xp[i] + min(c0 + c4 + c, n16 - 1u) * 16u);
+                for (uint32_t i = 0; i < FT; ++i) a[c][i] = *reinterpret_cast<const float4 *>(xp[i] + (c0 + c4 + c) * 16u);
 #pragma unroll
-            for (uint32_t c = 0; c < 4u; ++c) if (c0 + c4 + c < c1) multiply(a[c], b[c4 + c]);
+            for (uint32_t c = 0; c < N; ++c) multiply(a[c], b[c4 + c]);
         }
     } else {
 #pragma unroll 4
@@ -500,12 +501,17 @@ int launch_router_logits(const float *w, const float *x, uint32_t x_stride, uint
     // the tile grows while the blocks still fill the chip about twice: a larger one converts and reads less per product
     auto blocks = [&](uint32_t tt, uint32_t te) { return (uint64_t)((ntok + tt - 1u) / tt) * ((n_expert + te - 1u) / te); };
     // up to two blocks per SM the loads of a warp's whole share go out together (ALL): HBM is waited for once instead of once per four steps
-    const bool all = ncols <= 128u * RL_ALL;
+    // for the row lengths that give every warp 2, 4, 8 or 16 steps (the ones that the expert layouts take); other rows go by steps.
+    // us a layer, 16 steps of every row of up to 2048 columns and these: 6 tokens 56.4 and 54.6, 24 110.2 and 105.9; hidden 1024, 2 tokens 43.7 and 41.7 (by
+    // steps 42.4); hidden 512, 2 tokens 39.2 and 37.9 (38.0). (16 predicated steps took 172 and 196 registers, one block an SM: 64 tokens 162.7 against 160.8.)
+    const uint32_t all = ncols == 256u || ncols == 512u || ncols == 1024u || ncols == 2048u ? ncols / 128u : 0u;
+#define RC_RL_ALL(FT, FE) switch (all) { case 2u: RC_RL(FT, FE, 2u); break; case 4u: RC_RL(FT, FE, 4u); break; case 8u: RC_RL(FT, FE, 8u); break; case 16u: RC_RL(FT, FE, 16u); break; default: RC_RL(FT, FE, 0u); }
 #define RC_RL(FT, FE, ALL) RC_LAUNCH((k_router_logits<FT, FE, ALL>), dim3((ntok + 8u * FT - 1u) / (8u * FT), (n_expert + 8u * FE - 1u) / (8u * FE)), 256, 0, stream, w, x, x_stride, ntok, n_expert, ncols, logits)
-    if (ntok <= 8u) { if (all) RC_RL(1u, 1u, true); else RC_RL(1u, 1u, false); }
-    else if (blocks(16u, 8u) <= 296u) { if (all) RC_RL(2u, 1u, true); else RC_RL(2u, 1u, false); }
-    else RC_RL(2u, 2u, false);
+    if (ntok <= 8u) { RC_RL_ALL(1u, 1u) }
+    else if (blocks(16u, 8u) <= 296u) { RC_RL_ALL(2u, 1u) }
+    else RC_RL(2u, 2u, 0u);
 #undef RC_RL
+#undef RC_RL_ALL
     prof_end(stream);
     RC_LAUNCHED();
     return 1;
