@@ -259,6 +259,7 @@ int launch_gemv(GemvArgs &A, cudaStream_t stream) {
         total_rows += A.job[j].nrows;
     }
     if (gemv1_ok(A)) return launch_gemv1(A, stream);
+    RC_REQUIRE(!A.norm.w, "gemv: only rows of F32 / F16 / Q6_K of a single token are normalised on the way");
     RC_REQUIRE(!A.tail.ticket, "gemv: the routing tail needs F32 / F16 / Q6_K rows of at most 8192 columns and a 16-byte aligned vector");
     uint32_t lpr = 32u;
     while (lpr > (ncols >> 6)) lpr >>= 1;

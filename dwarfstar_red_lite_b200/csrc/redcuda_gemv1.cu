@@ -257,6 +257,12 @@ bool gemv1_ok(const GemvArgs &A) {
 bool gemv1_norm_ok(const GemvArgs &A) {
     for (uint32_t j = 0; j < A.njobs; ++j) if (A.job[j].ncols != A.job[0].ncols || A.job[j].ncols % 4u) return false;
     auto al = [](const void *p) { return ((uintptr_t)p & 15u) == 0u; };
+    // one block writes normed and resid while the others still read x, branch and w
+    const uintptr_t bytes = (uintptr_t)A.job[0].ncols * sizeof(float);
+    auto apart = [&](const float *p, const float *q) { return !p || !q || (uintptr_t)p + bytes <= (uintptr_t)q || (uintptr_t)q + bytes <= (uintptr_t)p; };
+    for (const float *o : {A.norm.normed, A.norm.resid})
+        if (!apart(o, A.x) || !apart(o, A.norm.branch) || !apart(o, A.norm.w)) return false;
+    if (!apart(A.norm.normed, A.norm.resid)) return false;
     return gemv1_ok(A) && A.job[0].ncols <= G1_NCOLS && A.norm.normed && al(A.norm.w) && al(A.norm.branch) && al(A.norm.resid) && al(A.norm.normed);
 }
 

@@ -34,7 +34,7 @@ struct RouteTail {
 };
 
 // The input of a single-token GEMV as RMSNorm(x [+ branch]) * w, computed by every block for itself: normed and resid (may be null) are
-// written by one of them. w null: x as it is.
+// written by one of them, while others still read, so they overlap neither x, branch and w nor each other. w null: x as it is.
 struct GemvNorm { const float *w, *branch; float eps; float *resid, *normed; };
 #define RC_MAX_JOBS 6u
 struct GemvArgs {

@@ -397,8 +397,8 @@ static int moe_shared_tc_gemm(redcuda_moe *m, uint32_t ntok, const float *x, con
     return launch_tc_gemm(A, tn, tag, s);
 }
 
-// x_quantised: xq_x / sx_x already hold the digits of x. norm (one token): x is normalised on the way; -1 with nothing launched where a
-// kernel would take part that reads x as it is
+// x_quantised: xq_x / sx_x already hold the digits of x. norm (one token): x is normalised on the way; -1 with nothing launched where the
+// GEMV cannot do that, or a kernel would take part that reads x as it is
 static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with_router, bool with_shared, bool x_quantised, cudaStream_t s,
                         const int8_t *xq = nullptr, const float *sx = nullptr, const RouteTail *tail = nullptr, const GemvNorm *norm = nullptr) {
     if (norm && moe_router_tc(m, ntok)) return -1;
@@ -441,7 +441,7 @@ static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with
     A.njobs = j;
     A.tag = "moe_pre_gemv";
     if (tail) A.tail = *tail;
-    if (norm) A.norm = *norm;
+    if (norm) { A.norm = *norm; if (!gemv1_norm_ok(A)) return -1; }
     return launch_gemv(A, s);
 }
 
@@ -648,11 +648,7 @@ namespace rc {
 // One token whose input is RMSNorm(x + N.branch) * N.w: 1 done, 0 failed, -1 this layer has no kernel that normalises its input (the
 // caller does it). resid: N.resid or another row.
 int moe_forward_norm1(redcuda_moe *m, const float *x, const GemvNorm &N, const float *resid, float *out, cudaStream_t s) {
-    if (!moe_fused1_ok(m) || m->router.type != RC_F32 || m->sh_gate_inp.type != RC_F32) return -1;
-    GemvArgs A{};
-    A.ntok = 1u; A.x = x; A.njobs = 1u; A.norm = N;
-    A.job[0].type = RC_F32; A.job[0].ncols = m->d.hidden;
-    if (!gemv1_norm_ok(A)) return -1;
+    if (!moe_fused1_ok(m)) return -1;
     return moe_forward_fused1(m, x, nullptr, resid, out, s, &N);
 }
 }
