@@ -749,6 +749,7 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
     if (!require_books(d.type_gu) || !require_books(d.type_down) || !require_books(d.type_sh)) return nullptr;
 
     status_words();        // allocated here, never inside a stream capture
+    if (!q6k_mma_init()) return nullptr;
     redcuda_moe *m = new (std::nothrow) redcuda_moe();
     if (!m) return fail("out of host memory");
     m->d = d;

@@ -129,5 +129,6 @@ __device__ __forceinline__ void actw_planes(const uint32_t (&w)[4], uint32_t (&p
 // Q6_K matrix (or gate/up pair with SiLU*mul when w1 != nullptr) x ntok activation rows given as digits (redcuda_q6k_mma.cu)
 int launch_q6k_mma(const uint8_t *w0, const uint8_t *w1, uint64_t nb, uint32_t nrows, uint32_t ncols, uint32_t ntok,
                    const int8_t *xq, const float *sx, float *out, uint32_t out_stride, const char *tag, cudaStream_t s);
+int q6k_mma_init();      // before the first launch on a device
 
 }  // namespace rc

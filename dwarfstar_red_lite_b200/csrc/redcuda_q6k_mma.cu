@@ -167,6 +167,13 @@ __global__ void __launch_bounds__(256, 2) k_q6k_mma(const __grid_constant__ Q6Ar
     }
 }
 
+// Once per layer or engine, on its device: a launch may then take what shared memory it needs. (Asked for at every launch it cost the host
+// about half a microsecond, twice a layer, where the host's queueing is what a small batch waits for.)
+int q6k_mma_init() {
+    RC_CUDA(cudaFuncSetAttribute(k_q6k_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Q6M_SMEM));
+    return 1;
+}
+
 // out[t][r] = W0[r].x[t]   or   SiLU(W0[r].x[t]) * (W1[r].x[t]) for Q6_K matrices and activations already in digit form.
 int launch_q6k_mma(const uint8_t *w0, const uint8_t *w1, uint64_t nb, uint32_t nrows, uint32_t ncols, uint32_t ntok,
                    const int8_t *xq, const float *sx, float *out, uint32_t out_stride, const char *tag, cudaStream_t s) {
@@ -181,7 +188,6 @@ int launch_q6k_mma(const uint8_t *w0, const uint8_t *w1, uint64_t nb, uint32_t n
     const uint32_t tok_block = 8u * (8u / (P.MS * P.KS));
     const dim3 grid(nrows / 16u, (ntok + tok_block - 1u) / tok_block);
     prof_begin(tag, s);
-    RC_CUDA(cudaFuncSetAttribute(k_q6k_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
     RC_LAUNCH((k_q6k_mma), grid, 256, P.smem, s, A);
     prof_end(s);
     RC_LAUNCHED();

@@ -12,6 +12,7 @@
 namespace rc {
 
 constexpr uint32_t Q6M_PANEL = 4096u;       // most columns staged at a time
+constexpr uint32_t Q6M_SMEM = 216u * 1024u; // most shared memory of a block
 // bytes of a staged panel of pc columns: 16 rows of a matrix, 8 tokens
 Q6M_HD constexpr uint32_t q6m_a_bytes(uint32_t pc) { return 16u * (pc / 2u + 16u + pc / 4u + 16u + pc / 16u + 16u); }
 Q6M_HD constexpr uint32_t q6m_b_bytes(uint32_t pc) { return 24u * (pc + 16u); }
@@ -30,7 +31,7 @@ inline Q6Plan q6m_plan(bool pair, uint32_t nrows, uint32_t ncols, uint32_t ntok)
     const uint32_t TGB = 8u / (P.MS * KS);
     P.groups = TGB < tgroups ? TGB : tgroups;
     auto bytes = [&](uint32_t pc) { return (size_t)P.MS * q6m_a_bytes(pc) + (size_t)P.groups * q6m_b_bytes(pc); };
-    for (P.panel = ncols < Q6M_PANEL ? ncols : Q6M_PANEL; bytes(P.panel) > 216u * 1024u;) P.panel = (P.panel / 2u + 255u) / 256u * 256u;
+    for (P.panel = ncols < Q6M_PANEL ? ncols : Q6M_PANEL; bytes(P.panel) > Q6M_SMEM;) P.panel = (P.panel / 2u + 255u) / 256u * 256u;
     P.smem = bytes(P.panel);
     return P;
 }
