@@ -388,9 +388,12 @@ int launch_nib_batch(MmaArgs &A, uint32_t max_items, cudaStream_t s) {
     const uint64_t pieces = (uint64_t)max_items * ((pairs + tpp - 1u) / tpp);
     const uint32_t grid = (uint32_t)(pieces < (uint64_t)sm_count ? (pieces ? pieces : 1u) : (uint64_t)sm_count);
     prof_begin(gateup ? "moe_gateup" : "moe_down", s);
+    // Down is launched ahead of the end of the kernel before it, the short one that makes its digits, so that its blocks set themselves up beside that.
+    // us a layer, plainly and so: 2 tokens 50.6 and 48.4, 6 54.7 and 52.5, 24 105.3 and 103.3, 64 161.1 and 159.4, 300 308.2 and 306.6, 1400 957.9
+    // and 957.2. Gate/up, behind an event that another stream records, gains nothing by it: 2 50.6, 24 105.3, 64 161.4.
 #define RC_NBB_LAUNCH(GU, NC) do { \
         RC_CUDA(cudaFuncSetAttribute(k_nib_batch<FMT, GU, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nbb_smem(NC))); \
-        RC_LAUNCH((k_nib_batch<FMT, GU, NC>), grid, NBB_WARPS * 32u, nbb_smem(NC), s, A); } while (0)
+        RC_LAUNCH_PDL_IF(!GU, (k_nib_batch<FMT, GU, NC>), grid, NBB_WARPS * 32u, nbb_smem(NC), s, A); } while (0)
     auto launch = [&](auto fmt) -> int {
         constexpr uint32_t FMT = decltype(fmt)::value;
         if (gateup) {
