@@ -1,12 +1,13 @@
 """Batch form of the expert kernels, against the CPU oracle: items of every size from one pair to more than a full one, the row lengths
-the layout takes, runs that leave blocks without work and runs that cut an item, and the shared expert's batch kernel around its
-panels of 2048 columns. Bounds: operands are exact, activations are 24-bit fixed point per row and sums of up to 4096 products are
+the layout takes, runs that leave blocks without work and runs that cut an item, and the shared expert's batch kernel, with its
+columns staged at once and in several panels. Bounds: operands are exact, activations are 24-bit fixed point per row and sums of up to 4096 products are
 fp32, so a layer output is good to a few 1e-6 of its range; 2e-5 leaves room for the order of the sums."""
 import numpy as np
 import pytest
 
 import dwarfstar_red_lite_b200 as rc
 import oracle_lib as ol
+import q6k_panels_lib as qp
 from dwarfstar_red_lite_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -41,3 +42,12 @@ def test_row_lengths(hidden, ffn, ntok):
 @pytest.mark.parametrize("ntok", [3, 8, 9, 37])
 def test_shared_expert_panels(hidden, ffn_sh, ntok):
     _check(synth.MoeDims(hidden=hidden, n_expert=8, top_k=2, ffn=256, ffn_sh=ffn_sh), ntok, 900 + ntok, False)
+
+
+# hidden, ffn_sh, tokens, panels of gate/up and of down: the second panel whole and ragged, column splits without work in a panel
+@pytest.mark.parametrize("hidden,ffn_sh,ntok,panels", [(2048, 2048, 75, (2, 2)), (2048, 2048, 127, (2, 2)), (2048, 4096, 64, (2, 2)), (2048, 1536, 99, (2, 1)),
+                                                      (4352, 512, 8, (2, 1)), (5120, 512, 8, (2, 1)), (8192, 256, 9, (2, 1))])
+def test_shared_expert_in_several_panels(hidden, ffn_sh, ntok, panels):
+    cut = lambda pair, nrows, ncols: -(-ncols // qp.plan(pair, nrows, ncols, ntok)["panel"])  # noqa: E731
+    assert (cut(1, ffn_sh, hidden), cut(0, hidden, ffn_sh)) == panels
+    _check(synth.MoeDims(hidden=hidden, n_expert=8, top_k=2, ffn=256, ffn_sh=ffn_sh), ntok, 1000 + ntok, False)
