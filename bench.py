@@ -980,13 +980,13 @@ def main():
     # 66): `achieved` / `frac` are on the ALGORITHMIC bytes, `bytes_read_per_launch` is what the kernel really reads.
     nib = not os.environ.get("RC_EXPERT_FMT", "nib4").startswith("i")
     real = dom_bytes * (138.0 / 66.0) if (nib and key) else dom_bytes
-    # DRAM traffic per launch: ncu (dram__bytes_read + dram__bytes_write) of the nibble-layout kernels on a 2-layer
-    # capture: 231.2 MB read + 4.8 MB written by a gate/up launch whose expert records are 230.6 MB, 116.3 + 6.2 MB by a
+    # DRAM traffic per launch: ncu (dram__bytes_read + dram__bytes_write) of k_nib_batch on a 2-layer
+    # capture: 232.4 MB read + 4.5 MB written by a gate/up launch whose expert records are 230.6 MB, 116.4 + 4.1 MB by a
     # down launch of 115.3 MB; traffic grows with the distinct experts read, so it is scaled by the bytes read.
-    ncu_ratio = ({"moe_gateup": 236.0 / 230.6, "moe_down": 122.5 / 115.3} if nib else {"moe_gateup": 114.93 / 105.41, "moe_down": 51.39 / 52.4}).get(dom)
+    ncu_ratio = ({"moe_gateup": 236.9 / 230.6, "moe_down": 120.5 / 115.3} if nib else {"moe_gateup": 114.93 / 105.41, "moe_down": 51.39 / 52.4}).get(dom)
     roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                 "frac_of_nominal_8000": achieved / 8000.0, "traffic": real * ncu_ratio if ncu_ratio else None,
-                "traffic_source": ("ncu capture of a 2-layer run of the %s kernels, scaled by the bytes read" % ("nibble-layout" if nib else "planar-format")) if ncu_ratio else None,
+                "traffic_source": ("ncu capture of a 2-layer run of the %s kernels, scaled by the bytes read" % ("nibble-layout batch" if nib else "planar-format")) if ncu_ratio else None,
                 "expert_layout": "nib4 (138 B per 256 weights)" if nib else "iq2 (66 B per 256 weights)",
                 "bytes_read_per_launch": real, "read_GBps": real / (dom_ms * 1e-3) / 1e9, "read_frac": real / (dom_ms * 1e-3) / 1e9 / peak,
                 "bytes_per_launch": dom_bytes, "ms_per_launch": dom_ms,
