@@ -116,7 +116,7 @@ __device__ __forceinline__ uint32_t shard_local(uint32_t g, uint32_t begin, uint
     return i < count ? i : 0xffffffffu;
 }
 
-template <uint32_t GP_KEEP>
+constexpr uint32_t GP_KEEP = 20u;
 __global__ void __launch_bounds__(1024) k_group_pairs(const uint32_t *__restrict__ pair_expert, uint32_t npairs, uint32_t expert_begin, uint32_t expert_stride,
                                                       uint32_t skip_foreign, uint32_t expert_count, uint32_t item_tok, uint32_t *__restrict__ sorted, uint32_t *__restrict__ uexp,
                                                       uint32_t *__restrict__ ustart, uint32_t *__restrict__ n_unique, uint32_t *__restrict__ item_u,
@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(1024) k_group_pairs(const uint32_t *__restrict
     __syncthreads();
     // A thread's first GP_KEEP pairs stay in registers with the rank that the count gave them: their ids are requested
     // together (a load per step of the counting loop is a round trip each) and placing them needs no second round of atomics.
-    // Keeping 20 instead of 3 takes the kernel from 18.9 to 16.9 us at 10000 pairs and from 28 to 25 at 20480; up to 3072, which 3 hold, there
-    // is nothing to gain and the larger form costs a layer of 24 tokens 0.8 us (120.7 -> 121.5).
+    // Keeping 20 takes the kernel from 18.9 to 16.9 us at 10000 pairs and from 28 to 25 at 20480 against keeping 3; a layer of 6, 24 and 300 tokens takes as
+    // long with either (52.7, 104.2 and 308.1 us).
     uint32_t pe[GP_KEEP], pr[GP_KEEP];
 #pragma unroll
     for (uint32_t i = 0; i < GP_KEEP; ++i) { if (1024u * i >= npairs) break; pe[i] = tid + 1024u * i < npairs ? pair_expert[tid + 1024u * i] : 0u; }
@@ -327,7 +327,7 @@ struct redcuda_moe {
 // Layers with IQ3_S matrices take their activations as wide digits: they ran on fp32 activations before the nibble layout held them,
 // and the 24-bit form per row is less than that (relative error of an expert's output against 64-bit sums, hidden 2048: fp32 1.6e-7 on any
 // row; three digits 3.1e-7 on Gaussian rows, 2.2e-6 with one element of 100, 4.7e-4 with a large one where the weights vanish; wide
-// digits 1.0e-7 on any). A layer of 24 tokens takes 109 us, of 2048 1714 (the fp32
+// digits 1.0e-7 on any). A layer of 24 tokens takes 104 us, of 2048 1693 (the fp32
 // kernel: 557 and 11693).
 static bool moe_wide_types(const redcuda_moe_desc &d) { return d.type_gu == RC_IQ3_S || d.type_down == RC_IQ3_S; }
 static bool moe_wide(const redcuda_moe *m);
@@ -355,8 +355,8 @@ static uint32_t moe_item_tokens(const redcuda_moe *m, bool single_token, uint32_
 // expert_count / n_expert of them): the tcgen05 kernel works on items of up to 64 pairs of one expert and decodes an
 // expert's weights once per item, so it needs experts that see many pairs each (prefill chunks of 2048 tokens: 40 pairs
 // per expert). RC_MOE_TC_MIN = pairs per expert from which it is used (default 32; 0 = never): its error against
-// 64-bit sums is 8.9e-7 where the integer kernels have 3.7e-7, so it takes over only where it gains much. A layer of 1400 tokens takes 965 us
-// on the integer kernels, one of 1700 990 on this.
+// 64-bit sums is 8.9e-7 where the integer kernels have 3.7e-7, so it takes over only where it gains much. A layer of 1400 tokens takes 944 to 957 us
+// on the integer kernels, one of 1700 991 on this.
 static void moe_choose_path(redcuda_moe *m, uint32_t npairs, bool all_local) {
     const char *v = getenv("RC_MOE_TC_MIN");
     const uint32_t min_avg = v ? (uint32_t)atoi(v) : 32u;
@@ -541,9 +541,7 @@ static int moe_group(redcuda_moe *m, const uint32_t *pair_expert, uint32_t npair
     if (distinct && npairs <= 64u && !skip_foreign) {
         RC_LAUNCH((k_group_trivial), 1, 64, 0, s, pair_expert, npairs, m->sorted, m->uexp, m->ustart, m->n_unique, m->item_u, m->item_p0, m->n_items, m->work);
     } else {
-#define RC_GROUP(KEEP) RC_LAUNCH_PDL_IF(npairs <= MOE_PDL_PAIRS, (k_group_pairs<KEEP>), 1, 1024, 0, s, pair_expert, npairs, m->d.expert_begin, m->d.expert_stride, skip_foreign ? 1u : 0u, m->d.expert_count, moe_item_tokens(m, false, npairs), m->sorted, m->uexp, m->ustart, m->n_unique, m->item_u, m->item_p0, m->n_items, m->bad, m->work, m->wait)
-        if (npairs <= 3072u) RC_GROUP(3u); else RC_GROUP(20u);
-#undef RC_GROUP
+        RC_LAUNCH_PDL_IF(npairs <= MOE_PDL_PAIRS, (k_group_pairs), 1, 1024, 0, s, pair_expert, npairs, m->d.expert_begin, m->d.expert_stride, skip_foreign ? 1u : 0u, m->d.expert_count, moe_item_tokens(m, false, npairs), m->sorted, m->uexp, m->ustart, m->n_unique, m->item_u, m->item_p0, m->n_items, m->bad, m->work, m->wait);
     }
     prof_end(s);
     RC_LAUNCHED();
