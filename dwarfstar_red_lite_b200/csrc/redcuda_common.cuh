@@ -81,8 +81,9 @@ inline cudaError_t launch_kernel(int file_default, uint32_t cluster_x, K kernel,
 #endif
 
 // The small kernels between the expert kernels (grouping, combine) are launched ahead of their predecessor's end up to this
-// many (token, expert) pairs. us a layer, plain -> early: 20 pairs 56.4 -> 54.4, 60 67.9 -> 66.7, 160 98.1 -> 96.1, 240 119.8 -> 118.7, 640 195.3 ->
-// 194.3, 3000 379.7 -> 379.3, 10000 894 -> 893: the two microseconds are 2 % and more of a layer up to here and lost in the expert kernels beyond.
+// many (token, expert) pairs. us a layer, plain -> early: 20 pairs 48.1 -> 48.1, 60 54.2 -> 52.4, 160 86.9 -> 84.3, 240 104.1 -> 101.3, 640 159.3 ->
+// 165.8, 1500 241.4 -> 237.7, 3000 308.1 -> 307.6, 10000 712.6 -> 711.7: two microseconds and more up to here; somewhere beyond 240 pairs it costs 4 %,
+// later it is lost in the expert kernels.
 constexpr uint32_t MOE_PDL_PAIRS = 160u;
 
 struct DevMem {

@@ -8,7 +8,7 @@
 // (prmt against an 8-byte table held in two registers). IQ3_S experts take the same layout (NIB_IQ3): their magnitudes are the
 // odd numbers 1 .. 15, so a signed weight is 2 n + 1 with n in -8 .. 7 and the code is n itself in two's complement; as the
 // high nibble of a byte with 8 below it, it IS the int8 operand 8 (2 n + 1) - one mask-and-or per 4 weights, and the block
-// scale d / 8 serves both formats. A layer of IQ3_S experts took 549 us for 24 tokens on the CUDA-core kernel, 109 here.
+// scale d / 8 serves both formats. A layer of IQ3_S experts took 549 us for 24 tokens on the CUDA-core kernel, 104 here.
 // Dequantised values are unchanged bit for bit
 // (redcuda_nib_dequant_rows against rl_quant_dequant_row, native/redlite_native_quant_cpu.c:166-191). The price is bytes:
 // 138 per 256 weights instead of 66 (IQ3_S: 110), i.e. 2.09x (1.25x) the HBM footprint and traffic of the routed experts.
@@ -26,8 +26,7 @@
 // Layers with IQ3_S matrices take the wide form of the digits (actw_scale in redcuda_moe_mma.cuh): four per value and a scale per
 // 256-column block, applied with d / 8. On the CUDA-core kernel they had fp32 rows; relative errors of an expert's output against
 // 64-bit sums (hidden 2048, ffn 512, rows from Gaussian to one element of 10000): fp32 rows 1.3e-7 to 2.1e-7, wide digits 0.8e-7
-// to 1.2e-7. The fourth digit costs nothing where items hold one or two pairs, which fill one tile either way (24 tokens: 118 us a
-// layer with four, 120 with three).
+// to 1.2e-7. The fourth digit costs nothing where items hold one or two pairs, which fill one tile either way.
 //
 // Here: the re-coding and the two kernels of a single token (k_nib_one for gate/up, k_nib_down_tail); batches are in
 // redcuda_moe_nib_batch.cu. Every warp streams its 16-row tiles through a private ring of records (one cp.async.bulk and one mbarrier
@@ -472,7 +471,7 @@ int launch_nib_down_tail(NibTailArgs &A, cudaStream_t s) {
     const size_t smem = (size_t)A.top_k * bpr * NIB_REC + (size_t)A.top_k * (A.fmt == NIB_IQ2 ? 3u : 4u) * bpitch + bpitch + (size_t)x_padded(A.ncols) * 4u + 16u;
     const uint32_t threads = (A.top_k + 2u) * 32u, grid = A.nrows / 16u;
     // launched plainly: ahead of time its blocks would gather on the SMs that the 80 gate / up blocks of a top-10 layer leave free
-    // (28.9 against 26.7 us a layer)
+    // (28.9 against 26.7 us a layer, measured when it took that long; 24.5 now)
     prof_begin("moe_down_tail", s);
 #define RC_TAIL_LAUNCH(NC) do { \
         RC_CUDA(cudaFuncSetAttribute(k_nib_down_tail<FMT, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \

@@ -26,7 +26,7 @@
 
 namespace rc {
 
-constexpr uint32_t NBB_WARPS = 12u;               // 168 registers: two records' sums and results for a full item, and a step's fragments
+constexpr uint32_t NBB_WARPS = 12u;               // 168 registers: two records' sums and results for a full item, and a step's fragments; ten of the 24 forms spill 8 to 24 bytes
 constexpr uint32_t NBB_COLS = 24u;                // digit columns of an item
 // tile pairs of a piece: enough that drawing it is small beside it, few enough that a small batch still reaches every warp
 __host__ __device__ constexpr uint32_t nbb_pairs(uint32_t ncols) { return ncols >= 1024u ? 1u : ncols == 512u ? 2u : 4u; }
@@ -225,7 +225,8 @@ __global__ void __launch_bounds__(NBB_WARPS * 32u, 1) k_nib_batch(const __grid_c
     auto load_d = [&](const uint8_t *a, const uint8_t *b) { F.d[0] = nbb_ldg1(a + lane_d); F.d[1] = nbb_ldg1(b + lane_d); };
     // A fragment is loaded half a step before its use, which a few warps on an SM cannot hide from HBM: where fewer than half of a block's
     // warps get a piece, the piece's records, which lie together, are sent for in L2 at once. us a layer without and with: 2 tokens (5 pieces
-    // a block) 52.1 and 50.4, but 3 tokens (7) 48.5 and 49.7, 6 (13) 56.4 and 60.0.
+    // a block) 49.6 and 48.1, but 3 tokens (7) 44.2 and 45.3, 6 (13) 52.3 and 56.1. (Sent for by the warp that fills the buffer, before the others know of
+    // the part, they take the first loads' place: 2 tokens 51.0 against 50.5.)
     auto send_for = [&](const Piece &P) {
         if (lane == 0) {
             const uint32_t bytes = P.steps * NIB_REC;

@@ -23,7 +23,9 @@ inline Q6Plan q6m_plan(bool pair, uint32_t nrows, uint32_t ncols, uint32_t ntok)
     Q6Plan P{};
     P.MS = pair ? 2u : 1u;
     const uint32_t nsteps = ncols / 16u, tgroups = (ntok + 7u) / 8u, tiles = nrows / 16u;
-    // column splits while the launch would leave SMs or warps idle and every split keeps 256 columns or more (whole runs of 128)
+    // Column splits while the launch would leave SMs or warps idle and every split keeps 256 columns or more (whole runs of 128). Warps idle
+    // where there are fewer groups of tokens than warps, as in a prompt of 3 to 7 tokens, even if the blocks fill the chip: a projection of 8192 rows
+    // is split by eight there. The order of a row's fp32 sums follows from the split.
     uint32_t KS = 1u;
     while (P.MS * KS * 2u <= 8u && nsteps / (KS * 2u) >= 16u && nsteps % (KS * 16u) == 0 &&
            ((uint64_t)tiles * ((tgroups + 8u / (P.MS * KS) - 1u) / (8u / (P.MS * KS))) < 148u * 2u || tgroups < 8u / (P.MS * KS))) KS <<= 1;
