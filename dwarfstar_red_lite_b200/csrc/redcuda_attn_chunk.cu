@@ -51,9 +51,9 @@ __device__ __forceinline__ void ac_split2(float a, float b, uint32_t &hi, uint32
 
 // KV = __half: K/V tiles are copied as they are (one digit). KV = float: split into hi / lo tiles on the way in.
 template <typename KV, int HD, int G>
-__global__ void __launch_bounds__(AC_THREADS, 1) k_attn_chunk(const float *__restrict__ query, const KV *__restrict__ kcache, const KV *__restrict__ vcache,
-                                                               uint32_t n_kv, const uint32_t *__restrict__ pos_p, uint32_t ntok, float scale,
-                                                               const float *__restrict__ gate, float *__restrict__ gated) {
+__global__ void __launch_bounds__(AC_THREADS, 1) k_attn_chunk(const float *query, const KV *kcache, const KV *vcache,
+                                                               uint32_t n_kv, const uint32_t *pos_p, uint32_t ntok, float scale,
+                                                               const float *gate, float *__restrict__ gated) {
     pdl_prologue();
     constexpr bool HALF = sizeof(KV) == 2;
     constexpr uint32_t PITCH = HD * 2u, CH = HD / 8u;                 // bytes and 16-byte chunks per row of a tile

@@ -50,6 +50,9 @@ bool books_iq3s_odd();       // every magnitude of the IQ3_S codebook is one of 
 // next kernel's blocks are scheduled (and run their prologue up to pdl_prologue's wait) while the previous kernel drains.
 // Every kernel calls pdl_prologue() first: it lets its own dependents start launching once all of its blocks have begun,
 // then waits until the kernels before it have completed and their writes are visible. RC_PDL=0 launches plainly.
+// What a kernel before it may have written is no const __restrict__ argument: that lets the compiler load it by the non-coherent path, which
+// is for memory that nobody writes while the kernel runs (it has begun before its predecessor's end), and such loads are moved across the
+// wait. Weights that were in place before are.
 // Programmatic dependent launch: RC_PDL=0 never, RC_PDL=1 every kernel, unset = per source file (RC_PDL_DEFAULT:
 // on for the short latency-bound kernels, off for the expert kernels, where early-resident blocks measured slower).
 int pdl_mode();
@@ -61,14 +64,14 @@ __device__ __forceinline__ void pdl_prologue() {
     asm volatile("griddepcontrol.launch_dependents;" ::);
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-// cluster_x: blocks along x that form a thread-block cluster (1: none)
+// cluster_x: blocks along x that form a thread-block cluster (1: none); file_default: 1 early, 0 not, -1 never
 template <typename K, typename... Args>
 inline cudaError_t launch_kernel(int file_default, uint32_t cluster_x, K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = (pdl_mode() < 0 ? file_default : pdl_mode()) ? 1 : 0;
+    at[0].val.programmaticStreamSerializationAllowed = file_default < 0 ? 0 : (pdl_mode() < 0 ? file_default : pdl_mode()) ? 1 : 0;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = cluster_x; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = cluster_x > 1u ? 2 : 1;
@@ -77,6 +80,7 @@ inline cudaError_t launch_kernel(int file_default, uint32_t cluster_x, K kernel,
 #define RC_LAUNCH(kernel, grid, block, smem, stream, ...) rc::launch_kernel(RC_PDL_DEFAULT, 1u, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)
 #define RC_LAUNCH_PDL(kernel, grid, block, smem, stream, ...) rc::launch_kernel(1, 1u, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)      // whatever the file's default
 #define RC_LAUNCH_PDL_IF(cond, kernel, grid, block, smem, stream, ...) rc::launch_kernel((cond) ? 1 : RC_PDL_DEFAULT, 1u, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)
+#define RC_LAUNCH_BEHIND_IF(cond, kernel, grid, block, smem, stream, ...) rc::launch_kernel((cond) ? -1 : RC_PDL_DEFAULT, 1u, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)      // never early where cond holds
 #define RC_LAUNCH_CLUSTER(cluster_x, kernel, grid, block, smem, stream, ...) rc::launch_kernel(RC_PDL_DEFAULT, cluster_x, kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)
 #endif
 

@@ -120,7 +120,7 @@ const uint32_t *books_iq3s() { int dev = 0; cudaGetDevice(&dev); return g_iq3s_p
 bool books_iq3s_odd() { int dev = 0; cudaGetDevice(&dev); return g_iq3s_odd[dev & 63]; }
 
 // ---- raw GGUF blocks -> planar ----
-__global__ void k_repack(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, uint32_t type, uint64_t nb, uint32_t units_per_block) {
+__global__ void k_repack(const uint8_t *src, uint8_t *__restrict__ dst, uint32_t type, uint64_t nb, uint32_t units_per_block) {
     pdl_prologue();
     // one thread per 2-byte unit of the raw matrix (every field of the three formats starts on an even offset)
     const uint64_t total = nb * units_per_block;
@@ -162,7 +162,7 @@ int upload_matrix(uint32_t type, uint32_t nrows, uint32_t ncols, const void *src
 }
 
 // ---- dequantisation: one thread per group of 8 values ----
-__global__ void k_dequant(const uint8_t *__restrict__ base, uint32_t type, uint64_t nb, const uint8_t *iq2, const uint32_t *iq3s, float *__restrict__ out) {
+__global__ void k_dequant(const uint8_t *base, uint32_t type, uint64_t nb, const uint8_t *iq2, const uint32_t *iq3s, float *__restrict__ out) {
     pdl_prologue();
     const RcBooks bk{iq2, iq3s};
     const uint64_t total = nb * 32u;
@@ -281,10 +281,10 @@ int launch_gemv(GemvArgs &A, cudaStream_t stream) {
     prof_begin(A.tag ? A.tag : "gemv", stream);
     if (nt == 1) {
         if (smem > 48u * 1024u) RC_CUDA(cudaFuncSetAttribute(k_gemv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        RC_LAUNCH((k_gemv<1>), tiles, 256, smem, stream, A);
+        RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv<1>), tiles, 256, smem, stream, A);
     } else {
         if (smem > 48u * 1024u) RC_CUDA(cudaFuncSetAttribute(k_gemv<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        RC_LAUNCH((k_gemv<4>), tiles, 256, smem, stream, A);
+        RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv<4>), tiles, 256, smem, stream, A);
     }
     prof_end(stream);
     RC_LAUNCHED();
@@ -292,7 +292,7 @@ int launch_gemv(GemvArgs &A, cudaStream_t stream) {
 }
 
 // ---- router: softmax + top-k, one block per token (router_exec.c:102-184 semantics, ties -> lower id) ----
-__global__ void __launch_bounds__(256) k_route(const float *__restrict__ logits, uint32_t n_expert, uint32_t top_k,
+__global__ void __launch_bounds__(256) k_route(const float *logits, uint32_t n_expert, uint32_t top_k,
                                                uint32_t *__restrict__ ids, float *__restrict__ weights, float *__restrict__ probs_out,
                                                uint32_t *__restrict__ status) {
     pdl_prologue();
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(256) k_route(const float *__restrict__ logits,
 // Warp-per-token variant for n_expert <= 1024: the probabilities of a token live in the warp's registers (32 per lane
 // at most), every selection round is an integer maximum over them and two warp reductions (redcuda_route.cuh) — no block
 // barriers. Same arithmetic and tie rule as k_route, and as there a non-finite softmax selects id 0 in every round.
-__global__ void __launch_bounds__(256) k_route_warp(const float *__restrict__ logits, uint32_t ntok, uint32_t n_expert, uint32_t top_k,
+__global__ void __launch_bounds__(256) k_route_warp(const float *logits, uint32_t ntok, uint32_t n_expert, uint32_t top_k,
                                                     uint32_t *__restrict__ ids, float *__restrict__ weights, float *__restrict__ probs_out,
                                                     RouteGroup1 G, uint32_t *__restrict__ status) {
     pdl_prologue();
@@ -378,7 +378,7 @@ int launch_route(const float *logits_dev, uint32_t ntok, uint32_t n_expert, uint
 }
 
 // out[t] = sigmoid(w . x[t]) for one F32 row w (the shared-expert gate), fp64 accumulation; one block per token.
-__global__ void __launch_bounds__(256) k_vec_sigmoid(const float *__restrict__ w, const float *__restrict__ x, uint32_t x_stride, uint32_t ncols,
+__global__ void __launch_bounds__(256) k_vec_sigmoid(const float *__restrict__ w, const float *x, uint32_t x_stride, uint32_t ncols,
                                                      float *__restrict__ out) {
     pdl_prologue();
     __shared__ double red[8];
@@ -413,8 +413,6 @@ __device__ __forceinline__ float4 ldg_now(const float *p) {
 // successive instructions are one float4 (k order within 16 columns is the same permutation for both operands, and a sum
 // does not depend on it), which costs no shared-memory staging, no barrier per K tile and one conversion per element. The
 // eight partial tiles meet in shared memory once, in a fixed order. Block = 8 FT tokens x 8 FE experts.
-// (x is not __restrict__: a load that the compiler may take for one of constant memory could move ahead of the wait in the middle of the form
-// that requests its weights first, and the kernel before this one may write x. Without it the loads stay behind the wait's memory clobber.)
 // ALL: the steps of 16 columns of a warp's eighth of a row, whose weights it requests together; 0: by steps
 template <uint32_t FT, uint32_t FE, uint32_t ALL>
 __global__ void __launch_bounds__(256) k_router_logits(const float *__restrict__ w, const float *x, uint32_t x_stride, uint32_t ntok,

@@ -25,7 +25,7 @@ __device__ __forceinline__ double softplus_stable(double x) { if (x > 20.0) retu
 
 // grid.x = 2*groups (q/k heads) + d_inner/S (v runs) + 1 (beta/gate); grid.y = batch; block = S threads
 __global__ void k_dn_prep(DnDims D, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,
-                          const float *__restrict__ qkv, const float *__restrict__ ba, float *__restrict__ conv_state,
+                          const float *qkv, const float *ba, float *__restrict__ conv_state,
                           float *__restrict__ qk, float *__restrict__ v, float *__restrict__ beta, float *__restrict__ gate) {
     pdl_prologue();
     __shared__ double red[32];
@@ -65,8 +65,8 @@ __global__ void k_dn_prep(DnDims D, const float *__restrict__ conv_kernel, const
 
 // one warp per (seq, value head, state row); VPL = S / 32 values per lane, element i = lane + 32 * v
 template <int VPL>
-__global__ void __launch_bounds__(256) k_dn_state(DnDims D, uint32_t batch, const float *__restrict__ qk, const float *__restrict__ v,
-                                                  const float *__restrict__ beta, const float *__restrict__ gate,
+__global__ void __launch_bounds__(256) k_dn_state(DnDims D, uint32_t batch, const float *qk, const float *v,
+                                                  const float *beta, const float *gate,
                                                   float *__restrict__ state, float *__restrict__ core) {
     pdl_prologue();
     const uint32_t lane = threadIdx.x & 31u;
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256) k_dn_state(DnDims D, uint32_t batch, cons
 }
 
 // grid (rank, batch), block S threads
-__global__ void k_dn_tail(DnDims D, const float *__restrict__ core, const float *__restrict__ z, const float *__restrict__ norm_w, float *__restrict__ out) {
+__global__ void k_dn_tail(DnDims D, const float *core, const float *z, const float *__restrict__ norm_w, float *__restrict__ out) {
     pdl_prologue();
     __shared__ double red[32];
     const uint32_t h = blockIdx.x, seq = blockIdx.y, i = threadIdx.x, S = D.S;
@@ -124,8 +124,8 @@ __global__ void k_dn_tail(DnDims D, const float *__restrict__ core, const float 
 // DC: conv taps known at compile time (0: D.d_conv); MINB: blocks per SM that the registers allow
 template <int VPL, uint32_t DC, uint32_t SPLIT, int MINB, uint32_t RING>
 __global__ void __launch_bounds__(256, MINB) k_dn_step(DnDims D, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,
-                                                    const float *__restrict__ qkv, const float *__restrict__ ba, float *conv_state, float *__restrict__ state,
-                                                    const float *__restrict__ z, const float *__restrict__ norm_w, float *__restrict__ out) {
+                                                    const float *qkv, const float *ba, float *conv_state, float *__restrict__ state,
+                                                    const float *z, const float *__restrict__ norm_w, float *__restrict__ out) {
     pdl_prologue();
     constexpr uint32_t S = VPL * 32u, SB = S / SPLIT, RPW = SB / 8u, TAPS = DC ? DC : 1u;        // SB: state rows of this block
     __shared__ float s_q[S], s_k[S], s_v[SB], s_core[SB], s_beta, s_gate;
@@ -166,9 +166,13 @@ __global__ void __launch_bounds__(256, MINB) k_dn_step(DnDims D, const float *__
     };
     auto roll = [&](uint32_t c) {
         float *cs = cs_base + (size_t)c * ns;
+        const float newest = x_base[c];
         for (uint32_t j = 0; j + 1u < ns; ++j) cs[j] = cs[j + 1u];
-        cs[ns - 1u] = x_base[c];
+        cs[ns - 1u] = newest;
     };
+    // used at the end: on its way with the rest
+    const size_t idx = (size_t)seq * D.d_inner + (size_t)h * S + part * SB + tid;
+    const float g = tid < SB ? z[idx] : 0.f;
     const float y = has_qk ? conv_silu(c_qk, wq, kq) : 0.f;
     __syncwarp();
     if (SPLIT > 1u || width > 1u) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // this block has read the key head's windows
@@ -216,10 +220,9 @@ __global__ void __launch_bounds__(256, MINB) k_dn_step(DnDims D, const float *__
     }
     __syncthreads();
     // gated RMSNorm over the head (the arithmetic of k_dn_tail)
-    const size_t idx = (size_t)seq * D.d_inner + (size_t)h * S + part * SB + tid;
-    float x = 0.f, g = 0.f;
+    float x = 0.f;
     ss = 0.0;
-    if (tid < SB) { x = s_core[tid]; g = z[idx]; ss = (double)x * (double)x; }
+    if (tid < SB) { x = s_core[tid]; ss = (double)x * (double)x; }
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if (SPLIT == 1u) {
         if (lane == 0) red2[warp] = ss;
@@ -259,7 +262,7 @@ __global__ void __launch_bounds__(256, MINB) k_dn_step(DnDims D, const float *__
 // scheduling: 133,000 blocks of 128 threads for a 2048-token chunk)
 constexpr uint32_t DN_PREP_TOK = 8u;
 __global__ void k_dn_prep_seq(DnDims D, uint32_t T, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,
-                              const float *__restrict__ qkv, const float *__restrict__ ba, const float *__restrict__ conv_state,
+                              const float *qkv, const float *ba, const float *conv_state,
                               float *__restrict__ qk, float *__restrict__ v, float *__restrict__ beta, float *__restrict__ gate) {
     pdl_prologue();
     __shared__ double red[2][32];
@@ -303,7 +306,7 @@ __global__ void k_dn_prep_seq(DnDims D, uint32_t T, const float *__restrict__ co
 }
 
 // conv state <- the last d_conv-1 samples of [state, chunk]; one thread per channel
-__global__ void k_dn_conv_roll(DnDims D, uint32_t T, const float *__restrict__ qkv, float *__restrict__ conv_state) {
+__global__ void k_dn_conv_roll(DnDims D, uint32_t T, const float *qkv, float *__restrict__ conv_state) {
     pdl_prologue();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, ns = D.d_conv - 1u;
     if (c >= D.channels) return;
@@ -319,8 +322,8 @@ __global__ void k_dn_conv_roll(DnDims D, uint32_t T, const float *__restrict__ q
 // of the one being applied (a warp that fetched them itself waited for L2 on every token of its sequential chain).
 constexpr uint32_t DN_TB = 8u;          // tokens per staged block
 template <int VPL>
-__global__ void __launch_bounds__(256) k_dn_state_seq(DnDims D, uint32_t T, const float *__restrict__ qk, const float *__restrict__ v,
-                                                      const float *__restrict__ beta, const float *__restrict__ gate,
+__global__ void __launch_bounds__(256) k_dn_state_seq(DnDims D, uint32_t T, const float *qk, const float *v,
+                                                      const float *beta, const float *gate,
                                                       float *__restrict__ state, float *__restrict__ core) {
     pdl_prologue();
     constexpr uint32_t S = VPL * 32u;
@@ -423,8 +426,8 @@ __global__ void __launch_bounds__(256) k_dn_state_seq(DnDims D, uint32_t T, cons
 // token, a token's q and the next token's k before the exchange that the chain waits for, and the eight output sums are
 // reduced together after the block. RC_DN_SCAN=warp selects k_dn_state_seq for comparison.
 template <uint32_t S, uint32_t CPT, uint32_t RPT, uint32_t WARPS>
-__global__ void __launch_bounds__(WARPS * 32u) k_dn_scan(DnDims D, uint32_t T, const float *__restrict__ qk, const float *__restrict__ v,
-                                                         const float *__restrict__ beta, const float *__restrict__ gate,
+__global__ void __launch_bounds__(WARPS * 32u) k_dn_scan(DnDims D, uint32_t T, const float *qk, const float *v,
+                                                         const float *beta, const float *gate,
                                                          float *__restrict__ state, float *__restrict__ core) {
     pdl_prologue();
     constexpr uint32_t LPR = S / CPT, RPW = 32u / LPR, RB = RPW * RPT * WARPS, NP = CPT / 4u, NT = WARPS * 32u, V4 = S / 4u;
@@ -633,7 +636,7 @@ __global__ void __launch_bounds__(WARPS * 32u) k_dn_scan(DnDims D, uint32_t T, c
 // the token-by-token kernel (a chain of about 1100 cycles per token and row).
 // k_dn_pairdots  the 16 scalars of a group per key head: k_s . k_t (s < t) and k_s . q_t (s <= t); grid (groups of 4, key heads)
 constexpr uint32_t DN_MC = 4u;
-__global__ void __launch_bounds__(32) k_dn_pairdots(DnDims D, uint32_t T, const float *__restrict__ qk, float *__restrict__ pd) {
+__global__ void __launch_bounds__(32) k_dn_pairdots(DnDims D, uint32_t T, const float *qk, float *__restrict__ pd) {
     pdl_prologue();
     const uint32_t c = blockIdx.x, kh = blockIdx.y, lane = threadIdx.x, S = D.S;
     const size_t tok_qk = (size_t)2u * D.groups * S;
@@ -666,8 +669,8 @@ __global__ void __launch_bounds__(32) k_dn_pairdots(DnDims D, uint32_t T, const 
 // Block and staging as k_dn_state_seq (8 warps = 8 rows of one head, eight tokens staged at a time); T4 = the tokens that
 // form whole groups of four (the caller runs the rest through k_dn_state_seq).
 template <int VPL>
-__global__ void __launch_bounds__(256) k_dn_state_seq4(DnDims D, uint32_t T4, const float *__restrict__ qk, const float *__restrict__ v,
-                                                       const float *__restrict__ beta, const float *__restrict__ gate, const float *__restrict__ pd,
+__global__ void __launch_bounds__(256) k_dn_state_seq4(DnDims D, uint32_t T4, const float *qk, const float *v,
+                                                       const float *beta, const float *gate, const float *pd,
                                                        float *__restrict__ state, float *__restrict__ core) {
     pdl_prologue();
     constexpr uint32_t S = VPL * 32u;

@@ -36,7 +36,7 @@ static double now_ms() { return std::chrono::duration<double, std::milli>(std::c
 
 // ---- small kernels ----
 // out[b] = dequantised embedding row of token[b] (grid = tokens, block = 256 threads)
-__global__ void k_embed_row(const uint8_t *__restrict__ base, uint32_t type, uint64_t nb, uint32_t ncols, uint32_t nrows, const uint32_t *__restrict__ token,
+__global__ void k_embed_row(const uint8_t *__restrict__ base, uint32_t type, uint64_t nb, uint32_t ncols, uint32_t nrows, const uint32_t *token,
                             const uint8_t *iq2, const uint32_t *iq3s, float *__restrict__ out, uint32_t *__restrict__ status) {
     pdl_prologue();
     uint64_t row = token[blockIdx.x];
@@ -72,7 +72,7 @@ __device__ __forceinline__ double block_sum_d(double v, double *red) {
 // normed = RMSNorm(x [+ branch]) * w (engine_cpu.c:96-101, 418-424); resid_out (optional) = x + branch. One block of THREADS per token: 1024 where the token is
 // alone, its row is the chain; 256 for the rows of a chunk, where the barriers of one block are hidden by the others of its SM.
 template <uint32_t THREADS>
-__global__ void __launch_bounds__(THREADS) k_rmsnorm(const float *__restrict__ x, const float *__restrict__ branch, const float *__restrict__ w,
+__global__ void __launch_bounds__(THREADS) k_rmsnorm(const float *x, const float *branch, const float *__restrict__ w,
                                                   uint32_t n, float eps, float *__restrict__ resid_out, float *__restrict__ normed) {
     pdl_prologue();
     __shared__ double red[32];
@@ -123,9 +123,9 @@ __device__ __forceinline__ float from_kv(__half v) { return __half2float(v); }
 // Per-head RMSNorm of q and k, NeoX RoPE on the first rope_dims, K/V rows appended to the cache (engine_cpu.c:277-296).
 // grid = (n_head + 2 * n_kv, tokens) blocks of head_dim threads; token z sits at position pos_p[z].
 template <typename KV>
-__global__ void k_attn_prep(const float *__restrict__ qg, const float *__restrict__ kraw, const float *__restrict__ vraw,
+__global__ void k_attn_prep(const float *qg, const float *kraw, const float *vraw,
                             const float *__restrict__ qn, const float *__restrict__ kn, uint32_t n_head, uint32_t n_kv, uint32_t hd,
-                            uint32_t rope_dims, float freq_base, float eps, const uint32_t *__restrict__ pos_p, float *__restrict__ query, float *__restrict__ gate,
+                            uint32_t rope_dims, float freq_base, float eps, const uint32_t *pos_p, float *__restrict__ query, float *__restrict__ gate,
                             KV *__restrict__ kcache, KV *__restrict__ vcache) {
     pdl_prologue();
     extern __shared__ float sh[];
@@ -187,8 +187,8 @@ struct KvRaw {
 // K/V head over a slice of positions (K and V rows are read once for all G heads); a warp takes every 8th position,
 // a lane VPL = head_dim/32 consecutive dimensions; online softmax per head. Partials: m, l and the accumulator.
 template <typename KV, int VPL, int G>
-__global__ void __launch_bounds__(256) k_attn_decode(const float *__restrict__ query, const KV *__restrict__ kcache, const KV *__restrict__ vcache,
-                                                     uint32_t n_kv, const uint32_t *__restrict__ pos_p, uint32_t nsplit, float scale,
+__global__ void __launch_bounds__(256) k_attn_decode(const float *query, const KV *kcache, const KV *vcache,
+                                                     uint32_t n_kv, const uint32_t *pos_p, uint32_t nsplit, float scale,
                                                      float *__restrict__ part_m, float *__restrict__ part_l, float *__restrict__ part_acc) {
     pdl_prologue();
     extern __shared__ float sm[];            // [8][G][hd] accumulators, then [8][G] m, [8][G] l
@@ -262,8 +262,8 @@ __global__ void __launch_bounds__(256) k_attn_decode(const float *__restrict__ q
 }
 
 // merge the split partials, normalise, apply the sigmoid output gate (engine_cpu.c:312-317). grid = (n_head, tokens), block = hd
-__global__ void k_attn_merge(const float *__restrict__ part_m, const float *__restrict__ part_l, const float *__restrict__ part_acc,
-                             const float *__restrict__ gate, uint32_t nsplit, uint32_t hd, float *__restrict__ gated) {
+__global__ void k_attn_merge(const float *part_m, const float *part_l, const float *part_acc,
+                             const float *gate, uint32_t nsplit, uint32_t hd, float *__restrict__ gated) {
     pdl_prologue();
     const uint32_t h = blockIdx.x, d = threadIdx.x;
     const size_t zoff = (size_t)blockIdx.y * gridDim.x;
@@ -298,7 +298,7 @@ __global__ void k_advance(uint32_t *pos) {
     pdl_prologue(); if (threadIdx.x == 0 && blockIdx.x == 0) *pos += 1u; }
 
 // gen_log / gen_count (optional): the chosen id is also appended to gen_log[*gen_count]
-__global__ void __launch_bounds__(1024) k_argmax(const float *__restrict__ v, uint32_t n, uint32_t *__restrict__ out, uint32_t *__restrict__ gen_log,
+__global__ void __launch_bounds__(1024) k_argmax(const float *v, uint32_t n, uint32_t *__restrict__ out, uint32_t *__restrict__ gen_log,
                                                  uint32_t *__restrict__ gen_count, uint32_t *__restrict__ status) {
     pdl_prologue();
     __shared__ float bv[32];

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256) k_ep_push(const __grid_constant__ EpPushA
 }
 
 // out[t] = (resid[t] +) shared[t] + sum over ranks r of slot[r][t], once every rank's combine has delivered. grid = (hidden / 1024, tokens)
-__global__ void __launch_bounds__(256) k_ep_reduce(const float *__restrict__ slots, const float *__restrict__ shared, const float *__restrict__ resid, uint32_t world, uint32_t tokens,
+__global__ void __launch_bounds__(256) k_ep_reduce(const float *slots, const float *shared, const float *resid, uint32_t world, uint32_t tokens,
                                                    uint32_t hidden, const EpWait wait, float *__restrict__ out) {
     pdl_prologue();
     ep_wait_all(wait);
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(256) k_ep_reduce(const float *__restrict__ slo
 }
 
 // io[i] += resid[i], n4 float4s (the residual of the NCCL and single-rank paths, whose sums end in the caller's buffer)
-__global__ void __launch_bounds__(256) k_ep_add_resid(float4 *__restrict__ io, const float4 *__restrict__ resid, uint32_t n4) {
+__global__ void __launch_bounds__(256) k_ep_add_resid(float4 *__restrict__ io, const float4 *resid, uint32_t n4) {
     pdl_prologue();
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i >= n4) return;

@@ -294,8 +294,9 @@ int launch_gemv1(GemvArgs &A, cudaStream_t stream) {
     A.part_doubles = (uint32_t)(smem / sizeof(double));
     if (q6 || A.norm.w) smem += (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + 16u;
     prof_begin(A.tag ? A.tag : "gemv", stream);
-    if (A.norm.w) RC_LAUNCH((k_gemv1<true>), tiles, G1_WARPS * 32u, smem, stream, A);
-    else RC_LAUNCH((k_gemv1<false>), tiles, G1_WARPS * 32u, smem, stream, A);
+    // weights that a kernel before this one has just laid out are read by the non-coherent path like others: then behind that kernel's end
+    if (A.norm.w) RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1<true>), tiles, G1_WARPS * 32u, smem, stream, A);
+    else RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1<false>), tiles, G1_WARPS * 32u, smem, stream, A);
     prof_end(stream);
     RC_LAUNCHED();
     return 1;

@@ -117,7 +117,7 @@ __device__ __forceinline__ uint32_t shard_local(uint32_t g, uint32_t begin, uint
 }
 
 constexpr uint32_t GP_KEEP = 20u;
-__global__ void __launch_bounds__(1024) k_group_pairs(const uint32_t *__restrict__ pair_expert, uint32_t npairs, uint32_t expert_begin, uint32_t expert_stride,
+__global__ void __launch_bounds__(1024) k_group_pairs(const uint32_t *pair_expert, uint32_t npairs, uint32_t expert_begin, uint32_t expert_stride,
                                                       uint32_t skip_foreign, uint32_t expert_count, uint32_t item_tok, uint32_t *__restrict__ sorted, uint32_t *__restrict__ uexp,
                                                       uint32_t *__restrict__ ustart, uint32_t *__restrict__ n_unique, uint32_t *__restrict__ item_u,
                                                       uint32_t *__restrict__ item_p0, uint32_t *__restrict__ n_items, uint32_t *__restrict__ bad, uint32_t *__restrict__ work, const EpWait wait) {
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(1024) k_group_pairs(const uint32_t *__restrict
 }
 
 // Single-token case: the k selected experts are distinct, so every pair is its own group and its own work item.
-__global__ void k_group_trivial(const uint32_t *__restrict__ pair_expert, uint32_t npairs, uint32_t *__restrict__ sorted,
+__global__ void k_group_trivial(const uint32_t *pair_expert, uint32_t npairs, uint32_t *__restrict__ sorted,
                                 uint32_t *__restrict__ uexp, uint32_t *__restrict__ ustart, uint32_t *__restrict__ n_unique,
                                 uint32_t *__restrict__ item_u, uint32_t *__restrict__ item_p0, uint32_t *__restrict__ n_items, uint32_t *__restrict__ work) {
     pdl_prologue();
@@ -197,10 +197,10 @@ __global__ void k_group_trivial(const uint32_t *__restrict__ pair_expert, uint32
 }
 
 // out[t] = resid[t] + (sum_k w[t][k] * pair_out[t*k + kk] + shared[t] * scalar[t]); k may be 0 (shared part only).
-__global__ void __launch_bounds__(256) k_moe_combine(const float *__restrict__ pair_out, const float *__restrict__ w, uint32_t top_k,
-                                                     const float *__restrict__ shared, const float *__restrict__ scalar,
-                                                     const float *__restrict__ resid, float *__restrict__ out, uint32_t hidden,
-                                                     const uint32_t *__restrict__ pair_row) {
+__global__ void __launch_bounds__(256) k_moe_combine(const float *pair_out, const float *w, uint32_t top_k,
+                                                     const float *shared, const float *scalar,
+                                                     const float *resid, float *__restrict__ out, uint32_t hidden,
+                                                     const uint32_t *pair_row) {
     pdl_prologue();
     const uint32_t t = blockIdx.y;
     const uint32_t r = (blockIdx.x * 256u + threadIdx.x) * 4u;
@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(256) k_moe_combine(const float *__restrict__ p
 // out[t] = sum over the pairs of token t whose expert THIS shard holds of w * pair_out[t * top_k + k], plus add[t - add_begin]
 // for the add_count tokens from add_begin on (the rank's own tokens: their shared-expert part rides along in the
 // reduce-scatter). A token without local pairs gets zeros (or its add row).
-__global__ void __launch_bounds__(256) k_ep_combine(const float *__restrict__ pair_out, const uint32_t *__restrict__ ids, const float *__restrict__ w, uint32_t top_k,
-                                                    uint32_t begin, uint32_t stride, uint32_t count, const float *__restrict__ add, uint32_t add_begin, uint32_t add_count,
+__global__ void __launch_bounds__(256) k_ep_combine(const float *pair_out, const uint32_t *ids, const float *w, uint32_t top_k,
+                                                    uint32_t begin, uint32_t stride, uint32_t count, const float *add, uint32_t add_begin, uint32_t add_count,
                                                     float *__restrict__ out, uint32_t hidden) {
     pdl_prologue();
     const uint32_t t = blockIdx.y;
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(256) k_ep_combine(const float *__restrict__ pa
 
 // The same sum delivered through peer memory: token t's row is stored into the slot its owner keeps for this rank
 // (NVLink stores; zeros when no local expert served the token, so that the owner can add all slots), then the flag.
-__global__ void __launch_bounds__(256) k_ep_combine_push(const float *__restrict__ pair_out, const uint32_t *__restrict__ ids, const float *__restrict__ w, uint32_t top_k,
+__global__ void __launch_bounds__(256) k_ep_combine_push(const float *pair_out, const uint32_t *ids, const float *w, uint32_t top_k,
                                                          uint32_t begin, uint32_t stride, uint32_t count, const __grid_constant__ EpPush P, uint32_t hidden) {
     pdl_prologue();
     const uint32_t t = blockIdx.y;
@@ -902,7 +902,7 @@ int redcuda_moe_experts_device(redcuda_moe *m, uint32_t npairs, const float *pai
 
 // Contiguous copies of the pairs' expert ids and of their router weights, the weight zeroed when the expert lives on
 // another shard (ids / w rows are meta_stride elements apart)
-__global__ void k_mask_weights(const uint32_t *__restrict__ ids, const float *__restrict__ w, uint32_t ntok, uint32_t top_k, uint32_t meta_stride,
+__global__ void k_mask_weights(const uint32_t *ids, const float *w, uint32_t ntok, uint32_t top_k, uint32_t meta_stride,
                                uint32_t begin, uint32_t stride, uint32_t count, uint32_t *__restrict__ ids_out, float *__restrict__ w_local) {
     pdl_prologue();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;

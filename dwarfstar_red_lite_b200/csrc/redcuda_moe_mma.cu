@@ -74,7 +74,7 @@ uint32_t act_digit_bits() {
 
 // ---- activation rows -> three balanced digit planes of `bits` bits + one fp32 scale per row ----
 // grid = rows, block = 256. xq[row][3][ncols] (digit 0 = least significant), sx[row]. Digits lie in [-2^(bits-1), 2^(bits-1)).
-__global__ void __launch_bounds__(256) k_quant_act(const float *__restrict__ x, uint32_t x_stride, uint32_t ncols,
+__global__ void __launch_bounds__(256) k_quant_act(const float *x, uint32_t x_stride, uint32_t ncols,
                                                    int8_t *__restrict__ xq, float *__restrict__ sx, uint32_t bits) {
     pdl_prologue();
     __shared__ uint32_t red[8];
@@ -119,7 +119,7 @@ int launch_quant_act(const float *x, uint32_t x_stride, uint32_t rows, uint32_t 
 }
 
 // The wide form: one warp per row and 256-column block, 8 values a lane. xq[row][4][ncols], sx[row][ncols / 256]
-__global__ void __launch_bounds__(256) k_quant_act_wide(const float *__restrict__ x, uint32_t x_stride, uint32_t nblocks, uint32_t bpr,
+__global__ void __launch_bounds__(256) k_quant_act_wide(const float *x, uint32_t x_stride, uint32_t nblocks, uint32_t bpr,
                                                         int8_t *__restrict__ xq, float *__restrict__ sx) {
     pdl_prologue();
     const uint32_t i = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;

@@ -55,7 +55,7 @@ bool nib_shape_ok(uint32_t nrows, uint32_t ncols) { return nrows % 16u == 0 && (
 // another in memory are repacked as one (their row counts are multiples of 16): a layer's 512 experts take one launch per
 // projection, where a planar repack and a recoding per matrix took 1024 ----
 template <uint32_t FMT>
-__global__ void k_nib_repack(const uint8_t *__restrict__ raw, uint64_t nb, uint32_t bpr, const RcBooks bk, uint8_t *__restrict__ dst) {
+__global__ void k_nib_repack(const uint8_t *raw, uint64_t nb, uint32_t bpr, const RcBooks bk, uint8_t *__restrict__ dst) {
     pdl_prologue();
     const uint64_t total = nb * 32u;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -112,7 +112,7 @@ int launch_nib_repack(uint32_t fmt, const uint8_t *raw, uint64_t nrows, uint32_t
 }
 
 // ---- nibble layout -> fp32, the float operations of rl_quant_dequant_row in the same order (exact) ----
-__global__ void k_nib_dequant(const uint8_t *__restrict__ nib, uint64_t nb, uint32_t nrows, uint32_t bpr, float *__restrict__ out) {
+__global__ void k_nib_dequant(const uint8_t *nib, uint64_t nb, uint32_t nrows, uint32_t bpr, float *__restrict__ out) {
     pdl_prologue();
     const uint64_t total = nb * 32u;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {

@@ -62,7 +62,7 @@ __device__ __forceinline__ uint4 tcx_decode8(uint32_t word, uint32_t sc) {
 // the memory is what bounds it, and a block per row (two passes, 64 of 256 threads busy in the second) took 58 us where
 // 20480 rows of 512 move 126 MB. grid = rows / 8, block = 256; ncols a multiple of 256, at most 256 NCH
 template <uint32_t NCH>
-__global__ void __launch_bounds__(256) k_tc_prep_rows(const float *__restrict__ a, const float *__restrict__ b, uint32_t stride, uint32_t nrows, uint32_t ncols,
+__global__ void __launch_bounds__(256) k_tc_prep_rows(const float *a, const float *b, uint32_t stride, uint32_t nrows, uint32_t ncols,
                                                       __half *__restrict__ xd, float *__restrict__ x_inv) {
     pdl_prologue();
     const uint32_t r = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;

@@ -180,7 +180,7 @@ __device__ __forceinline__ void tc_decode_stage_f32(const float *w, uint32_t nco
 // x [ntok][ncols] fp32 (or SiLU(x) * x2 when x2 is given) -> fp16 digits in the order the GEMM stages consume them:
 // xs[token tile][k stage][k chunk of 8 (8)][digit hi/lo][token group of 8 (TN/8)][token in group (8)][8 halves];
 // x_inv[t] = 2^-e_t undoes the per-token scale. Tokens beyond ntok are zero. grid = token tiles * TN, block = 256
-__global__ void k_tc_prep_x(const float *__restrict__ x, const float *__restrict__ x2, uint32_t x_stride, uint32_t ntok, uint32_t ncols, uint32_t tn,
+__global__ void k_tc_prep_x(const float *x, const float *x2, uint32_t x_stride, uint32_t ntok, uint32_t ncols, uint32_t tn,
                             __half *__restrict__ xs, float *__restrict__ x_inv) {
     pdl_prologue();
     __shared__ float red[8];
