@@ -70,16 +70,26 @@ __global__ void __launch_bounds__(AC_THREADS, 1) k_attn_chunk(const float *query
     const uint32_t n_head = n_kv * G, tok0 = qb * TPB;
 
     // ---- Q rows of the block -> two fp16 digit tiles; row r = (token tok0 + r / G, head kvh * G + r % G)
-    for (uint32_t i = tid; i < AC_ROWS * CH; i += AC_THREADS) {
-        const uint32_t r = i / CH, c = i - r * CH, z = tok0 + r / G, h = kvh * G + r % G;
-        uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
-        if (z < ntok) {
+    // (four pieces requested together, as are eight gate pairs at the end: the launches of a prompt of 3501 tokens 2787 -> 2605 us)
+    static_assert(AC_ROWS * CH % (4u * AC_THREADS) == 0u, "pieces of a thread");
+    for (uint32_t i0 = tid; i0 < AC_ROWS * CH; i0 += 4u * AC_THREADS) {
+        float4 a[4], b[4];
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+            const uint32_t i = i0 + q * AC_THREADS, r = i / CH, c = i - r * CH, z = tok0 + r / G, h = kvh * G + r % G;
+            a[q] = b[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (z >= ntok) continue;
             const float4 *src = reinterpret_cast<const float4 *>(query + ((size_t)z * n_head + h) * HD + c * 8u);
-            const float4 a = src[0], b = src[1];
-            ac_split2(a.x, a.y, hi.x, lo.x); ac_split2(a.z, a.w, hi.y, lo.y); ac_split2(b.x, b.y, hi.z, lo.z); ac_split2(b.z, b.w, hi.w, lo.w);
+            a[q] = src[0]; b[q] = src[1];
         }
-        *reinterpret_cast<uint4 *>(q_hi + ac_off(r, c, PITCH)) = hi;
-        *reinterpret_cast<uint4 *>(q_lo + ac_off(r, c, PITCH)) = lo;
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+            const uint32_t i = i0 + q * AC_THREADS, r = i / CH, c = i - r * CH;
+            uint4 hi, lo;
+            ac_split2(a[q].x, a[q].y, hi.x, lo.x); ac_split2(a[q].z, a[q].w, hi.y, lo.y); ac_split2(b[q].x, b[q].y, hi.z, lo.z); ac_split2(b[q].z, b[q].w, hi.w, lo.w);
+            *reinterpret_cast<uint4 *>(q_hi + ac_off(r, c, PITCH)) = hi;
+            *reinterpret_cast<uint4 *>(q_lo + ac_off(r, c, PITCH)) = lo;
+        }
     }
     if (tid < AC_ROWS) { const uint32_t z = tok0 + tid / G; s_lim[tid] = z < ntok ? pos_p[z] : 0u; }
     const uint32_t z_last = min(tok0 + TPB, ntok) - 1u;
@@ -216,13 +226,17 @@ __global__ void __launch_bounds__(AC_THREADS, 1) k_attn_chunk(const float *query
         const size_t base = ((size_t)z * n_head + h) * HD;
         const double L = (double)l_run[half];
 #pragma unroll
-        for (uint32_t n = 0; n < NT_O; ++n) {
-            const uint32_t d = n * 8u + 2u * (lane & 3u);
-            const float2 g = *reinterpret_cast<const float2 *>(gate + base + d);
-            const double a0 = (double)o_acc[n][half * 2] / L, a1 = (double)o_acc[n][half * 2 + 1] / L;
-            float2 o;
-            o.x = (float)(a0 / (1.0 + exp(-(double)g.x))); o.y = (float)(a1 / (1.0 + exp(-(double)g.y)));
-            *reinterpret_cast<float2 *>(gated + base + d) = o;
+        for (uint32_t n0 = 0; n0 < NT_O; n0 += 8u) {
+            float2 g[8];                          // eight requested together
+#pragma unroll
+            for (uint32_t n = 0; n < 8u; ++n) g[n] = *reinterpret_cast<const float2 *>(gate + base + (n0 + n) * 8u + 2u * (lane & 3u));
+#pragma unroll
+            for (uint32_t n = 0; n < 8u; ++n) {
+                const double a0 = (double)o_acc[n0 + n][half * 2] / L, a1 = (double)o_acc[n0 + n][half * 2 + 1] / L;
+                float2 o;
+                o.x = (float)(a0 / (1.0 + exp(-(double)g[n].x))); o.y = (float)(a1 / (1.0 + exp(-(double)g[n].y)));
+                *reinterpret_cast<float2 *>(gated + base + (n0 + n) * 8u + 2u * (lane & 3u)) = o;
+            }
         }
     }
 }

@@ -55,7 +55,7 @@ bool nib_shape_ok(uint32_t nrows, uint32_t ncols) { return nrows % 16u == 0 && (
 // another in memory are repacked as one (their row counts are multiples of 16): a layer's 512 experts take one launch per
 // projection, where a planar repack and a recoding per matrix took 1024 ----
 template <uint32_t FMT>
-__global__ void k_nib_repack(const uint8_t *raw, uint64_t nb, uint32_t bpr, const RcBooks bk, uint8_t *__restrict__ dst) {
+__global__ void k_nib_repack(const uint8_t *__restrict__ raw, uint64_t nb, uint32_t bpr, const RcBooks bk, uint8_t *__restrict__ dst) {
     pdl_prologue();
     const uint64_t total = nb * 32u;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -104,8 +104,9 @@ int launch_nib_repack(uint32_t fmt, const uint8_t *raw, uint64_t nrows, uint32_t
     const uint32_t grid = (uint32_t)((total + 255u) / 256u < 148u * 16u ? (total + 255u) / 256u : 148u * 16u);
     prof_begin("nib_repack", s);
     const RcBooks bk{books_iq2(), books_iq3s()};
-    if (fmt != NIB_IQ3) RC_LAUNCH((k_nib_repack<NIB_IQ2>), grid ? grid : 1u, 256, 0, s, raw, nb, ncols / 256u, bk, dst);
-    else RC_LAUNCH((k_nib_repack<NIB_IQ3>), grid ? grid : 1u, 256, 0, s, raw, nb, ncols / 256u, bk, dst);
+    // never early: its reads are non-coherent (452 us for a matrix of 512 experts against 462 by the other path)
+    if (fmt != NIB_IQ3) RC_LAUNCH_BEHIND_IF(true, (k_nib_repack<NIB_IQ2>), grid ? grid : 1u, 256, 0, s, raw, nb, ncols / 256u, bk, dst);
+    else RC_LAUNCH_BEHIND_IF(true, (k_nib_repack<NIB_IQ3>), grid ? grid : 1u, 256, 0, s, raw, nb, ncols / 256u, bk, dst);
     prof_end(s);
     RC_LAUNCHED();
     return 1;

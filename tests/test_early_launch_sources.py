@@ -8,7 +8,8 @@ import re
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "dwarfstar_red_lite_b200", "csrc")
 RESIDENT = {"k_router_logits": {"w"}, "k_vec_sigmoid": {"w"}, "k_rmsnorm": {"w"}, "k_attn_prep": {"qn", "kn"}, "k_embed_row": {"base"}, "k_dn_prep": {"conv_kernel", "dt_bias", "ssm_a"},
-            "k_dn_tail": {"norm_w"}, "k_dn_step": {"conv_kernel", "dt_bias", "ssm_a", "norm_w"}, "k_dn_prep_seq": {"conv_kernel", "dt_bias", "ssm_a"}}
+            "k_dn_tail": {"norm_w"}, "k_dn_step": {"conv_kernel", "dt_bias", "ssm_a", "norm_w"}, "k_dn_prep_seq": {"conv_kernel", "dt_bias", "ssm_a"},
+            "k_nib_repack": {"raw"}}      # never launched early
 KERNEL = re.compile(r"__global__[^;{]*?\b(k_\w+)\(([^{]*?)\)\s*\{", re.S)
 CONST_RESTRICT = re.compile(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)")
 
