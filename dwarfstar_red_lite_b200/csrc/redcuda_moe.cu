@@ -661,7 +661,8 @@ static size_t moe_ws_layout(const redcuda_moe_desc &d, redcuda_moe *m, uint8_t *
     redcuda_moe scratch_names;            // pointer members to aim at when only the size is wanted
     redcuda_moe &r = m ? *m : scratch_names;
     put(r.x, T * d.hidden * 4u); put(r.logits, T * d.n_expert * 4u); put(r.wk, P * 4u); put(r.scalar, T * 4u);
-    put(r.sh_act, T * d.ffn_sh * 4u); put(r.sh_out, T * d.hidden * 4u); put(r.act, P * d.ffn * 4u); put(r.tmp, P * d.hidden * 4u);
+    put(r.sh_act, T * d.ffn_sh * 4u); put(r.sh_out, T * d.hidden * 4u); put(r.act, P * d.ffn * 4u);
+    put(r.tmp, P * std::max(d.hidden, d.ffn) * 4u);      // the expert outputs, and before them the up rows of the tcgen05 kernel
     put(r.out, T * d.hidden * 4u); put(r.ids, P * 4u); put(r.sorted, P * 4u); put(r.uexp, (size_t)(d.expert_count + 1u) * 4u);
     put(r.ustart, (size_t)(d.expert_count + 2u) * 4u); put(r.n_unique, 16); put(r.bad, 16);
     // digits of the routed experts' inputs: three or four int8 digits per value (mma.sync kernels) or two fp16 digits (tcgen05 kernel)
