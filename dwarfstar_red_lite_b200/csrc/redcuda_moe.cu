@@ -352,14 +352,16 @@ static uint32_t moe_item_tokens(const redcuda_moe *m, bool single_token, uint32_
     return mma_item_tokens(single_token, npairs, m->d.expert_count);
 }
 // Which expert kernels serve a call of npairs pairs (all_local: every pair belongs to this shard; otherwise the share
-// expert_count / n_expert of them): the tcgen05 kernel works on items of up to 64 pairs of one expert and decodes an
-// expert's weights once per item, so it needs experts that see many pairs each (prefill chunks of 2048 tokens: 40 pairs
-// per expert). RC_MOE_TC_MIN = pairs per expert from which it is used (default 32; 0 = never): its error against
-// 64-bit sums is 8.9e-7 where the integer kernels have 3.7e-7, so it takes over only where it gains much. A layer of 1400 tokens takes 944 to 957 us
-// on the integer kernels, one of 1700 991 on this.
+// expert_count / n_expert of them): the tcgen05 kernel works on items of up to 48 pairs of one expert and decodes an
+// expert's weights once per item, so it needs experts that see several pairs each. RC_MOE_TC_MIN = pairs per expert from which it is
+// used (default 11; 0 = never). Its error against 64-bit sums is no larger than that of the integer kernels (outputs of an expert, rows of 2048
+// Gaussian values 2.98e-7 and 2.99e-7; with one element of 1000 3.1e-7 and 2.2e-6; log-normal 3.7e-7 and 2.0e-6), so the line lies where it gets
+// faster. us a layer of 512 experts, integer kernels -> this: 400 tokens 358 -> 407, 500 413 -> 420, 600 468 -> 453, 700 525 -> 472, 1000 697 -> 513,
+// 1400 943 -> 612, 2048 1343 -> 763; Zipf routing 400 341 -> 373, 600 443 -> 425; 256 experts 300 tokens 275 -> 254; 128 experts (hidden 1024) 200
+// tokens 129 -> 113.
 static void moe_choose_path(redcuda_moe *m, uint32_t npairs, bool all_local) {
     const char *v = getenv("RC_MOE_TC_MIN");
-    const uint32_t min_avg = v ? (uint32_t)atoi(v) : 32u;
+    const uint32_t min_avg = v ? (uint32_t)atoi(v) : 11u;
     const uint64_t local = all_local ? npairs : (uint64_t)npairs * m->d.expert_count / m->d.n_expert;
     m->tc_now = m->tc_ok && min_avg && local >= (uint64_t)min_avg * m->d.expert_count;
 }
@@ -478,7 +480,7 @@ static int moe_launch_experts(redcuda_moe *m, bool gateup, uint32_t npairs, bool
         T.expert_begin = m->d.expert_begin; T.n_local = m->d.expert_count;
         T.sorted = m->sorted; T.uexp = m->uexp; T.ustart = m->ustart; T.item_u = m->item_u; T.item_p0 = m->item_p0; T.n_items = m->n_items;
         T.xd = xd; T.x_inv = xinv; T.x_div = gateup ? x_div : 1u;
-        T.out[0] = out; T.out[1] = gateup ? m->tmp : nullptr; T.out_stride = out_stride;
+        T.out[0] = out; T.out[1] = gateup ? m->tmp : nullptr; T.out_stride = out_stride; T.work = m->work + (gateup ? 0 : 1);
         T.err = m->tc_err; T.status = status_words();
         const uint32_t live = npairs < m->d.expert_count ? npairs : m->d.expert_count;
         return launch_tc_experts(T, npairs / TCX_TN + live, gateup ? "moe_gateup_tc" : "moe_down_tc", s);
@@ -828,7 +830,7 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
     if (B) m->ws_shared = true;
     else { if (!m->ws.alloc(w)) return bail(); B = m->ws.as<uint8_t>(); }
     moe_ws_layout(d, m, B);
-    // the tcgen05 expert kernel works on 22-bit digits and truncating accumulators (8.2e-7 against 64-bit sums): not for layers that had fp32
+    // the tcgen05 expert kernel works on 22-bit digits and truncating accumulators (3.0e-7 against 64-bit sums): not for layers that had fp32
     m->tc_ok = m->nib && !moe_wide(m) && tcx_shape_ok(d.ffn, d.hidden) && tcx_shape_ok(d.hidden, d.ffn);
     {   // RC_MOE_PATH=cuda keeps the IQ2_XXS experts on the CUDA-core kernels (A/B switch for profiling)
         const char *pth = getenv("RC_MOE_PATH");

@@ -39,23 +39,24 @@ int launch_tc_gemm(TcArgs &A, uint32_t tn, const char *tag, cudaStream_t s);   /
 
 // ---- routed experts of a prefill chunk on the tensor cores (redcuda_tc_experts.cu) ----
 // Nibble-layout IQ2_XXS expert matrices against the pairs grouped by expert. One work item = up to TCX_TN pairs of one
-// expert (k_group_pairs cut with item_tok = TCX_TN).
-constexpr uint32_t TCX_TN = 64u;
+// expert (k_group_pairs cut with item_tok = TCX_TN; 48 leaves room for six stages of activations, 64 for four, and 40 pairs are the mean of a full chunk).
+constexpr uint32_t TCX_TN = 48u;
 struct TcxArgs {
     const uint8_t *w[2];            // nibble-layout matrices of the shard: (gate, up) or (down, null)
     uint64_t mat_bytes;             // bytes of one expert matrix
     uint32_t nmat, nrows, ncols;    // matrices in this launch (1 or 2), rows / columns of one expert matrix
     uint32_t expert_begin, n_local;
     const uint32_t *sorted, *uexp, *ustart, *item_u, *item_p0, *n_items;    // grouping (k_group_pairs)
-    const __half *xd;               // activation digits [row][hi / lo][ncols] from launch_tc_prep_rows
+    const __half *xd;               // activation digits [row][ncols / 128][hi / lo][128] from launch_tc_prep_rows
     const float *x_inv;             // per-row inverse scale
     uint32_t x_div;                 // activation row of pair p = p / x_div
     float *out[2];                  // out[m][p * out_stride + row]
     uint32_t out_stride;
-    uint32_t cta_blocks;            // filled by launch_tc_experts
+    uint32_t *work;                 // the launch's unit counter, zeroed by the grouping kernel
+    uint32_t upg;                   // groups of a unit, filled by launch_tc_experts
     uint32_t *err, *status;         // timeout flag of the launch; sticky status words (may be null)
 };
-// v[r][k] = b ? SiLU(a[r][k]) * b[r][k] : a[r][k]  ->  fp16 digits xd[r][2][ncols] and x_inv[r]
+// v[r][k] = b ? SiLU(a[r][k]) * b[r][k] : a[r][k]  ->  fp16 digits xd[r][ncols / 128][2][128] and x_inv[r]
 int launch_tc_prep_rows(const float *a, const float *b, uint32_t stride, uint32_t nrows, uint32_t ncols, __half *xd, float *x_inv, cudaStream_t s);
 bool tcx_shape_ok(uint32_t nrows, uint32_t ncols);
 int launch_tc_experts(TcxArgs &A, uint32_t max_items, const char *tag, cudaStream_t s);
