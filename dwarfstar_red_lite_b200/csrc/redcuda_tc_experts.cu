@@ -130,41 +130,13 @@ __device__ __forceinline__ void tcx_mma_ts(uint32_t leader, uint32_t d_tmem, uin
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
         :: "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
-__device__ __forceinline__ void tcx_commit(uint32_t leader, uint32_t mbar) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" :: "r"(mbar), "r"(leader) : "memory");
-}
-__device__ __forceinline__ uint32_t tcx_elect() {
-    uint32_t l;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(l));
-    return l;
-}
-__device__ __forceinline__ uint32_t tcx_try(uint32_t mbar, uint32_t parity) {
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                 : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
-    return done;
-}
-// A warp's wait, with one answer for all its lanes. One that gives up raises the flag, which every other wait looks at, so the CTA winds
-// down within a few waits. A dozen instructions: five programs of a CTA share an instruction cache.
-__device__ __forceinline__ bool tcx_wait(uint32_t mbar, uint32_t parity, uint32_t fail) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .u32 i, f;\n\tmov.u32 i, %4;\n"
-        "POLL_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE_%=;\n\t"
-        "ld.volatile.shared.u32 f, [%3];\n\tsub.u32 i, i, 1;\n\tsetp.eq.u32 q, i, 0;\n\t@q st.volatile.shared.u32 [%3], 1;\n\tsetp.ne.or.u32 q, f, 0, q;\n\t@!q bra POLL_%=;\n"
-        "DONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done) : "r"(mbar), "r"(parity), "r"(fail), "n"(TC_SPIN_LIMIT) : "memory");
-    return __all_sync(0xffffffffu, done);
-}
-// the same without being put to sleep until the barrier moves on
+// one poll, without being put to sleep until the barrier moves on
 __device__ __forceinline__ uint32_t tcx_test(uint32_t mbar, uint32_t parity) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
                  : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
     return done;
 }
-__device__ __forceinline__ void tcx_arrive(uint32_t mbar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(mbar) : "memory"); }
 
 constexpr uint32_t TCX_NB = 6u, TCX_NRAW = 4u, TCX_NI = 4u;                                // buffers: activation stages, records of a block, units
 constexpr uint32_t TCX_W_RAW = 2u, TCX_W_GATHER = 3u, TCX_W_DECODE = 4u, TCX_N_DECODE = 8u, TCX_W_DRAIN = 12u, TCX_N_DRAIN = 8u;
@@ -231,13 +203,13 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     const uint32_t fail_at = smem_u32(const_cast<uint32_t *>(&fail));
-    auto wait = [&](uint64_t *bar, uint32_t parity) { return tcx_wait(smem_u32(bar), parity, fail_at); };
+    auto wait = [&](uint64_t *bar, uint32_t parity) { return tc_wait(smem_u32(bar), parity, fail_at); };
     auto unit_wait = [&](uint32_t n) { return wait(&unit_full[n % TCX_NI], (n / TCX_NI) & 1u); };
-    auto unit_done = [&](uint32_t n) { __syncwarp(); if (lane == 0) tcx_arrive(smem_u32(&unit_empty[n % TCX_NI])); };
+    auto unit_done = [&](uint32_t n) { __syncwarp(); if (lane == 0) tc_arrive(smem_u32(&unit_empty[n % TCX_NI])); };
 
     if (warp < TCX_T) {
         // ------------------------------------------------------------------ MMA issue
-        const uint32_t leader = tcx_elect();
+        const uint32_t leader = tc_elect();
         const uint64_t desc0 = tcx_desc_sw128(smem_u32(b_base));
         uint32_t kb = warp, ka = 0u, b = 0u, bph = 0u;       // block; accumulations of this tile so far; activation stage buffer and its phase
         bool ok = true;
@@ -264,9 +236,9 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
                         for (uint32_t kk = 0; kk < 8u; ++kk)         // + 32 bytes per k-step; the first MMA overwrites
                             tcx_mma_ts(leader, tmem + (warp * TCX_SUBS + j) * TCX_TN, tmem + TCX_TM_A + a * TCX_A_COLS + 32u * j + 8u * (kk & 3u),
                                        desc0 + b * (TCX_B_BUF >> 4) + j * (TCX_B_SUB >> 4) + (kk < 4u ? TCX_B_DIGIT >> 4 : 0u) + 2u * (kk & 3u), idesc, kk ? 1u : 0u);
-                    tcx_commit(leader, smem_u32(&acc_full[warp]));
-                    tcx_commit(leader, smem_u32(&b_empty[b]));
-                    tcx_commit(leader, smem_u32(&a_empty[a]));
+                    tc_commit_if(leader, smem_u32(&acc_full[warp]));
+                    tc_commit_if(leader, smem_u32(&b_empty[b]));
+                    tc_commit_if(leader, smem_u32(&a_empty[a]));
                     if (++b == TCX_NB) { b = 0u; bph ^= 1u; }
                 }
             }
@@ -309,7 +281,7 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
                     for (uint32_t i = 0; i < 2u; ++i)
                         if (lane + 32u * i < TCX_TN) { U.row[lane + 32u * i] = f_row[i]; U.pair[lane + 32u * i] = f_pair[i]; U.xinv[lane + 32u * i] = f_inv[i]; }
                     __syncwarp();
-                    if (lane == 0) tcx_arrive(smem_u32(&unit_full[n % TCX_NI]));
+                    if (lane == 0) tc_arrive(smem_u32(&unit_full[n % TCX_NI]));
                 }
             }
         };
@@ -360,7 +332,7 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
         auto hand = [&]() {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) tcx_arrive(smem_u32(&b_full[gb]));
+            if (lane == 0) tc_arrive(smem_u32(&b_full[gb]));
             ++given;
             gb = gb + 1u == TCX_NB ? 0u : gb + 1u;
         };
@@ -415,7 +387,7 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
             for (uint32_t t = 0; t < 4u; ++t) wd[t] = *reinterpret_cast<const uint4 *>(raw + nib_code_off(rr, t, kg0));
             sc4 = *reinterpret_cast<const uint32_t *>(raw + nib_sc_off(rr, kg0));
             __syncwarp();
-            if (lane == 0) tcx_arrive(smem_u32(&raw_empty[k]));
+            if (lane == 0) tc_arrive(smem_u32(&raw_empty[k]));
             ++kl;
             return true;
         };
@@ -444,7 +416,7 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) tcx_arrive(smem_u32(&a_full[a]));
+                if (lane == 0) tc_arrive(smem_u32(&a_full[a]));
             }
         }
     } else {
@@ -493,7 +465,7 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
                     }
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) tcx_arrive(smem_u32(&acc_empty[half]));
+                    if (lane == 0) tc_arrive(smem_u32(&acc_empty[half]));
                 }
                 if (!ok) break;
                 if (last) {                               // store the group's results

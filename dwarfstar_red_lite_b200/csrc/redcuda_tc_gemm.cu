@@ -279,13 +279,16 @@ __global__ void __launch_bounds__(TC_THREADS) k_tc_decode_w(const __grid_constan
 }
 
 // ---- the GEMM proper: one CTA = 128 weight rows (MMA M) x TN tokens (MMA N) x all columns, K in stages of 64 -------------
-//   warp 0, one thread   producer: per stage ONE mbarrier transaction of two bulk copies (the stage's weight digits from wd,
+//   warp 0               producer: per stage ONE mbarrier transaction of two bulk copies (the stage's weight digits from wd,
 //                        its activation digits from xs), NS stages ahead of the MMAs
-//   warp 1, one thread   issues 4 k-steps x 2 tcgen05.mma per stage (A_hi x [B_hi | B_lo], N = 2 TN; A_lo x B_hi, N = TN), a
+//   warp 1               issues 4 k-steps x 2 tcgen05.mma per stage (A_hi x [B_hi | B_lo], N = 2 TN; A_lo x B_hi, N = TN), a
 //                        tcgen05.commit that frees the stage's buffers, and after every fourth stage one that hands the
 //                        256-column block's accumulator pair to the drain warps
 //   warps 2..9           tcgen05.ld of a finished block's two accumulators into fp32 register sums while the next block
 //                        multiplies into the other pair; scaling and stores at the end
+// The MMAs are issued by a converged warp (tc_mma_if): from a lane of its own the in-projections of a 2048-token chunk took 270 us (now 224), the
+// out-projection 102 (81), the out-projection of 93 tokens 39 (24). What bounds it now is shared memory: of its 128 bytes a cycle a stage wants 80 KB for the
+// MMAs and 64 KB for the copies in 768 cycles of MMAs.
 // No block-wide barrier inside the loop; every wait on an mbarrier is bounded, and a wait that gives up raises a flag that
 // every role reads before its next wait, so the CTA winds down, frees its tensor memory and reports the timeout.
 constexpr uint32_t TCG_THREADS = 320u, TCG_DRAIN_WARPS = 8u;
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(TCG_THREADS, 1) k_tc_gemm(const __grid_constan
     __shared__ __align__(8) uint64_t acc_empty[2];   // the drain warps have read accumulator pair b
     __shared__ uint32_t tmem_slot;
     __shared__ volatile uint32_t fail;               // a bounded wait ran out
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31u;
 
     // token tile = blockIdx.x (fastest: the CTAs that share a weight tile run together and read it from L2), row tile = blockIdx.y
     const uint32_t rt = blockIdx.y;
@@ -332,73 +335,52 @@ __global__ void __launch_bounds__(TCG_THREADS, 1) k_tc_gemm(const __grid_constan
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_slot;
-    auto wait = [&](uint64_t *bar, uint32_t parity) -> bool {
-        if (fail) return false;
-        if (mbar_wait(smem_u32(bar), parity)) return true;
-        fail = 1u;
-        return false;
-    };
-    // for the roles that are far ahead of their producer: longer sleeps between polls, so that their spinning takes no issue
-    // slots from the MMA thread
-    auto wait_idle = [&](uint64_t *bar, uint32_t parity) -> bool {
-        if (fail) return false;
-        const uint32_t addr = smem_u32(bar);
-        for (uint32_t i = 0; i < TC_SPIN_LIMIT / 8u; ++i) {
-            uint32_t done;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                         : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-            if (done) return true;
-            __nanosleep(256);
-        }
-        fail = 1u;
-        return false;
-    };
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0), fail_at = smem_u32(const_cast<uint32_t *>(&fail));
+    auto wait = [&](uint64_t *bar, uint32_t parity) { return tc_wait(smem_u32(bar), parity, fail_at); };
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
-        if (lane == 0) {
-            uint32_t issued = 0u;
-            for (uint32_t s = 0; s < nstage; ++s) {
-                const uint32_t j = s % NS;
-                if (s >= NS && !wait_idle(&empty[j], ((s / NS) - 1u) & 1u)) break;
+        uint32_t s = 0u;
+        for (; s < nstage; ++s) {
+            const uint32_t j = s % NS;
+            if (s >= NS && !wait(&empty[j], ((s / NS) - 1u) & 1u)) break;
+            if (lane == 0) {
                 const uint32_t bar = smem_u32(&full[j]), dst = smem_u32(smem + j * STAGE);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(STAGE) : "memory");
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                              :: "r"(dst), "l"(wd_tile + (size_t)s * A_BUF), "r"(A_BUF), "r"(bar) : "memory");
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                              :: "r"(dst + A_BUF), "l"(xs_tile + (size_t)s * (B_BUF / 2u)), "r"(B_BUF), "r"(bar) : "memory");
-                issued = s + 1u;
             }
-            // after a timeout elsewhere, copies that nobody waits for may still be writing into this CTA's shared memory
-            if (fail) for (uint32_t s = issued >= NS ? issued - NS : 0u; s < issued; ++s) mbar_wait(smem_u32(&full[s % NS]), (s / NS) & 1u);
+            __syncwarp();
         }
+        // after a timeout elsewhere, copies that nobody waits for may still be writing into this CTA's shared memory
+        if (fail && lane == 0) for (uint32_t k = s >= NS ? s - NS : 0u; k < s; ++k) mbar_wait(smem_u32(&full[k % NS]), (k / NS) & 1u);
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issue
-        if (lane == 0) {
-            const uint32_t idesc = tc_idesc((uint32_t)TN), idesc2 = tc_idesc(2u * (uint32_t)TN);
-            constexpr uint32_t A_LBO = TC_M * 16u, B_LBO = 2u * (uint32_t)TN * 16u, SBO = 128u;
-            const uint64_t da0 = tc_smem_desc(0u, A_LBO, SBO), db0 = tc_smem_desc(0u, B_LBO, SBO);
-            for (uint32_t s = 0; s < nstage; ++s) {
-                const uint32_t j = s % NS, c = s >> 2;
-                if (!wait(&full[j], (s / NS) & 1u)) break;
-                if ((s & 3u) == 0u && c >= 2u && !wait(&acc_empty[c & 1u], ((c >> 1) - 1u) & 1u)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // Two MMAs per k-step: A_hi x [B_hi | B_lo] (N = 2 TN: the hi*hi sums land in the first TN accumulator
-                // columns, hi*lo in the next TN) and A_lo x B_hi (N = TN, added to the cross-product columns).
-                const uint32_t a_st = smem_u32(smem + j * STAGE);
-                const uint32_t a_hi = a_st >> 4, a_lo = (a_st + TC_A_DIGIT) >> 4, b_st = (a_st + A_BUF) >> 4;
-                const uint32_t d_main = tmem + (c & 1u) * 2u * (uint32_t)TN, d_cross = d_main + (uint32_t)TN;
+        const uint32_t leader = tc_elect();
+        const uint32_t idesc = tc_idesc((uint32_t)TN), idesc2 = tc_idesc(2u * (uint32_t)TN);
+        constexpr uint32_t A_LBO = TC_M * 16u, B_LBO = 2u * (uint32_t)TN * 16u, SBO = 128u;
+        const uint64_t da0 = tc_smem_desc(smem_u32(smem), A_LBO, SBO), db0 = tc_smem_desc(smem_u32(smem) + A_BUF, B_LBO, SBO);
+        uint32_t j = 0u, ph = 0u;
+#pragma unroll 1
+        for (uint32_t s = 0; s < nstage; ++s) {
+            const uint32_t c = s >> 2;
+            if (!wait(&full[j], ph)) break;
+            if ((s & 3u) == 0u && c >= 2u && !wait(&acc_empty[c & 1u], ((c >> 1) - 1u) & 1u)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // Two MMAs per k-step: A_hi x [B_hi | B_lo] (N = 2 TN: the hi*hi sums land in the first TN accumulator
+            // columns, hi*lo in the next TN) and A_lo x B_hi (N = TN, added to the cross-product columns).
+            const uint64_t da = da0 + j * (STAGE >> 4), db = db0 + j * (STAGE >> 4);
+            const uint32_t d_main = tmem + (c & 1u) * 2u * (uint32_t)TN, d_cross = d_main + (uint32_t)TN;
 #pragma unroll
-                for (uint32_t kk = 0; kk < TC_KS / 16u; ++kk) {
-                    const uint64_t dah = da0 + ((a_hi + kk * (2u * A_LBO >> 4)) & 0x3fffu), dal = da0 + ((a_lo + kk * (2u * A_LBO >> 4)) & 0x3fffu);
-                    const uint64_t db = db0 + ((b_st + kk * (2u * B_LBO >> 4)) & 0x3fffu);
-                    tc_mma(d_main, dah, db, idesc2, ((s & 3u) | kk) ? 1u : 0u);      // a block's first MMA overwrites its accumulators
-                    tc_mma(d_cross, dal, db, idesc, 1u);
-                }
-                tc_commit(smem_u32(&empty[j]));
-                if ((s & 3u) == 3u) tc_commit(smem_u32(&acc_full[c & 1u]));
+            for (uint32_t kk = 0; kk < TC_KS / 16u; ++kk) {
+                tc_mma_if(leader, d_main, da + kk * (2u * A_LBO >> 4), db + kk * (2u * B_LBO >> 4), idesc2, (s & 3u) | kk);      // a block's first MMA overwrites its accumulators
+                tc_mma_if(leader, d_cross, da + (TC_A_DIGIT >> 4) + kk * (2u * A_LBO >> 4), db + kk * (2u * B_LBO >> 4), idesc, 1u);
             }
+            tc_commit_if(leader, smem_u32(&empty[j]));
+            if ((s & 3u) == 3u) tc_commit_if(leader, smem_u32(&acc_full[c & 1u]));
+            if (++j == NS) { j = 0u; ph ^= 1u; }
         }
     } else {
         // ------------------------------------------------------------------ accumulator drain and epilogue (256 threads)
@@ -410,7 +392,7 @@ __global__ void __launch_bounds__(TCG_THREADS, 1) k_tc_gemm(const __grid_constan
         for (uint32_t j = 0; j < PER; ++j) acc[j] = 0.f;
         bool ok = true;
         for (uint32_t blk = 0; blk < nblk && ok; ++blk) {
-            ok = wait_idle(&acc_full[blk & 1u], (blk >> 1) & 1u);
+            ok = wait(&acc_full[blk & 1u], (blk >> 1) & 1u);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t base = tmem + (qlane << 16) + (blk & 1u) * 2u * (uint32_t)TN + c_begin;
@@ -427,7 +409,7 @@ __global__ void __launch_bounds__(TCG_THREADS, 1) k_tc_gemm(const __grid_constan
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(&acc_empty[blk & 1u])) : "memory");
+            if (lane == 0) tc_arrive(smem_u32(&acc_empty[blk & 1u]));
         }
         if (ok && !fail) {
             const uint32_t row = row0 + qlane + lane;

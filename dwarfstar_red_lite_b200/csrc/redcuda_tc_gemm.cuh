@@ -78,17 +78,37 @@ __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr, uint32_t lbo, ui
 // instruction descriptor, kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = n
 __device__ __forceinline__ uint32_t tc_idesc(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((TC_M >> 4) << 24); }
 
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[smem] * B[smem], issued from a converged warp by the lane whose `leader` is set (tc_elect): addresses and descriptors stay in uniform registers. In code of one
+// lane they do not, and bringing them there for every MMA took longer than the MMA.
+__device__ __forceinline__ void tc_mma_if(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+        :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(uint32_t leader, uint32_t mbar) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" :: "r"(mbar), "r"(leader) : "memory");
+}
+__device__ __forceinline__ uint32_t tc_elect() {
+    uint32_t l;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(l));
+    return l;
 }
 
-__device__ __forceinline__ void tc_commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(mbar) : "memory");
+__device__ __forceinline__ void tc_arrive(uint32_t mbar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(mbar) : "memory"); }
+// A warp's wait, with one answer for all its lanes. One that gives up raises the flag, which every other wait looks at, so the CTA winds
+// down within a few waits. A dozen instructions: five programs of a CTA share an instruction cache.
+__device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity, uint32_t fail) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 i, f;\n\tmov.u32 i, %4;\n"
+        "POLL_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE_%=;\n\t"
+        "ld.volatile.shared.u32 f, [%3];\n\tsub.u32 i, i, 1;\n\tsetp.eq.u32 q, i, 0;\n\t@q st.volatile.shared.u32 [%3], 1;\n\tsetp.ne.or.u32 q, f, 0, q;\n\t@!q bra POLL_%=;\n"
+        "DONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done) : "r"(mbar), "r"(parity), "r"(fail), "n"(TC_SPIN_LIMIT) : "memory");
+    return __all_sync(0xffffffffu, done);
 }
-
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
     for (uint32_t i = 0; i < TC_SPIN_LIMIT; ++i) {
         uint32_t done;
