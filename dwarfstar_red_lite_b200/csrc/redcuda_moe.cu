@@ -602,7 +602,8 @@ static int moe_forward_on(redcuda_moe *m, uint32_t ntok, const float *x, const f
     // one quantisation of the token activations serves the routed gate/up and the shared gate/up
     // (a wide layer has digits of its own for the routed experts: `wide` makes those, `xq` the shared expert's)
     const bool wide = moe_wide(m);
-    const bool xq = wide ? moe_shared_mma(m, ntok) && !moe_shared_tc(m, ntok) : moe_experts_mma(m) || moe_shared_mma(m, ntok);
+    const bool sh_xq = moe_shared_mma(m, ntok) && !moe_shared_tc(m, ntok);
+    const bool xq = wide ? sh_xq : (moe_experts_mma(m) && !m->tc_now) || sh_xq;
     // The shared expert needs nothing from the router, so it runs on a side stream next to the routed
     // experts and joins before the combine (both edges are events, so the fork is kept when the caller captures a graph).
     // With profiling on, everything stays on one stream so that per-kernel times are not overlapped.
