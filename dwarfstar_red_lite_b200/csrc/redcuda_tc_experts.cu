@@ -161,16 +161,18 @@ struct TcxUnit { uint32_t live, expert, group0, ntok, ncol, pad[3]; uint32_t row
 //                 (warps 4-7 the first stage of a block, 8-11 the second)
 //   warps 12-19   read a stage's accumulators (12-15 those of the first tile, 16-19 of the second), add them, scaled by d / 8, to fp32
 //                 register sums, and store these at the end of a group
-// What bounds it is the decode warps' chain: two barriers, the record out of shared memory, 190 instructions, four stores and an arrival, some 1400
-// cycles a block where the MMAs of 48 pairs take 770 (with the arithmetic left out 700; HBM delivers a block to every SM in 770).
+// What bounds it is the decode warps' chain (two barriers, the record out of shared memory, 190 instructions, four stores and an arrival, some 1500
+// cycles a block where the MMAs of 48 pairs take 770 and HBM delivers a block to every SM in 770), and with full items the MMAs' wait for the drain.
 // How it came here, us for gate/up and down of 2048 tokens (40 pairs an expert): decoded weights in shared memory, one CTA per item and up to 32
 // blocks, items of 64 pairs, 128-column stages: 463 and 304, bound by shared memory (operand A written and read, 64 KB a stage of the 128
 // bytes a cycle that it moves, beside 64 KB of B) and by an issuing lane outside converged code, whose addresses have to be brought to
 // uniform registers for every MMA. Operand A in tensor memory, persistent, two tiles a gather: 391 and 208; MMAs issued from converged code: 272 and 167;
 // waits of a dozen instructions instead of loops inlined twenty times (120 KB of code: five programs share an instruction cache): 240 and 136
-// with accumulators of 256 columns. Accumulators of 64 columns cost 20 us of each layer and take the error from 8.6e-7 to 3.0e-7. Taken back: decode and
-// drain by the same eight warps (322 and 196), items of 64 pairs with four stages of activations instead of six (260 and 152), a decode warp
-// per tile instead of per stage (the same time, and barrier phases can be passed unseen).
+// with accumulators of 256 columns. Accumulators of 64 columns cost 20 us of each launch and take the error from 8.6e-7 to 3.0e-7. Records requested from
+// converged code (eight lanes with an address each are served one after the other) and barriers polled ahead of their use: 254 and 153 for
+// 2048 tokens, 700 tokens 207 and 112 -> 179 and 104. Taken back: decode and drain by the same eight warps (322 and 196), items of 64 pairs with four stages
+// of activations instead of six (260 and 152 against 240 and 136), a decode warp per tile instead of per stage (the same time, and barrier phases can
+// be passed unseen).
 __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_constant__ TcxArgs A) {
     pdl_prologue();
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -204,6 +206,9 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     const uint32_t fail_at = smem_u32(const_cast<uint32_t *>(&fail));
     auto wait = [&](uint64_t *bar, uint32_t parity) { return tc_wait(smem_u32(bar), parity, fail_at); };
+    // a poll ahead of the place where its answer is needed (a barrier's answer takes some hundred cycles, a role's turn has two or three), and the wait there
+    auto poll = [&](uint64_t *bar, uint32_t parity) { return tcx_test(smem_u32(bar), parity); };
+    auto wait_polled = [&](uint32_t polled, uint64_t *bar, uint32_t parity) { return __all_sync(0xffffffffu, polled) || wait(bar, parity); };
     auto unit_wait = [&](uint32_t n) { return wait(&unit_full[n % TCX_NI], (n / TCX_NI) & 1u); };
     auto unit_done = [&](uint32_t n) { __syncwarp(); if (lane == 0) tc_arrive(smem_u32(&unit_empty[n % TCX_NI])); };
 
@@ -211,7 +216,7 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
         // ------------------------------------------------------------------ MMA issue
         const uint32_t leader = tc_elect();
         const uint64_t desc0 = tcx_desc_sw128(smem_u32(b_base));
-        uint32_t kb = warp, ka = 0u, b = 0u, bph = 0u;       // block; accumulations of this tile so far; activation stage buffer and its phase
+        uint32_t ka = 0u, b = 0u, bph = 0u, a = warp * TCX_SPB, aph = 0u;       // accumulations of this tile so far; activation and weight stage buffers and their phases
         bool ok = true;
         for (uint32_t n = 0; ok && (ok = unit_wait(n)); ++n) {
             const TcxUnit &U = s_unit[n % TCX_NI];
@@ -220,12 +225,11 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
             if (!live) break;
             const uint32_t idesc = tc_idesc(ncol);
 #pragma unroll 1
-            for (uint32_t i = 0; i < ncb; ++i, kb += TCX_T) {
+            for (uint32_t i = 0; i < ncb && ok; ++i) {
 #pragma unroll 1
                 for (uint32_t h = 0; h < TCX_SPB && ok; ++h, ++ka) {
-                    const uint32_t q = kb * TCX_SPB + h, a = q % TCX_NA;
-                    if (!(ok = wait(&b_full[b], bph) && wait(&a_full[a], (q / TCX_NA) & 1u))) break;
-                    if (ka && !(ok = wait(&acc_empty[warp], (ka - 1u) & 1u))) break;
+                    const uint32_t b_there = poll(&b_full[b], bph), a_there = poll(&a_full[a], aph), d_free = ka ? poll(&acc_empty[warp], (ka - 1u) & 1u) : 1u;
+                    if (!(ok = wait_polled(b_there, &b_full[b], bph) && wait_polled(a_there, &a_full[a], aph) && wait_polled(d_free, &acc_empty[warp], (ka - 1u) & 1u))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     // An accumulator covers 64 columns, the lo digits first: the adder truncates, so what is lost grows with the steps that meet large
                     // sums. Relative error of an expert's output against 64-bit sums (rows of 2048 Gaussian values): 8.6e-7 with accumulators of 256 columns
@@ -240,6 +244,7 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
                     tc_commit_if(leader, smem_u32(&b_empty[b]));
                     tc_commit_if(leader, smem_u32(&a_empty[a]));
                     if (++b == TCX_NB) { b = 0u; bph ^= 1u; }
+                    if ((a += h == TCX_SPB - 1u ? TCX_SPB * (TCX_T - 1u) + 1u : 1u) >= TCX_NA) { a -= TCX_NA; aph ^= 1u; }      // behind a block, over the other tile's
                 }
             }
         }
@@ -285,25 +290,28 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
                 }
             }
         };
+        const uint32_t leader = tc_elect();
+        const uint64_t tile_step = (uint64_t)bpr * NIB_REC;      // from a 16-row tile to the next
         uint32_t kb = 0u, step = 0u;
 #pragma unroll 1
         while (step < 6u) look(step++, 0u);
         for (uint32_t n = 0; ok && f_live; ++n) {
-            const uint32_t e = f_e, group0 = (f_u % upi) * A.upg;
+            const uint32_t e = __shfl_sync(0xffffffffu, f_e, 0), group0 = __shfl_sync(0xffffffffu, (f_u % upi) * A.upg, 0);
             step = 0u;
-            const uint64_t base = (uint64_t)e * A.mat_bytes + (uint64_t)(group0 * gtiles * 8u + lane) * bpr * NIB_REC;      // record (16-row tile j, block c) of a matrix at (j * bpr + c) * NIB_REC
-            const uint8_t *src0 = A.w[0] + base, *src1 = A.nmat == 2u ? A.w[1] + base : src0 + (uint64_t)8u * bpr * NIB_REC;
+            const uint64_t base = (uint64_t)e * A.mat_bytes + (uint64_t)(group0 * gtiles * 8u) * tile_step;      // record (16-row tile j, block c) of a matrix at (j * bpr + c) * NIB_REC
+            const uint8_t *src0 = A.w[0] + base, *src1 = A.nmat == 2u ? A.w[1] + base : src0 + 8u * tile_step;
             uint32_t c = 0u;
 #pragma unroll 1
             for (uint32_t i = 0; i < ncb * TCX_T && ok; ++i, ++kb) {
                 const uint32_t k = kb % TCX_NRAW;
                 if (kb >= TCX_NRAW && !(ok = wait(&raw_empty[k], ((kb / TCX_NRAW) - 1u) & 1u))) break;
                 const uint32_t bar = smem_u32(&raw_full[k]), dst = smem_u32(raw_base + k * TCX_RAW);
-                if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(TCX_RAW) : "memory");
-                __syncwarp();
-                if (lane < 8u)
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                 :: "r"(dst + lane * NIB_REC), "l"(src0), "r"(NIB_REC), "r"(bar) : "memory");
+                asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}\n" :: "r"(bar), "r"(TCX_RAW), "r"(leader) : "memory");
+                // by one lane of a converged warp, its addresses uniform: eight lanes with an address each are served one after the other
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; ++j)
+                    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}\n"
+                                 :: "r"(dst + j * NIB_REC), "l"(src0 + (uint64_t)j * tile_step), "r"(NIB_REC), "r"(bar), "r"(leader) : "memory");
                 const uint8_t *other = src1;              // the other tile's turn; after both, the next block of the row or the next group
                 src1 = src0;
                 if (i & 1u) {
@@ -377,11 +385,11 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
         const uint32_t ta0 = tmem + (((warp & 3u) * 32u) << 16) + TCX_TM_A;
         const uint8_t *raw0 = raw_base + (row >> 4) * NIB_REC;
         uint4 wd[4];                                      // piece t: code words of the columns 32 kg + 8 t .. + 7, kg = kg0 .. kg0 + 3, of the next block
-        uint32_t sc4 = 0u, kl = 0u, kb = 0u;              // their four scales; blocks read from shared memory, blocks decoded
+        uint32_t sc4 = 0u, kl = 0u, a = half, aph = 1u;   // their four scales; blocks read from shared memory; weight stage buffer, and the phase that must have ended before it is filled (at first, the one before the barrier's first)
         bool ok = true;
-        auto load = [&]() -> bool {
+        auto load = [&](uint32_t polled) -> bool {
             const uint32_t k = kl % TCX_NRAW;
-            if (!wait(&raw_full[k], (kl / TCX_NRAW) & 1u)) return false;
+            if (!wait_polled(polled, &raw_full[k], (kl / TCX_NRAW) & 1u)) return false;
             const uint8_t *raw = raw0 + k * TCX_RAW;
 #pragma unroll
             for (uint32_t t = 0; t < 4u; ++t) wd[t] = *reinterpret_cast<const uint4 *>(raw + nib_code_off(rr, t, kg0));
@@ -394,10 +402,10 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
         for (uint32_t n = 0; ok && (ok = unit_wait(n)); ++n) {
             const uint32_t live = s_unit[n % TCX_NI].live;
             unit_done(n);
-            if (!live || !(ok = load())) break;
+            if (!live || !(ok = load(0u))) break;
 #pragma unroll 1
-            for (uint32_t i = 0; i < ncb * TCX_T; ++i, ++kb) {
-                const uint32_t q = kb * TCX_SPB + half, a = q % TCX_NA;
+            for (uint32_t i = 0; i < ncb * TCX_T; ++i) {
+                const uint32_t raw_there = poll(&raw_full[kl % TCX_NRAW], (kl / TCX_NRAW) & 1u), a_free = poll(&a_empty[a], aph);
                 uint32_t h[4][16];                        // all of them before the first store: a register that a store still has to read cannot be written
 #pragma unroll
                 for (uint32_t kg = 0; kg < 4u; ++kg) {
@@ -405,8 +413,8 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
 #pragma unroll
                     for (uint32_t t = 0; t < 4u; ++t) tcx_decode8(kg == 0u ? wd[t].x : kg == 1u ? wd[t].y : kg == 2u ? wd[t].z : wd[t].w, hs, hb, h[kg] + 4u * t);
                 }
-                if (i + 1u < ncb * TCX_T && !(ok = load())) break;        // on its way while this block is stored
-                if (q >= TCX_NA && !(ok = wait(&a_empty[a], ((q / TCX_NA) - 1u) & 1u))) break;
+                if (i + 1u < ncb * TCX_T && !(ok = load(raw_there))) break;        // on its way while this block is stored
+                if (!(ok = wait_polled(a_free, &a_empty[a], aph))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (uint32_t kg = 0; kg < 4u; ++kg)
@@ -417,6 +425,7 @@ __global__ void __launch_bounds__(TCX_THREADS, 1) k_tc_experts(const __grid_cons
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) tc_arrive(smem_u32(&a_full[a]));
+                if ((a += TCX_SPB) >= TCX_NA) { a -= TCX_NA; aph ^= 1u; }
             }
         }
     } else {
