@@ -291,7 +291,7 @@ using namespace rc;
 struct redcuda_moe {
     redcuda_moe_desc d;
     int device = 0;
-    DevMem wmem, ws;
+    DevMem wmem, ws, rt_mem;
     DMat router, sh_gate_inp, sh_gate, sh_up, sh_down;
     uint8_t *gate = nullptr, *up = nullptr, *down = nullptr;
     uint64_t gu_bytes = 0, down_bytes = 0, gu_nb = 0, down_nb = 0;
@@ -316,6 +316,8 @@ struct redcuda_moe {
     __half *sh_xs = nullptr; float *sh_xinv = nullptr;   // shared expert on the tcgen05 GEMM: activation digits and inverse scales
     uint8_t *sh_wd = nullptr; float *sh_winv = nullptr;  // and the weight digits of one launch (gate + up, or down)
     __half *rt_xs = nullptr; float *rt_xinv = nullptr; uint8_t *rt_wd = nullptr; float *rt_winv = nullptr;   // the same for the router logits of a large chunk
+    uint8_t *rt_q = nullptr; double *rt_ws = nullptr;       // the router's digits and row scales for the integer logits of a chunk (null: not a shape they tile)
+    uint8_t *rt_xq = nullptr; double *rt_xsc = nullptr;     // and those of the chunk's rows
     bool tc_ok = false;         // the tcgen05 expert kernel can serve this layer's shapes
     bool tc_now = false;        // ... and serves the call in progress (set by moe_choose_path, read by the grouping and the launches)
     bool ws_shared = false;     // the workspace belongs to the caller (rc::moe_create_shared)
@@ -386,6 +388,15 @@ static bool moe_router_tc(const redcuda_moe *m, uint32_t ntok) {
     const uint32_t min_tok = v ? (uint32_t)atoi(v) : 0u;
     return min_tok && ntok >= min_tok && m->router.type == RC_F32 && m->d.hidden % 256u == 0 && m->rt_wd;
 }
+// Router logits of a chunk by exact integer products (redcuda_router_i8.cu): from 640 tokens and 512 experts on; RC_ROUTER_I8_MIN = tokens (0: never, and then
+// for every expert count it tiles). us a layer, double sums -> this: 512 experts 400 tokens 349 -> 350, 512 414 -> 409, 700 411 -> 394, 2048 689 -> 637; 256 experts
+// 700 tokens 284 -> 286, 1024 335 -> 350, 2048 574 -> 587; 128 experts 2048 tokens 310 -> 320: the double kernel runs beside the shared expert's tcgen05
+// GEMMs, this one takes turns with them for the SMs.
+static bool moe_router_i8(const redcuda_moe *m, uint32_t ntok) {
+    if (!m->rt_q) return false;
+    if (const char *v = getenv("RC_ROUTER_I8_MIN")) return atoi(v) && ntok >= (uint32_t)atoi(v);
+    return ntok >= 640u && m->d.n_expert >= 512u;
+}
 // out[j][t][row] = W_j x[t] for one or two matrices that share x (x2: the input is SiLU(x) * x2)
 static int moe_shared_tc_gemm(redcuda_moe *m, uint32_t ntok, const float *x, const float *x2, uint32_t ncols, const DMat *w0, float *out0, const DMat *w1, float *out1,
                               const char *tag, cudaStream_t s) {
@@ -403,7 +414,7 @@ static int moe_shared_tc_gemm(redcuda_moe *m, uint32_t ntok, const float *x, con
 // GEMV cannot do that, or a kernel would take part that reads x as it is
 static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with_router, bool with_shared, bool x_quantised, cudaStream_t s,
                         const int8_t *xq = nullptr, const float *sx = nullptr, const RouteTail *tail = nullptr, const GemvNorm *norm = nullptr) {
-    if (norm && moe_router_tc(m, ntok)) return -1;
+    if (norm && (moe_router_tc(m, ntok) || moe_router_i8(m, ntok))) return -1;
     if (!xq) { xq = m->xq_x; sx = m->sx_x; }
     GemvArgs A{};
     A.ntok = ntok; A.x = x; A.x_stride = m->d.hidden; A.resident = 1u;
@@ -424,6 +435,8 @@ static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with
             T.wd = m->rt_wd; T.w_inv = m->rt_winv;
             T.job[0] = TcJob{m->router.base, 0u, RC_F32, m->d.n_expert, m->logits, m->d.n_expert, 0u};
             if (!launch_tc_gemm(T, tn, "moe_router_logits_tc", s)) return 0;
+        } else if (moe_router_i8(m, ntok)) {
+            if (!launch_rt_logits(m->rt_q, m->rt_ws, x, m->d.hidden, ntok, m->d.n_expert, m->d.hidden, m->rt_xq, m->rt_xsc, m->logits, m->tc_err, s)) return 0;
         } else if (ntok >= 2u && m->router.type == RC_F32) {
             if (!launch_router_logits((const float *)m->router.base, x, m->d.hidden, ntok, m->d.n_expert, m->d.hidden, m->logits, s)) return 0;
         } else add(m->router, nullptr, m->logits, m->d.n_expert, GEMV_STORE);
@@ -682,6 +695,7 @@ static size_t moe_ws_layout(const redcuda_moe_desc &d, redcuda_moe *m, uint8_t *
         put(r.rt_xs, tc_xs_halves((uint32_t)T, d.hidden, 128u) * 2u); put(r.rt_xinv, (T + 128u) * 4u);
         put(r.rt_wd, tc_wd_bytes(tc_row_tiles(d.n_expert), d.hidden)); put(r.rt_winv, (size_t)tc_row_tiles(d.n_expert) * 4u);
     }
+    if (rt_shape_ok(d.n_expert, d.hidden)) { put(r.rt_xq, rt_xq_bytes((uint32_t)T, d.hidden)); put(r.rt_xsc, rt_xs_doubles((uint32_t)T) * sizeof(double)); }
     if (m) { m->ticket = m->work + 2; m->tc_err = m->work + 3; }
     return w;
 }
@@ -823,6 +837,12 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
     ok = ok && put(d.type_gu, d.ffn, d.hidden, raw_gu, d.gate_exps, m->gate, m->gu_bytes) && put(d.type_gu, d.ffn, d.hidden, raw_gu, d.up_exps, m->up, m->gu_bytes) &&
          put(d.type_down, d.hidden, d.ffn, raw_down, d.down_exps, m->down, m->down_bytes);
     if (!ok) return bail();
+    if (rt_shape_ok(d.n_expert, d.hidden)) {
+        const size_t q = align_up(rt_wq_bytes(d.n_expert, d.hidden), 256);
+        if (!m->rt_mem.alloc(q + d.n_expert * sizeof(double))) return bail();
+        m->rt_q = m->rt_mem.as<uint8_t>(); m->rt_ws = reinterpret_cast<double *>(m->rt_q + q);
+        if (!launch_rt_digits_w((const float *)m->router.base, d.n_expert, d.hidden, m->rt_q, m->rt_ws, s)) return bail();
+    }
 
     // workspace: this layer's own, or the caller's (shared by layers whose calls are ordered on one stream)
     m->max_pairs = d.max_tokens * d.top_k;
