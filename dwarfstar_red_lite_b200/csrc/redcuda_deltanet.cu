@@ -257,52 +257,114 @@ __global__ void __launch_bounds__(256, MINB) k_dn_step(DnDims D, const float *__
 // k_dn_state_seq  the delta rule over the T tokens with the state row held in registers: one read and one write of
 //                 the state per chunk instead of per token; the next token's q/k/v/beta/gate are fetched while the
 //                 current one is reduced
-// the tail kernel is k_dn_tail with the token as its batch index
-// a block serves DN_PREP_TOK consecutive tokens of its channel group (one token per block left the kernel bound by block
-// scheduling: 133,000 blocks of 128 threads for a 2048-token chunk)
+// A block serves DN_PREP_TOK consecutive tokens of its channel group: a thread keeps its channel's samples and results of all of them, so that a sample is
+// read once and the eight L2 norms are reduced together, their roots taken by one thread each. Double-precision arithmetic bounds it (some 25 operations a
+// value; with exp() and a division of doubles for every value, a root and a division in every thread and a barrier per token it was 65, and 119 us for
+// 2048 tokens where this takes 62).
 constexpr uint32_t DN_PREP_TOK = 8u;
-__global__ void k_dn_prep_seq(DnDims D, uint32_t T, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,
-                              const float *qkv, const float *ba, const float *conv_state,
-                              float *__restrict__ qk, float *__restrict__ v, float *__restrict__ beta, float *__restrict__ gate) {
+
+// a / (1 + exp(-a)) to within 2^-40 of itself before it is rounded to fp32, whose half unit is 2^-25: exp(-a) = 2^n exp(r), |r| <= ln 2 / 2, exp(r) by its Taylor
+// polynomial of degree 10 (the remainder is below 2^-41), the reciprocal by one Newton step in double from an fp32 one (2^-22 squared)
+__device__ __forceinline__ float dn_silu(double a) {
+    if (!(fabs(a) < 80.0)) return (float)(a / (1.0 + exp(-a)));
+    const double magic = 6755399441055744.0, t = fma(a, -1.4426950408889634, magic), n = t - magic;       // 1.5 2^52: n is the nearest integer
+    const double r = fma(n, -1.9082149292705877e-10, fma(n, -0.693147180369123816490, -a));
+    double p = 2.7557319223985893e-07;                               // 1 / 10!
+    p = fma(p, r, 2.7557319223985888e-06); p = fma(p, r, 2.4801587301587302e-05); p = fma(p, r, 1.9841269841269841e-04); p = fma(p, r, 1.3888888888888889e-03);
+    p = fma(p, r, 8.3333333333333333e-03); p = fma(p, r, 4.1666666666666667e-02); p = fma(p, r, 1.6666666666666667e-01); p = fma(p, r, 0.5); p = fma(p, r, 1.0); p = fma(p, r, 1.0);
+    const double d = fma(p, __hiloint2double((__double2loint(t) + 1023) << 20, 0), 1.0);
+    double y = (double)(1.0f / (float)d);
+    y = fma(y, fma(-d, y, 1.0), y);
+    return (float)(a * y);
+}
+
+__global__ void __launch_bounds__(256) k_dn_prep_seq(DnDims D, uint32_t T, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,
+                                                     const float *qkv, const float *ba, const float *conv_state,
+                                                     float *__restrict__ qk, float *__restrict__ v, float *__restrict__ beta, float *__restrict__ gate) {
     pdl_prologue();
-    __shared__ double red[2][32];
-    const uint32_t tid = threadIdx.x, S = D.S, ns = D.d_conv - 1u;
+    __shared__ double red[8][DN_PREP_TOK], s_inv[DN_PREP_TOK];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, S = D.S, ns = D.d_conv - 1u;
     const uint32_t n_qk = 2u * D.groups, n_v = D.d_inner / S;
-    const uint32_t t_begin = blockIdx.y * DN_PREP_TOK, t_end = min(T, t_begin + DN_PREP_TOK);
+    const uint32_t t_begin = blockIdx.y * DN_PREP_TOK, n = min(DN_PREP_TOK, T - t_begin);
     if (blockIdx.x == n_qk + n_v) {
         const uint32_t width = D.rank / D.groups, stride = 2u * width;
-        for (uint32_t ti = t_begin; ti < t_end; ++ti)
-            for (uint32_t h = tid; h < D.rank; h += blockDim.x) {
-                const uint32_t g = h / width, l = h - g * width;
-                const float *b = ba + (size_t)ti * 2u * D.rank;
-                beta[(size_t)ti * D.rank + h] = (float)sigmoid_stable((double)b[g * stride + l]);
-                gate[(size_t)ti * D.rank + h] = (float)(softplus_stable((double)b[g * stride + width + l] + (double)dt_bias[h]) * (double)ssm_a[h]);
-            }
+        for (uint32_t i = tid; i < n * D.rank; i += blockDim.x) {
+            const uint32_t ti = t_begin + i / D.rank, h = i % D.rank, g = h / width, l = h - g * width;
+            const float *b = ba + (size_t)ti * 2u * D.rank;
+            beta[(size_t)ti * D.rank + h] = (float)sigmoid_stable((double)b[g * stride + l]);
+            gate[(size_t)ti * D.rank + h] = (float)(softplus_stable((double)b[g * stride + width + l] + (double)dt_bias[h]) * (double)ssm_a[h]);
+        }
         return;
     }
     const uint32_t c = blockIdx.x * S + tid;
     const float *cs = conv_state + (size_t)c * ns;
     const float *kr = conv_kernel + (size_t)c * D.d_conv;
-    for (uint32_t ti = t_begin; ti < t_end; ++ti) {
-        double acc = 0.0;
-        for (uint32_t j = 0; j < ns; ++j) {
-            const int tau = (int)ti + (int)j - (int)ns;        // time of tap j relative to the chunk start
-            const float smp = tau < 0 ? cs[(int)ns + tau] : qkv[(size_t)tau * D.channels + c];
-            acc += (double)smp * (double)kr[j];
+    auto sample = [&](int tau) { return tau < 0 ? cs[(int)ns + tau] : qkv[(size_t)tau * D.channels + c]; };        // tau: time relative to the chunk start
+    float y[DN_PREP_TOK];
+    if (D.d_conv == 4u) {                                  // the window slides over registers
+        float x[DN_PREP_TOK + 3u];
+#pragma unroll
+        for (uint32_t i = 0; i < DN_PREP_TOK + 3u; ++i) x[i] = i < n + 3u ? sample((int)(t_begin + i) - 3) : 0.f;
+        const double k0 = (double)kr[0], k1 = (double)kr[1], k2 = (double)kr[2], k3 = (double)kr[3];
+#pragma unroll
+        for (uint32_t i = 0; i < DN_PREP_TOK; ++i) y[i] = dn_silu(fma((double)x[i + 3u], k3, fma((double)x[i + 2u], k2, fma((double)x[i + 1u], k1, (double)x[i] * k0))));
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < DN_PREP_TOK; ++i) {
+            double acc = 0.0;
+            if (i < n) for (uint32_t j = 0; j <= ns; ++j) acc = fma((double)sample((int)(t_begin + i + j) - (int)ns), (double)kr[j], acc);
+            y[i] = dn_silu(acc);
         }
-        acc += (double)qkv[(size_t)ti * D.channels + c] * (double)kr[ns];
-        const float y = (float)(acc / (1.0 + exp(-acc)));
-        if (blockIdx.x >= n_qk) { v[(size_t)ti * D.d_inner + (c - n_qk * S)] = y; continue; }
-        double ss = (double)y * (double)y;
-        for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        double *rd = red[ti & 1u];                             // alternating buffers: one barrier per token
-        if ((tid & 31u) == 0) rd[tid >> 5] = ss;
-        __syncthreads();
-        double tot = 0.0;
-        for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) tot += rd[w];
-        const double inv = 1.0 / fmax(sqrt(tot), (double)D.eps);
-        qk[(size_t)ti * n_qk * S + c] = (float)((double)y * inv);
     }
+    if (blockIdx.x >= n_qk) {
+#pragma unroll
+        for (uint32_t i = 0; i < DN_PREP_TOK; ++i) if (i < n) v[(size_t)(t_begin + i) * D.d_inner + (c - n_qk * S)] = y[i];
+        return;
+    }
+    // the sums of the eight tokens over the warp: while a lane carries more than one, each exchange halves them
+    double a4[4], a2[2], a1;
+    const bool hi4 = lane & 16u, hi3 = lane & 8u, hi2 = lane & 4u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double lo = (double)y[i] * (double)y[i], hi = (double)y[i + 4] * (double)y[i + 4];
+        a4[i] = (hi4 ? hi : lo) + __shfl_xor_sync(0xffffffffu, hi4 ? lo : hi, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) a2[i] = (hi3 ? a4[i + 2] : a4[i]) + __shfl_xor_sync(0xffffffffu, hi3 ? a4[i] : a4[i + 2], 8);
+    a1 = (hi2 ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, hi2 ? a2[0] : a2[1], 4);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, 1);
+    if ((lane & 3u) == 0u) red[tid >> 5][((lane >> 4) & 1u) * 4u + ((lane >> 3) & 1u) * 2u + ((lane >> 2) & 1u)] = a1;
+    __syncthreads();
+    if (tid < DN_PREP_TOK) {
+        double tot = 0.0;
+        for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) tot += red[w][tid];
+        s_inv[tid] = 1.0 / fmax(sqrt(tot), (double)D.eps);
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = 0; i < DN_PREP_TOK; ++i) if (i < n) qk[(size_t)(t_begin + i) * n_qk * S + c] = (float)((double)y[i] * s_inv[i]);
+}
+
+// the gated RMSNorm of a chunk (the arithmetic of k_dn_tail): a warp per token and value head, VPL values a lane. grid = tokens * heads / 8; the rows are the
+// engine's, so aligned. A block of S threads per row with a barrier in it was bound by the scheduling of its blocks: 59 us for 2048 tokens, now 15
+template <uint32_t VPL>
+__global__ void __launch_bounds__(256) k_dn_tail_seq(DnDims D, uint32_t rows, const float *core, const float *z, const float *__restrict__ norm_w, float *__restrict__ out) {
+    pdl_prologue();
+    const uint32_t r = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (r >= rows) return;
+    const size_t idx = (size_t)r * (VPL * 32u) + lane * VPL;
+    struct __align__(VPL > 4u ? 16u : VPL * 4u) Vec { float f[VPL]; };
+    const Vec x = *reinterpret_cast<const Vec *>(core + idx), g = *reinterpret_cast<const Vec *>(z + idx);
+    double ss = 0.0;
+#pragma unroll
+    for (uint32_t i = 0; i < VPL; ++i) ss = fma((double)x.f[i], (double)x.f[i], ss);
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float inv = 1.0f / sqrtf((float)(ss / (double)(VPL * 32u)) + D.eps);
+    Vec o;
+#pragma unroll
+    for (uint32_t i = 0; i < VPL; ++i) o.f[i] = x.f[i] * inv * norm_w[lane * VPL + i] * (g.f[i] / (1.0f + expf(-g.f[i])));
+    *reinterpret_cast<Vec *>(out + idx) = o;
 }
 
 // conv state <- the last d_conv-1 samples of [state, chunk]; one thread per channel
@@ -851,7 +913,13 @@ int launch_deltanet_seq(const DnDims &D, uint32_t T, const float *conv_kernel, c
         RC_LAUNCHED();
     }
     prof_begin("dn_tail", s);
-    RC_LAUNCH((k_dn_tail), dim3(D.rank, T), D.S, 0, s, D, core, z, norm_w, out);
+    const uint32_t rows = D.rank * T, tail_grid = (rows + 7u) / 8u;
+    switch (D.S) {
+        case 32: RC_LAUNCH((k_dn_tail_seq<1>), tail_grid, 256, 0, s, D, rows, (const float *)core, z, norm_w, out); break;
+        case 64: RC_LAUNCH((k_dn_tail_seq<2>), tail_grid, 256, 0, s, D, rows, (const float *)core, z, norm_w, out); break;
+        case 128: RC_LAUNCH((k_dn_tail_seq<4>), tail_grid, 256, 0, s, D, rows, (const float *)core, z, norm_w, out); break;
+        default: RC_LAUNCH((k_dn_tail_seq<8>), tail_grid, 256, 0, s, D, rows, (const float *)core, z, norm_w, out); break;
+    }
     prof_end(s);
     RC_LAUNCHED();
     return 1;

@@ -1,4 +1,4 @@
-"""The row norms of a chunk at the full width: one block of 256 threads a row from 148 rows on, of 1024 below. The same prompt in one chunk
+"""The row norms of a chunk at the full width: a warp a row from 148 rows on, a block of 1024 threads below. The same prompt in one chunk
 and in chunks that take the other form, against the CPU oracle."""
 import os
 
