@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(256) k_dn_prep_seq(DnDims D, uint32_t T, const
 // the gated RMSNorm of a chunk (the arithmetic of k_dn_tail): a warp per token and value head, VPL values a lane. grid = tokens * heads / 8; the rows are the
 // engine's, so aligned. A block of S threads per row with a barrier in it was bound by the scheduling of its blocks: 59 us for 2048 tokens, now 15
 template <uint32_t VPL>
-__global__ void __launch_bounds__(256) k_dn_tail_seq(DnDims D, uint32_t rows, const float *core, const float *z, const float *__restrict__ norm_w, float *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_dn_tail_seq(DnDims D, uint32_t rows, const float *core, const float *z, const float *norm_w, float *__restrict__ out) {
     pdl_prologue();
     const uint32_t r = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (r >= rows) return;
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(256) k_dn_tail_seq(DnDims D, uint32_t rows, co
     const float inv = 1.0f / sqrtf((float)(ss / (double)(VPL * 32u)) + D.eps);
     Vec o;
 #pragma unroll
-    for (uint32_t i = 0; i < VPL; ++i) o.f[i] = x.f[i] * inv * norm_w[lane * VPL + i] * (g.f[i] / (1.0f + expf(-g.f[i])));
+    for (uint32_t i = 0; i < VPL; ++i) o.f[i] = x.f[i] * inv * __ldg(norm_w + lane * VPL + i) * (g.f[i] / (1.0f + expf(-g.f[i])));
     *reinterpret_cast<Vec *>(out + idx) = o;
 }
 

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(THREADS) k_rmsnorm(const float *x, const float
 // The same for the rows of a chunk, a warp each: its loads go out together and no barrier is met. grid = tokens / 4, rows of NV * 128 values, 16-byte aligned.
 // 2048 rows of 2048 values, with and without a branch: 11 and 7 us, a block of 256 threads per row 30 and 21
 template <uint32_t NV>
-__global__ void __launch_bounds__(128) k_rmsnorm_rows(const float *x, const float *branch, const float *__restrict__ w, uint32_t rows, float eps,
+__global__ void __launch_bounds__(128) k_rmsnorm_rows(const float *x, const float *branch, const float *w, uint32_t rows, float eps,
                                                       float *__restrict__ resid_out, float *__restrict__ normed) {
     pdl_prologue();
     const uint32_t r = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
@@ -199,7 +199,7 @@ __global__ void k_attn_prep(const float *qg, const float *kraw, const float *vra
 // The same for the tokens of a chunk (a block each, heads over its warps): the angles are computed once per token instead of by every head, which
 // made the double-precision pow, cos and sin most of the kernel (2048 tokens x 20 heads of 256: 84 us, now 53). hd = 32 VPL, rope_dims <= hd
 template <typename KV, uint32_t VPL>
-__global__ void __launch_bounds__(256) k_attn_prep_rows(const float *qg, const float *kraw, const float *vraw, const float *__restrict__ qn, const float *__restrict__ kn,
+__global__ void __launch_bounds__(256) k_attn_prep_rows(const float *qg, const float *kraw, const float *vraw, const float *qn, const float *kn,
                                                         uint32_t n_head, uint32_t n_kv, uint32_t rope_dims, float freq_base, float eps, const uint32_t *pos_p,
                                                         float *__restrict__ query, float *__restrict__ gate, KV *__restrict__ kcache, KV *__restrict__ vcache) {
     pdl_prologue();
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(256) k_attn_prep_rows(const float *qg, const f
         const double inv = 1.0 / sqrt(ss / (double)hd + (double)eps);
         __syncwarp();                  // the row of the head before has been read
 #pragma unroll
-        for (uint32_t i = 0; i < VPL; ++i) { v[i] = (float)((double)v[i] * inv * (double)nw[lane + 32u * i]); s_row[warp][lane + 32u * i] = v[i]; }
+        for (uint32_t i = 0; i < VPL; ++i) { v[i] = (float)((double)v[i] * inv * (double)__ldg(nw + lane + 32u * i)); s_row[warp][lane + 32u * i] = v[i]; }
         __syncwarp();
 #pragma unroll
         for (uint32_t i = 0; i < VPL; ++i) {

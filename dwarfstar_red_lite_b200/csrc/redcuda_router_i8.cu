@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(512) k_rt_digits_x(const float *x, uint32_t x_
     rt_digits_rows(x + (size_t)t * x_stride, x_stride, t < ntok ? ntok - t : 0u, ncols, xq + (size_t)tile * (ncols / RT_KS) * stage + tt * 16u, stage, tok * 16u, RT_D * tok * 16u, xs + t);
 }
 // grid = experts / 8
-__global__ void __launch_bounds__(512) k_rt_digits_w(const float *__restrict__ w, uint32_t ncols, uint8_t *__restrict__ wq, double *__restrict__ ws) {
+__global__ void __launch_bounds__(512) k_rt_digits_w(const float *w, uint32_t ncols, uint8_t *__restrict__ wq, double *__restrict__ ws) {
     pdl_prologue();
     const uint32_t e = blockIdx.x * 8u, tile = e / 128u, r = e % 128u;
     rt_digits_rows(w + (size_t)e * ncols, ncols, 8u, ncols, wq + (size_t)tile * (ncols / RT_KS) * RT_A_BUF + r * 16u, RT_A_BUF, RT_A_DIGIT, 128u * 16u, ws + e);
