@@ -13,6 +13,7 @@
 // Plain rows (router, scalar gate) are accumulated in double, as everywhere: they decide discrete outcomes.
 #include "redcuda_common.cuh"
 #include "redcuda_kernels.cuh"
+#include "redcuda_moe_mma.cuh"
 #include "redcuda_route.cuh"
 
 namespace rc {
@@ -243,6 +244,109 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1(const __grid_consta
     if (A.tail.ticket) route_tail(A.tail);
 }
 
+// ---- one large Q6_K matrix (the LM head) -------------------------------------------------------------------------------
+// Instruction issue bounds the products of a matrix of that size in floats: a byte permute per weight to make it one. Here x is four 8-bit digits with a
+// power-of-two scale per 256 columns (actw_digits: closer to the row than the rounding of one fp32 product), its digit words in place of the floats, and
+// a word of four 6-bit weights meets them in four dp4a: the sums of 16 columns are exact. The weights stay unsigned (q + 32), an accumulator begins
+// with -32 times its digits' sum. Lanes, rows and loads as in gemv1_q6k. 151936 x 2048: 61 us (floats: 72; 255 MB take 39 at the copy rate)
+constexpr uint32_t G1_DIGIT_ROWS = 16384u;       // rows from which a matrix is taken here; below, quantising x in every block costs more than it saves
+__device__ __forceinline__ int g1_dp4a(uint32_t q, uint32_t x, int c) { int d; asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(q), "r"(x), "r"(c)); return d; }
+
+template <bool NORM>
+__global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1_digits(const __grid_constant__ GemvArgs A) {
+    pdl_trigger();
+    extern __shared__ __align__(16) float g1_xs[];         // x, then its digit words; behind it -32 times the digit sums of every 16 columns
+    __shared__ float s_scale[G1_NCOLS / 256u];
+    const GemvJob &J = A.job[0];
+    const uint32_t row0 = blockIdx.x * J.rows_per_tile, nrow = min(J.rows_per_tile, J.nrows - row0);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, cpr = J.ncols >> 6, bpr = J.ncols >> 8;
+    const uint32_t lpr = g1_lanes(RC_Q6_K, J.ncols), rw = 32u / lpr, slot = lane / lpr, sub = lane % lpr, step = G1_WARPS * rw, first = warp * rw;
+    const uint64_t o_h = rc_q6_qh(J.nb), o_s = rc_q6_sc(J.nb), o_d = rc_q6_d(J.nb);
+    const bool on = sub < cpr;                              // lanes past the row's end repeat its last chunk and add nothing
+    const uint32_t cc = on ? sub : cpr - 1u, bcol = cc >> 2, half = (cc >> 1) & 1u, l0 = (cc & 1u) * 16u;
+    int4 *corr = reinterpret_cast<int4 *>(g1_xs + g1_xi(J.ncols));
+    auto load = [&](uint32_t vr) {
+        vr = min(vr, nrow - 1u);
+        const uint64_t blk = (uint64_t)(row0 + vr) * bpr + bcol;
+        const uint8_t *wl = J.w0 + blk * 128u + half * 64u + l0;
+        Q6Frag f;
+        f.a = __ldg(reinterpret_cast<const uint4 *>(wl));
+        f.b = __ldg(reinterpret_cast<const uint4 *>(wl + 32u));
+        f.h = __ldg(reinterpret_cast<const uint4 *>(J.w0 + o_h + blk * 64u + half * 32u + l0));
+        f.sc = __ldg(reinterpret_cast<const uint2 *>(J.w0 + o_s + blk * 16u + half * 8u));
+        f.d = __ldg(reinterpret_cast<const unsigned short *>(J.w0 + o_d) + blk);
+        return f;
+    };
+    Q6Frag f[2];
+    if (A.resident) { f[0] = load(first + slot); f[1] = load(first + step + slot); }
+    pdl_wait();
+    gemv1_stage<NORM>(A, J.ncols, g1_xs);
+    if (!A.resident) { f[0] = load(first + slot); f[1] = load(first + step + slot); }
+    __syncthreads();
+    for (uint32_t b = warp; b < bpr; b += G1_WARPS) {       // a warp per 256 columns, eight neighbouring values a lane
+        float4 *p = reinterpret_cast<float4 *>(g1_xs + g1_xi(b * 256u + lane * 8u));
+        const float4 v0 = p[0], v1 = p[1];
+        float up;
+        const float scale = actw_scale(__reduce_max_sync(0xffffffffu, max(act_mag4(v0), act_mag4(v1))), up);
+        if (lane == 0) s_scale[b] = scale;
+        const uint32_t w0[4] = {actw_digits(v0.x, up), actw_digits(v0.y, up), actw_digits(v0.z, up), actw_digits(v0.w, up)};
+        const uint32_t w1[4] = {actw_digits(v1.x, up), actw_digits(v1.y, up), actw_digits(v1.z, up), actw_digits(v1.w, up)};
+        uint32_t p0[4], p1[4];
+        actw_planes(w0, p0); actw_planes(w1, p1);
+        reinterpret_cast<uint4 *>(p)[0] = make_uint4(p0[0], p0[1], p0[2], p0[3]); reinterpret_cast<uint4 *>(p)[1] = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+        int c[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            c[i] = __dp4a((int)p0[i], 0x01010101, __dp4a((int)p1[i], 0x01010101, 0));
+            c[i] = -32 * (c[i] + __shfl_xor_sync(0xffffffffu, c[i], 1));
+        }
+        if (!(lane & 1u)) corr[b * 16u + (lane >> 1)] = make_int4(c[0], c[1], c[2], c[3]);
+    }
+    __syncthreads();
+    const uint4 *xl = reinterpret_cast<const uint4 *>(g1_xs + bcol * 268u + half * 136u + l0);
+    const int4 *cl = corr + (bcol * 256u + half * 128u + l0) / 16u;
+    const float xscale = s_scale[bcol];
+    for (uint32_t base = first; base < nrow; base += 2u * step) {
+        float acc[2] = {0.f, 0.f};
+        const uint32_t sq = l0 ? 8u : 0u;                   // the four scales of this lane's runs of 16 sit in every other byte of its half block
+#pragma unroll
+        for (int qd = 0; qd < 4; ++qd) {
+            const int4 c0 = cl[2 * qd];
+            int s[2][4] = {{c0.x, c0.y, c0.z, c0.w}, {c0.x, c0.y, c0.z, c0.w}};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const uint4 xd = xl[8 * qd + w];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const uint32_t a = w == 0 ? f[r].a.x : w == 1 ? f[r].a.y : w == 2 ? f[r].a.z : f[r].a.w, b = w == 0 ? f[r].b.x : w == 1 ? f[r].b.y : w == 2 ? f[r].b.z : f[r].b.w;
+                    const uint32_t h = w == 0 ? f[r].h.x : w == 1 ? f[r].h.y : w == 2 ? f[r].h.z : f[r].h.w;
+                    const uint32_t v = qd == 0 ? (a & 0x0F0F0F0Fu) | ((h << 4) & 0x30303030u) : qd == 1 ? (b & 0x0F0F0F0Fu) | ((h << 2) & 0x30303030u)
+                                     : qd == 2 ? ((a >> 4) & 0x0F0F0F0Fu) | (h & 0x30303030u) : ((b >> 4) & 0x0F0F0F0Fu) | ((h >> 2) & 0x30303030u);
+                    s[r][0] = g1_dp4a(v, xd.x, s[r][0]); s[r][1] = g1_dp4a(v, xd.y, s[r][1]); s[r][2] = g1_dp4a(v, xd.z, s[r][2]); s[r][3] = g1_dp4a(v, xd.w, s[r][3]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {                   // |digit sum| < 2^18: the upper and the lower two are exact as integers, the lower as a float too
+                const uint32_t word = qd < 2 ? f[r].sc.x : f[r].sc.y;
+                const float sc = (float)(int)(signed char)(word >> (sq + 16u * (qd & 1)));
+                acc[r] = fmaf(sc, fmaf(65536.0f, (float)(256 * s[r][3] + s[r][2]), (float)(256 * s[r][1] + s[r][0])), acc[r]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) acc[r] = on ? acc[r] * (__half2float(__ushort_as_half(f[r].d)) * xscale) : 0.f;
+        if (base + 2u * step < nrow) { f[0] = load(base + 2u * step + slot); f[1] = load(base + 3u * step + slot); }      // on the way during the reduction
+        for (uint32_t o = lpr >> 1; o; o >>= 1) { acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o); acc[1] += __shfl_xor_sync(0xffffffffu, acc[1], o); }
+        if (sub == 0u) {
+            if (base + slot < nrow) J.out[row0 + base + slot] = acc[0];
+            if (base + step + slot < nrow) J.out[row0 + base + step + slot] = acc[1];
+        }
+    }
+}
+static bool gemv1_digits_ok(const GemvArgs &A) {
+    const GemvJob &J = A.job[0];
+    return A.njobs == 1u && J.type == RC_Q6_K && J.epi == GEMV_STORE && J.ncols <= G1_NCOLS && J.nrows >= G1_DIGIT_ROWS && !A.tail.ticket;
+}
+
 // One token and rows that k_gemv1 holds; the other block types stay with the general kernel.
 bool gemv1_ok(const GemvArgs &A) {
     if (A.ntok != 1u || ((uintptr_t)A.x & 15u)) return false;
@@ -294,6 +398,14 @@ int launch_gemv1(GemvArgs &A, cudaStream_t stream) {
     A.part_doubles = (uint32_t)(smem / sizeof(double));
     if (q6 || A.norm.w) smem += (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + 16u;
     prof_begin(A.tag ? A.tag : "gemv", stream);
+    if (gemv1_digits_ok(A)) {
+        smem = (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + (size_t)(A.job[0].ncols / 16u) * sizeof(int4) + 16u;
+        if (A.norm.w) RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1_digits<true>), tiles, G1_WARPS * 32u, smem, stream, A);
+        else RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1_digits<false>), tiles, G1_WARPS * 32u, smem, stream, A);
+        prof_end(stream);
+        RC_LAUNCHED();
+        return 1;
+    }
     // weights that a kernel before this one has just laid out are read by the non-coherent path like others: then behind that kernel's end
     if (A.norm.w) RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1<true>), tiles, G1_WARPS * 32u, smem, stream, A);
     else RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1<false>), tiles, G1_WARPS * 32u, smem, stream, A);
