@@ -179,42 +179,95 @@ __device__ __forceinline__ void tc_decode_stage_f32(const float *w, uint32_t nco
 
 // x [ntok][ncols] fp32 (or SiLU(x) * x2 when x2 is given) -> fp16 digits in the order the GEMM stages consume them:
 // xs[token tile][k stage][k chunk of 8 (8)][digit hi/lo][token group of 8 (TN/8)][token in group (8)][8 halves];
-// x_inv[t] = 2^-e_t undoes the per-token scale. Tokens beyond ntok are zero. grid = token tiles * TN, block = 256
-__global__ void k_tc_prep_x(const float *x, const float *x2, uint32_t x_stride, uint32_t ntok, uint32_t ncols, uint32_t tn,
-                            __half *__restrict__ xs, float *__restrict__ x_inv) {
+// x_inv[t] = 2^-e_t undoes the per-token scale. Tokens beyond ntok are zero. A warp per token, a block per group of eight: a row is read
+// once (up to 256 NCH columns stay in registers; NCH = 0: read again for the digits) in 16-byte pieces, and the group's 16-byte chunks are
+// turned in shared memory so that eight tokens write the 128 bytes that lie together. Memory bounds it: 2048 tokens of 2048 columns (and 512 of the shared
+// expert's down) 17.0 -> 10.7 us a launch on average, a prompt's launches of 512 to 4096 columns 20.6 -> 13.2, against a block per token that
+// read its row twice and stored 16 bytes at a time. grid = token tiles * TN / 8, block = 256
+template <uint32_t NCH>
+__global__ void __launch_bounds__(256) k_tc_prep_x(const float *x, const float *x2, uint32_t x_stride, uint32_t ntok, uint32_t ncols, uint32_t tn,
+                                                   __half *xs, float *x_inv) {
     pdl_prologue();
-    __shared__ float red[8];
-    const uint32_t t = blockIdx.x, tid = threadIdx.x;
+    __shared__ uint4 turn[2][2][32][9];                        // [step parity][digit][chunk of the step][token + pad]
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, t = blockIdx.x * 8u + warp;
     const bool live = t < ntok;
+    const float *xr = x + (size_t)(live ? t : 0u) * x_stride, *x2r = x2 ? x2 + (size_t)(live ? t : 0u) * x_stride : nullptr;
+    const bool vec = ((size_t)xr & 15u) == 0u;                 // a caller's rows may begin at any float
+    auto load = [&](uint32_t k, float (&v)[8]) {
+#pragma unroll
+        for (uint32_t h = 0; h < 2u; ++h) {
+            const float *q = xr + k + 4u * h;
+            const float4 a = vec ? *reinterpret_cast<const float4 *>(q) : make_float4(q[0], q[1], q[2], q[3]);
+            v[4 * h] = a.x; v[4 * h + 1] = a.y; v[4 * h + 2] = a.z; v[4 * h + 3] = a.w;
+            if (x2r) {
+                const float4 b = *reinterpret_cast<const float4 *>(x2r + k + 4u * h);
+                v[4 * h] = silu_mul(a.x, b.x); v[4 * h + 1] = silu_mul(a.y, b.y); v[4 * h + 2] = silu_mul(a.z, b.z); v[4 * h + 3] = silu_mul(a.w, b.w);
+            }
+        }
+    };
+    float row[NCH ? NCH : 1u][8];
     float mx = 0.f;
-    auto val = [&](uint32_t k) { const size_t i = (size_t)t * x_stride + k; return x2 ? silu_mul(x[i], x2[i]) : x[i]; };
-    if (live) for (uint32_t k = tid; k < ncols; k += blockDim.x) mx = fmaxf(mx, fabsf(val(k)));
+    if constexpr (NCH != 0u) {
+#pragma unroll
+        for (uint32_t i = 0; i < NCH; ++i) {
+            const uint32_t k = i * 256u + lane * 8u;
+            if (live && k < ncols) load(k, row[i]);
+            else
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; ++j) row[i][j] = 0.f;
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < NCH; ++i)
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; ++j) mx = fmaxf(mx, fabsf(row[i][j]));
+    } else if (live) {
+        for (uint32_t k = lane * 8u; k < ncols; k += 256u) {
+            load(k, row[0]);
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; ++j) mx = fmaxf(mx, fabsf(row[0][j]));
+        }
+    }
     for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31u) == 0) red[tid >> 5] = mx;
-    __syncthreads();
-    mx = 0.f;
-    for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) mx = fmaxf(mx, red[w]);
     int e = 0;
     if (mx > 0.f && mx < INFINITY) { int ex; frexpf(mx, &ex); e = 14 - ex; }     // max |x| * 2^e in [2^13, 2^14)
     e = e > 100 ? 100 : e < -100 ? -100 : e;
     const float sc = exp2f((float)e);
-    if (tid == 0) x_inv[t] = exp2f((float)-e);
-    const uint32_t tile = t / tn, tt = t - tile * tn, nstage = ncols / TC_KS;
+    if (lane == 0) x_inv[t] = exp2f((float)-e);
+    const uint32_t g = blockIdx.x * 8u / tn, tt = blockIdx.x * 8u - g * tn, nstage = ncols / TC_KS;      // token tile, the group's first token in it
     const size_t digit = (size_t)tn * TC_KS;                   // halves of one digit of one stage
-    for (uint32_t c = tid; c < ncols / 8u; c += blockDim.x) {  // one 16-byte k-chunk per iteration
-        const uint32_t stage = c >> 3, kc = c & 7u;
-        __half hi[8], lo[8];
+    auto step = [&](uint32_t i, const float (&v)[8]) {         // columns [256 i, 256 i + 256)
+        uint4 d[2];
+        __half *hi = reinterpret_cast<__half *>(&d[0]), *lo = reinterpret_cast<__half *>(&d[1]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float v = live ? val(c * 8u + j) * sc : 0.f;
-            hi[j] = __float2half_rn(v);
-            lo[j] = __float2half_rn(v - __half2float(hi[j]));
+        for (uint32_t j = 0; j < 8u; ++j) {
+            const float s = v[j] * sc;
+            hi[j] = __float2half_rn(s);
+            lo[j] = __float2half_rn(s - __half2float(hi[j]));
         }
+        turn[i & 1u][0][lane][warp] = d[0];
+        turn[i & 1u][1][lane][warp] = d[1];
+        __syncthreads();                                       // one a step: the other parity's readers are past the step before
+        const uint32_t c = tid >> 3, stage = i * (256u / TC_KS) + (c >> 3), kc = c & 7u;
         // inside a stage: [k chunk][2 tn rows: the hi digits of the tn tokens, then their lo digits][8 halves], so that one MMA
         // of N = 2 tn takes both digits and one of N = tn the hi digits alone
-        __half *dst = xs + ((size_t)tile * nstage + stage) * 2u * digit + ((size_t)kc * (tn >> 2) + (tt >> 3)) * 64u + (tt & 7u) * 8u;
-        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(hi);
-        *reinterpret_cast<uint4 *>(dst + (size_t)tn * 8u) = *reinterpret_cast<const uint4 *>(lo);
+        if (stage < nstage) {
+            __half *dst = xs + ((size_t)g * nstage + stage) * 2u * digit + ((size_t)kc * (tn >> 2) + (tt >> 3)) * 64u + (tid & 7u) * 8u;
+            *reinterpret_cast<uint4 *>(dst) = turn[i & 1u][0][c][tid & 7u];
+            *reinterpret_cast<uint4 *>(dst + (size_t)tn * 8u) = turn[i & 1u][1][c][tid & 7u];
+        }
+    };
+    if constexpr (NCH != 0u) {
+#pragma unroll
+        for (uint32_t i = 0; i < NCH; ++i) if (i * 256u < ncols) step(i, row[i]);
+    } else {
+        for (uint32_t i = 0; i * 256u < ncols; ++i) {
+            const uint32_t k = i * 256u + lane * 8u;
+            if (live && k < ncols) load(k, row[0]);
+            else
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; ++j) row[0][j] = 0.f;
+            step(i, row[0]);
+        }
     }
 }
 
@@ -450,7 +503,12 @@ int launch_tc_prep_x(const float *x, const float *x2, uint32_t x_stride, uint32_
     RC_REQUIRE(tn == 32u || tn == 64u || tn == 128u, "tc gemm: token tile %u is not 32, 64 or 128", tn);
     const uint32_t tiles = (ntok + tn - 1u) / tn;
     prof_begin("tc_prep_x", s);
-    RC_LAUNCH((k_tc_prep_x), tiles * tn, 256, 0, s, x, x2, x_stride, ntok, ncols, tn, xs, x_inv);
+    const uint32_t grid = tiles * tn / 8u;
+    // rows of 2048 columns read a second time: 11.9 us a launch where registers take 10.7; rows of 4096 in registers (158 a thread): 13.7 on
+    // average over a prompt's launches where reading them again takes 13.2
+    if (ncols <= 512u) RC_LAUNCH((k_tc_prep_x<2>), grid, 256, 0, s, x, x2, x_stride, ntok, ncols, tn, xs, x_inv);
+    else if (ncols <= 2048u) RC_LAUNCH((k_tc_prep_x<8>), grid, 256, 0, s, x, x2, x_stride, ntok, ncols, tn, xs, x_inv);
+    else RC_LAUNCH((k_tc_prep_x<0>), grid, 256, 0, s, x, x2, x_stride, ntok, ncols, tn, xs, x_inv);
     prof_end(s);
     RC_LAUNCHED();
     return 1;
