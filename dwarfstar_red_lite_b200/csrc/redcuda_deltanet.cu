@@ -487,14 +487,19 @@ __global__ void __launch_bounds__(256) k_dn_state_seq(DnDims D, uint32_t T, cons
 // eight tokens run through a branch-free unrolled body; the block's decays, betas and v are fetched before its first
 // token, a token's q and the next token's k before the exchange that the chain waits for, and the eight output sums are
 // reduced together after the block. RC_DN_SCAN=warp selects k_dn_state_seq for comparison.
+// What bounds it is one warp per scheduler with a chain of about 400 cycles a token, 161 instructions of which 64 are packed fp32 (two cycles each). One
+// block an SM is said to the compiler (the second launch bound): it then takes 206 registers instead of 128 and has loads and the rows' chains further ahead.
+// With the token in two halves over arrays of the rows, up to the exchange and from it: 2048 tokens 501 -> 447 us (471 by the bound alone); 512 tokens
+// of states 256, 64, 32 wide 224 -> 214, 129 -> 121, 77 -> 70. The same to the bit. Tried on that: k of eight tokens as separate values 473; one exchange of three
+// steps for both rows 492; one barrier a block with a third buffer 484; loads pinned to their token 455; the rows half a token apart: the same code.
 template <uint32_t S, uint32_t CPT, uint32_t RPT, uint32_t WARPS>
-__global__ void __launch_bounds__(WARPS * 32u) k_dn_scan(DnDims D, uint32_t T, const float *qk, const float *v,
+__global__ void __launch_bounds__(WARPS * 32u, 1) k_dn_scan(DnDims D, uint32_t T, const float *qk, const float *v,
                                                          const float *beta, const float *gate,
                                                          float *__restrict__ state, float *__restrict__ core) {
     pdl_prologue();
     constexpr uint32_t LPR = S / CPT, RPW = 32u / LPR, RB = RPW * RPT * WARPS, NP = CPT / 4u, NT = WARPS * 32u, V4 = S / 4u;
     static_assert(LPR == 2u || LPR == 4u || LPR == 8u || LPR == 16u || LPR == 32u, "lanes per row");
-    static_assert(S % RB == 0u && RB % 4u == 0u && DN_TB == 8u, "rows per block");
+    static_assert(S % RB == 0u && RB % 4u == 0u && DN_TB == 8u && RPT <= 2u, "rows per block");
     __shared__ __align__(16) float s_q[2][DN_TB][S], s_k[2][DN_TB][S];
     __shared__ __align__(16) float s_v[2][RB][DN_TB];            // v by (row, token): a thread reads its row's eight values as two float4
     __shared__ __align__(16) float s_b[2][DN_TB], s_g[2][DN_TB];
@@ -560,83 +565,77 @@ __global__ void __launch_bounds__(WARPS * 32u) k_dn_scan(DnDims D, uint32_t T, c
                 vv[a][0] = v0.x; vv[a][1] = v0.y; vv[a][2] = v0.z; vv[a][3] = v0.w; vv[a][4] = v1.x; vv[a][5] = v1.y; vv[a][6] = v1.z; vv[a][7] = v1.w;
             }
         }
-        float op[RPT][DN_TB];
-        float4 kc[NP], kn[NP], qc[NP];
+        float op[RPT][DN_TB], x[RPT][LPR <= 8u ? LPR : 1u];
+        float4 kk[2][NP], qq[NP];                                // k by token parity
+        auto load = [&](float4 (&to)[NP], const float *from) {
 #pragma unroll
-        for (uint32_t i = 0; i < NP; ++i) kc[i] = *reinterpret_cast<const float4 *>(&s_k[buf][0][4u * (i * LPR + p)]);
+            for (uint32_t i = 0; i < NP; ++i) to[i] = *reinterpret_cast<const float4 *>(from + 4u * (i * LPR + p));
+        };
+        auto dot = [&](const float2 (&mr)[CPT / 2u], const float4 (&c)[NP]) {
+            float2 s2 = __fmul2_rn(mr[0], make_float2(c[0].x, c[0].y));
+            if constexpr (NP == 1u) {
+                s2 = __ffma2_rn(mr[1], make_float2(c[0].z, c[0].w), s2);
+            } else {
+                float2 pb = __fmul2_rn(mr[1], make_float2(c[0].z, c[0].w));
+#pragma unroll
+                for (uint32_t i = 1; i < NP; ++i) {
+                    s2 = __ffma2_rn(mr[2u * i], make_float2(c[i].x, c[i].y), s2);
+                    pb = __ffma2_rn(mr[2u * i + 1u], make_float2(c[i].z, c[i].w), pb);
+                }
+                s2 = __fadd2_rn(s2, pb);
+            }
+            return s2.x + s2.y;
+        };
+        // row a, token tt, up to the exchange: decay, dot with k, partial sums on their way
+        auto begin = [&](uint32_t a, uint32_t tt) {
+            const float2 d2 = make_float2(dec[tt], dec[tt]);
+#pragma unroll
+            for (uint32_t i = 0; i < 2u * NP; ++i) m[a][i] = __fmul2_rn(m[a][i], d2);
+            float sum = dot(m[a], kk[tt & 1u]);
+            if constexpr (LPR <= 8u) {
+                // one exchange step instead of log2(LPR) dependent ones: every lane of the row fetches all LPR partial sums
+                // and adds them in the same order (so the row's lanes agree to the bit)
+#pragma unroll
+                for (uint32_t l = 0; l < LPR; ++l) x[a][l] = __shfl_sync(0xffffffffu, sum, (int)((lane & ~(LPR - 1u)) + l));
+            } else {
+#pragma unroll
+                for (uint32_t o = LPR / 2u; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, (int)o);
+                x[a][0] = sum;
+            }
+        };
+        // ... and from there: correction, update, dot with q
+        auto finish = [&](uint32_t a, uint32_t tt) {
+            if constexpr (LPR <= 8u) {
+#pragma unroll
+                for (uint32_t w = LPR; w > 1u; w >>= 1)
+#pragma unroll
+                    for (uint32_t l = 0; l < w / 2u; ++l) x[a][l] = x[a][2u * l] + x[a][2u * l + 1u];
+            }
+            const float delta = (vv[a][tt] - x[a][0]) * bt[tt];
+            const float2 e2 = make_float2(delta, delta);
+#pragma unroll
+            for (uint32_t i = 0; i < NP; ++i) {
+                m[a][2u * i] = __ffma2_rn(make_float2(kk[tt & 1u][i].x, kk[tt & 1u][i].y), e2, m[a][2u * i]);
+                m[a][2u * i + 1u] = __ffma2_rn(make_float2(kk[tt & 1u][i].z, kk[tt & 1u][i].w), e2, m[a][2u * i + 1u]);
+            }
+            op[a][tt] = dot(m[a], qq);
+        };
+        load(kk[0], &s_k[buf][0][0]);
 #pragma unroll
         for (uint32_t tt = 0; tt < DN_TB; ++tt) {
 #pragma unroll
             for (uint32_t a = 0; a < RPT; ++a) op[a][tt] = 0.f;
+        }
+#pragma unroll
+        for (uint32_t tt = 0; tt < DN_TB; ++tt) {
             if (FULL || tt < n) {
-                // this token's q and the next token's k are requested before the reduction that the chain waits for
+                // this token's q and the next token's k are requested before the exchange that the chain waits for
+                load(qq, &s_q[buf][tt][0]);
+                if (tt + 1u < DN_TB) load(kk[(tt + 1u) & 1u], &s_k[buf][tt + 1u][0]);
 #pragma unroll
-                for (uint32_t i = 0; i < NP; ++i) {
-                    qc[i] = *reinterpret_cast<const float4 *>(&s_q[buf][tt][4u * (i * LPR + p)]);
-                    if (tt + 1u < DN_TB) kn[i] = *reinterpret_cast<const float4 *>(&s_k[buf][tt + 1u][4u * (i * LPR + p)]);
-                }
-                const float2 d2 = make_float2(dec[tt], dec[tt]);
-                float delta[RPT];
+                for (uint32_t a = 0; a < RPT; ++a) begin(a, tt);
 #pragma unroll
-                for (uint32_t a = 0; a < RPT; ++a) {
-#pragma unroll
-                    for (uint32_t i = 0; i < 2u * NP; ++i) m[a][i] = __fmul2_rn(m[a][i], d2);
-                    float2 s2 = __fmul2_rn(m[a][0], make_float2(kc[0].x, kc[0].y));
-                    if constexpr (NP == 1u) {
-                        s2 = __ffma2_rn(m[a][1], make_float2(kc[0].z, kc[0].w), s2);
-                    } else {
-                        float2 pb = __fmul2_rn(m[a][1], make_float2(kc[0].z, kc[0].w));
-#pragma unroll
-                        for (uint32_t i = 1; i < NP; ++i) {
-                            s2 = __ffma2_rn(m[a][2u * i], make_float2(kc[i].x, kc[i].y), s2);
-                            pb = __ffma2_rn(m[a][2u * i + 1u], make_float2(kc[i].z, kc[i].w), pb);
-                        }
-                        s2 = __fadd2_rn(s2, pb);
-                    }
-                    float sum = s2.x + s2.y;
-                    if constexpr (LPR <= 8u) {
-                        // one exchange step instead of log2(LPR) dependent ones: every lane of the row fetches all LPR partial sums
-                        // and adds them in the same order (so the row's lanes agree to the bit)
-                        float x[LPR];
-#pragma unroll
-                        for (uint32_t l = 0; l < LPR; ++l) x[l] = __shfl_sync(0xffffffffu, sum, (int)((lane & ~(LPR - 1u)) + l));
-#pragma unroll
-                        for (uint32_t w = LPR; w > 1u; w >>= 1)
-#pragma unroll
-                            for (uint32_t l = 0; l < w / 2u; ++l) x[l] = x[2u * l] + x[2u * l + 1u];
-                        sum = x[0];
-                    } else {
-#pragma unroll
-                        for (uint32_t o = LPR / 2u; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, (int)o);
-                    }
-                    delta[a] = (vv[a][tt] - sum) * bt[tt];
-                }
-#pragma unroll
-                for (uint32_t a = 0; a < RPT; ++a) {
-                    const float2 e2 = make_float2(delta[a], delta[a]);
-#pragma unroll
-                    for (uint32_t i = 0; i < NP; ++i) {
-                        m[a][2u * i] = __ffma2_rn(make_float2(kc[i].x, kc[i].y), e2, m[a][2u * i]);
-                        m[a][2u * i + 1u] = __ffma2_rn(make_float2(kc[i].z, kc[i].w), e2, m[a][2u * i + 1u]);
-                    }
-                    float2 s2 = __fmul2_rn(m[a][0], make_float2(qc[0].x, qc[0].y));
-                    if constexpr (NP == 1u) {
-                        s2 = __ffma2_rn(m[a][1], make_float2(qc[0].z, qc[0].w), s2);
-                    } else {
-                        float2 pb = __fmul2_rn(m[a][1], make_float2(qc[0].z, qc[0].w));
-#pragma unroll
-                        for (uint32_t i = 1; i < NP; ++i) {
-                            s2 = __ffma2_rn(m[a][2u * i], make_float2(qc[i].x, qc[i].y), s2);
-                            pb = __ffma2_rn(m[a][2u * i + 1u], make_float2(qc[i].z, qc[i].w), pb);
-                        }
-                        s2 = __fadd2_rn(s2, pb);
-                    }
-                    op[a][tt] = s2.x + s2.y;
-                }
-                if (tt + 1u < DN_TB) {
-#pragma unroll
-                    for (uint32_t i = 0; i < NP; ++i) kc[i] = kn[i];
-                }
+                for (uint32_t a = 0; a < RPT; ++a) finish(a, tt);
             }
         }
         // the eight output sums over the row's LPR lanes: while a lane carries more than one value each exchange halves them,
@@ -891,7 +890,7 @@ int launch_deltanet_seq(const DnDims &D, uint32_t T, const float *conv_kernel, c
             case 32: RC_LAUNCH((k_dn_scan<32, 16, 1, 2>), D.rank, 64, 0, s, D, Tr, qk_r, v_r, b_r, g_r, rec_state, core_r); break;
             case 64: RC_LAUNCH((k_dn_scan<64, 16, 1, 8>), D.rank, 256, 0, s, D, Tr, qk_r, v_r, b_r, g_r, rec_state, core_r); break;
             // 128-wide states: two rows per thread halve the shared-memory reads of k and q per multiply-add; measured on 2048-token
-            // chunks this tile took 0.50 ms, one row per thread 0.53-0.54 ms, wider lane groups (4 or 8 columns per thread) 0.58-0.70 ms
+            // chunks this tile takes 0.45 ms, one row of 16 or 32 columns per thread 0.52 and 0.48 ms, two rows of 8 columns 0.47 ms
             case 128: RC_LAUNCH((k_dn_scan<128, 16, 2, 4>), D.rank * 4u, 128, 0, s, D, Tr, qk_r, v_r, b_r, g_r, rec_state, core_r); break;
             default: RC_LAUNCH((k_dn_scan<256, 32, 1, 8>), D.rank * 8u, 256, 0, s, D, Tr, qk_r, v_r, b_r, g_r, rec_state, core_r); break;
         }
