@@ -356,16 +356,16 @@ static uint32_t moe_item_tokens(const redcuda_moe *m, bool single_token, uint32_
 // Which expert kernels serve a call of npairs pairs (all_local: every pair belongs to this shard; otherwise the share
 // expert_count / n_expert of them): the tcgen05 kernel works on items of up to 48 pairs of one expert and decodes an
 // expert's weights once per item, so it needs experts that see several pairs each. RC_MOE_TC_MIN = pairs per expert from which it is
-// used (default 11; 0 = never). Its error against 64-bit sums is no larger than that of the integer kernels (outputs of an expert, rows of 2048
+// used (0 = never; by default 8 an expert and 400 more, since what it adds besides the experts' decode does not shrink with their number). Its error against 64-bit sums is no larger than that of the integer kernels (outputs of an expert, rows of 2048
 // Gaussian values 2.98e-7 and 2.99e-7; with one element of 1000 3.1e-7 and 2.2e-6; log-normal 3.7e-7 and 2.0e-6), so the line lies where it gets
-// faster. us a layer of 512 experts, integer kernels -> this: 400 tokens 358 -> 407, 500 413 -> 420, 600 468 -> 453, 700 525 -> 472, 1000 697 -> 513,
-// 1400 943 -> 612, 2048 1343 -> 763; Zipf routing 400 341 -> 373, 600 443 -> 425; 256 experts 300 tokens 275 -> 254; 128 experts (hidden 1024) 200
-// tokens 129 -> 113.
+// faster. us a layer, integer kernels -> this: 512 experts 400 tokens 345 -> 355, 430 361 -> 372, 470 388 -> 367, 500 405 -> 370, 700 525 -> 472, 1000
+// 697 -> 513, 2048 1343 -> 690; Zipf routing 400 330 -> 329, 450 349 -> 342; hidden 1024 400 213 -> 211, 450 225 -> 219; 256 experts 256 tokens 234 -> 218,
+// hidden 1024 240 tokens 141 -> 138; 128 experts 110 tokens 130 -> 149, 141 152 -> 145, 200 180 -> 148, hidden 1024 141 tokens 103 -> 104, 180 113 -> 103.
 static void moe_choose_path(redcuda_moe *m, uint32_t npairs, bool all_local) {
     const char *v = getenv("RC_MOE_TC_MIN");
-    const uint32_t min_avg = v ? (uint32_t)atoi(v) : 11u;
+    const uint32_t min_avg = v ? (uint32_t)atoi(v) : 8u;
     const uint64_t local = all_local ? npairs : (uint64_t)npairs * m->d.expert_count / m->d.n_expert;
-    m->tc_now = m->tc_ok && min_avg && local >= (uint64_t)min_avg * m->d.expert_count;
+    m->tc_now = m->tc_ok && min_avg && local >= (uint64_t)min_avg * m->d.expert_count + (v ? 0u : 400u);
 }
 // tensor-core path of the shared expert: Q6_K and at least 3 tokens (below that the CUDA-core GEMV wins)
 static bool moe_shared_mma(const redcuda_moe *m, uint32_t ntok) {
