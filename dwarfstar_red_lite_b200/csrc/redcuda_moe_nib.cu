@@ -333,8 +333,9 @@ __global__ void __launch_bounds__(NIB_WARPS * 32u, 1) k_nib_one(const __grid_con
 // records arrive by bulk copy while the warp quantises expert k's activation row), the last two warps take the shared
 // expert's 16 rows (Q6_K, CUDA cores). Partial rows meet in shared memory and are summed in router order.
 constexpr uint32_t NIB_TAIL_MAX_K = 14u;
+// One block an SM is all there is (the second launch bound): with registers for loads further ahead a decode step of 16 layers takes 597 us instead of 609
 template <uint32_t FMT, uint32_t NCOLS>
-__global__ void __launch_bounds__((NIB_TAIL_MAX_K + 2u) * 32u) k_nib_down_tail(const __grid_constant__ NibTailArgs A) {
+__global__ void __launch_bounds__((NIB_TAIL_MAX_K + 2u) * 32u, 1) k_nib_down_tail(const __grid_constant__ NibTailArgs A) {
     pdl_prologue();
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr uint32_t BPR = NCOLS / 256u, BPITCH = NCOLS + 32u, PER_LANE = NCOLS / 32u, ND = FMT == NIB_IQ2 ? 3u : 4u;      // ND: digits of a value
