@@ -326,6 +326,11 @@ struct redcuda_moe {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_quant = nullptr;
 };
 
+// integer router logits (moe_router_i8): the digits of the router are made only for a layer that can see so many tokens at once, or where RC_ROUTER_I8_MIN asks
+constexpr uint32_t RT_MIN_TOKENS = 640u, RT_MIN_EXPERTS = 512u;
+static bool moe_wants_rt(const redcuda_moe_desc &d) {
+    return rt_shape_ok(d.n_expert, d.hidden) && (getenv("RC_ROUTER_I8_MIN") || (d.max_tokens >= RT_MIN_TOKENS && d.n_expert >= RT_MIN_EXPERTS));
+}
 // Layers with IQ3_S matrices take their activations as wide digits: they ran on fp32 activations before the nibble layout held them,
 // and the 24-bit form per row is less than that (relative error of an expert's output against 64-bit sums, hidden 2048: fp32 1.6e-7 on any
 // row; three digits 3.1e-7 on Gaussian rows, 2.2e-6 with one element of 100, 4.7e-4 with a large one where the weights vanish; wide
@@ -395,7 +400,7 @@ static bool moe_router_tc(const redcuda_moe *m, uint32_t ntok) {
 static bool moe_router_i8(const redcuda_moe *m, uint32_t ntok) {
     if (!m->rt_q) return false;
     if (const char *v = getenv("RC_ROUTER_I8_MIN")) return atoi(v) && ntok >= (uint32_t)atoi(v);
-    return ntok >= 640u && m->d.n_expert >= 512u;
+    return ntok >= RT_MIN_TOKENS && m->d.n_expert >= RT_MIN_EXPERTS;
 }
 // out[j][t][row] = W_j x[t] for one or two matrices that share x (x2: the input is SiLU(x) * x2)
 static int moe_shared_tc_gemm(redcuda_moe *m, uint32_t ntok, const float *x, const float *x2, uint32_t ncols, const DMat *w0, float *out0, const DMat *w1, float *out1,
@@ -695,7 +700,7 @@ static size_t moe_ws_layout(const redcuda_moe_desc &d, redcuda_moe *m, uint8_t *
         put(r.rt_xs, tc_xs_halves((uint32_t)T, d.hidden, 128u) * 2u); put(r.rt_xinv, (T + 128u) * 4u);
         put(r.rt_wd, tc_wd_bytes(tc_row_tiles(d.n_expert), d.hidden)); put(r.rt_winv, (size_t)tc_row_tiles(d.n_expert) * 4u);
     }
-    if (rt_shape_ok(d.n_expert, d.hidden)) { put(r.rt_xq, rt_xq_bytes((uint32_t)T, d.hidden)); put(r.rt_xsc, rt_xs_doubles((uint32_t)T) * sizeof(double)); }
+    if (moe_wants_rt(d)) { put(r.rt_xq, rt_xq_bytes((uint32_t)T, d.hidden)); put(r.rt_xsc, rt_xs_doubles((uint32_t)T) * sizeof(double)); }
     if (m) { m->ticket = m->work + 2; m->tc_err = m->work + 3; }
     return w;
 }
@@ -837,7 +842,7 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
     ok = ok && put(d.type_gu, d.ffn, d.hidden, raw_gu, d.gate_exps, m->gate, m->gu_bytes) && put(d.type_gu, d.ffn, d.hidden, raw_gu, d.up_exps, m->up, m->gu_bytes) &&
          put(d.type_down, d.hidden, d.ffn, raw_down, d.down_exps, m->down, m->down_bytes);
     if (!ok) return bail();
-    if (rt_shape_ok(d.n_expert, d.hidden)) {
+    if (moe_wants_rt(d)) {
         const size_t q = align_up(rt_wq_bytes(d.n_expert, d.hidden), 256);
         if (!m->rt_mem.alloc(q + d.n_expert * sizeof(double))) return bail();
         m->rt_q = m->rt_mem.as<uint8_t>(); m->rt_ws = reinterpret_cast<double *>(m->rt_q + q);
