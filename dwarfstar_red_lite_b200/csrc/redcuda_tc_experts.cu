@@ -1,4 +1,4 @@
-// Routed experts of a prefill chunk on the 5th-generation tensor cores (tcgen05): for every work item (up to 64 pairs of
+// Routed experts of a prefill chunk on the 5th-generation tensor cores (tcgen05): for every work item (up to TCX_TN pairs of
 // one expert) and every 128-row tile of the expert's matrix, out[pair][row] = sum_k W_e[row][k] * x[pair][k].
 //
 // The batched form of the expert GEMV (rl_quant_row_dot per row, native/redlite_native_quant_cpu.c:247-266, called per
