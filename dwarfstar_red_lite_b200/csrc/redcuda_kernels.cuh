@@ -138,15 +138,16 @@ int kq_dequant_rows(uint32_t type, const uint8_t *rows, uint32_t nrows, uint32_t
 int kq_matvec(uint32_t type, const uint8_t *w, uint32_t nrows, uint32_t ncols, const float *x, uint32_t ntok, float *out);
 
 int launch_vec_sigmoid(const float *w, const float *x, uint32_t x_stride, uint32_t ncols, uint32_t ntok, float *out, cudaStream_t stream);
-// The same logits for a chunk, as exact integer products of 40-bit fixed point on the tensor cores (redcuda_router_i8.cu). wq, ws: the router's digits and row
-// scales, made once (rt_wq_bytes bytes, n_expert doubles); xq, xs: scratch of rt_xq_bytes bytes and rt_xs_doubles doubles; err: the launch's timeout flag
+// The same logits for a chunk, by integer products of fixed-point rows on the tensor cores and, where these leave a logit less than the precision of fp32, summed in
+// double (redcuda_router_i8.cu). wq, ws: the router's digits and (quantum, what its elements lack in quanta) per row, made once (rt_wq_bytes bytes, n_expert of them); xq, xs: scratch of
+// rt_xq_bytes bytes and rt_rows of them; again: a bit per logit, rt_rows x n_expert; err: the launch's timeout flag
 bool rt_shape_ok(uint32_t n_expert, uint32_t ncols);
 size_t rt_wq_bytes(uint32_t n_expert, uint32_t ncols);
 size_t rt_xq_bytes(uint32_t ntok, uint32_t ncols);
-size_t rt_xs_doubles(uint32_t ntok);
-int launch_rt_digits_w(const float *w, uint32_t n_expert, uint32_t ncols, uint8_t *wq, double *ws, cudaStream_t s);
-int launch_rt_logits(const uint8_t *wq, const double *ws, const float *x, uint32_t x_stride, uint32_t ntok, uint32_t n_expert, uint32_t ncols, uint8_t *xq, double *xs, float *logits,
-                     uint32_t *err, cudaStream_t s);
+size_t rt_rows(uint32_t ntok);
+int launch_rt_digits_w(const float *w, uint32_t n_expert, uint32_t ncols, uint8_t *wq, double2 *ws, cudaStream_t s);
+int launch_rt_logits(const float *w, const uint8_t *wq, const double2 *ws, const float *x, uint32_t x_stride, uint32_t ntok, uint32_t n_expert, uint32_t ncols, uint8_t *xq, double2 *xs, uint32_t *again,
+                     float *logits, uint32_t *err, cudaStream_t s);
 // logits[t][e] = dot(w[e], x[t]) accumulated in double, F32 weights [n_expert][ncols]; for batches (tiled fp64 GEMM)
 int launch_router_logits(const float *w, const float *x, uint32_t x_stride, uint32_t ntok, uint32_t n_expert, uint32_t ncols, float *logits, cudaStream_t stream);
 

@@ -316,8 +316,9 @@ struct redcuda_moe {
     __half *sh_xs = nullptr; float *sh_xinv = nullptr;   // shared expert on the tcgen05 GEMM: activation digits and inverse scales
     uint8_t *sh_wd = nullptr; float *sh_winv = nullptr;  // and the weight digits of one launch (gate + up, or down)
     __half *rt_xs = nullptr; float *rt_xinv = nullptr; uint8_t *rt_wd = nullptr; float *rt_winv = nullptr;   // the same for the router logits of a large chunk
-    uint8_t *rt_q = nullptr; double *rt_ws = nullptr;       // the router's digits and row scales for the integer logits of a chunk (null: not a shape they tile)
-    uint8_t *rt_xq = nullptr; double *rt_xsc = nullptr;     // and those of the chunk's rows
+    uint8_t *rt_q = nullptr; double2 *rt_ws = nullptr;      // the router's digits and row scales for the integer logits of a chunk (null: not a shape they tile)
+    uint8_t *rt_xq = nullptr; double2 *rt_xsc = nullptr;    // and those of the chunk's rows
+    uint32_t *rt_again = nullptr;                           // the logits that are summed again in double, a bit each
     bool tc_ok = false;         // the tcgen05 expert kernel can serve this layer's shapes
     bool tc_now = false;        // ... and serves the call in progress (set by moe_choose_path, read by the grouping and the launches)
     bool ws_shared = false;     // the workspace belongs to the caller (rc::moe_create_shared)
@@ -393,10 +394,10 @@ static bool moe_router_tc(const redcuda_moe *m, uint32_t ntok) {
     const uint32_t min_tok = v ? (uint32_t)atoi(v) : 0u;
     return min_tok && ntok >= min_tok && m->router.type == RC_F32 && m->d.hidden % 256u == 0 && m->rt_wd;
 }
-// Router logits of a chunk by exact integer products (redcuda_router_i8.cu): from 640 tokens and 512 experts on; RC_ROUTER_I8_MIN = tokens (0: never, and then
-// for every expert count it tiles). us a layer, double sums -> this: 512 experts 400 tokens 349 -> 350, 512 414 -> 409, 700 411 -> 394, 2048 689 -> 637; 256 experts
-// 700 tokens 284 -> 286, 1024 335 -> 350, 2048 574 -> 587; 128 experts 2048 tokens 310 -> 320: the double kernel runs beside the shared expert's tcgen05
-// GEMMs, this one takes turns with them for the SMs.
+// Router logits of a chunk by integer products (redcuda_router_i8.cu): from 640 tokens and 512 experts on; RC_ROUTER_I8_MIN = tokens (0: never, and then
+// for every expert count it tiles). us a layer, double sums -> this: 512 experts 640 tokens 395 -> 390, 700 405 -> 397, 1024 452 -> 447, 1400 534 -> 513, 2048 679 -> 641;
+// 256 experts 1024 tokens 355 -> 349, 2048 570 -> 591: the double kernel runs beside the shared expert's tcgen05 GEMMs, this one takes turns with them for the
+// SMs. Where every logit of a chunk has to be summed again (rows with an element of 1e5 and more among ones) 2048 tokens take 330 us here instead of 138.
 static bool moe_router_i8(const redcuda_moe *m, uint32_t ntok) {
     if (!m->rt_q) return false;
     if (const char *v = getenv("RC_ROUTER_I8_MIN")) return atoi(v) && ntok >= (uint32_t)atoi(v);
@@ -441,7 +442,7 @@ static int moe_gemv_pre(redcuda_moe *m, uint32_t ntok, const float *x, bool with
             T.job[0] = TcJob{m->router.base, 0u, RC_F32, m->d.n_expert, m->logits, m->d.n_expert, 0u};
             if (!launch_tc_gemm(T, tn, "moe_router_logits_tc", s)) return 0;
         } else if (moe_router_i8(m, ntok)) {
-            if (!launch_rt_logits(m->rt_q, m->rt_ws, x, m->d.hidden, ntok, m->d.n_expert, m->d.hidden, m->rt_xq, m->rt_xsc, m->logits, m->tc_err, s)) return 0;
+            if (!launch_rt_logits((const float *)m->router.base, m->rt_q, m->rt_ws, x, m->d.hidden, ntok, m->d.n_expert, m->d.hidden, m->rt_xq, m->rt_xsc, m->rt_again, m->logits, m->tc_err, s)) return 0;
         } else if (ntok >= 2u && m->router.type == RC_F32) {
             if (!launch_router_logits((const float *)m->router.base, x, m->d.hidden, ntok, m->d.n_expert, m->d.hidden, m->logits, s)) return 0;
         } else add(m->router, nullptr, m->logits, m->d.n_expert, GEMV_STORE);
@@ -700,7 +701,7 @@ static size_t moe_ws_layout(const redcuda_moe_desc &d, redcuda_moe *m, uint8_t *
         put(r.rt_xs, tc_xs_halves((uint32_t)T, d.hidden, 128u) * 2u); put(r.rt_xinv, (T + 128u) * 4u);
         put(r.rt_wd, tc_wd_bytes(tc_row_tiles(d.n_expert), d.hidden)); put(r.rt_winv, (size_t)tc_row_tiles(d.n_expert) * 4u);
     }
-    if (moe_wants_rt(d)) { put(r.rt_xq, rt_xq_bytes((uint32_t)T, d.hidden)); put(r.rt_xsc, rt_xs_doubles((uint32_t)T) * sizeof(double)); }
+    if (moe_wants_rt(d)) { put(r.rt_xq, rt_xq_bytes((uint32_t)T, d.hidden)); put(r.rt_xsc, rt_rows((uint32_t)T) * sizeof(double2)); put(r.rt_again, rt_rows((uint32_t)T) * (d.n_expert / 8u)); }
     if (m) { m->ticket = m->work + 2; m->tc_err = m->work + 3; }
     return w;
 }
@@ -844,8 +845,8 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
     if (!ok) return bail();
     if (moe_wants_rt(d)) {
         const size_t q = align_up(rt_wq_bytes(d.n_expert, d.hidden), 256);
-        if (!m->rt_mem.alloc(q + d.n_expert * sizeof(double))) return bail();
-        m->rt_q = m->rt_mem.as<uint8_t>(); m->rt_ws = reinterpret_cast<double *>(m->rt_q + q);
+        if (!m->rt_mem.alloc(q + d.n_expert * sizeof(double2))) return bail();
+        m->rt_q = m->rt_mem.as<uint8_t>(); m->rt_ws = reinterpret_cast<double2 *>(m->rt_q + q);
         if (!launch_rt_digits_w((const float *)m->router.base, d.n_expert, d.hidden, m->rt_q, m->rt_ws, s)) return bail();
     }
 

@@ -1,17 +1,25 @@
-// Router logits of a chunk as exact integer products on the 5th-generation tensor cores (tcgen05, kind::i8).
+// Router logits of a chunk as integer products on the 5th-generation tensor cores (tcgen05, kind::i8), and in double where these do not give the sum.
 //
 // The logits loop of the reference (native/redlite_native_engine_cpu.c:347-355) sums in double, and so does k_router_logits, whose fp64 tensor
 // instructions run at 64 FMA per SM and clock: 133 us for 2048 tokens x 512 experts x 2048 columns, 119 of them the instructions themselves. Here a
-// row of x and a row of W are 40-bit fixed point, five balanced 8-bit digits d_i with a power-of-two scale per row: v 2^e = sum_i d_i 2^(8 (4 - i)).
-// A value down to 2^-16 of its row's largest is exact, a smaller one is within 2^-40 of the largest. The products of two digits and their sums over
-// a row are exact in 32 bits (5 x 2048 x 2^14 < 2^31), so that digits with the same i + j = s share an accumulator. s up to 5 is kept (19 of 25
-// products; the rest is below 2^-46 of the largest product), the six sums are added in double, scaled by powers of two and rounded once:
-// the logit is the rounded exact sum wherever that sum does not lie within 2^-16 of half a unit of it, as the double sums' logit is.
+// row of x and a row of W are fixed point, five balanced 8-bit digits d_i with a power-of-two scale per row: v 2^e = sum_i d_i 2^(8 (4 - i)), in steps of
+// a quantum q that is at most 2^-37 of the row's largest magnitude (and more than 2^-38): an element of 2^-14 of the largest or more is exact, a smaller one
+// off by at most q / 2. The products of two digits and their sums over a row are exact in 32 bits (5 x 8192 x 2^14 < 2^31), so that digits with the same
+// i + j = s share an accumulator. s up to 5 is kept (19 of 25 products); the six sums are added in double, scaled by powers of two and rounded once.
+// With r the sum of what a row's elements are off by, in quanta, a sum of n columns lacks at most
+//     E = q_x q_w (2^38 (r_x + r_w) + 3.1 2^30 n)
+// (no element exceeds 2^38 quanta; left out are three products of two digits of s = 6, at most 2^14 in units of 2^16 q_x q_w, and less below them). A logit with
+// E <= 2^-24 |logit| stands: its sum is right to the rounding of fp32, and nearly always by far more, since errors of both signs meet. Every other is
+// summed again in double (k_rt_exact): those that nearly cancel (eight in ten thousand with Gaussian rows of 2048), those of rows whose largest element stands out by so
+// much that the others lose digits, and the rows that are not finite, whose scale is NaN.
 //
-// k_rt_digits_x / _w   fp32 rows -> digits in the layout that a stage reads: [tile][stage of 64 columns][digit, 16-byte chunk, row], K-major core matrices
+// k_rt_digits_x / _w   fp32 rows -> digits in the layout that a stage reads: [tile][stage of 64 columns][digit, 16-byte chunk, row], K-major core matrices; and a
+//                      row's (q, r)
 // k_rt_logits<TOK>     one CTA = 128 experts x TOK tokens x all columns: a producer warp (two bulk copies a stage), an MMA warp (two k-steps of 32 columns
 //                      a stage, seven MMAs each: digit i of W against as many digits of x as keep s <= 5, side by side in N), four drain warps at the end.
-// The MMAs of a k-step take 608 cycles for 64 tokens and the operands 30 KB from L2, which delivers some 43 bytes a cycle to an SM: 700.
+//                      The MMAs of a k-step take 608 cycles for 64 tokens and the operands 30 KB from L2, which delivers some 43 bytes a cycle to an SM: 700.
+//                      These also set the bit of a logit whose E is too large.
+// k_rt_exact           the logits with their bit set, in double: a block per eight tokens, a warp per logit
 #define RC_PDL_DEFAULT 0
 #include "redcuda_common.cuh"
 #include "redcuda_kernels.cuh"
@@ -28,19 +36,22 @@ constexpr uint32_t RT_THREADS = 192u;
 // v 2^(38 - e) as a rounded integer, e the exponent of the row's largest magnitude (mx = f 2^e, f in [0.5, 1)), in two parts of 32 bits: a holds digits 0 to 2
 // (|v 2^(22 - e)| < 2^22), b the two below. Adding 1.5 2^23 leaves a float's rounded value in its mantissa; every difference here is exact.
 // Conversions to and from double are served at a few values a cycle, and 64-bit shifts are three instructions each.
-__device__ __forceinline__ void rt_fixed(float v, float up0, float up1, uint32_t &a, uint32_t &b) {
-    const float magic = 12582912.0f, t = (v * up0) * up1, ta = t + magic, r = (t - (ta - magic)) * 65536.0f;
-    int ia = __float_as_int(ta) - __float_as_int(magic), ib = __float_as_int(r + magic) - __float_as_int(magic);
+// Returned: what that is off by, in quanta.
+__device__ __forceinline__ float rt_fixed(float v, float up0, float up1, uint32_t &a, uint32_t &b) {
+    const float magic = 12582912.0f, t = (v * up0) * up1, ta = t + magic, r = (t - (ta - magic)) * 65536.0f, rb = r + magic;
+    int ia = __float_as_int(ta) - __float_as_int(magic), ib = __float_as_int(rb) - __float_as_int(magic);
     if (ib > 32639) { ib -= 65536; ++ia; }                           // what two balanced digits do not hold
     // adding 128 to every digit makes all bytes non-negative, so that the carries resolve themselves; digit 0 stays within 64
     a = ((uint32_t)ia + 0x808080u) ^ 0x808080u; b = ((uint32_t)ib + 0x8080u) ^ 0x8080u;
+    return fabsf(r - (rb - magic));
 }
 
 // Eight rows of ncols values (those from `live` on are zeros) -> digits at out + [stage][digit * dstride + chunk * cstride + row * 16], a chunk of 16 values a
 // thread and step: neighbouring lanes take neighbouring rows, whose chunks lie side by side. block = 512
 __device__ __forceinline__ void rt_digits_rows(const float *rows, uint32_t stride, uint32_t live, uint32_t ncols, uint8_t *out, size_t stage_bytes, uint32_t dstride, uint32_t cstride,
-                                               double *scale_out) {
+                                               double2 *row_out) {
     __shared__ uint32_t s_mag[16];
+    __shared__ float s_off[16][8];
     __shared__ float2 s_up[8];                                       // the multiplier 2^(22 - e) of a row as two factors; zero where every digit is to be zero
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     auto load4 = [&](uint32_t r, uint32_t k) {
@@ -62,7 +73,7 @@ __device__ __forceinline__ void rt_digits_rows(const float *rows, uint32_t strid
         mag = max(s_mag[2u * threadIdx.x], s_mag[2u * threadIdx.x + 1u]);
         int e = (int)(mag >> 23) - 126;
         if (mag < 0x00800000u) frexpf(__uint_as_float(mag), &e);     // subnormal
-        scale_out[threadIdx.x] = mag >= 0x7f800000u ? (double)NAN : mag ? __hiloint2double((e - 38 + 1023) << 20, 0) : 0.0;
+        row_out[threadIdx.x].x = mag >= 0x7f800000u ? (double)NAN : mag ? __hiloint2double((e - 38 + 1023) << 20, 0) : 0.0;
         const int h = (22 - e) / 2;
         auto pow2 = [](int x) { return __int_as_float((x + 127) << 23); };
         s_up[threadIdx.x] = mag && mag < 0x7f800000u ? make_float2(pow2(h), pow2(22 - e - h)) : make_float2(0.f, 0.f);
@@ -70,6 +81,7 @@ __device__ __forceinline__ void rt_digits_rows(const float *rows, uint32_t strid
     __syncthreads();
     const uint32_t r = threadIdx.x & 7u;
     const float2 up = s_up[r];
+    float off = 0.f;
 #pragma unroll 1
     for (uint32_t ch = threadIdx.x >> 3; ch < ncols / 16u; ch += 64u) {
         float4 v[4];
@@ -81,7 +93,7 @@ __device__ __forceinline__ void rt_digits_rows(const float *rows, uint32_t strid
             const float f[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
             uint32_t a[4], b[4];
 #pragma unroll
-            for (uint32_t j = 0; j < 4u; ++j) rt_fixed(up.x == 0.f ? 0.f : f[j], up.x, up.y, a[j], b[j]);
+            for (uint32_t j = 0; j < 4u; ++j) off += rt_fixed(up.x == 0.f ? 0.f : f[j], up.x, up.y, a[j], b[j]);
             // byte i of the four values side by side
             const uint32_t a01 = __byte_perm(a[0], a[1], 0x5140), a23 = __byte_perm(a[2], a[3], 0x5140), b01 = __byte_perm(b[0], b[1], 0x5140), b23 = __byte_perm(b[2], b[3], 0x5140);
             d[4][q] = __byte_perm(b01, b23, 0x5410); d[3][q] = __byte_perm(b01, b23, 0x7632); d[2][q] = __byte_perm(a01, a23, 0x5410); d[1][q] = __byte_perm(a01, a23, 0x7632);
@@ -91,17 +103,27 @@ __device__ __forceinline__ void rt_digits_rows(const float *rows, uint32_t strid
 #pragma unroll
         for (uint32_t i = 0; i < RT_D; ++i) *reinterpret_cast<uint4 *>(o + (size_t)i * dstride) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
     }
+    off += __shfl_xor_sync(0xffffffffu, off, 8);                     // the lanes of a row
+    off += __shfl_xor_sync(0xffffffffu, off, 16);
+    if (lane < 8u) s_off[warp][lane] = off;
+    __syncthreads();
+    if (threadIdx.x < 8u) {
+        float sum = 0.f;
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; ++i) sum += s_off[i][threadIdx.x];
+        row_out[threadIdx.x].y = (double)sum;
+    }
 }
 
 // grid = rows rounded up to the token tile / 8 (rows beyond ntok become zeros)
-__global__ void __launch_bounds__(512) k_rt_digits_x(const float *x, uint32_t x_stride, uint32_t ntok, uint32_t ncols, uint32_t tok, uint8_t *__restrict__ xq, double *__restrict__ xs) {
+__global__ void __launch_bounds__(512) k_rt_digits_x(const float *x, uint32_t x_stride, uint32_t ntok, uint32_t ncols, uint32_t tok, uint8_t *__restrict__ xq, double2 *__restrict__ xs) {
     pdl_prologue();
     const uint32_t t = blockIdx.x * 8u, tile = t / tok, tt = t - tile * tok;
     const size_t stage = (size_t)RT_D * RT_KS * tok;
     rt_digits_rows(x + (size_t)t * x_stride, x_stride, t < ntok ? ntok - t : 0u, ncols, xq + (size_t)tile * (ncols / RT_KS) * stage + tt * 16u, stage, tok * 16u, RT_D * tok * 16u, xs + t);
 }
 // grid = experts / 8
-__global__ void __launch_bounds__(512) k_rt_digits_w(const float *w, uint32_t ncols, uint8_t *__restrict__ wq, double *__restrict__ ws) {
+__global__ void __launch_bounds__(512) k_rt_digits_w(const float *w, uint32_t ncols, uint8_t *__restrict__ wq, double2 *__restrict__ ws) {
     pdl_prologue();
     const uint32_t e = blockIdx.x * 8u, tile = e / 128u, r = e % 128u;
     rt_digits_rows(w + (size_t)e * ncols, ncols, 8u, ncols, wq + (size_t)tile * (ncols / RT_KS) * RT_A_BUF + r * 16u, RT_A_BUF, RT_A_DIGIT, 128u * 16u, ws + e);
@@ -116,7 +138,7 @@ __device__ __forceinline__ void rt_mma_if(uint32_t leader, uint32_t d_tmem, uint
         :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
 
-struct RtArgs { const uint8_t *wq, *xq; const double *ws, *xs; float *logits; uint32_t ntok, n_expert, ncols; uint32_t *err, *status; };
+struct RtArgs { const uint8_t *wq, *xq; const double2 *ws, *xs; float *logits; uint32_t *again; uint32_t ntok, n_expert, ncols; uint32_t *err, *status; };
 
 template <uint32_t TOK>
 __global__ void __launch_bounds__(RT_THREADS, 1) k_rt_logits(const __grid_constant__ RtArgs A) {
@@ -199,7 +221,8 @@ __global__ void __launch_bounds__(RT_THREADS, 1) k_rt_logits(const __grid_consta
         // ------------------------------------------------------------------ drain (128 threads): a thread owns an expert
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t qlane = (warp & 3u) * 32u, e = blockIdx.y * 128u + qlane + lane;
-        const double ws = A.ws[e];
+        const double2 W = A.ws[e];
+        const double lacks = 0x1p38 * W.y + 3.1 * 0x1p30 * (double)A.ncols;
 #pragma unroll 1
         for (uint32_t c = 0; c < TOK && t0 + c < A.ntok; c += 8u) {
             uint32_t m[RT_S][8];
@@ -216,7 +239,12 @@ __global__ void __launch_bounds__(RT_THREADS, 1) k_rt_logits(const __grid_consta
                 double v = (double)(int)m[RT_S - 1u][i], p = 256.0;      // in units of 2^24 of the scaled values' product
 #pragma unroll
                 for (int s = (int)RT_S - 2; s >= 0; --s) { v = fma((double)(int)m[s][i], p, v); p *= 256.0; }
-                A.logits[(size_t)t * A.n_expert + e] = (float)(v * 16777216.0 * ws * A.xs[t]);
+                const double2 X = A.xs[t];
+                const double q = W.x * X.x;
+                v *= 0x1p24;
+                A.logits[(size_t)t * A.n_expert + e] = (float)(v * q);
+                const uint32_t again = __ballot_sync(0xffffffffu, !((lacks + 0x1p38 * X.y) * q <= fabs(0x1p-24 * v * q)));
+                if (lane == 0) A.again[((size_t)t * A.n_expert + e) >> 5] = again;
             }
         }
     }
@@ -229,28 +257,67 @@ __global__ void __launch_bounds__(RT_THREADS, 1) k_rt_logits(const __grid_consta
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
+// The logits that the integer sums do not settle, in double: a block lists those of its eight tokens, its warps take them in turn (each its own token's: the token with the
+// most of them made the others wait, 13.5 us for 2048 tokens where this takes 10.5; 23 with an element of 100 in every row, 263 if all are listed). grid = tokens / 8,
+// block = 256. The chain of a few rows' loads bounds it while they are few, conversions to double when they are many
+__global__ void __launch_bounds__(256, 2) k_rt_exact(const float *w, const float *x, uint32_t x_stride, uint32_t ntok, uint32_t n_expert, uint32_t ncols, const uint32_t *again, float *logits) {
+    pdl_prologue();
+    __shared__ uint16_t s_list[8192];                // token of the block, expert of the turn's 1024
+    __shared__ uint32_t s_n;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, words = n_expert >> 5, t0 = blockIdx.x * 8u;
+    for (uint32_t w0 = 0; w0 < words; w0 += 32u) {
+        if (threadIdx.x == 0) s_n = 0u;
+        __syncthreads();
+        uint32_t bits = t0 + warp < ntok && w0 + lane < words ? again[(size_t)(t0 + warp) * words + w0 + lane] : 0u;
+        uint32_t at = bits ? atomicAdd(&s_n, __popc(bits)) : 0u;
+        for (; bits; bits &= bits - 1u) s_list[at++] = (uint16_t)(warp << 10 | lane << 5 | ((uint32_t)__ffs((int)bits) - 1u));
+        __syncthreads();
+        const uint32_t n = s_n;
+        for (uint32_t k = warp; k < n; k += 8u) {
+            const uint32_t item = s_list[k], t = t0 + (item >> 10), e = w0 * 32u + (item & 1023u);
+            const float *wr = w + (size_t)e * ncols, *xr = x + (size_t)t * x_stride;
+            auto sum = [&](auto load) {
+                double a0 = 0.0, a1 = 0.0;
+#pragma unroll 8
+                for (uint32_t c = lane * 4u; c < ncols; c += 128u) {
+                    const float4 b = __ldg(reinterpret_cast<const float4 *>(wr + c)), a = load(xr + c);
+                    a0 = fma((double)a.x, (double)b.x, a0); a1 = fma((double)a.y, (double)b.y, a1);
+                    a0 = fma((double)a.z, (double)b.z, a0); a1 = fma((double)a.w, (double)b.w, a1);
+                }
+                return a0 + a1;
+            };
+            double v;                                // a caller's rows may begin at any float
+            if (((size_t)xr & 15u) == 0u) v = sum([](const float *p) { return *reinterpret_cast<const float4 *>(p); });
+            else v = sum([](const float *p) { return make_float4(p[0], p[1], p[2], p[3]); });
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) logits[(size_t)t * n_expert + e] = (float)v;
+        }
+        __syncthreads();
+    }
+}
+
 bool rt_shape_ok(uint32_t n_expert, uint32_t ncols) { return n_expert % 128u == 0 && n_expert && ncols % RT_KS == 0 && ncols && ncols <= 8192u; }
 size_t rt_wq_bytes(uint32_t n_expert, uint32_t ncols) { return (size_t)n_expert * ncols * RT_D; }
 static uint32_t rt_tok(uint32_t ntok, uint32_t n_expert) { return (ntok + 31u) / 32u * (n_expert / 128u) <= 148u ? 32u : 64u; }
 size_t rt_xq_bytes(uint32_t ntok, uint32_t ncols) { return (size_t)((ntok + 63u) / 64u) * 64u * ncols * RT_D; }
-size_t rt_xs_doubles(uint32_t ntok) { return (size_t)((ntok + 63u) / 64u) * 64u; }
+size_t rt_rows(uint32_t ntok) { return (size_t)((ntok + 63u) / 64u) * 64u; }
 
-int launch_rt_digits_w(const float *w, uint32_t n_expert, uint32_t ncols, uint8_t *wq, double *ws, cudaStream_t s) {
+int launch_rt_digits_w(const float *w, uint32_t n_expert, uint32_t ncols, uint8_t *wq, double2 *ws, cudaStream_t s) {
     RC_REQUIRE(rt_shape_ok(n_expert, ncols), "router digits: %u experts of %u columns are not tileable", n_expert, ncols);
     RC_LAUNCH((k_rt_digits_w), n_expert / 8u, 512, 0, s, w, ncols, wq, ws);
     RC_LAUNCHED();
     return 1;
 }
 
-int launch_rt_logits(const uint8_t *wq, const double *ws, const float *x, uint32_t x_stride, uint32_t ntok, uint32_t n_expert, uint32_t ncols, uint8_t *xq, double *xs, float *logits,
-                     uint32_t *err, cudaStream_t s) {
-    RC_REQUIRE(rt_shape_ok(n_expert, ncols) && ntok && wq && xq, "router logits: %u experts of %u columns are not tileable, or no tokens", n_expert, ncols);
+int launch_rt_logits(const float *w, const uint8_t *wq, const double2 *ws, const float *x, uint32_t x_stride, uint32_t ntok, uint32_t n_expert, uint32_t ncols, uint8_t *xq, double2 *xs, uint32_t *again,
+                     float *logits, uint32_t *err, cudaStream_t s) {
+    RC_REQUIRE(rt_shape_ok(n_expert, ncols) && ntok && w && wq && xq, "router logits: %u experts of %u columns are not tileable, or no tokens", n_expert, ncols);
     const uint32_t tok = rt_tok(ntok, n_expert), tiles = (ntok + tok - 1u) / tok;
     prof_begin("moe_router_digits", s);
     RC_LAUNCH((k_rt_digits_x), tiles * tok / 8u, 512, 0, s, x, x_stride, ntok, ncols, tok, xq, xs);
     prof_end(s);
     RC_LAUNCHED();
-    const RtArgs A{wq, xq, ws, xs, logits, ntok, n_expert, ncols, err, status_words()};
+    const RtArgs A{wq, xq, ws, xs, logits, again, ntok, n_expert, ncols, err, status_words()};
     const size_t smem = (size_t)RT_NS * (RT_A_BUF + RT_D * RT_KS * tok);
     prof_begin("moe_router_logits", s);
 #define RT_LAUNCH(TOK_) do { \
@@ -258,6 +325,10 @@ int launch_rt_logits(const uint8_t *wq, const double *ws, const float *x, uint32
         RC_LAUNCH((k_rt_logits<TOK_>), dim3(tiles, n_expert / 128u), RT_THREADS, smem, s, A); } while (0)
     if (tok == 64u) RT_LAUNCH(64u); else RT_LAUNCH(32u);
 #undef RT_LAUNCH
+    prof_end(s);
+    RC_LAUNCHED();
+    prof_begin("moe_router_exact", s);
+    RC_LAUNCH((k_rt_exact), (ntok + 7u) / 8u, 256, 0, s, w, x, x_stride, ntok, n_expert, ncols, (const uint32_t *)again, logits);
     prof_end(s);
     RC_LAUNCHED();
     return 1;
