@@ -83,14 +83,14 @@ __device__ __forceinline__ void gemv1_stage(const GemvArgs &A, uint32_t ncols, f
     }
 }
 
-template <bool NORM>
+template <bool NORM, bool STAGED = false>          // STAGED: x is in shared memory
 __device__ __forceinline__ void gemv1_q6k(const GemvArgs &A, const GemvJob &J, const G1Tile &T, double *part, float *xs) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t cpr = J.ncols >> 6, bpr = J.ncols >> 8, S = g1_slices(RC_Q6_K, J.ncols), ws = g1_slice_warps(S), lpr = g1_lanes(RC_Q6_K, J.ncols), rw = 32u / lpr;
     const uint32_t slot = lane / lpr, sub = lane % lpr, step = (G1_WARPS / ws) * rw, first = (warp / ws) * rw;
     const uint64_t o_h = rc_q6_qh(J.nb), o_s = rc_q6_sc(J.nb), o_d = rc_q6_d(J.nb);
     const uint64_t bias = f2_pack(__float_as_uint(-8388640.0f), __float_as_uint(-8388640.0f));      // 2^23 + 32
-    bool staged = false;
+    bool staged = STAGED;
     for (uint32_t sl = warp % ws; sl < S; sl += ws) {
         const uint32_t c = sl * (G1_QCOLS / 64u) + sub;
         const bool on = c < cpr;                                  // lanes past the row's end repeat its last chunk and add nothing
@@ -246,16 +246,36 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1(const __grid_consta
 
 // ---- one large Q6_K matrix (the LM head) -------------------------------------------------------------------------------
 // Instruction issue bounds the products of a matrix of that size in floats: a byte permute per weight to make it one. Here x is four 8-bit digits with a
-// power-of-two scale per 256 columns (actw_digits: closer to the row than the rounding of one fp32 product), its digit words in place of the floats, and
-// a word of four 6-bit weights meets them in four dp4a: the sums of 16 columns are exact. The weights stay unsigned (q + 32), an accumulator begins
-// with -32 times its digits' sum. Lanes, rows and loads as in gemv1_q6k. 151936 x 2048: 61 us (floats: 72; 255 MB take 39 at the copy rate)
-constexpr uint32_t G1_DIGIT_ROWS = 16384u;       // rows from which a matrix is taken here; below, quantising x in every block costs more than it saves
+// power-of-two scale per 256 columns (actw_digits), its digit words in place of the floats, and a word of four 6-bit weights meets them in four dp4a: the
+// sums of 16 columns are exact. The weights stay unsigned (q + 32), an accumulator begins with -32 times its digits' sum. Lanes, rows and loads as in
+// gemv1_q6k. 151936 x 2048: 61 us (floats: 72; 255 MB take 39 at the copy rate)
+//
+// The digits hold a value to 2^-30 of the largest of its 256, which is less than fp32 does for the small ones. So a row takes this form only if in each 256
+//   - at least 32 values lie within 2^-6 of the largest: these are exact, and what the others lack comes to less than the rounding of the fp32 sums that replace it
+//     (2^-23.3 of the block's product in the worst case, in the 2-norm over weights that do not follow the row). One value that stands out, which may meet a zero,
+//     is not enough;
+//   - the largest is at least 2^-60, so that neither the scale (2^-126 is the least) nor its product with d lose bits, and not above every number.
+// Every block sees the whole row and decides alike; a row that does not fit is multiplied as floats.
+__device__ __forceinline__ bool g1_digits_fit(const float4 &a, const float4 &b, uint32_t mx) {
+    if (mx == 0u) return true;
+    if (mx < (127u - 60u) << 23 || mx >= 0x7f800000u) return false;
+    const uint32_t least = mx - (6u << 23);
+    const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t n = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) n += act_mag(f[i]) >= least ? 1u : 0u;
+    return __reduce_add_sync(0xffffffffu, n) >= 32u;
+}
+// Rows from which a matrix is taken here; below, every block's digits of x cost what they save. us a decode step of 8 layers by rows of its LM head, floats -> digits: 4096
+// 496.2 -> 497.0, 8192 505.5 -> 505.1, 16384 514 -> 510, 32768 525 -> 520, 65536 547 -> 545, 151936 611 -> 597 (the kernel alone, with some 5 us of events: 76.3 -> 66.7)
+constexpr uint32_t G1_DIGIT_ROWS = 16384u;
 __device__ __forceinline__ int g1_dp4a(uint32_t q, uint32_t x, int c) { int d; asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(q), "r"(x), "r"(c)); return d; }
 
 template <bool NORM>
 __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1_digits(const __grid_constant__ GemvArgs A) {
     pdl_trigger();
-    extern __shared__ __align__(16) float g1_xs[];         // x, then its digit words; behind it -32 times the digit sums of every 16 columns
+    extern __shared__ __align__(16) double g1_part[];      // as in k_gemv1: results of a row that is multiplied as floats; behind them x, then its digit words; and -32 times the digit sums of every 16 columns
+    float *g1_xs = reinterpret_cast<float *>(g1_part + A.part_doubles);
     __shared__ float s_scale[G1_NCOLS / 256u];
     const GemvJob &J = A.job[0];
     const uint32_t row0 = blockIdx.x * J.rows_per_tile, nrow = min(J.rows_per_tile, J.nrows - row0);
@@ -283,12 +303,20 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1_digits(const __grid
     gemv1_stage<NORM>(A, J.ncols, g1_xs);
     if (!A.resident) { f[0] = load(first + slot); f[1] = load(first + step + slot); }
     __syncthreads();
-    for (uint32_t b = warp; b < bpr; b += G1_WARPS) {       // a warp per 256 columns, eight neighbouring values a lane
-        float4 *p = reinterpret_cast<float4 *>(g1_xs + g1_xi(b * 256u + lane * 8u));
-        const float4 v0 = p[0], v1 = p[1];
+    static_assert(G1_NCOLS / 256u <= G1_WARPS, "a warp per 256 columns, eight neighbouring values a lane");
+    float4 *p = reinterpret_cast<float4 *>(g1_xs + g1_xi(min(warp, bpr - 1u) * 256u + lane * 8u));
+    const float4 v0 = p[0], v1 = p[1];
+    const uint32_t mx = __reduce_max_sync(0xffffffffu, max(act_mag4(v0), act_mag4(v1)));
+    if (!__syncthreads_and(g1_digits_fit(v0, v1, mx))) {
+        gemv1_q6k<false, true>(A, J, G1Tile{row0, nrow, 0u, true}, g1_part, g1_xs);
+        __syncthreads();
+        for (uint32_t r = threadIdx.x; r < nrow; r += G1_WARPS * 32u) J.out[row0 + r] = (float)g1_part[r];
+        return;
+    }
+    if (warp < bpr) {
         float up;
-        const float scale = actw_scale(__reduce_max_sync(0xffffffffu, max(act_mag4(v0), act_mag4(v1))), up);
-        if (lane == 0) s_scale[b] = scale;
+        const float scale = actw_scale(mx, up);
+        if (lane == 0) s_scale[warp] = scale;
         const uint32_t w0[4] = {actw_digits(v0.x, up), actw_digits(v0.y, up), actw_digits(v0.z, up), actw_digits(v0.w, up)};
         const uint32_t w1[4] = {actw_digits(v1.x, up), actw_digits(v1.y, up), actw_digits(v1.z, up), actw_digits(v1.w, up)};
         uint32_t p0[4], p1[4];
@@ -300,7 +328,7 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1_digits(const __grid
             c[i] = __dp4a((int)p0[i], 0x01010101, __dp4a((int)p1[i], 0x01010101, 0));
             c[i] = -32 * (c[i] + __shfl_xor_sync(0xffffffffu, c[i], 1));
         }
-        if (!(lane & 1u)) corr[b * 16u + (lane >> 1)] = make_int4(c[0], c[1], c[2], c[3]);
+        if (!(lane & 1u)) corr[warp * 16u + (lane >> 1)] = make_int4(c[0], c[1], c[2], c[3]);
     }
     __syncthreads();
     const uint4 *xl = reinterpret_cast<const uint4 *>(g1_xs + bcol * 268u + half * 136u + l0);
@@ -399,7 +427,7 @@ int launch_gemv1(GemvArgs &A, cudaStream_t stream) {
     if (q6 || A.norm.w) smem += (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + 16u;
     prof_begin(A.tag ? A.tag : "gemv", stream);
     if (gemv1_digits_ok(A)) {
-        smem = (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + (size_t)(A.job[0].ncols / 16u) * sizeof(int4) + 16u;
+        smem += (size_t)(A.job[0].ncols / 16u) * sizeof(int4);
         if (A.norm.w) RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1_digits<true>), tiles, G1_WARPS * 32u, smem, stream, A);
         else RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1_digits<false>), tiles, G1_WARPS * 32u, smem, stream, A);
         prof_end(stream);

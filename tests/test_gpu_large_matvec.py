@@ -38,3 +38,36 @@ def test_a_row_that_is_not_finite():
         x = rng.normal(0, 1, size=(1, 512)).astype(np.float32)
         x[0, 300] = bad
         assert not np.isfinite(np.asarray(rc.quant_matvec(synth.Q6_K, w, ROWS, 512, x))).any()
+
+
+@pytest.mark.parametrize("kind", ["1e-25", "1e-33", "1e-35", "1e4 where the weights vanish", "1e6 where the weights vanish", "one of 256", "1e-37 beside ones"])
+@pytest.mark.parametrize("cols", [256, 768, 2048])
+def test_rows_that_digits_do_not_hold(cols, kind):
+    """Blocks of 256 values with one that stands out, with few that count, or near the least exponents: as right as the products of floats."""
+    rng = np.random.default_rng(cols + 1)
+    w = np.asarray(synth.quant_matrix(rng, synth.Q6_K, ROWS, cols, 1e-3, 5e-3, (-64, 63))).copy()
+    x = rng.normal(0, 1, size=cols)
+    if "vanish" in kind:
+        w.reshape(ROWS, cols // 256, 210)[:, -1, 192] = 0            # the 8-bit scale of the last block's first 16 columns
+        x[cols - 250] = float(kind[:3])
+    elif kind == "one of 256":
+        x[np.arange(cols) % 256 != 77] = 0.0
+    elif "beside" in kind:
+        x[-256:] *= 1e-37
+        w.reshape(ROWS, cols // 256, 210)[:, :-1, 208:] = 0          # the other blocks' d: what the small block gives is all there is
+    else:
+        x *= float(kind)
+    x = x.astype(np.float32)[None, :]
+    got = np.asarray(rc.quant_matvec(synth.Q6_K, w, ROWS, cols, x)).reshape(-1)
+    want = ol.dequant_rows(synth.Q6_K, w.reshape(ROWS, -1), cols).astype(np.float64) @ x[0].astype(np.float64)
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-7 + 2.0 ** -150 * ROWS ** 0.5 / np.linalg.norm(want)      # the last: rounding to a subnormal
+
+
+def test_an_infinity_keeps_its_sign():
+    rng = np.random.default_rng(1)
+    w = synth.quant_matrix(rng, synth.Q6_K, ROWS, 512, 1e-3, 5e-3, (-64, 63))
+    x = rng.normal(0, 1, size=(1, 512)).astype(np.float32)
+    x[0, 300] = np.inf
+    with np.errstate(invalid="ignore"):
+        want = (ol.dequant_rows(synth.Q6_K, np.asarray(w).reshape(ROWS, -1), 512)[:, 300] * np.float32(np.inf))
+    assert np.array_equal(np.asarray(rc.quant_matvec(synth.Q6_K, w, ROWS, 512, x)).reshape(-1), want, equal_nan=True)
