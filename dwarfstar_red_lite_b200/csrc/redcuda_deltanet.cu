@@ -10,6 +10,7 @@
 //   k_dn_step   all three in one launch, the usual form: the kernels above serve state sizes and head ratios beyond it
 #include "redcuda_common.cuh"
 #include "redcuda_kernels.cuh"
+#include "redcuda_silu.cuh"
 #include "redcuda_stage.cuh"
 #include "../../include/redcuda.h"
 
@@ -258,25 +259,10 @@ __global__ void __launch_bounds__(256, MINB) k_dn_step(DnDims D, const float *__
 //                 the state per chunk instead of per token; the next token's q/k/v/beta/gate are fetched while the
 //                 current one is reduced
 // A block serves DN_PREP_TOK consecutive tokens of its channel group: a thread keeps its channel's samples and results of all of them, so that a sample is
-// read once and the eight L2 norms are reduced together, their roots taken by one thread each. Double-precision arithmetic bounds it (some 25 operations a
+// read once and the eight L2 norms are reduced together, their roots taken by one thread each. Double-precision arithmetic bounds it (some 30 operations a
 // value; with exp() and a division of doubles for every value, a root and a division in every thread and a barrier per token it was 65, and 119 us for
-// 2048 tokens where this takes 62).
+// 2048 tokens where this takes 66).
 constexpr uint32_t DN_PREP_TOK = 8u;
-
-// a / (1 + exp(-a)) to within 2^-40 of itself before it is rounded to fp32, whose half unit is 2^-25: exp(-a) = 2^n exp(r), |r| <= ln 2 / 2, exp(r) by its Taylor
-// polynomial of degree 10 (the remainder is below 2^-41), the reciprocal by one Newton step in double from an fp32 one (2^-22 squared)
-__device__ __forceinline__ float dn_silu(double a) {
-    if (!(fabs(a) < 80.0)) return (float)(a / (1.0 + exp(-a)));
-    const double magic = 6755399441055744.0, t = fma(a, -1.4426950408889634, magic), n = t - magic;       // 1.5 2^52: n is the nearest integer
-    const double r = fma(n, -1.9082149292705877e-10, fma(n, -0.693147180369123816490, -a));
-    double p = 2.7557319223985893e-07;                               // 1 / 10!
-    p = fma(p, r, 2.7557319223985888e-06); p = fma(p, r, 2.4801587301587302e-05); p = fma(p, r, 1.9841269841269841e-04); p = fma(p, r, 1.3888888888888889e-03);
-    p = fma(p, r, 8.3333333333333333e-03); p = fma(p, r, 4.1666666666666667e-02); p = fma(p, r, 1.6666666666666667e-01); p = fma(p, r, 0.5); p = fma(p, r, 1.0); p = fma(p, r, 1.0);
-    const double d = fma(p, __hiloint2double((__double2loint(t) + 1023) << 20, 0), 1.0);
-    double y = (double)(1.0f / (float)d);
-    y = fma(y, fma(-d, y, 1.0), y);
-    return (float)(a * y);
-}
 
 __global__ void __launch_bounds__(256) k_dn_prep_seq(DnDims D, uint32_t T, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,
                                                      const float *qkv, const float *ba, const float *conv_state,
@@ -307,13 +293,13 @@ __global__ void __launch_bounds__(256) k_dn_prep_seq(DnDims D, uint32_t T, const
         for (uint32_t i = 0; i < DN_PREP_TOK + 3u; ++i) x[i] = i < n + 3u ? sample((int)(t_begin + i) - 3) : 0.f;
         const double k0 = (double)kr[0], k1 = (double)kr[1], k2 = (double)kr[2], k3 = (double)kr[3];
 #pragma unroll
-        for (uint32_t i = 0; i < DN_PREP_TOK; ++i) y[i] = dn_silu(fma((double)x[i + 3u], k3, fma((double)x[i + 2u], k2, fma((double)x[i + 1u], k1, (double)x[i] * k0))));
+        for (uint32_t i = 0; i < DN_PREP_TOK; ++i) y[i] = (float)silu_d(fma((double)x[i + 3u], k3, fma((double)x[i + 2u], k2, fma((double)x[i + 1u], k1, (double)x[i] * k0))));
     } else {
 #pragma unroll
         for (uint32_t i = 0; i < DN_PREP_TOK; ++i) {
             double acc = 0.0;
             if (i < n) for (uint32_t j = 0; j <= ns; ++j) acc = fma((double)sample((int)(t_begin + i + j) - (int)ns), (double)kr[j], acc);
-            y[i] = dn_silu(acc);
+            y[i] = (float)silu_d(acc);
         }
     }
     if (blockIdx.x >= n_qk) {
