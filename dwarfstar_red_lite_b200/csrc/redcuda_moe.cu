@@ -329,8 +329,10 @@ struct redcuda_moe {
 
 // integer router logits (moe_router_i8): the digits of the router are made only for a layer that can see so many tokens at once, or where RC_ROUTER_I8_MIN asks
 constexpr uint32_t RT_MIN_TOKENS = 640u, RT_MIN_EXPERTS = 512u;
+// (5 bytes a router weight, 5.2 MB of 512 experts x 2048 columns, and in the workspace 5 bytes a value of the chunk, 21 MB of 2048 x 2048)
 static bool moe_wants_rt(const redcuda_moe_desc &d) {
-    return rt_shape_ok(d.n_expert, d.hidden) && (getenv("RC_ROUTER_I8_MIN") || (d.max_tokens >= RT_MIN_TOKENS && d.n_expert >= RT_MIN_EXPERTS));
+    const char *v = getenv("RC_ROUTER_I8_MIN");
+    return rt_shape_ok(d.n_expert, d.hidden) && (v ? atoi(v) != 0 : d.max_tokens >= RT_MIN_TOKENS && d.n_expert >= RT_MIN_EXPERTS);
 }
 // Layers with IQ3_S matrices take their activations as wide digits: they ran on fp32 activations before the nibble layout held them,
 // and the 24-bit form per row is less than that (relative error of an expert's output against 64-bit sums, hidden 2048: fp32 1.6e-7 on any
@@ -885,7 +887,7 @@ void redcuda_moe_destroy(redcuda_moe *m) {
     delete m;
 }
 
-uint64_t redcuda_moe_resident_bytes(const redcuda_moe *m) { return m ? m->wmem.bytes : 0; }
+uint64_t redcuda_moe_resident_bytes(const redcuda_moe *m) { return m ? m->wmem.bytes + m->rt_mem.bytes : 0; }
 
 int redcuda_moe_forward_device(redcuda_moe *m, uint32_t ntok, const float *x_dev, const float *logits_in_dev, const float *resid_dev,
                                float *out_dev, void *stream) {

@@ -162,6 +162,8 @@ typedef struct {
 
 redcuda_moe *redcuda_moe_create(const redcuda_moe_desc *desc);
 void redcuda_moe_destroy(redcuda_moe *m);
+/* Device bytes of the layer's weights as they are held, without the workspace. A layer for 640 tokens and more with 512 experts
+ * and more keeps its router a second time, as digits for the tensor cores (5 bytes a weight). */
 uint64_t redcuda_moe_resident_bytes(const redcuda_moe *m);
 
 /* Expert parallelism, all-gather form (no reference counterpart: the reference is single-device; the pair layout is its
