@@ -145,6 +145,7 @@ bool rt_shape_ok(uint32_t n_expert, uint32_t ncols);
 size_t rt_wq_bytes(uint32_t n_expert, uint32_t ncols);
 size_t rt_xq_bytes(uint32_t ntok, uint32_t ncols);
 size_t rt_rows(uint32_t ntok);
+int rt_init();            // before the first launch on a device
 int launch_rt_digits_w(const float *w, uint32_t n_expert, uint32_t ncols, uint8_t *wq, double2 *ws, cudaStream_t s);
 int launch_rt_logits(const float *w, const uint8_t *wq, const double2 *ws, const float *x, uint32_t x_stride, uint32_t ntok, uint32_t n_expert, uint32_t ncols, uint8_t *xq, double2 *xs, uint32_t *again,
                      float *logits, uint32_t *err, cudaStream_t s);

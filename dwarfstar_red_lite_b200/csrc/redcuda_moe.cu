@@ -847,7 +847,7 @@ static redcuda_moe *moe_create_impl(const redcuda_moe_desc *desc, void *shared_w
     if (!ok) return bail();
     if (moe_wants_rt(d)) {
         const size_t q = align_up(rt_wq_bytes(d.n_expert, d.hidden), 256);
-        if (!m->rt_mem.alloc(q + d.n_expert * sizeof(double2))) return bail();
+        if (!rt_init() || !m->rt_mem.alloc(q + d.n_expert * sizeof(double2))) return bail();
         m->rt_q = m->rt_mem.as<uint8_t>(); m->rt_ws = reinterpret_cast<double2 *>(m->rt_q + q);
         if (!launch_rt_digits_w((const float *)m->router.base, d.n_expert, d.hidden, m->rt_q, m->rt_ws, s)) return bail();
     }

@@ -302,6 +302,14 @@ static uint32_t rt_tok(uint32_t ntok, uint32_t n_expert) { return (ntok + 31u) /
 size_t rt_xq_bytes(uint32_t ntok, uint32_t ncols) { return (size_t)((ntok + 63u) / 64u) * 64u * ncols * RT_D; }
 size_t rt_rows(uint32_t ntok) { return (size_t)((ntok + 63u) / 64u) * 64u; }
 
+static size_t rt_smem(uint32_t tok) { return (size_t)RT_NS * (RT_A_BUF + RT_D * RT_KS * tok); }
+// before the first launch on a device
+int rt_init() {
+    RC_CUDA(cudaFuncSetAttribute(k_rt_logits<32u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rt_smem(32u)));
+    RC_CUDA(cudaFuncSetAttribute(k_rt_logits<64u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rt_smem(64u)));
+    return 1;
+}
+
 int launch_rt_digits_w(const float *w, uint32_t n_expert, uint32_t ncols, uint8_t *wq, double2 *ws, cudaStream_t s) {
     RC_REQUIRE(rt_shape_ok(n_expert, ncols), "router digits: %u experts of %u columns are not tileable", n_expert, ncols);
     RC_LAUNCH((k_rt_digits_w), n_expert / 8u, 512, 0, s, w, ncols, wq, ws);
@@ -318,13 +326,10 @@ int launch_rt_logits(const float *w, const uint8_t *wq, const double2 *ws, const
     prof_end(s);
     RC_LAUNCHED();
     const RtArgs A{wq, xq, ws, xs, logits, again, ntok, n_expert, ncols, err, status_words()};
-    const size_t smem = (size_t)RT_NS * (RT_A_BUF + RT_D * RT_KS * tok);
+    const dim3 grid(tiles, n_expert / 128u);
     prof_begin("moe_router_logits", s);
-#define RT_LAUNCH(TOK_) do { \
-        RC_CUDA(cudaFuncSetAttribute(k_rt_logits<TOK_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        RC_LAUNCH((k_rt_logits<TOK_>), dim3(tiles, n_expert / 128u), RT_THREADS, smem, s, A); } while (0)
-    if (tok == 64u) RT_LAUNCH(64u); else RT_LAUNCH(32u);
-#undef RT_LAUNCH
+    if (tok == 64u) RC_LAUNCH((k_rt_logits<64u>), grid, RT_THREADS, rt_smem(64u), s, A);
+    else RC_LAUNCH((k_rt_logits<32u>), grid, RT_THREADS, rt_smem(32u), s, A);
     prof_end(s);
     RC_LAUNCHED();
     prof_begin("moe_router_exact", s);
