@@ -259,9 +259,9 @@ __global__ void __launch_bounds__(256, MINB) k_dn_step(DnDims D, const float *__
 //                 the state per chunk instead of per token; the next token's q/k/v/beta/gate are fetched while the
 //                 current one is reduced
 // A block serves DN_PREP_TOK consecutive tokens of its channel group: a thread keeps its channel's samples and results of all of them, so that a sample is
-// read once and the eight L2 norms are reduced together, their roots taken by one thread each. Double-precision arithmetic bounds it (some 30 operations a
-// value; with exp() and a division of doubles for every value, a root and a division in every thread and a barrier per token it was 65, and 119 us for
-// 2048 tokens where this takes 66).
+// read once and the eight L2 norms are reduced together, their roots taken by one thread each. Instruction issue bounds it (74 % of the slots, and three
+// cycles of waiting for a result between two instructions of a warp; a quarter of them are of doubles, some 30 a value. With exp() and a division of doubles for every
+// value, a root and a division in every thread and a barrier per token that was 65, and 119 us for 2048 tokens where this takes 66).
 constexpr uint32_t DN_PREP_TOK = 8u;
 
 __global__ void __launch_bounds__(256) k_dn_prep_seq(DnDims D, uint32_t T, const float *__restrict__ conv_kernel, const float *__restrict__ dt_bias, const float *__restrict__ ssm_a,

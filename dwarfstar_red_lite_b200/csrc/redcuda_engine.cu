@@ -70,7 +70,7 @@ __device__ __forceinline__ double block_sum_d(double v, double *red) {
 }
 
 // normed = RMSNorm(x [+ branch]) * w (engine_cpu.c:96-101, 418-424); resid_out (optional) = x + branch. One block of THREADS per token: 1024 where the token is
-// alone, its row is the chain; 256 for the rows of a chunk whose length k_rmsnorm_rows is not built for.
+// alone, its row is the chain; 256 for the rows of a chunk whose length k_rmsnorm_rows is not built for (it is for the lengths of the engine's models, 1024 and 2048).
 template <uint32_t THREADS>
 __global__ void __launch_bounds__(THREADS) k_rmsnorm(const float *x, const float *branch, const float *__restrict__ w,
                                                   uint32_t n, float eps, float *__restrict__ resid_out, float *__restrict__ normed) {

@@ -248,7 +248,8 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1(const __grid_consta
 // Instruction issue bounds the products of a matrix of that size in floats: a byte permute per weight to make it one. Here x is four 8-bit digits with a
 // power-of-two scale per 256 columns (actw_digits), its digit words in place of the floats, and a word of four 6-bit weights meets them in four dp4a: the
 // sums of 16 columns are exact. The weights stay unsigned (q + 32), an accumulator begins with -32 times its digits' sum. Lanes, rows and loads as in
-// gemv1_q6k. 151936 x 2048: 61 us (floats: 72; 255 MB take 39 at the copy rate)
+// gemv1_q6k. 151936 x 2048: 61 us (floats: 72; 255 MB take 39 at the copy rate). What bounds it now are waits for the digit words out of shared memory (half of
+// what a warp waits for); 57 % of the issue slots are taken.
 //
 // The digits hold a value to 2^-30 of the largest of its 256, which is less than fp32 does for the small ones. So a row takes this form only if in each 256
 //   - at least 32 values lie within 2^-6 of the largest: these are exact, and what the others lack comes to less than the rounding of the fp32 sums that replace it

@@ -369,6 +369,10 @@ static uint32_t moe_item_tokens(const redcuda_moe *m, bool single_token, uint32_
 // faster. us a layer, integer kernels -> this: 512 experts 400 tokens 345 -> 355, 430 361 -> 372, 470 388 -> 367, 500 405 -> 370, 700 525 -> 472, 1000
 // 697 -> 513, 2048 1343 -> 690; Zipf routing 400 330 -> 329, 450 349 -> 342; hidden 1024 400 213 -> 211, 450 225 -> 219; 256 experts 256 tokens 234 -> 218,
 // hidden 1024 240 tokens 141 -> 138; 128 experts 110 tokens 130 -> 149, 141 152 -> 145, 200 180 -> 148, hidden 1024 141 tokens 103 -> 104, 180 113 -> 103.
+// The grouping and the expert kernels alone, few experts (also what a shard of a larger layer has), hidden 2048: 2 experts 256 pairs 43 -> 54, 400 47 -> 55, 464 56 -> 55;
+// 8 experts 256 43 -> 54, 464 59 -> 56; 16 experts 400 47 -> 54, 528 59 -> 56, 900 93 -> 64; 32 experts 400 56 -> 57, 700 67 -> 61; 64 experts 600 68 -> 79, 700 80 -> 80,
+// 900 100 -> 82; hidden 1024 8 experts 464 45 -> 46, 64 experts 600 48 -> 56, 900 65 -> 59: a line of so many pairs an expert alone (32 before) took
+// up to 8 experts there too early.
 static void moe_choose_path(redcuda_moe *m, uint32_t npairs, bool all_local) {
     const char *v = getenv("RC_MOE_TC_MIN");
     const uint32_t min_avg = v ? (uint32_t)atoi(v) : 8u;

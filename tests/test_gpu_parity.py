@@ -220,7 +220,7 @@ def test_moe_layer_config1_ragged_zipf(full_layer):
 
 def test_moe_chunk_on_tcgen05_small(monkeypatch):
     """A chunk large enough for the tcgen05 expert kernel (>= 16 pairs per expert): 8 experts, 160 tokens, so that experts
-    get more than one 64-pair work item and ragged last items."""
+    get more than one 48-pair work item and ragged last items."""
     monkeypatch.setenv("RC_MOE_TC_MIN", "16")
     dims = synth.MoeDims(hidden=512, n_expert=8, top_k=2, ffn=256, ffn_sh=256)
     layer = synth.moe_layer(31, dims, expert_scale=0.5)
