@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1(const __grid_consta
 
 // ---- one large Q6_K matrix (the LM head) -------------------------------------------------------------------------------
 // Instruction issue bounds the products of a matrix of that size in floats: a byte permute per weight to make it one. Here x is four 8-bit digits with a
-// power-of-two scale per 256 columns (actw_digits), its digit words in place of the floats, and a word of four 6-bit weights meets them in four dp4a: the
+// power-of-two scale per 256 columns (actw_digits), and a word of four 6-bit weights meets them in four dp4a: the
 // sums of 16 columns are exact. The weights stay unsigned (q + 32), an accumulator begins with -32 times its digits' sum. Lanes, rows and loads as in
 // gemv1_q6k. 151936 x 2048: 61 us (floats: 72; 255 MB take 39 at the copy rate). What bounds it now are waits for the digit words out of shared memory (half of
 // what a warp waits for); 57 % of the issue slots are taken.
@@ -275,7 +275,7 @@ __device__ __forceinline__ int g1_dp4a(uint32_t q, uint32_t x, int c) { int d; a
 template <bool NORM>
 __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1_digits(const __grid_constant__ GemvArgs A) {
     pdl_trigger();
-    extern __shared__ __align__(16) double g1_part[];      // as in k_gemv1: results of a row that is multiplied as floats; behind them x, then its digit words; and -32 times the digit sums of every 16 columns
+    extern __shared__ __align__(16) double g1_part[];      // as in k_gemv1: results of a row that is multiplied as floats; behind them x, its digit words, and -32 times the digit sums of every 16 columns
     float *g1_xs = reinterpret_cast<float *>(g1_part + A.part_doubles);
     __shared__ float s_scale[G1_NCOLS / 256u];
     const GemvJob &J = A.job[0];
@@ -285,7 +285,8 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1_digits(const __grid
     const uint64_t o_h = rc_q6_qh(J.nb), o_s = rc_q6_sc(J.nb), o_d = rc_q6_d(J.nb);
     const bool on = sub < cpr;                              // lanes past the row's end repeat its last chunk and add nothing
     const uint32_t cc = on ? sub : cpr - 1u, bcol = cc >> 2, half = (cc >> 1) & 1u, l0 = (cc & 1u) * 16u;
-    int4 *corr = reinterpret_cast<int4 *>(g1_xs + g1_xi(J.ncols));
+    float *g1_xd = g1_xs + g1_xi(J.ncols);
+    int4 *corr = reinterpret_cast<int4 *>(g1_xd + g1_xi(J.ncols));
     auto load = [&](uint32_t vr) {
         vr = min(vr, nrow - 1u);
         const uint64_t blk = (uint64_t)(row0 + vr) * bpr + bcol;
@@ -305,16 +306,13 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1_digits(const __grid
     if (!A.resident) { f[0] = load(first + slot); f[1] = load(first + step + slot); }
     __syncthreads();
     static_assert(G1_NCOLS / 256u <= G1_WARPS, "a warp per 256 columns, eight neighbouring values a lane");
-    float4 *p = reinterpret_cast<float4 *>(g1_xs + g1_xi(min(warp, bpr - 1u) * 256u + lane * 8u));
-    const float4 v0 = p[0], v1 = p[1];
-    const uint32_t mx = __reduce_max_sync(0xffffffffu, max(act_mag4(v0), act_mag4(v1)));
-    if (!__syncthreads_and(g1_digits_fit(v0, v1, mx))) {
-        gemv1_q6k<false, true>(A, J, G1Tile{row0, nrow, 0u, true}, g1_part, g1_xs);
-        __syncthreads();
-        for (uint32_t r = threadIdx.x; r < nrow; r += G1_WARPS * 32u) J.out[row0 + r] = (float)g1_part[r];
-        return;
-    }
+    bool fit = true;
     if (warp < bpr) {
+        const uint32_t at = g1_xi(warp * 256u + lane * 8u);
+        const float4 *p = reinterpret_cast<const float4 *>(g1_xs + at);
+        const float4 v0 = p[0], v1 = p[1];
+        const uint32_t mx = __reduce_max_sync(0xffffffffu, max(act_mag4(v0), act_mag4(v1)));
+        fit = g1_digits_fit(v0, v1, mx);
         float up;
         const float scale = actw_scale(mx, up);
         if (lane == 0) s_scale[warp] = scale;
@@ -322,7 +320,8 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1_digits(const __grid
         const uint32_t w1[4] = {actw_digits(v1.x, up), actw_digits(v1.y, up), actw_digits(v1.z, up), actw_digits(v1.w, up)};
         uint32_t p0[4], p1[4];
         actw_planes(w0, p0); actw_planes(w1, p1);
-        reinterpret_cast<uint4 *>(p)[0] = make_uint4(p0[0], p0[1], p0[2], p0[3]); reinterpret_cast<uint4 *>(p)[1] = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+        uint4 *o = reinterpret_cast<uint4 *>(g1_xd + at);
+        o[0] = make_uint4(p0[0], p0[1], p0[2], p0[3]); o[1] = make_uint4(p1[0], p1[1], p1[2], p1[3]);
         int c[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -331,8 +330,13 @@ __global__ void __launch_bounds__(G1_WARPS * 32u, 3) k_gemv1_digits(const __grid
         }
         if (!(lane & 1u)) corr[warp * 16u + (lane >> 1)] = make_int4(c[0], c[1], c[2], c[3]);
     }
-    __syncthreads();
-    const uint4 *xl = reinterpret_cast<const uint4 *>(g1_xs + bcol * 268u + half * 136u + l0);
+    if (!__syncthreads_and(fit)) {
+        gemv1_q6k<false, true>(A, J, G1Tile{row0, nrow, 0u, true}, g1_part, g1_xs);
+        __syncthreads();
+        for (uint32_t r = threadIdx.x; r < nrow; r += G1_WARPS * 32u) J.out[row0 + r] = (float)g1_part[r];
+        return;
+    }
+    const uint4 *xl = reinterpret_cast<const uint4 *>(g1_xd + bcol * 268u + half * 136u + l0);
     const int4 *cl = corr + (bcol * 256u + half * 128u + l0) / 16u;
     const float xscale = s_scale[bcol];
     for (uint32_t base = first; base < nrow; base += 2u * step) {
@@ -428,7 +432,7 @@ int launch_gemv1(GemvArgs &A, cudaStream_t stream) {
     if (q6 || A.norm.w) smem += (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + 16u;
     prof_begin(A.tag ? A.tag : "gemv", stream);
     if (gemv1_digits_ok(A)) {
-        smem += (size_t)(A.job[0].ncols / 16u) * sizeof(int4);
+        smem += (size_t)g1_xi(A.job[0].ncols) * sizeof(float) + (size_t)(A.job[0].ncols / 16u) * sizeof(int4);
         if (A.norm.w) RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1_digits<true>), tiles, G1_WARPS * 32u, smem, stream, A);
         else RC_LAUNCH_BEHIND_IF(!A.resident, (k_gemv1_digits<false>), tiles, G1_WARPS * 32u, smem, stream, A);
         prof_end(stream);

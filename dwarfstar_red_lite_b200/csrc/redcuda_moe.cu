@@ -401,8 +401,8 @@ static bool moe_router_tc(const redcuda_moe *m, uint32_t ntok) {
     return min_tok && ntok >= min_tok && m->router.type == RC_F32 && m->d.hidden % 256u == 0 && m->rt_wd;
 }
 // Router logits of a chunk by integer products (redcuda_router_i8.cu): from 640 tokens and 512 experts on; RC_ROUTER_I8_MIN = tokens (0: never, and then
-// for every expert count it tiles). us a layer, double sums -> this: 512 experts 640 tokens 395 -> 390, 700 405 -> 397, 1024 452 -> 447, 1400 534 -> 513, 2048 679 -> 641;
-// 256 experts 1024 tokens 355 -> 349, 2048 570 -> 591: the double kernel runs beside the shared expert's tcgen05 GEMMs, this one takes turns with them for the
+// for every expert count it tiles). us a layer, double sums -> this: 512 experts 640 tokens 397 -> 395, 700 404 -> 398, 1024 451 -> 434, 1400 531 -> 495, 2048 668 -> 624;
+// 256 experts 1024 tokens 342 -> 340, 2048 566 -> 574: the double kernel runs beside the shared expert's tcgen05 GEMMs, this one takes turns with them for the
 // SMs. Where every logit of a chunk has to be summed again (rows with an element of 1e5 and more among ones) 2048 tokens take 330 us here instead of 138.
 static bool moe_router_i8(const redcuda_moe *m, uint32_t ntok) {
     if (!m->rt_q) return false;

@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1) k_rt_logits(const __grid_consta
     __shared__ __align__(8) uint64_t full[RT_NS], empty[RT_NS], done;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile uint32_t fail;               // a bounded wait ran out
+    __shared__ __align__(16) double2 s_xs[TOK];
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31u;
     const uint32_t nstage = A.ncols / RT_KS, t0 = blockIdx.x * TOK;
     const uint8_t *wq = A.wq + (size_t)blockIdx.y * nstage * RT_A_BUF, *xq = A.xq + (size_t)blockIdx.x * nstage * B_BUF;
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1) k_rt_logits(const __grid_consta
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (tid >= RT_THREADS - TOK) s_xs[tid - (RT_THREADS - TOK)] = A.xs[t0 + tid - (RT_THREADS - TOK)];       // rows beyond the tokens are there, as zeros
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -239,7 +241,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1) k_rt_logits(const __grid_consta
                 double v = (double)(int)m[RT_S - 1u][i], p = 256.0;      // in units of 2^24 of the scaled values' product
 #pragma unroll
                 for (int s = (int)RT_S - 2; s >= 0; --s) { v = fma((double)(int)m[s][i], p, v); p *= 256.0; }
-                const double2 X = A.xs[t];
+                const double2 X = s_xs[c + i];
                 const double q = W.x * X.x;
                 v *= 0x1p24;
                 A.logits[(size_t)t * A.n_expert + e] = (float)(v * q);
@@ -333,7 +335,7 @@ int launch_rt_logits(const float *w, const uint8_t *wq, const double2 *ws, const
     prof_end(s);
     RC_LAUNCHED();
     prof_begin("moe_router_exact", s);
-    RC_LAUNCH((k_rt_exact), (ntok + 7u) / 8u, 256, 0, s, w, x, x_stride, ntok, n_expert, ncols, (const uint32_t *)again, logits);
+    RC_LAUNCH_PDL((k_rt_exact), (ntok + 7u) / 8u, 256, 0, s, w, x, x_stride, ntok, n_expert, ncols, (const uint32_t *)again, logits);
     prof_end(s);
     RC_LAUNCHED();
     return 1;
