@@ -1,6 +1,8 @@
 """Decode attention where a warp takes several groups of four positions in turn (the rows of the next one requested ahead, the running maximum carried over, sums rescaled
 where it rises): a few tokens of a prompt in eight slices of 100 positions, one token in 64 slices of 63. Every head shape and both cache types against the chunk kernel
-(tests/test_gpu_attention_long.py holds that against the CPU oracle), two of them against the oracle itself (parity bound of a layer's output)."""
+(tests/test_gpu_attention_long.py holds that against the CPU oracle), two of them against the oracle itself. The parity bound of a layer's output, 1e-3, would not see a group that is left out: with
+one planted in the oracle (positions 340 to 343 of 402) the last layer differs by 6e-4 to 1.2e-3 of its largest value, and of 4001 positions it would be a
+tenth of that. Four layers of fp32 sums in two orders differ by 1e-7 to 4e-7; the bound is 5e-6."""
 import os
 
 import numpy as np
@@ -12,7 +14,7 @@ from dwarfstar_red_lite_b200.engine import Engine
 
 pytestmark = pytest.mark.gpu
 
-REL_OUT = 1e-3
+REL_OUT = 5e-6
 SHAPES = [(64, 4, 2), (64, 8, 2), (128, 8, 2), (128, 8, 1), (256, 4, 1), (256, 8, 1)]
 
 
@@ -27,7 +29,7 @@ def _model(tmp_path, shape, context):
 
 
 def _near(a, b):
-    assert np.max(np.abs(a - b)) <= REL_OUT * np.max(np.abs(b)) + 1e-6
+    assert np.max(np.abs(a - b)) <= REL_OUT * np.max(np.abs(b))
 
 
 def _state(eng, dims, logits):
